@@ -15,8 +15,8 @@ Before its warm-up the bench lets psi_autotune choose the sublist stride, the
 sublist walk's block size and the patch limit by timing trial solves of the
 same workload (--no-tune takes them from the flags); none of them changes a
 result.  After its timed regions it measures the random-access bound
-(psi_measure_random_access) at the size of the arrays the sublist walk and the
-switch read at random, and reports both kernels against it beside the
+(psi_measure_random_access) at the size of the array the switch reads at
+random, and reports the kernel against it beside the
 copy-bandwidth roofline.  On one GPU the line also carries, unless --no-extras:
 the n = 10,000 random game (out-degree U[2,10]) on the GPU beside the dense
 restatement of the reference's CPUParity on the host ("c1"); the 2^23 long-path
@@ -106,7 +106,7 @@ METHOD = {
     "solve_loop": "one CUDA graph per solve (device-side loop control); per-phase times for the roofline from the "
                   "same kernels in the host-driven loop",
     "evaluation": "incremental where few strategies changed (psi_options.incremental = auto: patches after steps "
-                  "that changed <= patch_limit strategies, else the full Euler-tour evaluation); results identical "
+                  "that changed <= patch_limit strategies, else a full evaluation by walks over the strategy graph); results identical "
                   "to full evaluations",
 }
 
@@ -293,6 +293,10 @@ def phase_bytes(phase, n, m, nsub, counters, calls, n_even, n_odd, iters, brs):
         # broadcast: vloc, solved, strategy, priority in; status, PathNode out (37 B);
         # root-path summaries: status and PathNode in, summary and key out (32 B)
         return 69 * n
+    if phase == "walk":
+        # records: strategy, priority, solved flag in, record out (25 B); walks: record and
+        # key in, status, summary, landmark record and key out (52 B)
+        return 77 * n
     if phase == "reduced":
         if nsub >= RULER_MIN:
             # ruling set: item entries in, (ruler, prefix) out and back in, the
@@ -307,15 +311,16 @@ def phase_bytes(phase, n, m, nsub, counters, calls, n_even, n_odd, iters, brs):
 
 # reduced lists at least this long are ranked through a ruling set (k_rank_ruled)
 RULER_MIN = 4096
-KERNEL_OF_PHASE = {"switch": "k_switch", "sublist": "k_walk_sublists", "tour": "k_tour_relink",
-                   "broadcast": "k_broadcast_depth", "reduced": "k_rank_ruled", "cycles": "k_cycles"}
+KERNEL_OF_PHASE = {"switch": "k_switch", "broadcast": "k_root_walk", "cycles": "k_root_settle"}
 # the kernels of a timed phase (for their DRAM traffic per launch)
-PHASE_KERNELS = {"sublist": ("k_walk_sublists",), "tour": ("k_dirty_list", "k_tour_relink", "k_sink_list"),
-                 "broadcast": ("k_broadcast_depth", "k_rootinfo")}
+PHASE_KERNELS = {"broadcast": ("k_root_init", "k_root_walk")}
 # phases of the full evaluation: their kernels work only in evaluations that
 # are not patches (in a patch they return at their gate), so their per-launch
 # time is their phase time over the full evaluations
-FULL_EVAL_PHASES = ("sublist", "tour", "broadcast", "reduced", "cycles")
+FULL_EVAL_PHASES = ("broadcast", "cycles")
+# the byte formula of a phase where it is not the phase's own name: the library
+# reports the evaluation's walks under "broadcast"
+BYTES_OF_PHASE = {"broadcast": "walk"}
 
 
 # ------------------------------------------------------------------ CPU legs
@@ -607,10 +612,10 @@ def run_gb300(args, rank, world, local):
 
     # roofline of the dominant kernel-level phase (the patch phase, a few
     # latency-bound cooperative launches per evaluation, is reported apart)
-    kernel_phases = ("switch", "sublist", "tour", "broadcast", "reduced", "cycles")
+    kernel_phases = ("switch", "broadcast", "cycles")
     dom = max(kernel_phases, key=lambda p: phases[p][0])
     dom_ms, dom_calls = phases[dom][0], launches_of(dom)
-    bpc = phase_bytes(dom, game.n, game.m, nsub, counters, dom_calls, n_even, n_odd, iters, brs)
+    bpc = phase_bytes(BYTES_OF_PHASE.get(dom, dom), game.n, game.m, nsub, counters, dom_calls, n_even, n_odd, iters, brs)
     peak, peak_kind = hbm_peak()
     roofline = None
     if bpc is not None and dom_calls:
@@ -628,13 +633,12 @@ def run_gb300(args, rank, world, local):
             roofline["traffic_GBps"] = traffic / (dom_ms / dom_calls / 1e3) / 1e9
             roofline["traffic_frac"] = roofline["traffic_GBps"] / peak
     # the random-access bound beside the copy bound, measured at the size of
-    # the array each phase reads at random (the tour's successors for the
-    # sublist walk, the comparison keys for the switch) and at 1 GiB (DRAM)
+    # the array the switch reads at random (the comparison keys) and at 1 GiB
+    # (DRAM)
     rpeak = {"how": "psi_measure_random_access: independent 4-byte loads at uniformly random positions of a "
                     "device array of the given size, 8 in flight per thread, every SM filled; median of 10 "
                     "launches (CUDA events); sector_GBps counts 32 B per load",
              "dram_1GiB": random_access_peak(local, 1 << 30),
-             "sublist": random_access_peak(local, 4 * (2 * game.n + 2)),
              "switch": random_access_peak(local, 4 * game.n)}
 
     def vs_random(p, ms_per_call):
@@ -651,9 +655,9 @@ def run_gb300(args, rank, world, local):
         if ra:
             roofline["random_access"] = ra
     lr = {}
-    for p in ("sublist", "tour", "broadcast"):
+    for p in ("broadcast",):
         pm, pc = phases[p][0], launches_of(p)
-        b = phase_bytes(p, game.n, game.m, nsub, counters, pc, n_even, n_odd, iters, brs)
+        b = phase_bytes(BYTES_OF_PHASE[p], game.n, game.m, nsub, counters, pc, n_even, n_odd, iters, brs)
         if pc:
             sec = pm / pc / 1e3
             lr[p] = {"ms_per_call": pm / pc, "GBps": b / sec / 1e9, "frac": b / sec / 1e9 / peak}

@@ -87,7 +87,8 @@ typedef struct {
     int32_t device;          /* CUDA device ordinal (default 0) */
     int32_t valuation_mode;  /* PSI_VAL_* (default PSI_VAL_PATH) */
     int32_t sublist_len;     /* Helman-JaJa node stride between sublist heads (default 64,
-                                the reference's gpu_list_ranking.cu:19) */
+                                the reference's gpu_list_ranking.cu:19); at least 2, without effect:
+                                evaluations walk the strategy graph and rank no list */
     int32_t timing;          /* 1: record per-phase CUDA-event times (default 1) */
     int32_t graph;           /* 1 (default): psi_solve runs the whole solve_si loop as one CUDA
                                 graph (device-side loop control, no host synchronisation per
@@ -99,8 +100,8 @@ typedef struct {
                                 the same as a full evaluation's) */
     int32_t patch_limit;     /* PSI_INCR_AUTO: the most changed strategies after which a
                                 patch is tried (0, the default: max(1024, n/64)) */
-    int32_t walk_block;      /* threads per block of the sublist walk (one thread per
-                                sublist): a multiple of 32 in [32, 1024]; 0, the default: 128 */
+    int32_t walk_block;      /* threads per block of the sublist walk: a multiple of 32 in
+                                [32, 1024] or 0 (the default); without effect, as sublist_len */
     int32_t switch_kernel;   /* PSI_SWITCH_*: how the all-switches step maps vertices to threads
                                 (the same results either way) */
 } psi_options;
@@ -187,10 +188,11 @@ int psi_solve(psi_solver *s, int32_t reset, int32_t *iter_count, int32_t *br_cou
 int psi_solver_times(psi_solver *s, double *eval_ms, double *switch_ms, int64_t *evals, int64_t *switches);
 int psi_solver_reset_times(psi_solver *s);
 /* Per-phase device times (ms) and call counts, phases in this order:
- * 0 evaluation (whole), 1 switch step, 2 tour build, 3 sublist walk,
- * 4 reduced-list ranking, 5 broadcast, 6 cycle parity, 7 incremental
- * evaluation (its kernels; they return at once when the full evaluation
- * runs, and the full evaluation's when a patch does). */
+ * 0 evaluation (whole), 1 switch step, 5 the full evaluation's walks, 6 the
+ * pointer jumping for the walks it cut short, 7 incremental evaluation (its
+ * kernels; they return at once when the full evaluation runs, and the full
+ * evaluation's when a patch does).  2 tour build, 3 sublist walk and 4
+ * reduced-list ranking stay at zero: no tour is built. */
 enum { PSI_PHASE_EVAL = 0, PSI_PHASE_SWITCH, PSI_PHASE_TOUR, PSI_PHASE_SUBLIST, PSI_PHASE_REDUCED,
        PSI_PHASE_BROADCAST, PSI_PHASE_CYCLES, PSI_PHASE_PATCH, PSI_PHASE_COUNT };
 int psi_solver_phase_times(psi_solver *s, double *ms, int64_t *calls, int32_t nphases);
@@ -214,10 +216,10 @@ int psi_solver_debug_inject_error(psi_solver *s, int32_t after_evals, uint32_t b
 /* Work counters since the last reset, in this order: evaluations, switch
  * steps, compared edges, parent/priority loads of the comparison walks,
  * vertices whose strategy changed, unreached vertices (summed over full
- * evaluations), pointer-jumping rounds, incremental evaluations (patches),
- * vertices the patches re-evaluated, and of the Euler-tour build and upkeep:
- * parents whose child lists were (re)linked, in-neighbour entries they
- * scanned, children they linked.  Writes min(k, 12) values. */
+ * evaluations), the rounds that pointer jumping over them would take,
+ * incremental evaluations (patches), vertices the patches re-evaluated, and
+ * three zeros (of the Euler-tour upkeep: no tour is built).  Writes min(k, 12)
+ * values. */
 int psi_solver_counters(psi_solver *s, int64_t *out, int32_t k);
 /* Kernel launches issued by this library in this process so far. */
 int64_t psi_launch_count(void);

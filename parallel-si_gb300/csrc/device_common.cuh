@@ -28,16 +28,32 @@ __host__ __device__ __forceinline__ int32_t st_infinite(int32_t st)
     return st == ST_POS_INF ? 1 : (st == ST_NEG_INF ? -1 : 0);
 }
 
-// Snapshot of a vertex the sink reached, written by an evaluation: its parent
-// in the sink tree (-1 = the sink), its priority, and a summary of its root
-// path (the path from the vertex to the sink): the highest priority on it and
-// how many vertices of the path carry that priority.  rmax == RM_UNKNOWN until
-// the summary has been computed.  16-byte aligned so one load fetches it all
-// and the (rmax, rcnt) pair is written as one 8-byte store.
+// Path record of a vertex, written by an evaluation: its successor in the
+// strategy (-1 = the sink), its priority, and a summary of its path to the
+// sink: the highest priority on it (rmax) and one word with the path's length
+// and how many of its vertices carry rmax (path_word).  rmax == RM_UNKNOWN
+// until the vertex is evaluated, RM_POS_INF / RM_NEG_INF where its valuation
+// is infinite.  16-byte aligned so one load fetches it all and the
+// (rmax, word) pair is published as one 8-byte store.
 struct __align__(16) PathNode {
-    int32_t parent, pri, rmax, rcnt;
+    int32_t parent, pri, rmax, word;
 };
 constexpr int32_t RM_UNKNOWN = INT32_MIN;
+constexpr int32_t RM_POS_INF = INT32_MIN + 1;
+constexpr int32_t RM_NEG_INF = INT32_MIN + 2;
+
+// Depth (path length) and count in one word, 16 bits each: a walk that meets
+// a finished ancestor takes both from the record it has loaded anyway, where
+// a separate depth array cost one more random access per vertex.  A path of
+// kDeepPath vertices or more has the word's depth at kDeepPath: its depth is
+// then in the status word and its count in the array rdeep.
+constexpr int32_t kDeepPath = 0xffff;
+__host__ __device__ __forceinline__ int32_t path_word(int32_t depth, int32_t count)
+{
+    return depth < kDeepPath ? (int32_t)((uint32_t)depth << 16 | (uint32_t)count) : (int32_t)((uint32_t)kDeepPath << 16);
+}
+__host__ __device__ __forceinline__ int32_t path_word_depth(int32_t w) { return (int32_t)((uint32_t)w >> 16); }
+__host__ __device__ __forceinline__ int32_t path_word_count(int32_t w) { return w & 0xffff; }
 
 // Comparison key of a vertex after an evaluation: 4 bytes, what the switch
 // step gathers per compared edge (n = 2^24 keys take 64 MiB and stay in L2).
@@ -180,7 +196,7 @@ __device__ __forceinline__ void top2_add_n(Top2 &t, int32_t p, int32_t count)
 // there (the sink at L = 0).  skip[v] = (landmark, top two priorities of the
 // segment from v up to the landmark, exclusive, and their counts packed as
 // c1 | c2 << 16; a segment holds at most SKIP_K vertices).  Written by the
-// root-summary pass of a full evaluation; a patch marks its vertices'
+// walks of a full evaluation (root_kernels.cu); a patch marks its vertices'
 // records unknown (the paths of all other vertices are unchanged).  SKIP_K
 // measured on GB300 (graph solve of the 2^24 random game, long-path 2^23):
 // 64: 63.8, 57.8 ms; 32: 62.8, 57.8; 16: 62.0, 57.0; 8: 61.6, 55.5; 4: 61.8,
@@ -199,11 +215,11 @@ __device__ __forceinline__ void skip_merge(Top2 &t, const int4 s)
     top2_add_n(t, s.z, (int32_t)((uint32_t)s.w >> 16));
 }
 
-// Release store of a root-path summary (rmax, rcnt) as one 8-byte word: the
-// skip record written before it is visible to any thread that acquires it.
-__device__ __forceinline__ void publish_summary(PathNode *p, int32_t m, int32_t c)
+// Release store of a summary (rmax, word) as one 8-byte word: what was written
+// before it (skip, status, rdeep) is visible to any thread that acquires it.
+__device__ __forceinline__ void publish_summary(PathNode *p, int32_t m, int32_t word)
 {
-    const unsigned long long w = (unsigned long long)(uint32_t)m | ((unsigned long long)(uint32_t)c << 32);
+    const unsigned long long w = (unsigned long long)(uint32_t)m | ((unsigned long long)(uint32_t)word << 32);
     asm volatile("st.release.gpu.global.b64 [%0], %1;" ::"l"(&p->rmax), "l"(w) : "memory");
 }
 __device__ __forceinline__ int32_t acquire_rmax(const PathNode *p)

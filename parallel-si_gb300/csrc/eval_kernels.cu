@@ -1,40 +1,27 @@
-// eval_kernels.cu -- strategy evaluation on sm_103a.
+// eval_kernels.cu -- initial strategies, mark_solved, and list ranking of an
+// Euler tour on sm_103a.
 //
-// One evaluation turns the current strategy (one successor per vertex, -1 for
-// the sink) into a per-vertex status word (device_common.cuh):
+// The list ranking serves the evaluation without allocation (noalloc.cu),
+// which wants path lengths only, from a fixed scratch array; solvers evaluate
+// by walks over the strategy graph (root_kernels.cu).
 //
-//  1. Euler tour of the sink tree (tour_init, tour_link, sink_chain).  Every
-//     vertex's up/down node pair is spliced into its parent's list of
-//     children -- the reference builds the same list with one atomic exchange
-//     per vertex (gpu_list_ranking.cu:52-92), which serialises on popular
-//     parents.  Here each live parent links its own children by scanning its
-//     in-neighbours in a reverse CSR built once per game: no atomics, and the
-//     child order (in-neighbour order) is deterministic; the sink's children,
-//     which can be millions, are compacted with one atomic per warp and
-//     chained.  After the first evaluation the tour is kept up to date
-//     instead (tour_relink): only parents whose children changed since -- the
-//     old and new successor of each switched vertex, each newly solved vertex
-//     -- are relinked, a few percent of them per step.
-//  2. Helman-JaJa list ranking: `nsub` sublist heads at fixed tour nodes
-//     (node j*stride, and the list start; gpu_list_ranking.cu:96-110 marks
-//     heads in the successor array, here a node's head index follows from its
-//     id so the tour is never modified); one thread per sublist walks to the
-//     next head accumulating +1/-1 depth steps (walk_sublists,
+//  1. Helman-JaJa list ranking of the tour: `nsub` sublist heads at fixed tour
+//     nodes (node j*stride, and the list start; gpu_list_ranking.cu:96-110
+//     marks heads in the successor array, here a node's head index follows
+//     from its id so the tour is never modified); one thread per sublist walks
+//     to the next head accumulating +1/-1 depth steps (walk_sublists,
 //     gpu_list_ranking.cu:114-193).  The reduced list of sublists is ranked on
 //     the device by Wyllie pointer jumping in one cooperative launch
 //     (rank_reduced) -- the reference copies it to the host and walks it
 //     serially (gpu_list_ranking.cu:197-240) -- giving every sublist its suffix
 //     sum and whether the list start reaches it.
-//  3. Broadcast (broadcast_depth, gpu_list_ranking.cu:244-277): a vertex the
-//     sink reaches gets its path length; its parent and priority are snapshot
-//     for the comparison walks of the following switch step.  Vertices the
-//     sink does not reach are collected.
-//  4. Those vertices end in a cycle or in a solved vertex.  Pointer jumping
+//  2. Broadcast (broadcast_depth, gpu_list_ranking.cu:244-277): a vertex the
+//     sink reaches gets its path length; the others are collected.
+//  3. Those vertices end in a cycle or in a solved vertex.  Pointer jumping
 //     with a running maximum (cycles, one cooperative launch) gives each the
-//     parity of its cycle's top priority, or the frozen value of the solved
-//     vertex, in every evaluation -- as the reference CPU solver does
-//     (cpu_parity.cpp:35-52, 80-104); the reference GPU list ranker marks all of
-//     them +inf (gpu_list_ranking.cu:254-276).
+//     parity of its cycle's top priority (cpu_parity.cpp:35-52, 80-104); the
+//     reference GPU list ranker marks all of them +inf
+//     (gpu_list_ranking.cu:254-276).
 #include <atomic>
 #include <climits>
 #include <cooperative_groups.h>
@@ -53,13 +40,6 @@ inline unsigned grid_for(int64_t items, int block = kBlock)
     int64_t g = ceil_div(items, block);
     return (unsigned)(g < 1 ? 1 : g);
 }
-
-// The scans of all vertices that compact a list (dirty parents, the sink's
-// children) give each thread kVec consecutive vertices per pass: their byte
-// flags arrive in one 16-byte load, int32 fields in four, so a warp reads 512
-// contiguous bytes of each array per load; the ragged end of the range (and
-// arrays not 16-byte aligned) go one vertex at a time.
-constexpr int kVec = 16;
 
 __device__ __forceinline__ int ceil_log2_dev(int64_t x)
 {
@@ -88,254 +68,6 @@ __global__ void k_reset_odd(int32_t n, const int8_t *__restrict__ owner, const i
             strat[v] = tgt[off[v]];
             if (need) need[v] = 1;   // its choice starts over
         }
-}
-
-// Up node of v points at its own down node; the down node of a vertex that no
-// parent links (solved, or child of a solved vertex) points back at its up
-// node.  The sink's down node ends the list.
-__global__ void k_tour_init(int32_t n, int32_t *__restrict__ succ, int2 *__restrict__ vloc,
-                            uint8_t *__restrict__ dirty, const int32_t *__restrict__ gate,
-                            const uint8_t *__restrict__ tie, uint8_t *__restrict__ need)
-{
-    if (gate && !*gate) return;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += (int64_t)gridDim.x * blockDim.x) {
-        succ[2 * i + 1] = (int32_t)(2 * i);
-        succ[2 * i] = (i == n) ? TOUR_END : (int32_t)(2 * i + 1);
-        if (i < n) {
-            vloc[i] = make_int2(-1, 0);
-            dirty[i] = 0;   // a full build leaves nothing to relink
-            if (tie && tie[i]) need[i] = 1;
-        }
-    }
-}
-
-// Work counters of the tour kernels, one set of atomics per block:
-// stats[0] += parents linked, [1] += in-neighbour entries scanned, [2] +=
-// children linked (stats == nullptr: none).  Every thread of the block calls it.
-__device__ __forceinline__ void add_relink_stats(unsigned long long *stats, int32_t parents, int32_t entries,
-                                                 int32_t children)
-{
-    if (!stats) return;
-    __shared__ unsigned long long acc[3];
-    if (threadIdx.x == 0) acc[0] = acc[1] = acc[2] = 0;
-    __syncthreads();
-    if (parents) atomicAdd(&acc[0], (unsigned long long)parents);
-    if (entries) atomicAdd(&acc[1], (unsigned long long)entries);
-    if (children) atomicAdd(&acc[2], (unsigned long long)children);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (acc[0]) atomicAdd(&stats[0], acc[0]);
-        if (acc[1]) atomicAdd(&stats[1], acc[1]);
-        if (acc[2]) atomicAdd(&stats[2], acc[2]);
-    }
-}
-
-// In-neighbours of a parent p in batches: the next kInBatch entries of its
-// reverse-CSR slice [eb, e1) and their strategies, all loads issued before any
-// is used (independent gathers in flight per thread); child[j] says whether
-// entry j is a child of p (strat[u] == p), false past the slice.
-constexpr int kInBatch = 4;
-__device__ __forceinline__ void in_batch(const int32_t *__restrict__ rev_src, const int32_t *__restrict__ strat,
-                                         int32_t eb, int32_t e1, int32_t p, int32_t (&us)[kInBatch],
-                                         bool (&child)[kInBatch])
-{
-#pragma unroll
-    for (int j = 0; j < kInBatch; j++) us[j] = (eb + j < e1) ? rev_src[eb + j] : -1;
-    int32_t ss[kInBatch];
-#pragma unroll
-    for (int j = 0; j < kInBatch; j++) ss[j] = (us[j] >= 0) ? strat[us[j]] : -1;
-#pragma unroll
-    for (int j = 0; j < kInBatch; j++) child[j] = us[j] >= 0 && ss[j] == p;
-}
-
-// Thread p: (a) if p is a live child of the sink, append it to the sink list;
-// (b) if p is live, link its children, found among its distinct in-neighbours
-// rev_src[rev_off[p] .. rev_off[p+1]), as
-// up(p) -> up(c0) ... down(c0) -> up(c1) ... down(c_last) -> down(p).
-// A solved child is linked like any other (checking would cost a second
-// random gather per in-neighbour): its up/down pair adds +1-1 to no one's
-// depth, its own children stay unlinked (a solved parent links nothing), and
-// the broadcast skips it.
-__global__ void k_tour_link(int32_t n, const int32_t *__restrict__ strat, const uint8_t *__restrict__ solved,
-                            const int32_t *__restrict__ rev_off, const int32_t *__restrict__ rev_src,
-                            int32_t *__restrict__ succ, int32_t *__restrict__ sinklist,
-                            int32_t *__restrict__ sinkcount, const int32_t *__restrict__ gate,
-                            unsigned long long *__restrict__ stats)
-{
-    if (gate && !*gate) return;
-    int32_t t_parents = 0, t_entries = 0, t_children = 0;
-    // grid-stride with block-uniform passes (block_append needs every thread)
-    for (int64_t b0 = (int64_t)blockIdx.x * blockDim.x; b0 < n; b0 += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t p = (int32_t)(b0 + threadIdx.x);
-        const bool live = p < n && !solved[p];
-        block_append(live && strat[p] < 0, p, sinklist, sinkcount);
-        if (!live) continue;
-        int32_t prev = -1;
-        const int32_t e0 = rev_off[p], e1 = rev_off[p + 1];
-        t_parents++;
-        t_entries += e1 - e0;
-        for (int32_t eb = e0; eb < e1; eb += kInBatch) {
-            int32_t us[kInBatch];
-            bool child[kInBatch];
-            in_batch(rev_src, strat, eb, e1, p, us, child);
-#pragma unroll
-            for (int j = 0; j < kInBatch; j++) {
-                if (!child[j]) continue;
-                const int32_t u = us[j];
-                if (prev < 0) succ[2 * (int64_t)p + 1] = 2 * u + 1;
-                else succ[2 * (int64_t)prev] = 2 * u + 1;
-                prev = u;
-                t_children++;
-            }
-        }
-        if (prev >= 0) succ[2 * (int64_t)prev] = 2 * p;
-    }
-    add_relink_stats(stats, t_parents, t_entries, t_children);
-}
-
-// Incremental tour maintenance.  Between evaluations the tour lists persist
-// in succ; the switch step and mark_solved flag as dirty every parent whose set
-// of children may have changed (the old and the new parent of each changed
-// strategy, each newly solved vertex).  Thread p relinks a dirty p from its
-// in-neighbours: a live p chains its current children exactly as k_tour_link
-// does; a solved p links none and turns each of its children into an isolated
-// 2-cycle (down -> own up), so they are unreached and the cycle pass gives
-// them p's frozen value.  Parents that are not dirty keep their lists, which
-// are still exact.  The dirty parents are compacted first (k_dirty_list, which
-// also clears the flags), so the relinking threads are all busy.
-__global__ void k_dirty_list(int32_t n, uint8_t *__restrict__ dirty, int32_t *__restrict__ list,
-                             int32_t *__restrict__ count, int2 *__restrict__ vloc, const int32_t *__restrict__ gate,
-                             const uint8_t *__restrict__ tie, uint8_t *__restrict__ need)
-{
-    if (gate && !*gate) return;
-    const bool vec = aligned16(dirty) && aligned16(vloc) && (!tie || (aligned16(tie) && aligned16(need)));
-    const int64_t pass = (int64_t)kVec * blockDim.x;
-    for (int64_t b0 = (int64_t)blockIdx.x * pass; b0 < n; b0 += (int64_t)gridDim.x * pass) {
-        const int64_t v0 = b0 + (int64_t)kVec * threadIdx.x;
-        int32_t v[kVec];
-        if (vec && v0 + kVec <= n) {
-            Bytes16 d;
-            d.q = *reinterpret_cast<const int4 *>(dirty + v0);
-            if (d.q.x | d.q.y | d.q.z | d.q.w) *reinterpret_cast<int4 *>(dirty + v0) = make_int4(0, 0, 0, 0);
-#pragma unroll
-            for (int k = 0; k < kVec; k++) v[k] = d.b[k] ? (int32_t)(v0 + k) : -1;
-            int4 *vl = reinterpret_cast<int4 *>(vloc + v0);   // on no walked sublist until the walk reaches it
-#pragma unroll
-            for (int k = 0; k < kVec / 2; k++) vl[k] = make_int4(-1, -1, -1, -1);
-            if (tie) {
-                const int4 t = *reinterpret_cast<const int4 *>(tie + v0);
-                if (t.x | t.y | t.z | t.w) {
-                    int4 *nd = reinterpret_cast<int4 *>(need + v0);
-                    const int4 o = *nd;
-                    *nd = make_int4(o.x | t.x, o.y | t.y, o.z | t.z, o.w | t.w);   // flags are 0 or 1
-                }
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < kVec; k++) {
-                const int64_t i = v0 + k;
-                v[k] = -1;
-                if (i < n) {
-                    if (dirty[i]) {
-                        dirty[i] = 0;
-                        v[k] = (int32_t)i;
-                    }
-                    vloc[i] = make_int2(-1, -1);
-                    if (tie && tie[i]) need[i] = 1;
-                }
-            }
-        }
-        block_append_k(v, list, count);
-    }
-}
-
-__global__ void k_tour_relink(const int32_t *__restrict__ list, const int32_t *__restrict__ count,
-                              const int32_t *__restrict__ strat, const uint8_t *__restrict__ solved,
-                              const int32_t *__restrict__ rev_off, const int32_t *__restrict__ rev_src,
-                              int32_t *__restrict__ succ, const int32_t *__restrict__ gate,
-                              unsigned long long *__restrict__ stats)
-{
-    if (gate && !*gate) return;
-    const int32_t k = *count;
-    int32_t t_parents = 0, t_entries = 0, t_children = 0;
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) {
-        const int32_t p = list[i];
-        const bool live = !solved[p];
-        int32_t prev = -1;
-        const int32_t e0 = rev_off[p], e1 = rev_off[p + 1];
-        t_parents++;
-        t_entries += e1 - e0;
-        for (int32_t eb = e0; eb < e1; eb += kInBatch) {
-            int32_t us[kInBatch];
-            bool child[kInBatch];
-            in_batch(rev_src, strat, eb, e1, p, us, child);
-#pragma unroll
-            for (int j = 0; j < kInBatch; j++) {
-                if (!child[j]) continue;
-                const int32_t u = us[j];
-                t_children++;
-                if (!live) {
-                    succ[2 * (int64_t)u] = 2 * u + 1;
-                    continue;
-                }
-                if (prev < 0) succ[2 * (int64_t)p + 1] = 2 * u + 1;
-                else succ[2 * (int64_t)prev] = 2 * u + 1;
-                prev = u;
-            }
-        }
-        if (prev >= 0) succ[2 * (int64_t)prev] = 2 * p;
-        else succ[2 * (int64_t)p + 1] = 2 * p;
-    }
-    add_relink_stats(stats, t_parents, t_entries, t_children);
-}
-
-// The sink's live children (the full build collects them in k_tour_link).
-__global__ void k_sink_list(int32_t n, const int32_t *__restrict__ strat, const uint8_t *__restrict__ solved,
-                            int32_t *__restrict__ sinklist, int32_t *__restrict__ sinkcount,
-                            const int32_t *__restrict__ gate)
-{
-    if (gate && !*gate) return;
-    const bool vec = aligned16(strat) && aligned16(solved);
-    const int64_t pass = (int64_t)kVec * blockDim.x;
-    for (int64_t b0 = (int64_t)blockIdx.x * pass; b0 < n; b0 += (int64_t)gridDim.x * pass) {
-        const int64_t v0 = b0 + (int64_t)kVec * threadIdx.x;
-        int32_t v[kVec];
-        if (vec && v0 + kVec <= n) {
-            Bytes16 so;
-            so.q = *reinterpret_cast<const int4 *>(solved + v0);
-            const int4 *sp = reinterpret_cast<const int4 *>(strat + v0);
-#pragma unroll
-            for (int k = 0; k < kVec / 4; k++) {
-                const int4 q = sp[k];
-                v[4 * k + 0] = (q.x < 0 && !so.b[4 * k + 0]) ? (int32_t)(v0 + 4 * k + 0) : -1;
-                v[4 * k + 1] = (q.y < 0 && !so.b[4 * k + 1]) ? (int32_t)(v0 + 4 * k + 1) : -1;
-                v[4 * k + 2] = (q.z < 0 && !so.b[4 * k + 2]) ? (int32_t)(v0 + 4 * k + 2) : -1;
-                v[4 * k + 3] = (q.w < 0 && !so.b[4 * k + 3]) ? (int32_t)(v0 + 4 * k + 3) : -1;
-            }
-        } else {
-#pragma unroll
-            for (int k = 0; k < kVec; k++) {
-                const int64_t i = v0 + k;
-                v[k] = (i < n && strat[i] < 0 && !solved[i]) ? (int32_t)i : -1;
-            }
-        }
-        block_append_k(v, sinklist, sinkcount);
-    }
-}
-
-// sink up -> up(c0) ... down(c0) -> up(c1) ... down(c_last) -> sink down
-__global__ void k_sink_chain(int32_t n, const int32_t *__restrict__ sinklist,
-                             const int32_t *__restrict__ sinkcount, int32_t *__restrict__ succ,
-                             const int32_t *__restrict__ gate)
-{
-    if (gate && !*gate) return;
-    int32_t k = *sinkcount;
-    if (k == 0 && blockIdx.x == 0 && threadIdx.x == 0) succ[2 * (int64_t)n + 1] = 2 * n;
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) {
-        int32_t v = sinklist[i];
-        succ[2 * (int64_t)v] = (i + 1 < k) ? 2 * sinklist[i + 1] + 1 : 2 * n;
-        if (i == 0) succ[2 * (int64_t)n + 1] = 2 * v + 1;
-    }
 }
 
 // Sublist heads are fixed tour nodes: node j*stride is head j for j < nsub-1
@@ -597,82 +329,6 @@ __global__ void k_broadcast_depth(int32_t n, const int2 *__restrict__ vloc, cons
     }
 }
 
-// Root-path summaries of the reached vertices.  Each thread walks from its
-// vertex towards the sink until it meets an ancestor whose summary is already
-// known (or the sink) and stores the summary of its own vertex only; with
-// threads in arbitrary order a walk is short on average (an ancestor has
-// usually been done already).  A concurrent reader sees either RM_UNKNOWN or
-// the final pair, which is written as one 8-byte store.  The key is written
-// only where it changed; all threads stay to the end (flag_in_neighbours is
-// warp-collective).
-// eight blocks per SM (at most 32 registers): the walks are latency-bound
-__global__ void __launch_bounds__(kBlock, 8) k_rootinfo(int32_t n, const int32_t *__restrict__ st,
-                                                        PathNode *__restrict__ node,
-                           int32_t *__restrict__ key, uint32_t *__restrict__ err, ChangeTrack track,
-                           const int32_t *__restrict__ gate, int4 *__restrict__ skip)
-{
-    if (gate && !*gate) return;
-    for (int64_t b0 = (int64_t)blockIdx.x * blockDim.x; b0 < n; b0 += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t v = (int32_t)(b0 + threadIdx.x);
-        bool changed = false;
-        if (v < n && st[v] >= 1) {
-            const int32_t old = key ? key[v] : 0;
-            const int32_t d = st[v], L = skip_landmark_depth(d);
-            PathNode q = node[v];
-            int32_t m = q.pri, c = 1, y = q.parent, dy = d - 1;
-            // the landmark segment: v, then the ancestors above it down to depth L + 1
-            Top2 seg = {q.pri, 1, -1, 0};
-            int32_t anc = (dy == L) ? y : SKIP_UNKNOWN;
-            int32_t steps = 0;
-            while (y >= 0) {
-                int4 r = *reinterpret_cast<const int4 *>(&node[y]);
-                if (r.z != RM_UNKNOWN) {
-                    top1_merge(m, c, r.z, r.w);
-                    break;
-                }
-                top1_merge(m, c, r.y, 1);
-                if (anc == SKIP_UNKNOWN) top2_add(seg, r.y);
-                y = r.x;
-                if (--dy == L && anc == SKIP_UNKNOWN) anc = y;
-                if (++steps > n) {
-                    atomicOr(err, DERR_WALK_CAP);
-                    break;
-                }
-            }
-            if (skip) {
-                // stopped inside the segment at y, whose summary is known: its skip was
-                // published before it (same landmark); if not yet visible, walk on
-                for (int32_t guard = 0; anc == SKIP_UNKNOWN && y >= 0 && guard <= SKIP_K; guard++) {
-                    // only a summary published in this evaluation vouches for the skip
-                    // (the broadcast reset every reached vertex's summary)
-                    if (acquire_rmax(&node[y]) != RM_UNKNOWN) {
-                        const int4 sy = __ldcg(&skip[y]);
-                        if (sy.x != SKIP_UNKNOWN) {
-                            skip_merge(seg, sy);
-                            anc = sy.x;
-                            break;
-                        }
-                    }
-                    const int2 r = *reinterpret_cast<const int2 *>(&node[y]);
-                    top2_add(seg, r.y);
-                    y = r.x;
-                    if (--dy == L) anc = y;
-                }
-                skip[v] = skip_pack(anc, seg);
-                publish_summary(&node[v], m, c);   // release: the skip before the summary that vouches for it
-            } else {
-                *reinterpret_cast<int2 *>(&node[v].rmax) = make_int2(m, c);
-            }
-            const int32_t k = finite_key(m, c);
-            if (key && k != old) {
-                key[v] = k;
-                changed = true;
-            }
-        }
-        flag_in_neighbours(track, changed, v);
-    }
-}
-
 // ---- cycle parity of the unreached vertices
 // Pointer jumping: after round r, jmp[u] = (the vertex 2^r steps ahead, the
 // largest (priority, vertex id) pair over the 2^r vertices starting at u, a
@@ -833,7 +489,7 @@ __global__ void __launch_bounds__(kCycleBlock, kCycleMinBlocks) k_cycles(const i
 // With game_of/gmask (served games), only vertices of games whose mask is set.
 __global__ void k_mark_solved(const int32_t *__restrict__ ucount, const int32_t *__restrict__ ulist,
                               int32_t player, const int32_t *__restrict__ st, uint8_t *__restrict__ solved,
-                              uint8_t *__restrict__ dirty, const int32_t *__restrict__ game_of,
+                              const int32_t *__restrict__ game_of,
                               const int32_t *__restrict__ gmask, const int32_t *__restrict__ gate,
                               int32_t *__restrict__ from, uint32_t *__restrict__ done)
 {
@@ -847,10 +503,7 @@ __global__ void k_mark_solved(const int32_t *__restrict__ ucount, const int32_t 
             int32_t g = game_of[u];
             if (g < 0 || !gmask[g]) continue;
         }
-        if (st[u] == target) {
-            solved[u] = 1;
-            dirty[u] = 1;
-        }
+        if (st[u] == target) solved[u] = 1;
     }
     if (!from) return;
     // the last block to finish (every block has read *from by then) moves
@@ -926,42 +579,6 @@ void launch_reset_odd(cudaStream_t s, int32_t n, const int8_t *owner, const int3
     k_reset_odd<<<capped_grid(n), kBlock, 0, s>>>(n, owner, off, tgt, strat, gate, need);
 }
 
-void launch_tour_build(cudaStream_t s, int32_t n, const int32_t *strat, const uint8_t *solved,
-                       const int32_t *rev_off, const int32_t *rev_src, int32_t *succ, int2 *vloc,
-                       int32_t *sinklist, int32_t *sinkcount, uint8_t *dirty, const int32_t *gate,
-                       const uint8_t *tie, uint8_t *need, unsigned long long *stats)
-{
-    count_launch();
-    k_tour_init<<<capped_grid((int64_t)n + 1), kBlock, 0, s>>>(n, succ, vloc, dirty, gate, tie, need);
-    count_launch();
-    k_tour_link<<<capped_grid(n), kBlock, 0, s>>>(n, strat, solved, rev_off, rev_src, succ, sinklist, sinkcount,
-                                                  gate, stats);
-    count_launch();
-    unsigned g = grid_for(n);
-    k_sink_chain<<<g < 1216u ? g : 1216u, kBlock, 0, s>>>(n, sinklist, sinkcount, succ, gate);
-}
-
-int launch_tour_update(cudaStream_t s, int32_t n, const int32_t *strat, const uint8_t *solved,
-                       const int32_t *rev_off, const int32_t *rev_src, uint8_t *dirty, int32_t *succ, int2 *vloc,
-                       int32_t *sinklist, int32_t *sinkcount, int32_t *dlist, int32_t *dcount,
-                       const int32_t *gate, const uint8_t *tie, uint8_t *need, unsigned long long *stats)
-{
-    cudaError_t e = cudaMemsetAsync(dcount, 0, sizeof(int32_t), s);
-    if (e != cudaSuccess) return (int)e;
-    count_launch();
-    k_dirty_list<<<capped_grid(ceil_div(n, kVec)), kBlock, 0, s>>>(n, dirty, dlist, dcount, vloc, gate, tie,
-                                                                        need);
-    count_launch();
-    unsigned g = grid_for(n);
-    g = g < 1216u ? g : 1216u;
-    k_tour_relink<<<g, kBlock, 0, s>>>(dlist, dcount, strat, solved, rev_off, rev_src, succ, gate, stats);
-    count_launch();
-    k_sink_list<<<capped_grid(ceil_div(n, kVec)), kBlock, 0, s>>>(n, strat, solved, sinklist, sinkcount, gate);
-    count_launch();
-    k_sink_chain<<<g, kBlock, 0, s>>>(n, sinklist, sinkcount, succ, gate);
-    return 0;
-}
-
 void launch_walk_sublists(cudaStream_t s, int32_t nsub, int32_t n, int64_t L, int32_t stride, const int32_t *succ,
                           int2 *vloc, int2 *red, uint32_t *err, const int32_t *gate, int block)
 {
@@ -1013,13 +630,6 @@ void launch_broadcast_depth(cudaStream_t s, int32_t n, const int2 *vloc, const i
                                                                            ulist, ucount, gate);
 }
 
-void launch_rootinfo(cudaStream_t s, int32_t n, const int32_t *st, PathNode *node, int32_t *key, uint32_t *err,
-                     ChangeTrack track, const int32_t *gate, int4 *skip)
-{
-    count_launch();
-    k_rootinfo<<<capped_grid(n), kBlock, 0, s>>>(n, st, node, key, err, track, gate, skip);
-}
-
 int launch_cycles(cudaStream_t s, const int32_t *ucount, const int32_t *ulist, const int32_t *strat,
                   const int32_t *pri, const uint8_t *solved, int32_t *st, int32_t *key, int4 *ja, int4 *jb,
                   int32_t *la, int32_t *lb, int32_t *cnt, uint32_t *err, ChangeTrack track, const int32_t *gate)
@@ -1035,11 +645,11 @@ int launch_cycles(cudaStream_t s, const int32_t *ucount, const int32_t *ulist, c
 }
 
 void launch_mark_solved(cudaStream_t s, const int32_t *ucount, const int32_t *ulist, int32_t player,
-                        const int32_t *st, uint8_t *solved, uint8_t *dirty, const int32_t *game_of,
+                        const int32_t *st, uint8_t *solved, const int32_t *game_of,
                         const int32_t *gmask, const int32_t *gate, int32_t *from, uint32_t *done)
 {
     count_launch();
-    k_mark_solved<<<608, kBlock, 0, s>>>(ucount, ulist, player, st, solved, dirty, game_of, gmask, gate, from,
+    k_mark_solved<<<608, kBlock, 0, s>>>(ucount, ulist, player, st, solved, game_of, gmask, gate, from,
                                          done);
 }
 

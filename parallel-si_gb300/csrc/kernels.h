@@ -37,9 +37,7 @@ struct ChangeTrack {
 // Device words deciding which kernels of an evaluation do work (their gates;
 // set by the host or by control kernels, patch_kernels.cu).
 struct EvalGates {
-    int32_t full = 0;        // the tour is built from scratch
-    int32_t incr = 0;        // the previous tour is brought up to date
-    int32_t eval = 1;        // the full evaluation's kernels after the tour run
+    int32_t eval = 1;        // the full evaluation's kernels run
     int32_t patch = 0;       // this evaluation is a patch (patch_kernels.cu)
     int32_t try_patch = 0;   // the next evaluation may be a patch: every strategy change since the
                              // last evaluation went through a switch step that listed it
@@ -48,7 +46,6 @@ struct EvalGates {
     int32_t acount = 0;      // vertices the current patch re-evaluates
     int32_t nseeds = 0;      // of them the changed ones (alist[0, nseeds))
     int32_t lcnt[3] = {0, 0, 0};              // per-level append counters of the patch's search
-    int32_t saved_full = 0, saved_incr = 0;   // tour gates while a patch holds them closed
     int32_t skip = 0, backoff = 1;            // evaluations not to try a patch after a failed one
     int32_t mfrom[2] = {0, 0};   // per player: unreached-list index its next mark_solved scans from
     uint32_t mdone = 0;          // blocks of the running mark_solved that have finished
@@ -126,25 +123,30 @@ void launch_reset_odd(cudaStream_t s, int32_t n, const int8_t *owner, const int3
                       const int32_t *tgt, int32_t *strat, const int32_t *gate = nullptr, uint8_t *need = nullptr);
 
 // ---- evaluation (gpu_list_ranking.cu:52-277)
-// Euler tour of the sink tree, built from scratch.  rev_off/rev_src: distinct
-// in-neighbours of each vertex.  *sinkcount must be 0 on entry; sinklist holds
-// n entries.
-void launch_tour_build(cudaStream_t s, int32_t n, const int32_t *strat, const uint8_t *solved,
-                       const int32_t *rev_off, const int32_t *rev_src, int32_t *succ, int2 *vloc,
-                       int32_t *sinklist, int32_t *sinkcount, uint8_t *dirty, const int32_t *gate = nullptr,
-                       const uint8_t *tie = nullptr, uint8_t *need = nullptr, unsigned long long *stats = nullptr);
-// The same tour brought up to date from the previous one: only the parents
-// flagged in dirty (cleared here; dlist: n entries of scratch, dcount: one
-// counter) are relinked and the sink's list is rebuilt.  Returns a
-// cudaError_t value.  Both set need[v] wherever tie[v] is set (a full
-// evaluation: ChangeTrack), when tie is given.  With stats (3 words), both
-// add the parents they linked, the in-neighbour entries they scanned and the
-// children they linked.
-int launch_tour_update(cudaStream_t s, int32_t n, const int32_t *strat, const uint8_t *solved,
-                       const int32_t *rev_off, const int32_t *rev_src, uint8_t *dirty, int32_t *succ, int2 *vloc,
-                       int32_t *sinklist, int32_t *sinkcount, int32_t *dlist, int32_t *dcount,
-                       const int32_t *gate = nullptr, const uint8_t *tie = nullptr, uint8_t *need = nullptr,
-                       unsigned long long *stats = nullptr);
+// A full evaluation of the current strategy (root_kernels.cu).
+struct EvalArgs {
+    int32_t n = 0;
+    const int32_t *strat = nullptr, *pri = nullptr;
+    const uint8_t *solved = nullptr;
+    int32_t *st = nullptr;        // status words (frozen where solved)
+    PathNode *node = nullptr;
+    int32_t *rdeep = nullptr;     // counts of paths too long for the record's word (n entries)
+    int4 *skip = nullptr;         // landmark skips (device_common.cuh)
+    int32_t *key = nullptr;       // comparison keys
+    int32_t *ulist = nullptr, *ucount = nullptr;   // the vertices the sink does not reach (*ucount 0 on entry)
+    int32_t *la = nullptr, *lb = nullptr, *lcount = nullptr;   // walks cut short: two lists (n entries), a counter
+    int4 *ja = nullptr, *jb = nullptr;             // their jump entries (n entries each)
+    int32_t *cnt = nullptr;       // three counters
+    ChangeTrack track;
+    const int32_t *gate = nullptr;
+};
+void launch_root_init(cudaStream_t s, const EvalArgs &a);
+void launch_root_walk(cudaStream_t s, const EvalArgs &a);
+// Cooperative launch; returns a cudaError_t value.
+int launch_root_settle(cudaStream_t s, const EvalArgs &a);
+
+// ---- list ranking of an Euler tour (gpu_list_ranking.cu:52-277), the
+// evaluation without allocation (noalloc.cu)
 // Sublist walks; heads are the nodes j*stride (j < nsub-1) and the list start.
 // One thread per sublist, `block` threads per block (a multiple of 32, <= 1024).
 constexpr int kWalkBlock = 128;
@@ -164,11 +166,6 @@ void launch_broadcast_depth(cudaStream_t s, int32_t n, const int2 *vloc, const i
                             const int32_t *strat, const int32_t *pri, const uint8_t *solved,
                             int32_t *st, PathNode *node, int32_t *ulist, int32_t *ucount,
                             const int32_t *gate = nullptr);
-// Root-path summaries (rmax, rcnt) of every reached vertex, also stored as its
-// comparison key when key != nullptr.
-// With skip (n entries), also each reached vertex's landmark skip (device_common.cuh).
-void launch_rootinfo(cudaStream_t s, int32_t n, const int32_t *st, PathNode *node, int32_t *key, uint32_t *err,
-                     ChangeTrack track = ChangeTrack(), const int32_t *gate = nullptr, int4 *skip = nullptr);
 // Cycle parity of the *ucount vertices in ulist (cooperative launch), also
 // stored as their comparison keys when key != nullptr.  ja, jb: n entries;
 // la, lb: n entries (active lists); cnt: 3 counters.  Returns a cudaError_t
@@ -183,9 +180,8 @@ int launch_cycles(cudaStream_t s, const int32_t *ucount, const int32_t *ulist, c
 // are scanned, and *from moves to the list's end: the entries before it were
 // scanned by this player's last mark_solved, and a vertex whose status has
 // changed since was appended again by a patch (EvalGates::mfrom).
-// Newly solved vertices are flagged in dirty (their children leave the tour).
 void launch_mark_solved(cudaStream_t s, const int32_t *ucount, const int32_t *ulist, int32_t player,
-                        const int32_t *st, uint8_t *solved, uint8_t *dirty, const int32_t *game_of = nullptr,
+                        const int32_t *st, uint8_t *solved, const int32_t *game_of = nullptr,
                         const int32_t *gmask = nullptr, const int32_t *gate = nullptr,
                         int32_t *from = nullptr, uint32_t *done = nullptr);
 
@@ -193,8 +189,7 @@ void launch_mark_solved(cudaStream_t s, const int32_t *ucount, const int32_t *ul
 // Switches the np vertices listed in plist (all owned by `player`).
 // stats[0..3] += compared edges, walk loads, changed vertices, strict
 // improvements; with game_of (batches) also gcount[game] += improvements,
-// and with gmask only vertices of games whose mask is set switch.  The old and
-// the new successor of every changed vertex are flagged in dirty.  With need
+// and with gmask only vertices of games whose mask is set switch.  With need
 // (and list: n entries, list_count: one counter) only the vertices of plist
 // whose need flag is set are examined (ChangeTrack); examined vertices get
 // need = 0, or 1 when a tie at their best successor leaves their choice to a
@@ -206,8 +201,9 @@ void launch_mark_solved(cudaStream_t s, const int32_t *ucount, const int32_t *ul
 // and owner bytes rather than through plist.
 void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t player,
                    const int32_t *off, const int32_t *tgt, int32_t *strat, const int32_t *st,
-                   const int32_t *key, const PathNode *node, unsigned long long *stats, const int32_t *game_of,
-                   unsigned long long *gcount, const int32_t *gmask, uint8_t *dirty, uint32_t *err,
+                   const int32_t *key, const PathNode *node, const int32_t *rdeep,
+                   unsigned long long *stats, const int32_t *game_of,
+                   unsigned long long *gcount, const int32_t *gmask, uint32_t *err,
                    const int32_t *gate = nullptr, uint8_t *need = nullptr, int32_t *list = nullptr,
                    int32_t *list_count = nullptr, ChangeList changes = ChangeList(), uint8_t *tie = nullptr,
                    uint8_t *watch = nullptr, const int4 *skip = nullptr, bool warp = false,
@@ -227,23 +223,17 @@ void launch_arena_place(cudaStream_t s, int32_t nu, int32_t k_games, const int32
                         const int32_t *u_off, const int32_t *u_tgt, const int32_t *u_roff, const int32_t *u_rsrc,
                         int8_t *owner, int32_t *pri, int32_t *off, int32_t *tgt, int32_t *rev_off, int32_t *rev_src,
                         int32_t *strat, int32_t *st, uint8_t *solved, int32_t *game_of, int4 *gstate,
-                        unsigned long long *gcount, int32_t *succ, uint8_t *dirty, uint8_t *need,
-                        ChangeList changes = ChangeList());
+                        unsigned long long *gcount, uint8_t *need, ChangeList changes = ChangeList());
 // Games copied as they are into a union (game k at vertices ub[k], edges
 // ue[k]): offsets and targets shifted to union numbering, u_off[nu] = ue[K],
 // and game_of[v] = v's game when game_of != nullptr.
 void launch_union_fixup(cudaStream_t s, int32_t nu, int64_t mu, int32_t k_games, const int32_t *ub, const int32_t *ue,
                         int32_t *u_off, int32_t *u_tgt, int32_t *game_of = nullptr);
-// Tour upkeep of the arena: every slot an isolated pair; the sink's nodes
-// following the vertex count from old_n to new_n.
-void launch_isolate_pairs(cudaStream_t s, int64_t count, int32_t *succ);
-void launch_move_extent(cudaStream_t s, int32_t old_n, int32_t new_n, int32_t *succ);
 // A finished game's strategy (its own ids) and infinite flags into out
 // (2 count entries).
 void launch_arena_export(cudaStream_t s, int32_t vb, int32_t count, const int32_t *strat, const int32_t *st,
                          int32_t *out);
-void launch_arena_clear(cudaStream_t s, int32_t vb, int32_t count, uint8_t *solved, int32_t *game_of, int32_t *st,
-                        int32_t *succ, uint8_t *dirty);
+void launch_arena_clear(cudaStream_t s, int32_t vb, int32_t count, uint8_t *solved, int32_t *game_of, int32_t *st);
 // Appends the vertices of `player` that belong to a game to plist (*count += k).
 void launch_build_plist(cudaStream_t s, int32_t n, int32_t player, const int8_t *owner, const int32_t *game_of,
                         int32_t *plist, int32_t *count);
@@ -255,7 +245,7 @@ void launch_serve_account(cudaStream_t s, int32_t slots, int32_t event, int4 *st
 // switched go back to their first successor.
 void launch_serve_reset_odd(cudaStream_t s, int32_t np, const int32_t *plist, const int32_t *game_of,
                             const int32_t *gmask, const unsigned long long *gcount, const int32_t *off,
-                            const int32_t *tgt, int32_t *strat, uint8_t *dirty, uint8_t *need,
+                            const int32_t *tgt, int32_t *strat, uint8_t *need,
                             ChangeList changes = ChangeList());
 
 // ---- dense valuation rows for export (the reference's ArrayVal layout)
@@ -267,7 +257,7 @@ void launch_materialize(cudaStream_t s, int32_t v0, int32_t count, int32_t d, co
 // changed since the last evaluation; the result equals a full evaluation's.
 struct PatchArgs {
     EvalGates *g = nullptr;
-    int32_t *ucount = nullptr, *sinkcount = nullptr;   // reset when the full evaluation runs
+    int32_t *ucount = nullptr;   // reset when the full evaluation runs
     const int32_t *clist = nullptr;                    // the changed vertices (ChangeList)
     const int32_t *strat = nullptr, *pri = nullptr, *rev_off = nullptr, *rev_src = nullptr;
     const uint8_t *solved = nullptr;
@@ -280,6 +270,7 @@ struct PatchArgs {
     int64_t ucap = 0;           // capacity of ulist
     int32_t *st = nullptr;
     PathNode *node = nullptr;
+    int32_t *rdeep = nullptr;
     int32_t *key = nullptr;
     int32_t *ulist = nullptr;   // unreached list, appended to (mark_solved scans it)
     unsigned long long *stats = nullptr;   // [0] += 1 per patch, [1] += vertices re-evaluated
@@ -287,7 +278,7 @@ struct PatchArgs {
     int4 *skip = nullptr;       // landmark skips: a patched vertex's record becomes unknown
 };
 // Sets the gates the host decides before an evaluation (one thread).
-void launch_eval_gates(cudaStream_t s, EvalGates *g, int32_t full, int32_t incr, int32_t try_patch);
+void launch_eval_gates(cudaStream_t s, EvalGates *g, int32_t try_patch);
 // One thread: decides between a patch and the full evaluation (gates).
 void launch_patch_begin(cudaStream_t s, const PatchArgs &a);
 // Cooperative launches, gated on g->patch; return a cudaError_t value.

@@ -10,14 +10,12 @@
 // with exactly the state a full evaluation (compute_valuation,
 // gpu_list_ranking.cu:279-326) would leave.  Most evaluations of a solve
 // follow such a step: in Odd's best-response loop the number of changed
-// strategies falls by about an order of magnitude per step.  The Euler tour
-// is not touched: the parents flagged dirty since its last update stay
-// flagged, and the next full evaluation relinks them all.
+// strategies falls by about an order of magnitude per step.
 //
 //  1. k_patch_begin (one thread) takes the changed vertices the switch steps
 //     listed since the last evaluation and opens either the patch's gate or
 //     the full evaluation's: a patch needs the list complete, the caller's
-//     permission (the tour and the list cover every change since the last
+//     permission (the list covers every change since the last
 //     evaluation) and room in the unreached list.
 //  2. k_patch_collect (cooperative) finds A level by level: the changed
 //     vertices (the seeds, level 0), then the in-neighbours u with
@@ -77,12 +75,7 @@ __device__ __forceinline__ int ceil_log2_i(int64_t x)
     return r;
 }
 
-__global__ void k_eval_gates(EvalGates *g, int32_t full, int32_t incr, int32_t try_patch)
-{
-    g->full = full;
-    g->incr = incr;
-    g->try_patch = try_patch;
-}
+__global__ void k_eval_gates(EvalGates *g, int32_t try_patch) { g->try_patch = try_patch; }
 
 __global__ void k_patch_begin(PatchArgs a)
 {
@@ -98,17 +91,12 @@ __global__ void k_patch_begin(PatchArgs a)
         ok = false;
     }
     if (ok) {
-        g->saved_full = g->full;
-        g->saved_incr = g->incr;
-        g->full = 0;
-        g->incr = 0;
         g->eval = 0;
         g->patch = 1;
     } else {
         g->eval = 1;
         g->patch = 0;
         *a.ucount = 0;      // the full evaluation collects the unreached vertices afresh
-        *a.sinkcount = 0;
         g->mfrom[0] = g->mfrom[1] = 0;
     }
 }
@@ -304,10 +292,7 @@ __global__ void __launch_bounds__(kPatchBlock) k_patch_collect(PatchArgs a)
     if (leader) {
         g->patch = 0;
         g->eval = 1;
-        g->full = g->saved_full;
-        g->incr = g->saved_incr;
         *a.ucount = 0;
-        *a.sinkcount = 0;
         g->mfrom[0] = g->mfrom[1] = 0;
         g->skip = g->backoff;
         g->backoff = g->backoff < kBackoffMax ? 2 * g->backoff : kBackoffMax;
@@ -373,7 +358,7 @@ __global__ void __launch_bounds__(kPatchBlock) k_patch_values(PatchArgs a)
             if (st >= 1) {
                 const PathNode q = a.node[t];
                 val.x += st;
-                top1_merge(val.y, val.z, q.rmax, q.rcnt);
+                top1_merge(val.y, val.z, q.rmax, st < kDeepPath ? path_word_count(q.word) : a.rdeep[t]);
             } else {
                 val.x = st;
             }
@@ -405,8 +390,10 @@ __global__ void __launch_bounds__(kPatchBlock) k_patch_values(PatchArgs a)
             if (sv.x >= 1) {
                 int32_t m = r.z, c = r.w;
                 top1_merge(m, c, sv.y, sv.z);
-                a.st[v] = r.y + sv.x;
-                a.node[v] = PathNode{sv_strat, sv_pri, m, c};
+                const int32_t d = r.y + sv.x;
+                a.st[v] = d;
+                a.node[v] = PathNode{sv_strat, sv_pri, m, path_word(d, c)};
+                if (d >= kDeepPath) a.rdeep[v] = c;
                 k = finite_key(m, c);
             } else {
                 a.st[v] = sv.x;
@@ -452,10 +439,10 @@ std::atomic<int> g_collect_blocks[kMaxCachedDevices], g_values_blocks[kMaxCached
 
 }  // namespace
 
-void launch_eval_gates(cudaStream_t s, EvalGates *g, int32_t full, int32_t incr, int32_t try_patch)
+void launch_eval_gates(cudaStream_t s, EvalGates *g, int32_t try_patch)
 {
     count_launch();
-    k_eval_gates<<<1, 1, 0, s>>>(g, full, incr, try_patch);
+    k_eval_gates<<<1, 1, 0, s>>>(g, try_patch);
 }
 
 void launch_patch_begin(cudaStream_t s, const PatchArgs &a)

@@ -37,8 +37,8 @@ __global__ void k_arena_place(int32_t nu, int32_t k_games, const int32_t *__rest
                               int32_t *__restrict__ rev_off, int32_t *__restrict__ rev_src,
                               int32_t *__restrict__ strat, int32_t *__restrict__ st, uint8_t *__restrict__ solved,
                               int32_t *__restrict__ game_of, int4 *__restrict__ gstate,
-                              unsigned long long *__restrict__ gcount, int32_t *__restrict__ succ,
-                              uint8_t *__restrict__ dirty, uint8_t *__restrict__ need, ChangeList changes)
+                              unsigned long long *__restrict__ gcount, uint8_t *__restrict__ need,
+                              ChangeList changes)
 {
     int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nu) return;
@@ -63,11 +63,6 @@ __global__ void k_arena_place(int32_t nu, int32_t k_games, const int32_t *__rest
     st[a] = 0;
     solved[a] = 0;
     game_of[a] = slot[k];
-    // tour: an isolated pair until the next evaluation relinks a (a dirty
-    // parent) and its parent links it
-    succ[2 * (int64_t)a] = 2 * a + 1;
-    succ[2 * (int64_t)a + 1] = 2 * a;
-    dirty[a] = 1;
     need[a] = 1;
     if (changes.list) note_change(changes, a);   // a new vertex: the next evaluation may patch it in
     if (i == u0) {
@@ -84,9 +79,6 @@ __global__ void k_arena_place(int32_t nu, int32_t k_games, const int32_t *__rest
         st[z] = 0;
         solved[z] = 1;
         game_of[z] = -1;
-        succ[2 * (int64_t)z] = 2 * z + 1;
-        succ[2 * (int64_t)z + 1] = 2 * z;
-        dirty[z] = 0;
     }
 }
 
@@ -121,28 +113,6 @@ __global__ void k_union_fixup(int32_t nu, int64_t mu, int32_t k_games, const int
     if (blockIdx.x == 0 && threadIdx.x == 0) u_off[nu] = ue[k_games];
 }
 
-// Every slot of a new arena starts as an isolated tour pair.
-__global__ void k_isolate_pairs(int64_t count, int32_t *__restrict__ succ)
-{
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < count; v += (int64_t)gridDim.x * blockDim.x) {
-        succ[2 * v] = (int32_t)(2 * v + 1);
-        succ[2 * v + 1] = (int32_t)(2 * v);
-    }
-}
-
-// The arena's vertex count moved from old_n to new_n: the sink's two nodes
-// are 2n and 2n+1, so vertex old_n gets an isolated pair back (placement may
-// overwrite it next) and the new sink's down node ends the list.
-__global__ void k_move_extent(int32_t old_n, int32_t new_n, int32_t *__restrict__ succ)
-{
-    if (old_n < new_n) {
-        succ[2 * (int64_t)old_n] = 2 * old_n + 1;
-        succ[2 * (int64_t)old_n + 1] = 2 * old_n;
-    }
-    succ[2 * (int64_t)new_n] = TOUR_END;
-    succ[2 * (int64_t)new_n + 1] = 2 * new_n;
-}
-
 // A finished game's results in its own vertex ids: out[0, count) its
 // strategy (-1 = the sink), out[count, 2 count) +1 where Even wins (valuation
 // +inf), -1 at -inf, 0 at a finite valuation (CPUParity's infinite[]).
@@ -157,10 +127,10 @@ __global__ void k_arena_export(int32_t vb, int32_t count, const int32_t *__restr
 }
 
 // A removed game's range becomes inert: solved, in no game, with no finite
-// depth left behind (the root-path summary pass visits every vertex with a
-// finite depth), and out of the tour.
+// depth left behind.  The whole game leaves at once and games never link to
+// each other, so no walk comes here again.
 __global__ void k_arena_clear(int32_t vb, int32_t count, uint8_t *__restrict__ solved, int32_t *__restrict__ game_of,
-                              int32_t *__restrict__ st, int32_t *__restrict__ succ, uint8_t *__restrict__ dirty)
+                              int32_t *__restrict__ st)
 {
     int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
@@ -168,11 +138,6 @@ __global__ void k_arena_clear(int32_t vb, int32_t count, uint8_t *__restrict__ s
     solved[v] = 1;
     game_of[v] = -1;
     st[v] = 0;
-    dirty[v] = 0;
-    // the whole game leaves at once (games never link to each other), so its
-    // pairs can be isolated without touching anyone else's list
-    succ[2 * (int64_t)v] = 2 * v + 1;
-    succ[2 * (int64_t)v + 1] = 2 * v;
 }
 
 // Vertices of `player` that belong to a game, appended in any order (the
@@ -236,8 +201,8 @@ __global__ void k_serve_account(int32_t slots, int32_t event, int4 *__restrict__
 __global__ void k_serve_reset_odd(int32_t np, const int32_t *__restrict__ plist, const int32_t *__restrict__ game_of,
                                   const int32_t *__restrict__ gmask, const unsigned long long *__restrict__ gcount,
                                   const int32_t *__restrict__ off, const int32_t *__restrict__ tgt,
-                                  int32_t *__restrict__ strat, uint8_t *__restrict__ dirty,
-                                  uint8_t *__restrict__ need, ChangeList changes)
+                                  int32_t *__restrict__ strat, uint8_t *__restrict__ need,
+                                  ChangeList changes)
 {
     int32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= np) return;
@@ -247,9 +212,7 @@ __global__ void k_serve_reset_odd(int32_t np, const int32_t *__restrict__ plist,
     int32_t old = strat[v], first = tgt[off[v]];
     if (old == first) return;
     strat[v] = first;
-    if (old >= 0) dirty[old] = 1;   // both parents' child lists change
-    dirty[first] = 1;
-    need[v] = 1;                    // its choice starts over
+    need[v] = 1;   // its choice starts over
     if (changes.list) note_change(changes, v);
 }
 
@@ -257,12 +220,11 @@ __global__ void k_serve_reset_odd(int32_t np, const int32_t *__restrict__ plist,
 
 void launch_serve_reset_odd(cudaStream_t s, int32_t np, const int32_t *plist, const int32_t *game_of,
                             const int32_t *gmask, const unsigned long long *gcount, const int32_t *off,
-                            const int32_t *tgt, int32_t *strat, uint8_t *dirty, uint8_t *need, ChangeList changes)
+                            const int32_t *tgt, int32_t *strat, uint8_t *need, ChangeList changes)
 {
     if (np <= 0) return;
     count_launch();
-    k_serve_reset_odd<<<grid_for(np), kBlock, 0, s>>>(np, plist, game_of, gmask, gcount, off, tgt, strat, dirty, need,
-                                                      changes);
+    k_serve_reset_odd<<<grid_for(np), kBlock, 0, s>>>(np, plist, game_of, gmask, gcount, off, tgt, strat, need, changes);
 }
 
 void launch_arena_place(cudaStream_t s, int32_t nu, int32_t k_games, const int32_t *ub, const int32_t *vb,
@@ -270,14 +232,13 @@ void launch_arena_place(cudaStream_t s, int32_t nu, int32_t k_games, const int32
                         const int32_t *u_off, const int32_t *u_tgt, const int32_t *u_roff, const int32_t *u_rsrc,
                         int8_t *owner, int32_t *pri, int32_t *off, int32_t *tgt, int32_t *rev_off, int32_t *rev_src,
                         int32_t *strat, int32_t *st, uint8_t *solved, int32_t *game_of, int4 *gstate,
-                        unsigned long long *gcount, int32_t *succ, uint8_t *dirty, uint8_t *need,
-                        ChangeList changes)
+                        unsigned long long *gcount, uint8_t *need, ChangeList changes)
 {
     if (nu <= 0) return;
     count_launch();
     k_arena_place<<<grid_for(nu), kBlock, 0, s>>>(nu, k_games, ub, vb, eb, slot, u_owner, u_pri, u_off, u_tgt, u_roff,
                                                   u_rsrc, owner, pri, off, tgt, rev_off, rev_src, strat, st, solved,
-                                                  game_of, gstate, gcount, succ, dirty, need, changes);
+                                                  game_of, gstate, gcount, need, changes);
 }
 
 void launch_union_fixup(cudaStream_t s, int32_t nu, int64_t mu, int32_t k_games, const int32_t *ub, const int32_t *ue,
@@ -289,21 +250,6 @@ void launch_union_fixup(cudaStream_t s, int32_t nu, int64_t mu, int32_t k_games,
     k_union_fixup<<<g, kBlock, 0, s>>>(nu, mu, k_games, ub, ue, u_off, u_tgt, game_of);
 }
 
-void launch_isolate_pairs(cudaStream_t s, int64_t count, int32_t *succ)
-{
-    if (count <= 0) return;
-    count_launch();
-    unsigned g = grid_for(count);
-    g = g < 2432u ? g : 2432u;
-    k_isolate_pairs<<<g, kBlock, 0, s>>>(count, succ);
-}
-
-void launch_move_extent(cudaStream_t s, int32_t old_n, int32_t new_n, int32_t *succ)
-{
-    count_launch();
-    k_move_extent<<<1, 1, 0, s>>>(old_n, new_n, succ);
-}
-
 void launch_arena_export(cudaStream_t s, int32_t vb, int32_t count, const int32_t *strat, const int32_t *st,
                          int32_t *out)
 {
@@ -312,12 +258,11 @@ void launch_arena_export(cudaStream_t s, int32_t vb, int32_t count, const int32_
     k_arena_export<<<grid_for(count), kBlock, 0, s>>>(vb, count, strat, st, out);
 }
 
-void launch_arena_clear(cudaStream_t s, int32_t vb, int32_t count, uint8_t *solved, int32_t *game_of, int32_t *st,
-                        int32_t *succ, uint8_t *dirty)
+void launch_arena_clear(cudaStream_t s, int32_t vb, int32_t count, uint8_t *solved, int32_t *game_of, int32_t *st)
 {
     if (count <= 0) return;
     count_launch();
-    k_arena_clear<<<grid_for(count), kBlock, 0, s>>>(vb, count, solved, game_of, st, succ, dirty);
+    k_arena_clear<<<grid_for(count), kBlock, 0, s>>>(vb, count, solved, game_of, st);
 }
 
 void launch_build_plist(cudaStream_t s, int32_t n, int32_t player, const int8_t *owner, const int32_t *game_of,

@@ -60,11 +60,9 @@ int Solver::create(const CsrView &g, const psi_options &opt, Solver **out, bool 
     Solver *s = new Solver();
     s->device_ = opt.device;
     s->timing_ = opt.timing != 0;
-    s->stride_ = opt.sublist_len;
     s->use_graph_ = opt.graph != 0;
     s->incremental_ = opt.incremental;
     s->patch_limit_ = opt.patch_limit;
-    s->walk_block_ = opt.walk_block ? opt.walk_block : kWalkBlock;
     s->switch_warp_ = opt.switch_kernel == PSI_SWITCH_WARP;
     rc = s->alloc_arrays(g.n, g.m);
     if (!rc) rc = s->upload_game(g, validate);
@@ -88,11 +86,9 @@ int Solver::create_arena(int64_t max_vertices, int64_t max_edges, int32_t slots,
     Solver *s = new Solver();
     s->device_ = opt.device;
     s->timing_ = opt.timing != 0;
-    s->stride_ = opt.sublist_len;
     // admissions list their new vertices as changed ones: a patch evaluates them
     s->incremental_ = opt.incremental;
     s->patch_limit_ = opt.patch_limit;
-    s->walk_block_ = opt.walk_block ? opt.walk_block : kWalkBlock;
     s->switch_warp_ = opt.switch_kernel == PSI_SWITCH_WARP;
     rc = s->alloc_arrays(max_vertices, max_edges);
     if (!rc) rc = s->init_arena(slots);
@@ -137,11 +133,9 @@ int Solver::create_union(const std::vector<const HostGame *> &gs, const psi_opti
     Solver *s = new Solver();
     s->device_ = opt.device;
     s->timing_ = opt.timing != 0;
-    s->stride_ = opt.sublist_len;
     s->use_graph_ = opt.graph != 0;
     s->incremental_ = opt.incremental;
     s->patch_limit_ = opt.patch_limit;
-    s->walk_block_ = opt.walk_block ? opt.walk_block : kWalkBlock;
     s->switch_warp_ = opt.switch_kernel == PSI_SWITCH_WARP;
     rc = s->alloc_arrays(n, m);
     if (!rc) rc = s->upload_union(gs, table, base->back());
@@ -158,7 +152,7 @@ int Solver::upload_union(const std::vector<const HostGame *> &gs, const std::vec
 {
     const int32_t K = (int32_t)gs.size();
     const int32_t *ub = table.data(), *ue = ub + K + 1;
-    set_extent((int32_t)n);
+    n_ = (int32_t)n;
     m_ = ue[K];
     np_ = n_;
     const struct {
@@ -191,16 +185,6 @@ int Solver::upload_union(const std::vector<const HostGame *> &gs, const std::vec
     return finish_upload();
 }
 
-// Vertex count the kernels process: the tour has 2n+2 nodes, the sublist
-// heads follow from the stride.
-void Solver::set_extent(int32_t n)
-{
-    n_ = n;
-    L_ = 2 * (int64_t)n_ + 2;
-    // heads at node j*stride for j < nsub-1, plus the list start (node L-1)
-    nsub_ = (int32_t)(ceil_div(L_ - 1, stride_) + 1);
-}
-
 // Device arrays for games of up to cap_n vertices and cap_m edges.
 int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
 {
@@ -208,8 +192,6 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
     if (rc) return rc;
     cap_n_ = cap_n;
     cap_m_ = cap_m;
-    const int64_t capL = 2 * cap_n + 2;
-    const int64_t cap_sub = ceil_div(capL - 1, stride_) + 1;
     // incremental evaluation: change-list capacity (larger lists mean a full
     // evaluation), re-evaluated set capacity, level cap of its search
     if (incremental_ != PSI_INCR_OFF) {
@@ -245,16 +227,13 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
         {(void **)&node_, sizeof(PathNode) * (size_t)cap_n},
         {(void **)&skip_, sizeof(int4) * (size_t)cap_n},
         {(void **)&key_, 4 * (size_t)cap_n},
-        {(void **)&succ_, 4 * (size_t)capL},
-        {(void **)&dirty_, (size_t)cap_n},
+        {(void **)&rdeep_, 4 * (size_t)cap_n},
         {(void **)&need_, (size_t)cap_n},
         {(void **)&tie_, (size_t)cap_n},
         {(void **)&watch_, (size_t)cap_n},
         {(void **)&ulist_, 4 * (size_t)ucap_},
-        {(void **)&vloc_, 8 * (size_t)cap_n},
-        {(void **)&redA_, 8 * (size_t)cap_sub},
-        {(void **)&redB_, 8 * (size_t)cap_sub},
-        {(void **)&redC_, 8 * (size_t)cap_sub},
+        {(void **)&la_, 4 * (size_t)cap_n},
+        {(void **)&lb_, 4 * (size_t)cap_n},
         {(void **)&jA_, sizeof(int4) * (size_t)cap_n},
         {(void **)&jB_, sizeof(int4) * (size_t)cap_n},
         {(void **)&dw_, sizeof(Words)},
@@ -288,7 +267,6 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
     const GraphCtl fresh;
     // pageable source: staged before the call returns
     PSI_CUDA_TRY(cudaMemcpyAsync(ctl_, &fresh, sizeof fresh, cudaMemcpyHostToDevice, stream_));
-    PSI_CUDA_TRY(cudaMemsetAsync(dirty_, 0, (size_t)cap_n, stream_));
     return PSI_OK;
 }
 
@@ -298,7 +276,7 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
 // partition on the device.
 int Solver::upload_game(const CsrView &g, bool validate)
 {
-    set_extent(g.n);
+    n_ = g.n;
     m_ = g.m;
     max_pri_ = g.max_pri;
     np_ = n_;
@@ -328,7 +306,7 @@ int Solver::upload_game(const CsrView &g, bool validate)
 int Solver::finish_upload()
 {
     launch_narrow_owner(stream_, n_, st_, owner_);
-    int ce = partition_players(stream_, n_, owner_, plist_, &dw_->sinkcount);
+    int ce = partition_players(stream_, n_, owner_, plist_, &dw_->selcount);
     if (ce) return fail(PSI_ERR_CUDA, std::string("player lists: ") + cudaGetErrorString((cudaError_t)ce));
     PSI_CUDA_TRY(cudaMemsetAsync(solved_, 0, n_, stream_));
     PSI_CUDA_TRY(cudaMemsetAsync(st_, 0, 4 * (size_t)n_, stream_));
@@ -339,7 +317,7 @@ int Solver::finish_upload()
     if (ce) return fail(PSI_ERR_CUDA, std::string("reverse CSR: ") + cudaGetErrorString((cudaError_t)ce));
     int rc = sync_and_check("upload");
     if (rc) return rc;
-    np0_ = hw_->sinkcount;
+    np0_ = hw_->selcount;
     return PSI_OK;
 }
 
@@ -419,9 +397,6 @@ int Solver::sync_and_check(const char *what)
     if (rc) return rc;
     times_.patches = (int64_t)hw_->patch[0];
     times_.patched = (int64_t)hw_->patch[1];
-    times_.tour_parents = (int64_t)hw_->relink[0];
-    times_.tour_entries = (int64_t)hw_->relink[1];
-    times_.tour_children = (int64_t)hw_->relink[2];
     if (hw_->err) {
         uint32_t bits = hw_->err;
         cudaMemsetAsync(dw_, 0, sizeof(Words), stream_);
@@ -435,8 +410,7 @@ void Solver::reset_times()
 {
     times_ = SolverTimes();
     cudaMemsetAsync(dw_->patch, 0, sizeof(dw_->patch), stream_);
-    cudaMemsetAsync(dw_->relink, 0, sizeof(dw_->relink), stream_);
-    if (hw_) hw_->patch[0] = hw_->patch[1] = hw_->relink[0] = hw_->relink[1] = hw_->relink[2] = 0;
+    if (hw_) hw_->patch[0] = hw_->patch[1] = 0;
 }
 
 void Solver::reset_tracking()
@@ -459,7 +433,7 @@ int Solver::init_strat()
     if (rc) return rc;
     strat_ready_ = true;
     val_ready_ = false;
-    tour_valid_ = false;
+    tracked_ = false;
     return PSI_OK;
 }
 
@@ -470,7 +444,7 @@ int Solver::reset_opponent_strategy()
     if (rc) return rc;
     launch_reset_odd(stream_, n_, owner_, off_, tgt_, strat_);
     reset_tracking();   // Odd's choices start over
-    tour_valid_ = false;
+    tracked_ = false;
     return sync_and_check("reset_opponent_strategy");
 }
 
@@ -479,7 +453,6 @@ PatchArgs Solver::patch_args()
     PatchArgs a;
     a.g = ctl_;
     a.ucount = &dw_->ucount;
-    a.sinkcount = &dw_->sinkcount;
     a.clist = clist_;
     a.strat = strat_;
     a.pri = pri_;
@@ -498,6 +471,7 @@ PatchArgs Solver::patch_args()
     a.ucap = ucap_;
     a.st = st_;
     a.node = node_;
+    a.rdeep = rdeep_;
     a.key = key_;
     a.ulist = ulist_;
     a.stats = dw_->patch;
@@ -531,51 +505,43 @@ int Solver::enqueue_patch(bool timed)
     return PSI_OK;
 }
 
-// The full evaluation, every kernel gated (ctl_->full / incr / eval).
+EvalArgs Solver::eval_args()
+{
+    EvalArgs a;
+    a.n = n_;
+    a.strat = strat_;
+    a.pri = pri_;
+    a.solved = solved_;
+    a.st = st_;
+    a.node = node_;
+    a.rdeep = rdeep_;
+    a.skip = skip_;
+    a.key = key_;
+    a.ulist = ulist_;
+    a.ucount = &dw_->ucount;
+    a.la = la_;
+    a.lb = lb_;
+    a.lcount = &dw_->lcount;
+    a.ja = jA_;
+    a.jb = jB_;
+    a.cnt = dw_->cnt;
+    a.track = track();
+    a.gate = &ctl_->eval;
+    return a;
+}
+
+// The full evaluation (root_kernels.cu), every kernel gated (ctl_->eval).
 int Solver::enqueue_full(bool timed)
 {
-    auto begin = [&](Phase p) {
-        if (timed) phase_begin(p);
-    };
-    auto end = [&](Phase p) {
-        if (timed) phase_end(p);
-    };
-    // 1. Euler tour of the sink tree: built afresh (gate full) or the previous
-    //    one relinked where strategies or solved flags changed (gate incr);
-    //    jA_ is free until the cycle pass: it holds the list of dirty parents
-    begin(PH_TOUR);
-    launch_tour_build(stream_, n_, strat_, solved_, rev_off_, rev_src_, succ_, vloc_, ulist_, &dw_->sinkcount, dirty_,
-                      &ctl_->full, tie_, need_, dw_->relink);
-    int ce = launch_tour_update(stream_, n_, strat_, solved_, rev_off_, rev_src_, dirty_, succ_, vloc_, ulist_,
-                                &dw_->sinkcount, reinterpret_cast<int32_t *>(jA_), &dw_->cnt[0], &ctl_->incr, tie_,
-                                need_, dw_->relink);
-    if (ce) return fail(PSI_ERR_CUDA, std::string("tour update: ") + cudaGetErrorString((cudaError_t)ce));
-    end(PH_TOUR);
-    // 2. Helman-JaJa sublists, then the reduced list ranked on the device
-    begin(PH_SUBLIST);
-    launch_walk_sublists(stream_, nsub_, n_, L_, stride_, succ_, vloc_, redA_, &dw_->err, &ctl_->eval,
-                         walk_block_);
-    end(PH_SUBLIST);
-    begin(PH_REDUCED);
-    const int2 *fin = nullptr;
-    ce = launch_rank_reduced(stream_, nsub_, redA_, redB_, redC_, &fin, &ctl_->eval, &dw_->err);
-    if (ce) return fail(PSI_ERR_CUDA, std::string("reduced-list kernel: ") + cudaGetErrorString((cudaError_t)ce));
-    end(PH_REDUCED);
-    // 3. broadcast depths; collect the vertices the sink does not reach
-    //    (ulist held the sink's children until here); root-path summaries
-    begin(PH_BROADCAST);
-    launch_broadcast_depth(stream_, n_, vloc_, fin, strat_, pri_, solved_, st_, node_, ulist_, &dw_->ucount,
-                           &ctl_->eval);
-    launch_rootinfo(stream_, n_, st_, node_, key_, &dw_->err, track(), &ctl_->eval, skip_);
-    end(PH_BROADCAST);
-    // 4. cycle parity by pointer jumping over the unreached vertices (the
-    //    tour's vloc array is free again: it holds the two active lists)
-    begin(PH_CYCLES);
-    int32_t *la = reinterpret_cast<int32_t *>(vloc_), *lb = la + n_;
-    ce = launch_cycles(stream_, &dw_->ucount, ulist_, strat_, pri_, solved_, st_, key_, jA_, jB_, la, lb, dw_->cnt,
-                       &dw_->err, track(), &ctl_->eval);
-    if (ce) return fail(PSI_ERR_CUDA, std::string("cycle kernel: ") + cudaGetErrorString((cudaError_t)ce));
-    end(PH_CYCLES);
+    const EvalArgs a = eval_args();
+    if (timed) phase_begin(PH_BROADCAST);
+    launch_root_init(stream_, a);
+    launch_root_walk(stream_, a);
+    if (timed) phase_end(PH_BROADCAST);
+    if (timed) phase_begin(PH_CYCLES);
+    int ce = launch_root_settle(stream_, a);
+    if (ce) return fail(PSI_ERR_CUDA, std::string("settling kernel: ") + cudaGetErrorString((cudaError_t)ce));
+    if (timed) phase_end(PH_CYCLES);
     return PSI_OK;
 }
 
@@ -584,10 +550,9 @@ int Solver::compute_valuation()
     if (!strat_ready_) return fail(PSI_ERR_STATE, "compute_valuation before init_strat");
     int rc = set_device();
     if (rc) return rc;
-    // the previous tour (and the switch steps' change list since) is usable
-    // only if no strategy changed outside a switch step since it was built
-    launch_eval_gates(stream_, ctl_, tour_valid_ ? 0 : 1, tour_valid_ ? 1 : 0,
-                      (tour_valid_ && incremental_ != PSI_INCR_OFF) ? 1 : 0);
+    // the last evaluation's state and the switch steps' change list since are
+    // usable only if no strategy changed outside a switch step
+    launch_eval_gates(stream_, ctl_, (tracked_ && incremental_ != PSI_INCR_OFF) ? 1 : 0);
     const unsigned long long patches_before = hw_->patch[0];
     phase_begin(PH_EVAL);
     rc = enqueue_eval(true);
@@ -603,7 +568,7 @@ int Solver::compute_valuation()
     }
     times_.evals++;
     val_ready_ = true;
-    tour_valid_ = true;
+    tracked_ = true;
     return PSI_OK;
 }
 
@@ -614,7 +579,7 @@ int Solver::mark_solved(int32_t player)
     int rc = set_device();
     if (rc) return rc;
     // a masked step (served games) scans the whole list
-    launch_mark_solved(stream_, &dw_->ucount, ulist_, player, st_, solved_, dirty_, gmask_ ? game_of_ : nullptr,
+    launch_mark_solved(stream_, &dw_->ucount, ulist_, player, st_, solved_, gmask_ ? game_of_ : nullptr,
                        gmask_, nullptr, gmask_ ? nullptr : &ctl_->mfrom[player], &ctl_->mdone);
     PSI_CUDA_TRY(cudaGetLastError());
     return PSI_OK;   // ordered on the stream before the next call
@@ -630,9 +595,9 @@ int Solver::switch_strategy(int32_t player, int64_t *switched)
     phase_begin(PH_SWITCH);
     const int32_t np = (player == 0) ? np0_ : np_ - np0_;
     const int32_t *pl = plist_ + (player == 0 ? 0 : np0_);
-    // jB_ is free until the next cycle pass: it holds the list of vertices to examine
-    launch_switch(stream_, np, pl, player, off_, tgt_, strat_, st_, key_, node_, dw_->sw, game_of_, gcount_, gmask_,
-                  dirty_, &dw_->err, nullptr, need_, reinterpret_cast<int32_t *>(jB_), &dw_->cnt[2], changes(), tie_,
+    // jB_ is free until the next full evaluation: it holds the list of vertices to examine
+    launch_switch(stream_, np, pl, player, off_, tgt_, strat_, st_, key_, node_, rdeep_, dw_->sw, game_of_, gcount_,
+                  gmask_, &dw_->err, nullptr, need_, reinterpret_cast<int32_t *>(jB_), &dw_->cnt[2], changes(), tie_,
                   watch_, skip_, switch_warp_, &dw_->claim, arena_ ? nullptr : owner_, n_);
     phase_end(PH_SWITCH);
     rc = sync_and_check("switch_strategy");
@@ -674,24 +639,24 @@ int Solver::get_winning(int32_t player, std::vector<int32_t> &out)
     return copy_winning(out.data(), k);
 }
 
-// The winning set of `player` selected on the device into succ_ (free between
+// The winning set of `player` selected on the device into la_ (free between
 // evaluations); *count receives its size.
 int Solver::winning_ids(int32_t player, int64_t *count)
 {
     if (player != 0 && player != 1) return fail(PSI_ERR_INVALID, "player must be 0 or 1");
     int rc = set_device();
     if (rc) return rc;
-    int ce = select_winning(stream_, n_, player, st_, succ_, &dw_->sinkcount);
+    int ce = select_winning(stream_, n_, player, st_, la_, &dw_->selcount);
     if (ce) return fail(PSI_ERR_CUDA, std::string("winning set: ") + cudaGetErrorString((cudaError_t)ce));
     rc = sync_and_check("get_winning");
     if (rc) return rc;
-    *count = hw_->sinkcount;
+    *count = hw_->selcount;
     return PSI_OK;
 }
 
 int Solver::copy_winning(int32_t *out, int64_t k)
 {
-    if (k > 0) PSI_CUDA_TRY(cudaMemcpyAsync(out, succ_, 4 * (size_t)k, cudaMemcpyDeviceToHost, stream_));
+    if (k > 0) PSI_CUDA_TRY(cudaMemcpyAsync(out, la_, 4 * (size_t)k, cudaMemcpyDeviceToHost, stream_));
     PSI_CUDA_TRY(cudaStreamSynchronize(stream_));
     return PSI_OK;
 }
@@ -741,16 +706,17 @@ int Solver::get_path_summary(int32_t *depth, int32_t *top, int32_t *count)
     if (!val_ready_) return fail(PSI_ERR_STATE, "get_path_summary before compute_valuation");
     int rc = set_device();
     if (rc) return rc;
-    std::vector<int32_t> st(n_);
+    std::vector<int32_t> st(n_), deep(n_);
     std::vector<PathNode> nd(n_);
     PSI_CUDA_TRY(cudaMemcpyAsync(st.data(), st_, 4 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
     PSI_CUDA_TRY(cudaMemcpyAsync(nd.data(), node_, sizeof(PathNode) * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
+    PSI_CUDA_TRY(cudaMemcpyAsync(deep.data(), rdeep_, 4 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
     PSI_CUDA_TRY(cudaStreamSynchronize(stream_));
     for (int32_t v = 0; v < n_; v++) {
         const bool fin = st[v] >= 1;
         if (depth) depth[v] = fin ? st[v] : 0;
         if (top) top[v] = fin ? nd[v].rmax : -1;
-        if (count) count[v] = fin ? nd[v].rcnt : 0;
+        if (count) count[v] = !fin ? 0 : (st[v] < kDeepPath ? path_word_count(nd[v].word) : deep[v]);
     }
     return PSI_OK;
 }
@@ -776,7 +742,7 @@ int Solver::set_strategy(const int32_t *in)
     reset_tracking();
     PSI_CUDA_TRY(cudaStreamSynchronize(stream_));
     strat_ready_ = true;
-    tour_valid_ = false;
+    tracked_ = false;
     return PSI_OK;
 }
 
@@ -902,7 +868,7 @@ int Solver::solve_batch(int32_t *iters, int32_t *brs)
 
 int Solver::init_arena(int32_t slots)
 {
-    set_extent(0);
+    n_ = 0;
     m_ = 0;
     max_pri_ = 0;
     np0_ = np_ = 0;
@@ -923,8 +889,6 @@ int Solver::init_arena(int32_t slots)
     PSI_CUDA_TRY(cudaMemsetAsync(solved_, 1, (size_t)cap_n_, stream_));          // every slot inert
     PSI_CUDA_TRY(cudaMemsetAsync(game_of_, 0xff, 4 * (size_t)cap_n_, stream_));   // -1: in no game
     PSI_CUDA_TRY(cudaMemsetAsync(st_, 0, 4 * (size_t)cap_n_, stream_));            // no finite depths
-    launch_isolate_pairs(stream_, cap_n_ + 1, succ_);                              // no slot in the tour
-    launch_move_extent(stream_, 0, 0, succ_);
     PSI_CUDA_TRY(cudaMemsetAsync(gstate_, 0, sizeof(int4) * (size_t)slots, stream_));
     PSI_CUDA_TRY(cudaMemsetAsync(gcount_, 0, sizeof(unsigned long long) * (size_t)slots, stream_));
     PSI_CUDA_TRY(cudaMemsetAsync(gmask_, 0, 4 * (size_t)slots, stream_));
@@ -936,8 +900,8 @@ int Solver::init_arena(int32_t slots)
 // Places the games admitted in one step: each game's arrays are copied as
 // they are into a device staging union (no host packing), shifted to union
 // numbering on the device, given one reverse-CSR build and placed by one
-// launch.  The tour stays valid: placed vertices start as isolated pairs and
-// dirty parents, which the next evaluation relinks.
+// launch.  They are listed as changed vertices, so the next evaluation may
+// be a patch.
 int Solver::arena_add(const std::vector<const HostGame *> &gs, const std::vector<int32_t> &vb,
                       const std::vector<int32_t> &eb, const std::vector<int32_t> &slot, int32_t extent)
 {
@@ -998,11 +962,10 @@ int Solver::arena_add(const std::vector<const HostGame *> &gs, const std::vector
         // with full evaluations only, the unreached list is rebuilt before its next use; after a
         // patch mark_solved reads it (the new vertices are appended by the patch)
         if (incremental_ == PSI_INCR_OFF) e = cudaMemsetAsync(&dw_->ucount, 0, sizeof(int32_t), stream_);
-        if (extent != n_) launch_move_extent(stream_, n_, extent, succ_);
         const int32_t *vbd = d_tab + 2 * K + 2, *ebd = d_tab + 3 * K + 2, *sld = d_tab + 4 * K + 2;
         launch_arena_place(stream_, (int32_t)n, K, d_tab, vbd, ebd, sld, u_owner, u_pri, u_off, u_tgt, u_roff, u_rsrc,
                            owner_, pri_, off_, tgt_, rev_off_, rev_src_, strat_, st_, solved_, game_of_, gstate_,
-                           gcount_, succ_, dirty_, need_, changes());
+                           gcount_, need_, changes());
         if (e == cudaSuccess) e = cudaGetLastError();
     }
     for (int i = 0; i < 7; i++)
@@ -1010,11 +973,11 @@ int Solver::arena_add(const std::vector<const HostGame *> &gs, const std::vector
     if (ce) return fail(PSI_ERR_CUDA, std::string("reverse CSR: ") + cudaGetErrorString((cudaError_t)ce));
     if (e != cudaSuccess) return fail(PSI_ERR_CUDA, std::string("arena_add: ") + cudaGetErrorString(e));
     if (top > max_pri_) max_pri_ = top;
-    set_extent(extent);
+    n_ = extent;
     return sync_and_check("arena_add");
 }
 
-// Retires games: their ranges become inert and leave the tour (one
+// Retires games: their ranges become inert (one
 // synchronisation for all of them).
 int Solver::arena_remove(const std::vector<int32_t> &vb, const std::vector<int32_t> &count,
                          const std::vector<int32_t> &slot, int32_t extent)
@@ -1028,13 +991,12 @@ int Solver::arena_remove(const std::vector<int32_t> &vb, const std::vector<int32
     int rc = set_device();
     if (rc) return rc;
     for (size_t k = 0; k < K; k++) {
-        launch_arena_clear(stream_, vb[k], count[k], solved_, game_of_, st_, succ_, dirty_);
+        launch_arena_clear(stream_, vb[k], count[k], solved_, game_of_, st_);
         PSI_CUDA_TRY(cudaMemsetAsync(gstate_ + slot[k], 0, sizeof(int4), stream_));
     }
     // the retired vertices left in the unreached list are solved: mark_solved passes them by
     if (incremental_ == PSI_INCR_OFF) PSI_CUDA_TRY(cudaMemsetAsync(&dw_->ucount, 0, sizeof(int32_t), stream_));
-    if (extent != n_) launch_move_extent(stream_, n_, extent, succ_);
-    set_extent(extent);
+    n_ = extent;
     return sync_and_check("arena_remove");
 }
 
@@ -1058,15 +1020,15 @@ int Solver::arena_rebuild_lists()
 {
     int rc = set_device();
     if (rc) return rc;
-    PSI_CUDA_TRY(cudaMemsetAsync(&dw_->sinkcount, 0, sizeof(int32_t), stream_));
-    launch_build_plist(stream_, n_, 0, owner_, game_of_, plist_, &dw_->sinkcount);
+    PSI_CUDA_TRY(cudaMemsetAsync(&dw_->selcount, 0, sizeof(int32_t), stream_));
+    launch_build_plist(stream_, n_, 0, owner_, game_of_, plist_, &dw_->selcount);
     rc = sync_and_check("arena_rebuild_lists");
     if (rc) return rc;
-    np0_ = hw_->sinkcount;
-    launch_build_plist(stream_, n_, 1, owner_, game_of_, plist_, &dw_->sinkcount);   // appends after Even's
+    np0_ = hw_->selcount;
+    launch_build_plist(stream_, n_, 1, owner_, game_of_, plist_, &dw_->selcount);   // appends after Even's
     rc = sync_and_check("arena_rebuild_lists");
     if (rc) return rc;
-    np_ = hw_->sinkcount;
+    np_ = hw_->selcount;
     return PSI_OK;
 }
 
@@ -1098,7 +1060,7 @@ int Solver::arena_step(bool reset, std::vector<int32_t> &done, std::vector<int32
     if (rc) return rc;
     if (reset)
         launch_serve_reset_odd(stream_, np_ - np0_, plist_ + np0_, game_of_, gmask_, gcount_, off_, tgt_, strat_,
-                               dirty_, need_, changes());
+                               need_, changes());
     launch_serve_account(stream_, games_, 2, gstate_, gcount_, gmask_);
     std::vector<int4> st((size_t)games_);
     PSI_CUDA_TRY(cudaMemcpyAsync(st.data(), gstate_, sizeof(int4) * (size_t)games_, cudaMemcpyDeviceToHost, stream_));

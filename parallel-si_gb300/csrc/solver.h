@@ -29,8 +29,6 @@ struct SolverTimes {
     int64_t unreached = 0, jump_rounds = 0;
     // incremental evaluations (patch_kernels.cu) and the vertices they re-evaluated
     int64_t patches = 0, patched = 0;
-    // tour build and upkeep: parents linked, in-neighbour entries scanned, children linked
-    int64_t tour_parents = 0, tour_entries = 0, tour_children = 0;
 };
 
 // Status word -> +1 / -1 / 0 as CPUParity's infinite[] (device_common.cuh:
@@ -108,7 +106,6 @@ public:
     int32_t n() const { return n_; }
     int64_t m() const { return m_; }
     int32_t max_pri() const { return max_pri_; }
-    int32_t sublists() const { return nsub_; }
     cudaStream_t stream() const { return stream_; }
     const SolverTimes &times() const { return times_; }
     void reset_times();
@@ -150,7 +147,6 @@ private:
     int upload_union(const std::vector<const HostGame *> &gs, const std::vector<int32_t> &table, int64_t n);
     int finish_upload();
     int init_arena(int32_t slots);
-    void set_extent(int32_t n);
     int sync_and_check(const char *what);
     // One SI step captured into the loop body of the solve graph.
     int enqueue_step(cudaGraph_t body, cudaGraphConditionalHandle loop, bool reset);
@@ -161,6 +157,7 @@ private:
     int enqueue_patch(bool timed);
     int enqueue_full(bool timed);
     PatchArgs patch_args();
+    EvalArgs eval_args();
     ChangeList changes() const { return clist_ ? ChangeList{clist_, &ctl_->ccount, ccap_} : ChangeList(); }
     int build_graph(bool reset);
     int get_range(const int32_t *src, int64_t v0, int64_t count, int32_t *out);
@@ -180,11 +177,11 @@ private:
     int collect_phases();
     SolverTimes times_;
 
-    int32_t n_ = 0, max_pri_ = 0, nsub_ = 0, stride_ = 64;
-    int64_t m_ = 0, L_ = 0, cap_n_ = 0, cap_m_ = 0;
+    int32_t n_ = 0, max_pri_ = 0;
+    int64_t m_ = 0, cap_n_ = 0, cap_m_ = 0;
     int32_t np_ = 0;   // entries in plist_ (Even's np0_ first)
     bool strat_ready_ = false, val_ready_ = false;
-    bool tour_valid_ = false;   // succ holds the last evaluation's tour (dirty_ lists what changed since)
+    bool tracked_ = false;      // every strategy change since the last evaluation went through a switch step
     int last_unreached_ = 0;
 
     // game (device); plist_ lists Even's vertices then Odd's (np0_ of them are Even's)
@@ -205,22 +202,20 @@ private:
     int4 *skip_ = nullptr;       // landmark skips of the comparison walks (device_common.cuh)
     int32_t *key_ = nullptr;   // comparison key per vertex (device_common.cuh)
     // evaluation scratch
-    int32_t *succ_ = nullptr, *ulist_ = nullptr;
-    uint8_t *dirty_ = nullptr;   // parents whose child lists changed since the last evaluation
+    int32_t *ulist_ = nullptr;
+    int32_t *rdeep_ = nullptr;   // counts of paths too long for the path record's word
+    int32_t *la_ = nullptr, *lb_ = nullptr;   // walks cut short (EvalArgs)
     uint8_t *need_ = nullptr;    // vertices their owner's next switch step must examine (ChangeTrack)
     uint8_t *tie_ = nullptr;     // vertices whose last examination rested on a walk (ChangeTrack)
     uint8_t *watch_ = nullptr;   // vertices such an examination rested on (ChangeTrack)
     ChangeTrack track() const { return ChangeTrack{need_, rev_off_, rev_src_, &ctl_->quiet, tie_, watch_}; }
     void reset_tracking();       // every vertex to be examined (need = 1, quiet until the next evaluation)
     int32_t *rev_off_ = nullptr, *rev_src_ = nullptr;   // distinct in-neighbours (static)
-    int2 *vloc_ = nullptr, *redA_ = nullptr, *redB_ = nullptr;
-    int4 *jA_ = nullptr, *jB_ = nullptr;   // the cycle pass's jump entries
-    int2 *redC_ = nullptr;
+    int4 *jA_ = nullptr, *jB_ = nullptr;   // jump entries of the walks cut short
     // incremental evaluation (patch_kernels.cu): the switch steps' change
     // list, the re-evaluated set and its positions, the jump entries
     int32_t incremental_ = 1;   // psi_options.incremental
     int32_t patch_limit_ = 0;   // psi_options.patch_limit
-    int32_t walk_block_ = kWalkBlock;   // psi_options.walk_block (0 there: kWalkBlock)
     bool switch_warp_ = false;          // psi_options.switch_kernel == PSI_SWITCH_WARP
     int32_t *clist_ = nullptr, *alist_ = nullptr, *apos_ = nullptr;
     int4 *pj_ = nullptr;
@@ -230,11 +225,11 @@ private:
     struct Words {
         unsigned long long sw[4];   // switch counters (launch_switch)
         unsigned long long patch[2];   // patches, vertices they re-evaluated (since reset_times)
-        unsigned long long relink[3];  // tour kernels: parents, in-list entries, children linked (since reset_times)
         uint32_t err;
         int32_t ucount;             // vertices the sink did not reach
-        int32_t sinkcount;          // children of the sink (tour build)
-        int32_t cnt[3];             // active-list counters of the cycle kernel
+        int32_t selcount;           // size of a selected list (players, winning set)
+        int32_t lcount;             // walks cut short in the last full evaluation
+        int32_t cnt[3];             // list counters (EvalArgs, launch_switch)
         uint32_t claim;             // the switch kernel's work counter (launch_switch)
     };
     Words *dw_ = nullptr, *hw_ = nullptr;

@@ -22,12 +22,9 @@ namespace psi {
 
 namespace {
 
-// after an evaluation: the tour is valid for updates (and the next
-// evaluation may be a patch), one more evaluation
+// after an evaluation: the next one may be a patch; one more evaluation
 __global__ void k_ctl_evaluated(GraphCtl *c, uint32_t *err)
 {
-    c->full = 0;
-    c->incr = 1;
     c->try_patch = c->patch_on;
     c->reset = 0;
     c->quiet = 0;
@@ -57,9 +54,7 @@ __global__ void k_ctl_even(GraphCtl *c, const unsigned long long *sw, const uint
             go = false;
         } else if (reset_variant) {   // main.cpp:25-26: Odd starts the next iteration afresh
             c->reset = 1;
-            c->full = 1;              // many Odd strategies change: rebuild the tour
-            c->incr = 0;
-            c->try_patch = 0;         // and no switch step lists those changes
+            c->try_patch = 0;         // no switch step lists those changes
         }
     }
     if (go && c->max_evals > 0 && c->brs >= c->max_evals) {
@@ -144,26 +139,26 @@ int Solver::enqueue_step(cudaGraph_t body, cudaGraphConditionalHandle loop, bool
     k_ctl_evaluated<<<1, 1, 0, stream_>>>(ctl_, &dw_->err);
     if (batch) launch_batch_account(stream_, games_, 0, gstate_, gcount_);
     // Odd: mark_solved(1), switch(1)
-    launch_mark_solved(stream_, &dw_->ucount, ulist_, 1, st_, solved_, dirty_, nullptr, nullptr, nullptr,
+    launch_mark_solved(stream_, &dw_->ucount, ulist_, 1, st_, solved_, nullptr, nullptr, nullptr,
                        &ctl_->mfrom[1], &ctl_->mdone);
     e = cudaMemsetAsync(dw_->sw, 0, sizeof(dw_->sw), stream_);
     if (e != cudaSuccess) return abort_capture(fail(PSI_ERR_CUDA, std::string("memset: ") + cudaGetErrorString(e)));
     int32_t *todo = reinterpret_cast<int32_t *>(jB_);   // free until the next cycle pass
     unsigned long long *gc = batch ? gcount_ : nullptr;
-    launch_switch(stream_, np_ - np0_, plist_ + np0_, 1, off_, tgt_, strat_, st_, key_, node_, dw_->sw,
-                  batch ? game_of_ : nullptr, gc, nullptr, dirty_, &dw_->err, nullptr, need_, todo, &dw_->cnt[2],
+    launch_switch(stream_, np_ - np0_, plist_ + np0_, 1, off_, tgt_, strat_, st_, key_, node_, rdeep_, dw_->sw,
+                  batch ? game_of_ : nullptr, gc, nullptr, &dw_->err, nullptr, need_, todo, &dw_->cnt[2],
                   changes(), tie_, watch_, skip_, switch_warp_, &dw_->claim, arena_ ? nullptr : owner_, n_);
     if (batch) launch_batch_account(stream_, games_, 1, gstate_, gcount_);
     count_launch();
     k_ctl_odd<<<1, 1, 0, stream_>>>(ctl_, dw_->sw);
     // Even, when Odd made no strict improvement: mark_solved(0), switch(0)
-    launch_mark_solved(stream_, &dw_->ucount, ulist_, 0, st_, solved_, dirty_, nullptr, nullptr, &ctl_->even,
+    launch_mark_solved(stream_, &dw_->ucount, ulist_, 0, st_, solved_, nullptr, nullptr, &ctl_->even,
                        &ctl_->mfrom[0], &ctl_->mdone);
     if (batch) launch_batch_account(stream_, games_, 2, gstate_, gcount_, &ctl_->even);
     e = cudaMemsetAsync(dw_->sw, 0, sizeof(dw_->sw), stream_);
     if (e != cudaSuccess) return abort_capture(fail(PSI_ERR_CUDA, std::string("memset: ") + cudaGetErrorString(e)));
-    launch_switch(stream_, np0_, plist_, 0, off_, tgt_, strat_, st_, key_, node_, dw_->sw,
-                  batch ? game_of_ : nullptr, gc, nullptr, dirty_, &dw_->err, &ctl_->even, need_, todo,
+    launch_switch(stream_, np0_, plist_, 0, off_, tgt_, strat_, st_, key_, node_, rdeep_, dw_->sw,
+                  batch ? game_of_ : nullptr, gc, nullptr, &dw_->err, &ctl_->even, need_, todo,
                   &dw_->cnt[2], changes(), tie_, watch_, skip_, switch_warp_, &dw_->claim,
                   arena_ ? nullptr : owner_, n_);
     if (batch) launch_batch_account(stream_, games_, 3, gstate_, gcount_, &ctl_->even);
@@ -218,8 +213,7 @@ int Solver::run_graph(bool reset, int64_t max_evals, GraphCtl *out, int4 *gstate
         if (rc) return rc;
     }
     GraphCtl init;
-    init.full = 1;   // init_strat: the first evaluation builds the tour
-    init.quiet = 1;  // and every need flag is set
+    init.quiet = 1;   // init_strat: every need flag is set
     init.patch_on = incremental_ != PSI_INCR_OFF ? 1 : 0;
     init.max_evals = max_evals > 0 && max_evals < INT32_MAX ? (int32_t)max_evals : 0;
     init.inject_at = inject_at_;
@@ -242,11 +236,11 @@ int Solver::run_graph(bool reset, int64_t max_evals, GraphCtl *out, int4 *gstate
     times_.switches += out->brs + out->iters;
     if (rc) {   // the device error word was set: the state is not trusted
         val_ready_ = false;
-        tour_valid_ = false;
+        tracked_ = false;
         return rc;
     }
     val_ready_ = true;
-    tour_valid_ = true;
+    tracked_ = true;
     if (out->stop == GraphCtl::kEvalCap) return fail(PSI_ERR_LIMIT, "evaluation cap reached");
     if (out->stop == GraphCtl::kDeviceError) return fail(PSI_ERR_LIMIT, "graph solve loop stopped by a device error");
     if (out->stop != GraphCtl::kConverged) return fail(PSI_ERR_LIMIT, "graph solve loop stopped by its guard");

@@ -142,14 +142,24 @@ __device__ int walk_compare(const PathNode *__restrict__ node, const int4 *__res
 // equal: the exact summaries decide, else a walk to the lowest common
 // ancestor (w = -1 is the sink).
 __device__ int compare_equal_keys(const PathNode *__restrict__ node, const int4 *__restrict__ skip,
-                                  const int32_t *__restrict__ st, int32_t u, int32_t w, int32_t &loads,
+                                  const int32_t *__restrict__ st, const int32_t *__restrict__ rdeep, int32_t u, int32_t w, int32_t &loads,
                                   uint32_t *__restrict__ err)
 {
     const int2 ru = *reinterpret_cast<const int2 *>(&node[u].rmax);
     const int2 rw = (w >= 0) ? *reinterpret_cast<const int2 *>(&node[w].rmax) : make_int2(-1, 0);
-    if (ru.x != rw.x) return ru.x > rw.x ? decide(ru.x, ru.y, 0) : decide(rw.x, 0, rw.y);
-    if (ru.y != rw.y) return decide(ru.x, ru.y, rw.y);
-    return walk_compare(node, skip, u, st[u], w, w >= 0 ? st[w] : 0, loads, err);
+    int32_t du = path_word_depth(ru.y), cu = path_word_count(ru.y);
+    int32_t dw = path_word_depth(rw.y), cw = path_word_count(rw.y);   // the sink: depth 0, count 0
+    if (du == kDeepPath) {
+        du = st[u];
+        cu = rdeep[u];
+    }
+    if (dw == kDeepPath) {
+        dw = st[w];
+        cw = rdeep[w];
+    }
+    if (ru.x != rw.x) return ru.x > rw.x ? decide(ru.x, cu, 0) : decide(rw.x, 0, cw);
+    if (cu != cw) return decide(ru.x, cu, cw);
+    return walk_compare(node, skip, u, du, w, dw, loads, err);
 }
 
 // One thread per vertex of plist (all owned by `player`).  Per compared edge
@@ -246,11 +256,12 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
                                                    int32_t *__restrict__ strat, const int32_t *__restrict__ st,
                                                    const int32_t *__restrict__ key,
                                                    const PathNode *__restrict__ node,
+                                                   const int32_t *__restrict__ rdeep,
                                                    unsigned long long *__restrict__ stats,
                                                    const int32_t *__restrict__ game_of,
                                                    unsigned long long *__restrict__ gcount,
                                                    const int32_t *__restrict__ gmask,
-                                                   uint8_t *__restrict__ dirty, uint32_t *__restrict__ err,
+                                                   uint32_t *__restrict__ err,
                                                    const int32_t *__restrict__ gate, uint8_t *__restrict__ need,
                                                    ChangeList changes, uint8_t *__restrict__ tie_out,
                                                    uint8_t *__restrict__ watch, const int4 *__restrict__ skip,
@@ -357,7 +368,7 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
                     int c;
                     if (ku != kc) c = ku > kc ? 1 : -1;
                     else if (u == cur || key_infinite(ku)) c = 0;
-                    else c = compare_equal_keys(node, skip, st, u, cur, t_loads, err);
+                    else c = compare_equal_keys(node, skip, st, rdeep, u, cur, t_loads, err);
                     if ((player == 0 && c > 0) || (player == 1 && c < 0)) {
                         cur = u;
                         kc = ku;
@@ -379,8 +390,6 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
             }
             if (moves) {   // strict improvements never return to cur0: cur != cur0
                 strat[v] = cur;
-                if (cur0 >= 0) dirty[cur0] = 1;
-                if (cur >= 0) dirty[cur] = 1;
                 if (game_of) atomicAdd(&gcount[game_of[v]], (unsigned long long)moves);
                 t_changed++;
                 t_moves += moves;
@@ -439,11 +448,12 @@ __global__ void __launch_bounds__(kBlock) k_switch_warp(int32_t np, const int32_
                                                         const int32_t *__restrict__ st,
                                                         const int32_t *__restrict__ key,
                                                         const PathNode *__restrict__ node,
+                                                        const int32_t *__restrict__ rdeep,
                                                         unsigned long long *__restrict__ stats,
                                                         const int32_t *__restrict__ game_of,
                                                         unsigned long long *__restrict__ gcount,
                                                         const int32_t *__restrict__ gmask,
-                                                        uint8_t *__restrict__ dirty, uint32_t *__restrict__ err,
+                                                        uint32_t *__restrict__ err,
                                                         const int32_t *__restrict__ gate, uint8_t *__restrict__ need,
                                                         ChangeList changes, uint8_t *__restrict__ tie_out,
                                                         uint8_t *__restrict__ watch, const int4 *__restrict__ skip)
@@ -586,7 +596,7 @@ __global__ void __launch_bounds__(kBlock) k_switch_warp(int32_t np, const int32_
                 int cmp;
                 if (ku != kc) cmp = ku > kc ? 1 : -1;
                 else if (uu == cur || key_infinite(ku)) cmp = 0;
-                else cmp = compare_equal_keys(node, skip, st, uu, cur, t_loads, err);
+                else cmp = compare_equal_keys(node, skip, st, rdeep, uu, cur, t_loads, err);
                 if ((player == 0 && cmp > 0) || (player == 1 && cmp < 0)) {
                     cur = uu;
                     kc = ku;
@@ -610,8 +620,6 @@ __global__ void __launch_bounds__(kBlock) k_switch_warp(int32_t np, const int32_
             }
             if (moves) {   // strict improvements never return to cur0: cur != cur0
                 strat[v] = cur;
-                if (cur0 >= 0) dirty[cur0] = 1;
-                if (cur >= 0) dirty[cur] = 1;
                 if (game_of) atomicAdd(&gcount[game_of[v]], (unsigned long long)moves);
                 t_changed++;
                 t_moves += moves;
@@ -715,8 +723,8 @@ int switch_grid()
 
 void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t player, const int32_t *off,
                    const int32_t *tgt, int32_t *strat, const int32_t *st, const int32_t *key, const PathNode *node,
-                   unsigned long long *stats, const int32_t *game_of, unsigned long long *gcount,
-                   const int32_t *gmask, uint8_t *dirty, uint32_t *err, const int32_t *gate, uint8_t *need,
+                   const int32_t *rdeep, unsigned long long *stats, const int32_t *game_of, unsigned long long *gcount,
+                   const int32_t *gmask, uint32_t *err, const int32_t *gate, uint8_t *need,
                    int32_t *list, int32_t *list_count, ChangeList changes, uint8_t *tie, uint8_t *watch,
                    const int4 *skip, bool warp, uint32_t *claim, const int8_t *owner, int32_t n_all)
 {
@@ -747,11 +755,11 @@ void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t pla
     }
     count_launch();
     if (warp)
-        k_switch_warp<<<g, kBlock, 0, s>>>(np, items, count, player, off, tgt, strat, st, key, node, stats, game_of,
-                                           gcount, gmask, dirty, err, gate, need, changes, tie, watch, skip);
+        k_switch_warp<<<g, kBlock, 0, s>>>(np, items, count, player, off, tgt, strat, st, key, node, rdeep, stats,
+                                           game_of, gcount, gmask, err, gate, need, changes, tie, watch, skip);
     else
-        k_switch<<<g, kBlock, 0, s>>>(np, items, count, player, off, tgt, strat, st, key, node, stats, game_of,
-                                      gcount, gmask, dirty, err, gate, need, changes, tie, watch, skip,
+        k_switch<<<g, kBlock, 0, s>>>(np, items, count, player, off, tgt, strat, st, key, node, rdeep, stats, game_of,
+                                      gcount, gmask, err, gate, need, changes, tie, watch, skip,
                                       count ? claim : nullptr);
 }
 
