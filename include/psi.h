@@ -90,9 +90,11 @@ typedef struct {
                                 the reference's gpu_list_ranking.cu:19); at least 2, without effect:
                                 evaluations walk the strategy graph and rank no list */
     int32_t timing;          /* 1: record per-phase CUDA-event times (default 1) */
-    int32_t graph;           /* 1 (default): psi_solve runs the whole solve_si loop as one CUDA
-                                graph (device-side loop control, no host synchronisation per
-                                step; same results; records no per-phase times); 0: the
+    int32_t graph;           /* 1 (default): psi_solve runs the whole solve_si loop on the device
+                                (no host synchronisation per step; same results; records no
+                                per-phase times): one persistent kernel, which evaluates in full
+                                every time, for single games below 2^20 vertices with neither
+                                PSI_INCR_ALWAYS nor PSI_SWITCH_WARP, else one CUDA graph; 0: the
                                 host-driven loop */
     int32_t incremental;     /* PSI_INCR_*: whether an evaluation after a switch step that
                                 changed few strategies re-evaluates only the vertices whose

@@ -1,0 +1,207 @@
+// compare.cuh -- the exact comparison of two finite valuations by walking
+// their paths to the lowest common ancestor (the third tier described in
+// switch_kernels.cu), for every kernel that switches strategies.
+#ifndef PSI_COMPARE_CUH
+#define PSI_COMPARE_CUH
+
+#include <climits>
+
+#include "device_common.cuh"
+
+namespace psi {
+
+// Even's view of a difference at priority p: +1 if side a is better.
+__device__ __forceinline__ int decide(int32_t p, int32_t ca, int32_t cb)
+{
+    if ((p & 1) == 0) return ca > cb ? 1 : -1;
+    return ca < cb ? 1 : -1;
+}
+
+// Tier 3: walks to the lowest common ancestor of u and w (depths du, dw; w may
+// be the sink, -1 with depth 0), collecting the top two priorities of each
+// side's segment below it; passes after the first repeat the walk counting
+// only priorities below the last tie.  With skip, the first pass jumps whole
+// landmark segments (device_common.cuh): the deeper side jumps while its
+// landmark is no shallower than the other side; at equal depths both jump
+// while their landmarks differ (the common ancestor is then above both);
+// once they share one, the common ancestor lies in that segment and both
+// step one vertex at a time.
+static __device__ int walk_compare(const PathNode *__restrict__ node, const int4 *__restrict__ skip, int32_t u, int32_t du,
+                            int32_t w, int32_t dw, int32_t &loads, uint32_t *__restrict__ err)
+{
+    int32_t thr = INT_MAX;
+    const int32_t max_pass = (du + dw) / 2 + 2;
+    for (int32_t pass = 0; pass < max_pass; pass++) {
+        Top2 A = {-1, 0, -1, 0}, B = {-1, 0, -1, 0};
+        int32_t a = u, b = w, da = du, db = dw;
+        bool jumps = skip != nullptr && pass == 0;
+        while (a != b || da != db) {
+            bool adv_a = da >= db, adv_b = db >= da;
+            if ((adv_a && (a < 0 || da <= 0)) || (adv_b && (b < 0 || db <= 0))) {   // inconsistent: cannot happen
+                atomicOr(err, DERR_WALK_CAP);
+                return 0;
+            }
+            if (jumps) {
+                if (adv_a && adv_b) {
+                    const int4 sa = skip[a], sb = skip[b];
+                    loads += 2;
+                    if (sa.x != SKIP_UNKNOWN && sb.x != SKIP_UNKNOWN) {
+                        if (sa.x != sb.x) {
+                            skip_merge(A, sa);
+                            skip_merge(B, sb);
+                            a = sa.x;
+                            b = sb.x;
+                            da = db = skip_landmark_depth(da);
+                            continue;
+                        }
+                        jumps = false;   // one landmark: the common ancestor is within this segment
+                    }
+                } else {
+                    const int32_t x = adv_a ? a : b, dx = adv_a ? da : db, other = adv_a ? db : da;
+                    const int32_t L = skip_landmark_depth(dx);
+                    if (L >= other) {
+                        const int4 sx = skip[x];
+                        loads++;
+                        if (sx.x != SKIP_UNKNOWN) {
+                            if (adv_a) {
+                                skip_merge(A, sx);
+                                a = sx.x;
+                                da = L;
+                            } else {
+                                skip_merge(B, sx);
+                                b = sx.x;
+                                db = L;
+                            }
+                            continue;
+                        }
+                    }
+                }
+            }
+            if (adv_a) {
+                int2 q = *reinterpret_cast<const int2 *>(&node[a]);
+                loads++;
+                if (q.y < thr) top2_add(A, q.y);
+                a = q.x;
+                da--;
+            }
+            if (adv_b) {
+                int2 q = *reinterpret_cast<const int2 *>(&node[b]);
+                loads++;
+                if (q.y < thr) top2_add(B, q.y);
+                b = q.x;
+                db--;
+            }
+        }
+        int32_t M1 = max(A.m1, B.m1);
+        if (M1 < 0) return 0;
+        int32_t ca = (A.m1 == M1) ? A.c1 : 0, cb = (B.m1 == M1) ? B.c1 : 0;
+        if (ca != cb) return decide(M1, ca, cb);
+        int32_t M2 = max(A.m2, B.m2);
+        if (M2 < 0) return 0;
+        ca = (A.m2 == M2) ? A.c2 : 0;
+        cb = (B.m2 == M2) ? B.c2 : 0;
+        if (ca != cb) return decide(M2, ca, cb);
+        thr = M2;
+    }
+    atomicOr(err, DERR_PASS_CAP);
+    return 0;
+}
+
+// The same comparison with one priority per pass, for kernels where a whole
+// phase waits for its longest walk: few instructions per step and no branches
+// on priorities (the two-priority update above diverges, about 0.12 us per
+// step on top of the loads).  Pass k finds the highest priority below the last
+// tie and its count on either side; with skip, whole landmark segments are
+// jumped where their record's two priorities tell the one sought.  path: per
+// vertex (parent, priority).  Once loads passes budget: kUndecided.
+constexpr int kUndecided = 2;
+__device__ __forceinline__ void top_add(int32_t &m, int32_t &c, int32_t p, int32_t k, int32_t below)
+{
+    p = p < below ? p : -1;
+    c = p > m ? k : (p == m ? c + k : c);
+    m = max(m, p);
+}
+__device__ __forceinline__ bool top_jump(int32_t &m, int32_t &c, const int4 s, int32_t below)
+{
+    if (s.x == SKIP_UNKNOWN || (s.y >= below && s.z >= below)) return false;
+    const bool first = s.y < below;
+    top_add(m, c, first ? s.y : s.z, first ? s.w & 0xffff : (int32_t)((uint32_t)s.w >> 16), below);
+    return true;
+}
+static __device__ __noinline__ int lean_compare(const int2 *path, const int4 *skip, int32_t u, int32_t du, int32_t w,
+                                                int32_t dw, int32_t &loads, int32_t budget, uint32_t *err)
+{
+    int32_t below = INT_MAX;
+    for (int32_t pass = 0; pass <= du + dw; pass++) {
+        int32_t a = u, b = w, da = du, db = dw, ma = -1, ca = 0, mb = -1, cb = 0;
+        bool swapped = false;
+        if (da < db) {   // a is the deeper side
+            a = w;
+            b = u;
+            da = dw;
+            db = du;
+            swapped = true;
+        }
+        while (da > db) {
+            if (a < 0 || ++loads > budget) break;
+            const int32_t l = skip_landmark_depth(da);
+            if (skip && l >= db) {
+                const int4 s = skip[a];
+                if (top_jump(ma, ca, s, below)) {
+                    a = s.x;
+                    da = l;
+                    continue;
+                }
+            }
+            const int2 q = path[a];
+            top_add(ma, ca, q.y, 1, below);
+            a = q.x;
+            da--;
+        }
+        bool jumps = skip != nullptr;
+        while (a != b) {
+            if (a < 0 || b < 0) break;
+            loads += 2;
+            if (loads > budget) break;
+            if (jumps) {
+                const int4 s = skip[a], t = skip[b];
+                int32_t m2 = ma, c2 = ca, m3 = mb, c3 = cb;
+                if (s.x != t.x && top_jump(m2, c2, s, below) && top_jump(m3, c3, t, below)) {
+                    ma = m2;
+                    ca = c2;
+                    mb = m3;
+                    cb = c3;
+                    a = s.x;
+                    b = t.x;
+                    da = skip_landmark_depth(da);
+                    continue;
+                }
+                // one landmark: the paths meet in this segment
+                jumps = s.x != t.x;
+            }
+            const int2 q = path[a], r = path[b];
+            top_add(ma, ca, q.y, 1, below);
+            top_add(mb, cb, r.y, 1, below);
+            a = q.x;
+            b = r.x;
+            da--;
+        }
+        if (loads > budget) return kUndecided;
+        if (a != b) {   // inconsistent: cannot happen
+            atomicOr(err, DERR_WALK_CAP);
+            return 0;
+        }
+        const int32_t m = max(ma, mb);
+        if (m < 0) return 0;
+        ca = ma == m ? ca : 0;
+        cb = mb == m ? cb : 0;
+        if (ca != cb) return swapped ? decide(m, cb, ca) : decide(m, ca, cb);
+        below = m;
+    }
+    atomicOr(err, DERR_PASS_CAP);
+    return 0;
+}
+
+}  // namespace psi
+
+#endif

@@ -10,6 +10,7 @@
 namespace psi {
 
 struct PathNode;   // device_common.cuh
+struct GraphCtl;   // solver.h
 
 // Change tracking between evaluations and switch steps: when an evaluation
 // changes a vertex's comparison key, its in-neighbours (rev_off/rev_src) get
@@ -144,6 +145,37 @@ void launch_root_init(cudaStream_t s, const EvalArgs &a);
 void launch_root_walk(cudaStream_t s, const EvalArgs &a);
 // Cooperative launch; returns a cudaError_t value.
 int launch_root_settle(cudaStream_t s, const EvalArgs &a);
+
+// A whole solve_si of one game in one persistent launch (solve_kernels.cu).
+struct SolveSync {
+    int32_t vote[3] = {0, 0, 0}, vote2[3] = {0, 0, 0};
+    uint32_t phase = 0;
+    uint32_t errs[3] = {0, 0, 0};
+    uint32_t err = 0;
+};
+struct SolveArgs {
+    int32_t n = 0, n_even = 0;    // plist: Even's n_even vertices, then Odd's
+    const int8_t *owner = nullptr;
+    const int32_t *pri = nullptr, *off = nullptr, *tgt = nullptr, *plist = nullptr;
+    int32_t *strat = nullptr, *st = nullptr, *key = nullptr, *rdeep = nullptr;
+    uint8_t *solved = nullptr;
+    PathNode *node = nullptr;
+    int4 *skip = nullptr;
+    int4 *jump[2] = {nullptr, nullptr};       // n entries each
+    int2 *path[2] = {nullptr, nullptr};       // (strategy, priority), n entries each
+    int32_t *ulist = nullptr, *ucount = nullptr;
+    SolveSync *sync = nullptr;    // zero before the first solve
+    GraphCtl *ctl = nullptr;      // receives iters, brs, stop
+    uint32_t *err = nullptr;
+    int32_t reset = 0, max_evals = 0, guard = 0;
+    int32_t inject_at = 0;
+    uint32_t inject_bits = 0;
+};
+// The largest game it takes on the current device (over a million vertices
+// from 32 SMs on).
+int64_t solve_capacity();
+// Returns a cudaError_t value.
+int launch_solve(cudaStream_t s, const SolveArgs &a);
 
 // ---- list ranking of an Euler tour (gpu_list_ranking.cu:52-277), the
 // evaluation without allocation (noalloc.cu)

@@ -1,0 +1,501 @@
+// solve_kernels.cu -- solve_si (main.cpp:20-55) of one game in one persistent
+// kernel on sm_103a, for games whose state stays in L2.
+//
+// What bounds such a solve is latency: a step of the loop touches a few MB,
+// but as a sequence of launches (about 18 per step, each with its own ramp)
+// it took 80 us whatever the size.  Here the whole loop is one cooperative
+// launch; a step is two phases with a grid barrier after each, three when
+// Even moves, and every evaluation is a full one.
+//
+//  - Jump phase.  Every vertex v has a record jump[v] = (target, top priority
+//    of the window from v up to the target, how many of the window's vertices
+//    carry it, the window's length), one 16-byte word that is read and
+//    written whole.  It starts as (successor, own priority, 1, 1).  v's
+//    thread reads its target's record, appends that window to its own and
+//    stores the result, until the target is the sink (the record is then v's
+//    summary) or a vertex known to be infinite.  All threads do so at once
+//    without barriers: whichever state of the target's record a reader
+//    finds, it is a window of the same path.  So a vertex at depth d is done
+//    after about log2 d reads, where a walk would take d (all vertices start
+//    together here: no ancestor is finished yet).  A window of n vertices or
+//    a return to a vertex seen before (Brent's marker) means that the target
+//    lies on a cycle; its top priority is collected along the records from
+//    there on, until they return to it or cover n vertices.
+//    A vertex makes at most kJumps reads per pass; should one be left, the
+//    pass is repeated (its windows are kept, so a few passes reach any depth).
+//  - Switch phase of one player.  mark_solved and the all-switches step touch
+//    different words, so they share a phase, and each vertex's thread also
+//    writes the next evaluation's initial records, into the other of two
+//    buffers (comparisons still read the current ones).
+//  - Comparisons that walk far (equal summaries, paths that meet late) would
+//    hold up a whole phase, 30 to 500 us where the others take 5.  A vertex
+//    whose walks pass their budget of steps is left over; only if there are any, all
+//    threads write landmark records (device_common.cuh) and those vertices
+//    are done again with them.
+//
+// A thread owns the same vertices in every phase (plist[tid], plist[tid +
+// threads], ...), so what a vertex's phases start from -- its id, CSR range,
+// priority, choice and first successors -- stays in shared memory, 40 bytes
+// per vertex; the first dependent load of a phase is then a key or a record.
+//
+// Every vertex of the player is examined in every switch phase: with all keys
+// in L2 that costs less than tracking which have changed.  What would cost is
+// to repeat the walks of ties that nothing has touched, so a record also says
+// whether a strategy on the vertex's path has changed since the last
+// evaluation (Odd's last examination) and since Even's last one.
+#include <climits>
+#include <cooperative_groups.h>
+
+#include "compare.cuh"
+#include "device_common.cuh"
+#include "kernels.h"
+#include "solver.h"
+
+namespace cg = cooperative_groups;
+
+namespace psi {
+
+namespace {
+
+// targets of finished records
+constexpr int32_t kSink = -1, kNegInf = -2, kPosInf = -3;
+// reads per vertex and pass
+constexpr int kJumps = 64;
+constexpr int kMaxPasses = 64;
+// a record's last word: the window's length (up to kMaxLen: n or more only say
+// "a cycle"; n < 2^20), whether a strategy in it has changed since the last
+// evaluation, and, once finished, since Even's last examination
+constexpr int32_t kMaxLen = 1 << 24, kLen = (1 << 25) - 1;
+constexpr int32_t kNew = 1 << 30, kNewEven = 1 << 29;
+
+__device__ __forceinline__ int4 load_jump(const int4 *p)
+{
+    int4 r;
+    asm volatile("{\n\t.reg .b128 t;\n\t.reg .b64 lo, hi;\n\t"
+                 "ld.relaxed.gpu.global.b128 t, [%4];\n\t"
+                 "mov.b128 {lo, hi}, t;\n\t"
+                 "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}"
+                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+                 : "l"(p)
+                 : "memory");
+    return r;
+}
+__device__ __forceinline__ void store_jump(int4 *p, const int4 r)
+{
+    asm volatile("{\n\t.reg .b128 t;\n\t.reg .b64 lo, hi;\n\t"
+                 "mov.b64 lo, {%1, %2};\n\tmov.b64 hi, {%3, %4};\n\t"
+                 "mov.b128 t, {lo, hi};\n\t"
+                 "st.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w)
+                 : "memory");
+}
+
+// One pass of v's record r; true when it is finished.
+__device__ __forceinline__ bool jump_pass(int4 *jump, int32_t n, int32_t v, int4 &r)
+{
+    if (r.x < 0) return true;
+    int32_t mark = v;
+    for (int i = 1; i <= kJumps; i++) {
+        bool cycle = (r.w & kLen) >= n;
+        if (!cycle) {
+            const int4 q = load_jump(&jump[r.x]);
+            if (q.x <= kNegInf) {
+                r = make_int4(q.x, 0, 0, 0);
+                store_jump(&jump[v], r);
+                return true;
+            }
+            top1_merge(r.y, r.z, q.y, q.z);
+            r.z = min(r.z, kMaxLen);
+            r.w = min((r.w & kLen) + (q.w & kLen), kMaxLen) | (r.w & kNewEven) | ((r.w | q.w) & kNew);
+            r.x = q.x;
+            cycle = r.x == mark;
+            if ((i & (i - 1)) == 0) mark = r.x;
+        }
+        if (cycle) {
+            // the target is on the cycle: the top priority of the windows from
+            // it, once around or n vertices
+            const int32_t t0 = r.x;
+            int32_t t = t0, len = 0, top = -1, code = 0;
+            for (int j = 0; j < kJumps; j++) {
+                const int4 q = load_jump(&jump[t]);
+                if (q.x <= kNegInf) {
+                    code = q.x;
+                    break;
+                }
+                top = max(top, q.y);
+                len = min(len + (q.w & kLen), kMaxLen);
+                t = q.x;
+                if (t == t0 || len >= n) {
+                    code = (top & 1) ? kNegInf : kPosInf;
+                    break;
+                }
+            }
+            if (code) {
+                r = make_int4(code, 0, 0, 0);
+                store_jump(&jump[v], r);
+                return true;
+            }
+            r.w = kMaxLen | (r.w & ~kLen);   // a later pass goes on from the cycle
+            store_jump(&jump[v], r);
+            return false;
+        }
+        if (r.x == kSink && (r.w & kNew)) r.w |= kNewEven;
+        store_jump(&jump[v], r);
+        if (r.x == kSink) return true;
+    }
+    return false;
+}
+
+// Steps of comparison walks per vertex before it is left over: a step is a
+// dependent read from L2, the second round costs the landmark records of all
+// vertices and two barriers.  Solve in us with 16, 64, 256 steps: 431, 382,
+// 323 (n = 10^4), 960, 940, 832 (10^5), 2782, 2537, 2640 (2^18 vertices, 8
+// priorities), but 5200, 5690, 6320 (10^6), where each thread has seven
+// vertices whose walks would add up.
+__device__ __forceinline__ int32_t walk_budget(int32_t n, int32_t threads) { return n <= 2 * threads ? 256 : 16; }
+
+// Even's view of finite u against finite w (distinct, equal keys; -1: the sink).
+__device__ __forceinline__ int compare_tied(const int4 *jump, const int2 *path, const int4 *skip, int32_t u, int32_t w,
+                                         int32_t &loads, int32_t budget, uint32_t *err)
+{
+    const int4 ru = jump[u];
+    const int4 rw = (w >= 0) ? jump[w] : make_int4(kSink, -1, 0, 0);   // w's length: 0
+    if (ru.y != rw.y) return ru.y > rw.y ? decide(ru.y, ru.z, 0) : decide(rw.y, 0, rw.z);
+    if (ru.z != rw.z) return decide(ru.y, ru.z, rw.z);
+    return lean_compare(path, skip, u, ru.w & kLen, w, rw.w & kLen, loads, budget, err);
+}
+
+constexpr int kSolveThreads = 1024;
+// low bits of a vertex's choice word: solved; its path touched since Even's
+// last examination
+constexpr int32_t kSolved = 1, kTouched = 2;
+__device__ __forceinline__ int32_t bits(int32_t t, bool fresh)
+{
+    return 1 | (fresh ? kNew | kNewEven : 0) | ((t & kTouched) ? kNewEven : 0);
+}
+constexpr int kFirst = 5;       // successors kept per vertex
+constexpr int kWords = 5 + kFirst;
+constexpr int kMinThreads = 128;
+constexpr int32_t kOneBlock = 1024;   // games up to this size run in one block
+constexpr int kMaxWaves = 32;   // vertices per thread (a bit mask)
+constexpr int kMaxCached = 5;   // vertices per thread kept (200 KB); further ones are read anew
+constexpr int kSharedBytes = 4 * kWords * kSolveThreads * kMaxCached;   // 200 KB
+
+// GRID: over the whole grid; otherwise one block with block barriers.
+template <bool GRID>
+__global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
+{
+    extern __shared__ int32_t own[];   // [wave][word][thread]
+    const int32_t n = a.n;
+    const int32_t tid = GRID ? (int32_t)(blockIdx.x * blockDim.x + threadIdx.x) : (int32_t)threadIdx.x;
+    const int32_t nth = GRID ? (int32_t)(gridDim.x * blockDim.x) : (int32_t)blockDim.x;
+    const int32_t budget = walk_budget(n, nth);
+    // Barrier with two votes: whether any thread passed true.  Phase k uses the
+    // words k % 3, which thread 0 clears in phase k - 1, when everyone has
+    // read their last use (phase k - 3); the count goes on from solve to
+    // solve.  err: the error bits thread 0 saw on its way into the barrier
+    // (the same for all threads, as the loop's control has to be).
+    uint32_t phase = a.sync->phase, err = 0;
+    bool voted = false, voted2 = false;
+    auto barrier = [&](bool mine, bool mine2) {
+        const uint32_t k = phase % 3, k1 = (phase + 1) % 3;
+        phase++;
+        if (tid == 0) {
+            a.sync->vote[k1] = a.sync->vote2[k1] = 0;
+            a.sync->errs[k] = *(volatile uint32_t *)&a.sync->err;
+        }
+        if (__syncthreads_or(mine) && threadIdx.x == 0) a.sync->vote[k] = 1;
+        if (__syncthreads_or(mine2) && threadIdx.x == 0) a.sync->vote2[k] = 1;
+        if (GRID) cg::this_grid().sync();
+        else __syncthreads();
+        err = __ldcg(&a.sync->errs[k]);
+        voted = __ldcg(&a.sync->vote[k]) != 0;
+        voted2 = __ldcg(&a.sync->vote2[k]) != 0;
+    };
+    // the thread's vertex in wave w (vertex i of plist): its words
+    struct Own {
+        int32_t v, e0, deg, pri, t;   // t: (choice + 1) * 4 + kTouched + solved
+    };
+    auto word = [&](int32_t w, int k) -> int32_t & { return own[(w * kWords + k) * (int32_t)blockDim.x + threadIdx.x]; };
+    auto get = [&](int32_t w, int32_t i) -> Own {
+        if (w < kMaxCached) return Own{word(w, 0), word(w, 1), word(w, 2), word(w, 3), word(w, 4)};
+        const int32_t v = a.plist[i], e0 = a.off[v];
+        return Own{v, e0, a.off[v + 1] - e0, a.pri[v], 4 * (a.strat[v] + 1) + a.solved[v]};
+    };
+    auto put = [&](int32_t w, int32_t v, int32_t t) {
+        if (w < kMaxCached) {
+            word(w, 4) = t;
+        } else {
+            a.strat[v] = (t >> 2) - 1;
+            a.solved[v] = t & 3;   // (with kTouched until the end)
+        }
+    };
+    auto successor = [&](int32_t w, int32_t e0, int32_t j) -> int32_t {
+        return (w < kMaxCached && j < kFirst) ? word(w, 5 + j) : a.tgt[e0 + j];
+    };
+    // the records of the current evaluation, and those that switch phases prepare
+    int4 *jump = a.jump[0], *jump_next = a.jump[1];
+    int2 *path = a.path[0], *path_next = a.path[1];
+    // fresh: the choice differs from the current evaluation's
+    auto prepare = [&](int4 *j, int2 *p, const Own &o, int32_t code, bool fresh) {
+        const int32_t t = (o.t >> 2) - 1;
+        p[o.v] = make_int2(t, o.pri);
+        store_jump(&j[o.v], (o.t & kSolved) ? make_int4(code, 0, 0, 0) : make_int4(t, o.pri, 1, bits(o.t, fresh)));
+    };
+    // The player's choice at a vertex (k_switch's rule): the successors in CSR
+    // order, moving only on a strict improvement; that is the first best one,
+    // the present choice counting first.  Keys decide; among distinct finite
+    // vertices that share the best key, exact comparisons.  The present choice
+    // was a best one at the last examination, so where it and the other path
+    // are as they were then (newbit; solved vertices' records do not tell), it
+    // stands.  False if the walks passed the budget.
+    auto choose = [&](int32_t w, const Own &o, int32_t player, const int4 *skip, int32_t budget, int32_t own_w,
+                      int32_t &choice) -> bool {
+        const int32_t cur0 = choice;
+        int32_t cur = cur0, kc = (cur0 >= 0) ? a.key[cur0] : 0;
+        bool tie = false;
+        for (int32_t b = 0; b < o.deg; b += kFirst) {
+            int32_t us[kFirst], ks[kFirst];
+#pragma unroll
+            for (int j = 0; j < kFirst; j++) us[j] = (b + j < o.deg) ? successor(w, o.e0, b + j) : -1;
+#pragma unroll
+            for (int j = 0; j < kFirst; j++) ks[j] = (us[j] >= 0) ? a.key[us[j]] : 0;
+#pragma unroll
+            for (int j = 0; j < kFirst; j++) {
+                if (us[j] < 0) continue;
+                if ((player == 0) ? ks[j] > kc : ks[j] < kc) {
+                    cur = us[j];
+                    kc = ks[j];
+                    tie = false;
+                } else if (ks[j] == kc && us[j] != cur) {
+                    tie = true;
+                }
+            }
+        }
+        if (tie && !key_infinite(kc)) {
+            const int32_t newbit = player == 0 ? kNewEven : kNew;
+            const bool settled = cur == cur0 && !(o.t & kSolved) && !(own_w & newbit);
+            int32_t loads = 0;
+            bool after = cur == cur0;   // the candidates follow the first best one
+            for (int32_t j = 0; j < o.deg; j++) {
+                const int32_t u = successor(w, o.e0, j);
+                if (!after) {
+                    after = u == cur;
+                    continue;
+                }
+                if (u == cur || a.key[u] != kc) continue;
+                if (settled && cur == cur0 && !(jump[u].w & newbit)) continue;
+                const int c = compare_tied(jump, path, skip, u, cur, loads, budget, &a.sync->err);
+                if (c == kUndecided) return false;
+                if ((player == 0) ? c > 0 : c < 0) cur = u;
+            }
+        }
+        choice = cur;
+        return true;
+    };
+
+    // init_strat (cpu_parity.cpp:276-286)
+    if (tid == 0) *a.ucount = 0;
+    for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
+        Own o;
+        o.v = a.plist[i];
+        o.e0 = a.off[o.v];
+        o.deg = a.off[o.v + 1] - o.e0;
+        o.pri = a.pri[o.v];
+        o.t = (i < a.n_even ? 0 : 4 * (a.tgt[o.e0] + 1)) | kTouched;
+        if (w < kMaxCached) {
+            word(w, 0) = o.v;
+            word(w, 1) = o.e0;
+            word(w, 2) = o.deg;
+            word(w, 3) = o.pri;
+#pragma unroll
+            for (int j = 0; j < kFirst; j++) word(w, 5 + j) = j < o.deg ? a.tgt[o.e0 + j] : 0;
+        }
+        put(w, o.v, o.t);
+        prepare(jump, path, o, 0, true);
+    }
+    barrier(false, false);
+
+    int32_t iters = 0, brs = 0, stop = GraphCtl::kRunning;
+    while (stop == GraphCtl::kRunning) {
+        // evaluation
+        voted = true;
+        for (int pass = 0; voted; pass++) {
+            if (pass == kMaxPasses) {   // cannot happen: windows grow at least kJumps-fold per pass
+                if (tid == 0) atomicOr(&a.sync->err, DERR_WALK_CAP);
+                break;
+            }
+            bool left = false;
+            for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
+                const Own o = get(w, i);
+                if (o.t & kSolved) continue;   // its record and key stay
+                int4 r = load_jump(&jump[o.v]);
+                if (!jump_pass(jump, n, o.v, r)) {
+                    left = true;
+                    continue;
+                }
+                if (r.w & kNew) put(w, o.v, o.t | kTouched);
+                a.key[o.v] = r.x == kSink ? finite_key(r.y, r.z) : (r.x == kPosInf ? KEY_POS_INF : KEY_NEG_INF);
+            }
+            barrier(left, false);
+        }
+        brs++;
+        if (tid == 0 && a.inject_at > 0 && brs == a.inject_at) atomicOr(&a.sync->err, a.inject_bits);
+        // mark_solved and switch: Odd, and Even when Odd made no move
+        int32_t player = 1;
+        bool go;
+        for (;; player = 0) {
+            const int32_t code = player == 0 ? kPosInf : kNegInf;
+            uint32_t over = 0;   // the thread's vertices that are left over
+            bool moved = false;
+            for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
+                Own o = get(w, i);
+                const int4 r = jump[o.v];   // own record
+                const int32_t t0 = o.t;
+                bool fresh = false;
+                if (r.x == code) o.t |= kSolved;
+                if (player == 0) o.t &= ~kTouched;
+                if ((i < a.n_even) == (player == 0)) {
+                    int32_t choice = (o.t >> 2) - 1;
+                    if (choose(w, o, player, nullptr, budget, r.w, choice)) o.t = 4 * (choice + 1) + (o.t & 3);
+                    else over |= 1u << w;
+                    fresh = (o.t >> 2) != (t0 >> 2);
+                    moved |= fresh;
+                }
+                if (o.t != t0) put(w, o.v, o.t);
+                prepare(jump_next, path_next, o, r.x, fresh);
+            }
+            barrier(moved, over != 0);
+            go = voted;
+            if (voted2) {
+                for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
+                    const int32_t v = w < kMaxCached ? word(w, 0) : a.plist[i];
+                    const int4 r = jump[v];
+                    if (r.x != kSink) continue;
+                    Top2 seg = {-1, 0, -1, 0};
+                    int32_t anc = v;
+                    const int32_t d = r.w & kLen;
+                    for (int32_t j = d - skip_landmark_depth(d); j > 0; j--) {
+                        const int2 q = path[anc];
+                        top2_add(seg, q.y);
+                        anc = q.x;
+                    }
+                    a.skip[v] = skip_pack(anc, seg);
+                }
+                barrier(false, false);
+                moved = false;
+                for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
+                    if (!(over >> w & 1)) continue;
+                    Own o = get(w, i);
+                    const int4 r = jump[o.v];
+                    int32_t choice = (o.t >> 2) - 1;
+                    choose(w, o, player, a.skip, INT_MAX, r.w, choice);
+                    if (choice != (o.t >> 2) - 1) {
+                        moved = true;
+                        o.t = 4 * (choice + 1) + (o.t & 3);
+                        put(w, o.v, o.t);
+                        prepare(jump_next, path_next, o, r.x, true);
+                    }
+                }
+                barrier(moved, false);
+                go |= voted;
+            }
+            if (go || player == 0) break;
+        }
+        // the loop's control, as k_ctl_even (solver_graph.cu)
+        if (err) {
+            stop = GraphCtl::kDeviceError;
+        } else if (player == 0) {
+            iters++;
+            if (!go) stop = GraphCtl::kConverged;
+        }
+        if (stop == GraphCtl::kRunning && a.max_evals > 0 && brs >= a.max_evals) stop = GraphCtl::kEvalCap;
+        if (stop == GraphCtl::kRunning && brs >= a.guard) stop = GraphCtl::kRunaway;
+        if (stop != GraphCtl::kRunning) break;
+        if (player == 0 && a.reset) {   // cpu_parity.cpp:300-307
+            for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
+                if (i < a.n_even) continue;
+                Own o = get(w, i);
+                o.t = 4 * (successor(w, o.e0, 0) + 1) + (o.t & 3);
+                put(w, o.v, o.t);
+                prepare(jump_next, path_next, o, jump_next[o.v].x, (o.t >> 2) - 1 != path[o.v].x);
+            }
+            barrier(false, false);
+        }
+        int4 *j = jump;
+        jump = jump_next;
+        jump_next = j;
+        int2 *p = path;
+        path = path_next;
+        path_next = p;
+    }
+
+    // the last evaluation as a solver leaves it (device_common.cuh); the
+    // landmark records are unknown, so later comparisons step
+    for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
+        const Own o = get(w, i);
+        const int32_t v = o.v;
+        const int4 r = jump[v];
+        const int2 q = path[v];
+        const bool fin = r.x == kSink;
+        if (w < kMaxCached) a.strat[v] = (o.t >> 2) - 1;
+        a.solved[v] = o.t & kSolved;
+        const int32_t d = r.w & kLen;
+        if (!fin && !(o.t & kSolved)) a.ulist[atomicAdd(a.ucount, 1)] = v;   // (none once the loop has converged)
+        a.st[v] = fin ? d : (r.x == kPosInf ? ST_POS_INF : ST_NEG_INF);
+        if (fin && d >= kDeepPath) a.rdeep[v] = r.z;
+        a.skip[v] = make_int4(SKIP_UNKNOWN, 0, 0, 0);
+        *reinterpret_cast<int4 *>(&a.node[v]) =
+            fin ? make_int4(q.x, q.y, r.y, path_word(d, r.z))
+                : make_int4(q.x, q.y, r.x == kPosInf ? RM_POS_INF : RM_NEG_INF, 0);
+    }
+    if (tid == 0) {
+        a.ctl->iters = iters;
+        a.ctl->brs = brs;
+        a.ctl->stop = stop;
+        a.ctl->mfrom[0] = a.ctl->mfrom[1] = 0;
+        *a.err = *(volatile uint32_t *)&a.sync->err;
+        a.sync->err = 0;
+        a.sync->phase = phase;
+    }
+}
+
+std::atomic<int> g_sms[kMaxCachedDevices];
+
+}  // namespace
+
+static int device_sms()
+{
+    return per_device(g_sms, [] {
+        int dev = 0, x = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&x, cudaDevAttrMultiProcessorCount, dev);
+        return x > 0 ? x : 1;
+    });
+}
+
+int64_t solve_capacity() { return (int64_t)kMaxWaves * kSolveThreads * device_sms(); }
+
+int launch_solve(cudaStream_t s, const SolveArgs &a)
+{
+    const int sms = device_sms();
+    // the vertices spread over all SMs, at least kMinThreads per block (n = 10^4:
+    // 0.63 ms per solve in ten blocks of 1,024, 0.53 ms in 79 of 128; one block
+    // up to kOneBlock vertices, where block barriers are worth more)
+    int threads = kSolveThreads;
+    while (threads > kMinThreads && ceil_div(a.n, threads / 2) <= sms) threads /= 2;
+    const int64_t need = ceil_div(a.n, threads);
+    const int grid = a.n <= kOneBlock ? 1 : (int)(need < sms ? need : sms);
+    if (grid == 1) threads = kSolveThreads;
+    const int64_t waves = ceil_div(a.n, (int64_t)grid * threads);
+    const size_t smem = 4 * (size_t)kWords * threads * (size_t)(waves < kMaxCached ? waves : kMaxCached);
+    const void *kernel = grid == 1 ? (const void *)k_solve<false> : (const void *)k_solve<true>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBytes);
+    if (e != cudaSuccess) return (int)e;
+    void *args[] = {(void *)&a};
+    count_launch();
+    if (grid == 1) return (int)cudaLaunchKernel(kernel, dim3(1), dim3(threads), args, smem, s);
+    return (int)cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, smem, s);
+}
+
+}  // namespace psi

@@ -232,12 +232,12 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
         {(void **)&tie_, (size_t)cap_n},
         {(void **)&watch_, (size_t)cap_n},
         {(void **)&ulist_, 4 * (size_t)ucap_},
-        {(void **)&la_, 4 * (size_t)cap_n},
-        {(void **)&lb_, 4 * (size_t)cap_n},
+        {(void **)&paths_, 2 * sizeof(int2) * (size_t)cap_n},
         {(void **)&jA_, sizeof(int4) * (size_t)cap_n},
         {(void **)&jB_, sizeof(int4) * (size_t)cap_n},
         {(void **)&dw_, sizeof(Words)},
         {(void **)&ctl_, sizeof(GraphCtl)},
+        {(void **)&sync_, sizeof(SolveSync)},
     };
     for (const auto &a : arrays) {
         cudaError_t e = device_alloc(a.ptr, a.bytes, stream_);
@@ -264,6 +264,7 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
     }
     PSI_CUDA_TRY(cudaMallocHost((void **)&hw_, sizeof(Words)));
     PSI_CUDA_TRY(cudaMemsetAsync(dw_, 0, sizeof(Words), stream_));
+    PSI_CUDA_TRY(cudaMemsetAsync(sync_, 0, sizeof(SolveSync), stream_));
     const GraphCtl fresh;
     // pageable source: staged before the call returns
     PSI_CUDA_TRY(cudaMemcpyAsync(ctl_, &fresh, sizeof fresh, cudaMemcpyHostToDevice, stream_));
@@ -416,10 +417,20 @@ void Solver::reset_times()
 void Solver::reset_tracking()
 {
     static const int32_t one = 1;
+    stale_ = false;
     cudaMemsetAsync(need_, 1, (size_t)n_, stream_);
     cudaMemsetAsync(tie_, 0, (size_t)n_, stream_);
     cudaMemsetAsync(watch_, 0, (size_t)n_, stream_);
     cudaMemcpyAsync(&ctl_->quiet, &one, sizeof one, cudaMemcpyHostToDevice, stream_);
+}
+
+// The same when a switch step may come before the next evaluation, which
+// then has to flag what it changes.
+void Solver::refresh_tracking()
+{
+    if (!stale_) return;
+    reset_tracking();
+    cudaMemsetAsync(&ctl_->quiet, 0, sizeof(int32_t), stream_);
 }
 
 int Solver::init_strat()
@@ -519,8 +530,8 @@ EvalArgs Solver::eval_args()
     a.key = key_;
     a.ulist = ulist_;
     a.ucount = &dw_->ucount;
-    a.la = la_;
-    a.lb = lb_;
+    a.la = reinterpret_cast<int32_t *>(paths_);
+    a.lb = a.la + n_;
     a.lcount = &dw_->lcount;
     a.ja = jA_;
     a.jb = jB_;
@@ -550,6 +561,7 @@ int Solver::compute_valuation()
     if (!strat_ready_) return fail(PSI_ERR_STATE, "compute_valuation before init_strat");
     int rc = set_device();
     if (rc) return rc;
+    refresh_tracking();
     // the last evaluation's state and the switch steps' change list since are
     // usable only if no strategy changed outside a switch step
     launch_eval_gates(stream_, ctl_, (tracked_ && incremental_ != PSI_INCR_OFF) ? 1 : 0);
@@ -591,6 +603,7 @@ int Solver::switch_strategy(int32_t player, int64_t *switched)
     if (!val_ready_) return fail(PSI_ERR_STATE, "switch_strategy before compute_valuation");
     int rc = set_device();
     if (rc) return rc;
+    refresh_tracking();
     PSI_CUDA_TRY(cudaMemsetAsync(dw_->sw, 0, sizeof(dw_->sw), stream_));
     phase_begin(PH_SWITCH);
     const int32_t np = (player == 0) ? np0_ : np_ - np0_;
@@ -639,14 +652,14 @@ int Solver::get_winning(int32_t player, std::vector<int32_t> &out)
     return copy_winning(out.data(), k);
 }
 
-// The winning set of `player` selected on the device into la_ (free between
+// The winning set of `player` selected on the device into paths_ (free between
 // evaluations); *count receives its size.
 int Solver::winning_ids(int32_t player, int64_t *count)
 {
     if (player != 0 && player != 1) return fail(PSI_ERR_INVALID, "player must be 0 or 1");
     int rc = set_device();
     if (rc) return rc;
-    int ce = select_winning(stream_, n_, player, st_, la_, &dw_->selcount);
+    int ce = select_winning(stream_, n_, player, st_, reinterpret_cast<int32_t *>(paths_), &dw_->selcount);
     if (ce) return fail(PSI_ERR_CUDA, std::string("winning set: ") + cudaGetErrorString((cudaError_t)ce));
     rc = sync_and_check("get_winning");
     if (rc) return rc;
@@ -656,7 +669,7 @@ int Solver::winning_ids(int32_t player, int64_t *count)
 
 int Solver::copy_winning(int32_t *out, int64_t k)
 {
-    if (k > 0) PSI_CUDA_TRY(cudaMemcpyAsync(out, la_, 4 * (size_t)k, cudaMemcpyDeviceToHost, stream_));
+    if (k > 0) PSI_CUDA_TRY(cudaMemcpyAsync(out, paths_, 4 * (size_t)k, cudaMemcpyDeviceToHost, stream_));
     PSI_CUDA_TRY(cudaStreamSynchronize(stream_));
     return PSI_OK;
 }

@@ -204,11 +204,12 @@ private:
     // evaluation scratch
     int32_t *ulist_ = nullptr;
     int32_t *rdeep_ = nullptr;   // counts of paths too long for the path record's word
-    int32_t *la_ = nullptr, *lb_ = nullptr;   // walks cut short (EvalArgs)
+    int2 *paths_ = nullptr;      // 2n entries: path records (SolveArgs), or the lists of walks cut short (EvalArgs)
     uint8_t *need_ = nullptr;    // vertices their owner's next switch step must examine (ChangeTrack)
     uint8_t *tie_ = nullptr;     // vertices whose last examination rested on a walk (ChangeTrack)
     uint8_t *watch_ = nullptr;   // vertices such an examination rested on (ChangeTrack)
     ChangeTrack track() const { return ChangeTrack{need_, rev_off_, rev_src_, &ctl_->quiet, tie_, watch_}; }
+    void refresh_tracking();     // after a fused solve: every vertex to be examined
     void reset_tracking();       // every vertex to be examined (need = 1, quiet until the next evaluation)
     int32_t *rev_off_ = nullptr, *rev_src_ = nullptr;   // distinct in-neighbours (static)
     int4 *jA_ = nullptr, *jB_ = nullptr;   // jump entries of the walks cut short
@@ -236,6 +237,12 @@ private:
     // graph-driven solve loop (solver_graph.cu)
     int run_graph(bool reset, int64_t max_evals, GraphCtl *out, int4 *gstate_out);
     int solve_batch_graph(std::vector<int4> &state);
+    // the loop as one persistent kernel (solve_kernels.cu), where fused() says so
+    bool fused();
+    int run_fused(bool reset, int64_t max_evals, GraphCtl *out);
+    static int loop_ended(const GraphCtl &out);
+    SolveSync *sync_ = nullptr;
+    bool stale_ = false;   // the tracking flags do not describe the state: reset before they are used
     bool use_graph_ = false, graph_reset_ = false;
     int32_t inject_at_ = 0;
     uint32_t inject_bits_ = 0;

@@ -78,6 +78,13 @@ inline int32_t eval_guard(int64_t n)
     return (int32_t)(g < (1 << 14) ? (1 << 14) : (g > (1 << 20) ? (1 << 20) : g));
 }
 
+// Games below 2^20 vertices are solved by one persistent kernel.  Solve and
+// read-back, graph -> kernel: n = 100 0.65 -> 0.17 ms, 10^4 1.41 -> 0.57 ms,
+// 10^5 (reset variant) 3.43 -> 1.18 ms, 10^6 9.0 -> 4.3 ms; at 2*10^6 both take
+// the same, and beyond, where full evaluations no longer run from L2, the
+// graph's patches win.
+constexpr int32_t kFusedVertices = (1 << 20) - 1;
+
 }  // namespace
 
 // Opens the full evaluation's conditional node iff this evaluation is not a
@@ -241,17 +248,79 @@ int Solver::run_graph(bool reset, int64_t max_evals, GraphCtl *out, int4 *gstate
     }
     val_ready_ = true;
     tracked_ = true;
-    if (out->stop == GraphCtl::kEvalCap) return fail(PSI_ERR_LIMIT, "evaluation cap reached");
-    if (out->stop == GraphCtl::kDeviceError) return fail(PSI_ERR_LIMIT, "graph solve loop stopped by a device error");
-    if (out->stop != GraphCtl::kConverged) return fail(PSI_ERR_LIMIT, "graph solve loop stopped by its guard");
+    return loop_ended(*out);
+}
+
+int Solver::loop_ended(const GraphCtl &out)
+{
+    if (out.stop == GraphCtl::kEvalCap) return fail(PSI_ERR_LIMIT, "evaluation cap reached");
+    if (out.stop == GraphCtl::kDeviceError) return fail(PSI_ERR_LIMIT, "graph solve loop stopped by a device error");
+    if (out.stop != GraphCtl::kConverged) return fail(PSI_ERR_LIMIT, "graph solve loop stopped by its guard");
     return PSI_OK;
 }
 
-// solve_si as one graph launch; the same results and counts as solve().
+// Whether psi_solve runs as one persistent kernel.  It evaluates in full
+// every time (so not with PSI_INCR_ALWAYS, which asks for patches) and has a
+// switch of its own (so not with the warp-cooperative kernel).
+bool Solver::fused()
+{
+    return games_ == 0 && n_ > 0 && n_ <= kFusedVertices && incremental_ != PSI_INCR_ALWAYS && !switch_warp_ &&
+           set_device() == PSI_OK && n_ <= solve_capacity();
+}
+
+int Solver::run_fused(bool reset, int64_t max_evals, GraphCtl *out)
+{
+    int rc = set_device();
+    if (rc) return rc;
+    SolveArgs a;
+    a.n = n_;
+    a.n_even = np0_;
+    a.owner = owner_;
+    a.pri = pri_;
+    a.off = off_;
+    a.tgt = tgt_;
+    a.plist = plist_;
+    a.strat = strat_;
+    a.st = st_;
+    a.key = key_;
+    a.rdeep = rdeep_;
+    a.solved = solved_;
+    a.node = node_;
+    a.skip = skip_;
+    a.jump[0] = jA_;
+    a.jump[1] = jB_;
+    a.path[0] = paths_;
+    a.path[1] = paths_ + n_;
+    a.ulist = ulist_;
+    a.ucount = &dw_->ucount;
+    a.sync = sync_;
+    a.ctl = ctl_;
+    a.err = &dw_->err;
+    a.reset = reset ? 1 : 0;
+    a.max_evals = max_evals > 0 && max_evals < INT32_MAX ? (int32_t)max_evals : 0;
+    a.guard = eval_guard(n_);
+    a.inject_at = inject_at_;
+    a.inject_bits = inject_bits_;
+    int ce = launch_solve(stream_, a);
+    if (ce) return fail(PSI_ERR_CUDA, std::string("solve kernel: ") + cudaGetErrorString((cudaError_t)ce));
+    PSI_CUDA_TRY(cudaMemcpyAsync(out, ctl_, sizeof *out, cudaMemcpyDeviceToHost, stream_));
+    rc = sync_and_check("solve (kernel)");
+    if (rc && rc != PSI_ERR_LIMIT) return rc;
+    times_.evals += out->brs;
+    times_.switches += out->brs + out->iters;
+    strat_ready_ = true;
+    tracked_ = false;   // no switch step listed the changes
+    stale_ = true;
+    val_ready_ = rc == PSI_OK;
+    if (rc) return rc;   // the device error word was set: the state is not trusted
+    return loop_ended(*out);
+}
+
+// solve_si on the device; the same results and counts as solve().
 int Solver::solve_graph(int32_t reset, int32_t *iters, int32_t *brs, int64_t max_evals)
 {
     GraphCtl out;
-    int rc = run_graph(reset != 0, max_evals, &out, nullptr);
+    int rc = fused() ? run_fused(reset != 0, max_evals, &out) : run_graph(reset != 0, max_evals, &out, nullptr);
     if (rc) return rc;
     *iters = out.iters;
     *brs = out.brs;

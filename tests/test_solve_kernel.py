@@ -1,0 +1,102 @@
+"""psi_solve as one persistent kernel (solve_kernels.cu) at the sizes where
+its launch or its phases change: one block up to 1,024 vertices, blocks of 128
+threads and more above, two vertices per thread past 155,648 (152 SMs), more
+than the five kept in shared memory past 778,240; jumps over deep chains and
+long cycles; and the state it leaves for the step-by-step calls."""
+import numpy as np
+import pytest
+
+import oracle
+import psi
+from games import make
+from test_root_walk import paths_game
+
+PSI_ERR_LIMIT = 8
+
+
+def _solved(s, reset=False):
+    out = s.solve(reset=reset), s.get_strategy(), s.get_infinite(), s.get_solved(), s.get_winning(0)
+    return out + s.get_summary()
+
+
+def _same(a, b):
+    assert a[0] == b[0]
+    for k, (x, y) in enumerate(zip(a[1:], b[1:])):
+        assert np.array_equal(x, y), f"output {k}: differ at {np.nonzero(x != y)[0][:10]}"
+
+
+GAMES = [("ring10", 10, 0)]
+GAMES += [("c4", n, n) for n in (20, 127, 128, 129, 1023, 1024, 1025, 2049, 19456, 19457)]
+GAMES += [("smallpri", n, n) for n in (64, 1024, 1025, 30000)]
+GAMES += [("c3", n, n) for n in (50, 1025, 20000)]
+GAMES += [("evencyc", 3000, 5), ("cycles", 12, 3), ("cycles", 24, 4)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("reset", [False, True])
+@pytest.mark.parametrize("fam,n,seed", GAMES)
+def test_solve_matches_the_oracle(fam, n, seed, reset):
+    g = make(fam, n, seed)
+    ref = oracle.Sparse(*g.csr())
+    s = psi.GPUList(g)
+    for _ in range(2):                        # a second solve starts afresh
+        assert s.solve(reset=reset) == ref.solve(reset=reset)
+        assert np.array_equal(s.get_strategy(), ref.get_strategy())
+        assert np.array_equal(s.get_infinite(), ref.get_infinite())
+        assert np.array_equal(s.get_winning(0), ref.get_winning(0))
+    s.close()
+    ref.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,pri", [(155648, 155648), (155649, 9), (778241, 778241), ((1 << 20) - 1, 1 << 20)])
+def test_solve_matches_the_graph_loop(n, pri):
+    """Against the same game through the graph (the warp-cooperative switch
+    selects it), which other tests hold to the oracle at these sizes."""
+    g = psi.Game.random(n, 2, 5, pri, n)
+    a, b = psi.GPUList(g), psi.GPUList(g, switch_kernel=1)
+    _same(_solved(a), _solved(b))
+    a.close()
+    b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("chains,cycle", [
+    ([1], 0), ([64], 0), ([65], 0), ([3000, 500], 0), ([0xFFFE], 0), ([0xFFFF], 0), ([70000], 0), ([100000] * 4, 0),
+    ([5], 1), ([100], 2), ([900], 63), ([900], 64), ([30], 4097), ([5000] * 40, 3), ([100], 200000),
+])
+def test_deep_chains_and_long_cycles(chains, cycle):
+    g = paths_game(chains, 7 * len(chains) + cycle, cycle=cycle)
+    a, b = psi.GPUList(g), psi.GPUList(g, graph=0)
+    _same(_solved(a), _solved(b))
+    a.close()
+    b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cap", [1, 2, 5, 9])
+@pytest.mark.parametrize("reset", [0, 1])
+def test_steps_after_a_capped_solve(cap, reset):
+    """A solve stopped by its evaluation cap leaves a state that the
+    step-by-step calls go on from, as after the host-driven loop."""
+    import ctypes as C
+
+    from psi._lib import lib
+    g = make("c1", 3000, 17)
+    a, b = psi.GPUList(g), psi.GPUList(g, graph=0)
+    for s in (a, b):
+        it, br = C.c_int32(), C.c_int32()
+        assert lib.psi_solve(s._h, reset, C.byref(it), C.byref(br), cap) == PSI_ERR_LIMIT
+    for step in range(4):
+        for s in (a, b):
+            if step:
+                s.compute_valuation()
+        for p in (1, 0):
+            a.mark_solved(p)
+            b.mark_solved(p)
+            assert a.switch_strategy(p) == b.switch_strategy(p)
+        assert np.array_equal(a.get_strategy(), b.get_strategy())
+        assert np.array_equal(a.get_infinite(), b.get_infinite())
+        assert np.array_equal(a.get_solved(), b.get_solved())
+    a.close()
+    b.close()
