@@ -18,102 +18,18 @@ __device__ __forceinline__ int decide(int32_t p, int32_t ca, int32_t cb)
 }
 
 // Tier 3: walks to the lowest common ancestor of u and w (depths du, dw; w may
-// be the sink, -1 with depth 0), collecting the top two priorities of each
-// side's segment below it; passes after the first repeat the walk counting
-// only priorities below the last tie.  With skip, the first pass jumps whole
-// landmark segments (device_common.cuh): the deeper side jumps while its
+// be the sink, -1 with depth 0).  Pass k finds the highest priority below the
+// last tie on each side's segment below the ancestor, and its count.  With
+// skip, whole landmark segments are jumped (device_common.cuh) where their
+// record's two priorities tell the one sought: the deeper side jumps while its
 // landmark is no shallower than the other side; at equal depths both jump
-// while their landmarks differ (the common ancestor is then above both);
-// once they share one, the common ancestor lies in that segment and both
-// step one vertex at a time.
-static __device__ int walk_compare(const PathNode *__restrict__ node, const int4 *__restrict__ skip, int32_t u, int32_t du,
-                            int32_t w, int32_t dw, int32_t &loads, uint32_t *__restrict__ err)
-{
-    int32_t thr = INT_MAX;
-    const int32_t max_pass = (du + dw) / 2 + 2;
-    for (int32_t pass = 0; pass < max_pass; pass++) {
-        Top2 A = {-1, 0, -1, 0}, B = {-1, 0, -1, 0};
-        int32_t a = u, b = w, da = du, db = dw;
-        bool jumps = skip != nullptr && pass == 0;
-        while (a != b || da != db) {
-            bool adv_a = da >= db, adv_b = db >= da;
-            if ((adv_a && (a < 0 || da <= 0)) || (adv_b && (b < 0 || db <= 0))) {   // inconsistent: cannot happen
-                atomicOr(err, DERR_WALK_CAP);
-                return 0;
-            }
-            if (jumps) {
-                if (adv_a && adv_b) {
-                    const int4 sa = skip[a], sb = skip[b];
-                    loads += 2;
-                    if (sa.x != SKIP_UNKNOWN && sb.x != SKIP_UNKNOWN) {
-                        if (sa.x != sb.x) {
-                            skip_merge(A, sa);
-                            skip_merge(B, sb);
-                            a = sa.x;
-                            b = sb.x;
-                            da = db = skip_landmark_depth(da);
-                            continue;
-                        }
-                        jumps = false;   // one landmark: the common ancestor is within this segment
-                    }
-                } else {
-                    const int32_t x = adv_a ? a : b, dx = adv_a ? da : db, other = adv_a ? db : da;
-                    const int32_t L = skip_landmark_depth(dx);
-                    if (L >= other) {
-                        const int4 sx = skip[x];
-                        loads++;
-                        if (sx.x != SKIP_UNKNOWN) {
-                            if (adv_a) {
-                                skip_merge(A, sx);
-                                a = sx.x;
-                                da = L;
-                            } else {
-                                skip_merge(B, sx);
-                                b = sx.x;
-                                db = L;
-                            }
-                            continue;
-                        }
-                    }
-                }
-            }
-            if (adv_a) {
-                int2 q = *reinterpret_cast<const int2 *>(&node[a]);
-                loads++;
-                if (q.y < thr) top2_add(A, q.y);
-                a = q.x;
-                da--;
-            }
-            if (adv_b) {
-                int2 q = *reinterpret_cast<const int2 *>(&node[b]);
-                loads++;
-                if (q.y < thr) top2_add(B, q.y);
-                b = q.x;
-                db--;
-            }
-        }
-        int32_t M1 = max(A.m1, B.m1);
-        if (M1 < 0) return 0;
-        int32_t ca = (A.m1 == M1) ? A.c1 : 0, cb = (B.m1 == M1) ? B.c1 : 0;
-        if (ca != cb) return decide(M1, ca, cb);
-        int32_t M2 = max(A.m2, B.m2);
-        if (M2 < 0) return 0;
-        ca = (A.m2 == M2) ? A.c2 : 0;
-        cb = (B.m2 == M2) ? B.c2 : 0;
-        if (ca != cb) return decide(M2, ca, cb);
-        thr = M2;
-    }
-    atomicOr(err, DERR_PASS_CAP);
-    return 0;
-}
-
-// The same comparison with one priority per pass, for kernels where a whole
-// phase waits for its longest walk: few instructions per step and no branches
-// on priorities (the two-priority update above diverges, about 0.12 us per
-// step on top of the loads).  Pass k finds the highest priority below the last
-// tie and its count on either side; with skip, whole landmark segments are
-// jumped where their record's two priorities tell the one sought.  path: per
-// vertex (parent, priority).  Once loads passes budget: kUndecided.
+// while their landmarks differ (the common ancestor is then above both); once
+// they share one, the common ancestor lies in that segment and both step one
+// vertex at a time.  One priority per pass keeps a step to a few instructions
+// without branches on priorities: updating two diverged, about 0.12 us per
+// step on top of the loads, where a whole launch or phase waits for its
+// longest walk.  path: per vertex a record that begins with (parent,
+// priority).  Once loads passes budget: kUndecided.
 constexpr int kUndecided = 2;
 __device__ __forceinline__ void top_add(int32_t &m, int32_t &c, int32_t p, int32_t k, int32_t below)
 {
@@ -125,10 +41,11 @@ __device__ __forceinline__ bool top_jump(int32_t &m, int32_t &c, const int4 s, i
 {
     if (s.x == SKIP_UNKNOWN || (s.y >= below && s.z >= below)) return false;
     const bool first = s.y < below;
-    top_add(m, c, first ? s.y : s.z, first ? s.w & 0xffff : (int32_t)((uint32_t)s.w >> 16), below);
+    top_add(m, c, first ? s.y : s.z, first ? skip_c1(s.w) : skip_c2(s.w), below);
     return true;
 }
-static __device__ __noinline__ int lean_compare(const int2 *path, const int4 *skip, int32_t u, int32_t du, int32_t w,
+template <class Rec>
+static __device__ __noinline__ int lean_compare(const Rec *path, const int4 *skip, int32_t u, int32_t du, int32_t w,
                                                 int32_t dw, int32_t &loads, int32_t budget, uint32_t *err)
 {
     int32_t below = INT_MAX;
@@ -153,7 +70,7 @@ static __device__ __noinline__ int lean_compare(const int2 *path, const int4 *sk
                     continue;
                 }
             }
-            const int2 q = path[a];
+            const int2 q = *reinterpret_cast<const int2 *>(&path[a]);
             top_add(ma, ca, q.y, 1, below);
             a = q.x;
             da--;
@@ -179,7 +96,7 @@ static __device__ __noinline__ int lean_compare(const int2 *path, const int4 *sk
                 // one landmark: the paths meet in this segment
                 jumps = s.x != t.x;
             }
-            const int2 q = path[a], r = path[b];
+            const int2 q = *reinterpret_cast<const int2 *>(&path[a]), r = *reinterpret_cast<const int2 *>(&path[b]);
             top_add(ma, ca, q.y, 1, below);
             top_add(mb, cb, r.y, 1, below);
             a = q.x;

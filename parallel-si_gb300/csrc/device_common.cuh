@@ -194,10 +194,11 @@ __device__ __forceinline__ void top2_add_n(Top2 &t, int32_t p, int32_t count)
 // Landmark skips for the comparison walks.  A finite vertex at depth d has
 // its landmark at depth L = SKIP_K * floor((d - 1) / SKIP_K): the ancestor
 // there (the sink at L = 0).  skip[v] = (landmark, top two priorities of the
-// segment from v up to the landmark, exclusive, and their counts packed as
-// c1 | c2 << 16; a segment holds at most SKIP_K vertices).  Written by the
-// walks of a full evaluation (root_kernels.cu); a patch marks its vertices'
-// records unknown (the paths of all other vertices are unchanged).  SKIP_K
+// segment from v up to the landmark, exclusive, one word: their counts, a
+// segment holds at most SKIP_K vertices, and the number of the evaluation that
+// wrote it).  Written by the walks of a full evaluation (root_kernels.cu) as
+// one 16-byte word; a patch marks its vertices' records unknown (the paths of
+// all other vertices are unchanged).  SKIP_K
 // measured on GB300 (graph solve of the 2^24 random game, long-path 2^23):
 // 64: 63.8, 57.8 ms; 32: 62.8, 57.8; 16: 62.0, 57.0; 8: 61.6, 55.5; 4: 61.8,
 // 55.5 ms: shorter segments shorten the steps after the last jump more than
@@ -205,22 +206,52 @@ __device__ __forceinline__ void top2_add_n(Top2 &t, int32_t p, int32_t count)
 constexpr int32_t SKIP_K = 8;
 constexpr int32_t SKIP_UNKNOWN = INT32_MIN;
 __host__ __device__ __forceinline__ int32_t skip_landmark_depth(int32_t d) { return ((d - 1) / SKIP_K) * SKIP_K; }
-__device__ __forceinline__ int4 skip_pack(int32_t anc, const Top2 &t)
+// the record's word: c1 - 1 (3 bits), c2 (4 bits), evaluation number (25 bits)
+constexpr uint32_t kEpochMask = (1u << 25) - 1;
+__device__ __forceinline__ int32_t skip_c1(int32_t w) { return (w & 7) + 1; }
+__device__ __forceinline__ int32_t skip_c2(int32_t w) { return (w >> 3) & 15; }
+__device__ __forceinline__ uint32_t skip_epoch(int32_t w) { return (uint32_t)w >> 7; }
+__device__ __forceinline__ int4 skip_pack(int32_t anc, const Top2 &t, uint32_t epoch = 0)
 {
-    return make_int4(anc, t.m1, t.m2, (t.c1 & 0xffff) | (t.c2 << 16));
+    return make_int4(anc, t.m1, t.m2, (int32_t)(epoch << 7 | (uint32_t)t.c2 << 3 | (uint32_t)(t.c1 - 1)));
 }
 __device__ __forceinline__ void skip_merge(Top2 &t, const int4 s)
 {
-    top2_add_n(t, s.y, s.w & 0xffff);
-    top2_add_n(t, s.z, (int32_t)((uint32_t)s.w >> 16));
+    top2_add_n(t, s.y, skip_c1(s.w));
+    top2_add_n(t, s.z, skip_c2(s.w));
 }
 
-// Release store of a summary (rmax, word) as one 8-byte word: what was written
-// before it (skip, status, rdeep) is visible to any thread that acquires it.
-__device__ __forceinline__ void publish_summary(PathNode *p, int32_t m, int32_t word)
+// 16-byte records read and written whole while other threads do the same.
+__device__ __forceinline__ int4 load_whole(const int4 *p)
+{
+    int4 r;
+    asm volatile("{\n\t.reg .b128 t;\n\t.reg .b64 lo, hi;\n\t"
+                 "ld.relaxed.gpu.global.b128 t, [%4];\n\t"
+                 "mov.b128 {lo, hi}, t;\n\t"
+                 "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}"
+                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+                 : "l"(p)
+                 : "memory");
+    return r;
+}
+__device__ __forceinline__ void store_whole(int4 *p, const int4 r)
+{
+    asm volatile("{\n\t.reg .b128 t;\n\t.reg .b64 lo, hi;\n\t"
+                 "mov.b64 lo, {%1, %2};\n\tmov.b64 hi, {%3, %4};\n\t"
+                 "mov.b128 t, {lo, hi};\n\t"
+                 "st.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w)
+                 : "memory");
+}
+
+// Publishes a summary (rmax, word) as one 8-byte word.  deep: what was written
+// before it (status, rdeep) is visible to any thread that acquires it; the
+// release costs a wait for all of the thread's stores, so others do without.
+__device__ __forceinline__ void publish_summary(PathNode *p, int32_t m, int32_t word, bool deep = false)
 {
     const unsigned long long w = (unsigned long long)(uint32_t)m | ((unsigned long long)(uint32_t)word << 32);
-    asm volatile("st.release.gpu.global.b64 [%0], %1;" ::"l"(&p->rmax), "l"(w) : "memory");
+    if (deep) asm volatile("st.release.gpu.global.b64 [%0], %1;" ::"l"(&p->rmax), "l"(w) : "memory");
+    else asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(&p->rmax), "l"(w) : "memory");
 }
 __device__ __forceinline__ int32_t acquire_rmax(const PathNode *p)
 {

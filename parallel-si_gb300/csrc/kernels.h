@@ -133,6 +133,7 @@ struct EvalArgs {
     PathNode *node = nullptr;
     int32_t *rdeep = nullptr;     // counts of paths too long for the record's word (n entries)
     int4 *skip = nullptr;         // landmark skips (device_common.cuh)
+    const uint32_t *epoch = nullptr;   // evaluation number (launch_patch_begin advances it)
     int32_t *key = nullptr;       // comparison keys
     int32_t *ulist = nullptr, *ucount = nullptr;   // the vertices the sink does not reach (*ucount 0 on entry)
     int32_t *la = nullptr, *lb = nullptr, *lcount = nullptr;   // walks cut short: two lists (n entries), a counter
@@ -152,6 +153,7 @@ struct SolveSync {
     uint32_t phase = 0;
     uint32_t errs[3] = {0, 0, 0};
     uint32_t err = 0;
+    uint32_t epoch = 0;   // evaluation number of the landmark records (EvalArgs)
 };
 struct SolveArgs {
     int32_t n = 0, n_even = 0;    // plist: Even's n_even vertices, then Odd's
@@ -220,7 +222,8 @@ void launch_mark_solved(cudaStream_t s, const int32_t *ucount, const int32_t *ul
 // ---- all-switches (gpu_parity.cu:191-317, cpu_parity.cpp:154-263)
 // Switches the np vertices listed in plist (all owned by `player`).
 // stats[0..3] += compared edges, walk loads, changed vertices, strict
-// improvements; with game_of (batches) also gcount[game] += improvements,
+// improvements (those only with count_moves; otherwise one per changed vertex,
+// for fewer comparisons); with game_of (batches) also gcount[game] += them,
 // and with gmask only vertices of games whose mask is set switch.  With need
 // (and list: n entries, list_count: one counter) only the vertices of plist
 // whose need flag is set are examined (ChangeTrack); examined vertices get
@@ -239,7 +242,8 @@ void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t pla
                    const int32_t *gate = nullptr, uint8_t *need = nullptr, int32_t *list = nullptr,
                    int32_t *list_count = nullptr, ChangeList changes = ChangeList(), uint8_t *tie = nullptr,
                    uint8_t *watch = nullptr, const int4 *skip = nullptr, bool warp = false,
-                   uint32_t *claim = nullptr, const int8_t *owner = nullptr, int32_t n_all = 0);
+                   uint32_t *claim = nullptr, const int8_t *owner = nullptr, int32_t n_all = 0,
+                   bool count_moves = true);
 // ---- batches: per-game accounting of solve_si (state[g] = brs, iters,
 // odd_done, done; gcount[g] = strict improvements of the last switch step);
 // with gate, only when *gate is set
@@ -308,6 +312,7 @@ struct PatchArgs {
     unsigned long long *stats = nullptr;   // [0] += 1 per patch, [1] += vertices re-evaluated
     ChangeTrack track;
     int4 *skip = nullptr;       // landmark skips: a patched vertex's record becomes unknown
+    uint32_t *epoch = nullptr;
 };
 // Sets the gates the host decides before an evaluation (one thread).
 void launch_eval_gates(cudaStream_t s, EvalGates *g, int32_t try_patch);

@@ -80,6 +80,7 @@ __global__ void k_eval_gates(EvalGates *g, int32_t try_patch) { g->try_patch = t
 __global__ void k_patch_begin(PatchArgs a)
 {
     EvalGates *g = a.g;
+    ++*a.epoch;
     const int32_t cc = g->ccount;
     g->ccount = 0;   // the next switch steps list their changes afresh
     g->csnap = cc;

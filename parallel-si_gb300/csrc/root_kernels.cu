@@ -56,12 +56,15 @@ __global__ void k_root_init(EvalArgs a)
 {
     if (a.gate && !*a.gate) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.lcount = 0;
+    // the evaluation number wraps around: no record of the last round may look current
+    const bool wrap = (*a.epoch & kEpochMask) == 0;
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < a.n; v += (int64_t)gridDim.x * blockDim.x) {
         const int32_t t = a.strat[v], p = a.pri[v];
         int4 q = make_int4(t, p, RM_UNKNOWN, 0);
         if (a.solved[v]) q = make_int4(-1, p, a.st[v] == ST_POS_INF ? RM_POS_INF : RM_NEG_INF, 0);
         else if (t < 0) q = make_int4(-1, p, p, path_word(1, 1));
         *reinterpret_cast<int4 *>(&a.node[v]) = q;
+        if (wrap) a.skip[v] = make_int4(SKIP_UNKNOWN, 0, 0, 0);
         if (a.track.tie && a.track.tie[v]) a.track.need[v] = 1;
     }
 }
@@ -80,15 +83,14 @@ __device__ __forceinline__ void path_depth_count(const EvalArgs &a, int32_t y, i
     }
 }
 
-// Publishes a finite vertex: status, skip, then the summary that vouches for
-// both (release).
+// Publishes a finite vertex: landmark record, status, summary.
 __device__ __forceinline__ void publish_finite(const EvalArgs &a, int32_t v, int32_t d, int32_t m, int32_t c,
-                                               int32_t anc, const Top2 &seg)
+                                               int32_t anc, const Top2 &seg, uint32_t epoch)
 {
+    store_whole(&a.skip[v], skip_pack(anc, seg, epoch));
     a.st[v] = d;
     if (d >= kDeepPath) a.rdeep[v] = c;
-    a.skip[v] = skip_pack(anc, seg);
-    publish_summary(&a.node[v], m, path_word(d, c));
+    publish_summary(&a.node[v], m, path_word(d, c), d >= kDeepPath);
 }
 
 // A walk's step cap: longer walks are left to k_root_settle.
@@ -98,10 +100,18 @@ constexpr int kWalkThreads = 256;
 // atomic (one atomic per warp and pass on the list's counter would serialise)
 constexpr int kUnreachedBuf = 128;
 
-__global__ void __launch_bounds__(kWalkThreads, 6) k_root_walk(EvalArgs a)
+// Bound by the latency of dependent loads (2^22 random game: DRAM 25%, L2 32%,
+// issue slots 45% busy), so by how many walks are in flight: eight blocks per
+// SM at 32 registers; a summary is stored as soon as it is known and without a
+// release (which waits for the thread's earlier stores: a third of the stalls),
+// the landmark record after it and tagged with the evaluation's number.  Walks
+// and init of a 2^24 solve 17.6 -> 14.1 ms (17 full evaluations), long-path
+// 11.0 -> 8.9 ms.
+__global__ void __launch_bounds__(kWalkThreads, 8) k_root_walk(EvalArgs a)
 {
     if (a.gate && !*a.gate) return;
     __shared__ int32_t ubuf[kWalkThreads / 32][kUnreachedBuf];
+    const uint32_t epoch = *a.epoch & kEpochMask;
     const int lane = threadIdx.x & 31;
     int32_t *buf = ubuf[threadIdx.x >> 5];
     int nbuf = 0;   // uniform over the warp
@@ -123,78 +133,71 @@ __global__ void __launch_bounds__(kWalkThreads, 6) k_root_walk(EvalArgs a)
             const int4 q = *reinterpret_cast<const int4 *>(&a.node[v]);
             old = a.key[v];
             if (q.z != RM_POS_INF && q.z != RM_NEG_INF) {   // not solved
-                int32_t m = q.y, c = 1;
-                Top2 seg = {q.y, 1, -1, 0};
                 if (q.x < 0) {   // a child of the sink, published by init: its skip and status are written here
                     a.st[v] = 1;
-                    a.skip[v] = skip_pack(-1, seg);
-                    k = finite_key(m, c);
+                    a.skip[v] = skip_pack(-1, Top2{q.y, 1, -1, 0}, epoch);
+                    k = finite_key(q.y, 1);
                     finite = true;
                 } else {
-                    int32_t y = q.x, s = 1;             // s vertices walked, y the next one
-                    int32_t mark = v, cm = q.y;         // marker, top priority from it up to y (exclusive)
-                    int32_t code = 0;                   // an infinity, once known
+                    int32_t m = q.y, c = 1;
+                    int32_t y = q.x, s = 1, mark = v;   // s vertices walked, y the next one; the marker
                     int4 r;
                     while (true) {
                         r = *reinterpret_cast<const int4 *>(&a.node[y]);
-                        if (r.z != RM_UNKNOWN) {
-                            if (r.z == RM_POS_INF || r.z == RM_NEG_INF) code = r.z;
-                            break;
-                        }
-                        if (y == mark) {
-                            code = (cm & 1) ? RM_NEG_INF : RM_POS_INF;
-                            break;
-                        }
-                        if (s >= kWalkCap) {
-                            left = true;
-                            break;
-                        }
-                        if ((s & (s - 1)) == 0) {       // after 1, 2, 4, ... vertices the marker moves here
-                            mark = y;
-                            cm = r.y;
-                        } else {
-                            cm = max(cm, r.y);
-                        }
+                        if (r.z != RM_UNKNOWN || y == mark || s >= kWalkCap) break;
+                        if ((s & (s - 1)) == 0) mark = y;   // after 1, 2, 4, ... vertices the marker moves here
                         top1_merge(m, c, r.y, 1);
-                        if (s < SKIP_K) top2_add(seg, r.y);
                         y = r.x;
                         s++;
+                    }
+                    int32_t code = 0;                       // an infinity, where it is one
+                    if (r.z == RM_POS_INF || r.z == RM_NEG_INF) {
+                        code = r.z;
+                    } else if (r.z == RM_UNKNOWN && y == mark) {   // a cycle of at most s vertices
+                        int32_t top = r.y;
+                        for (int32_t x = r.x; x != mark;) {
+                            const int2 e = *reinterpret_cast<const int2 *>(&a.node[x]);
+                            top = max(top, e.y);
+                            x = e.x;
+                        }
+                        code = (top & 1) ? RM_NEG_INF : RM_POS_INF;
                     }
                     if (code) {
                         a.st[v] = (code == RM_POS_INF) ? ST_POS_INF : ST_NEG_INF;
                         publish_summary(&a.node[v], code, 0);
                         k = (code == RM_POS_INF) ? KEY_POS_INF : KEY_NEG_INF;
                         infinite = true;
-                    } else if (!left) {
+                    } else if (r.z == RM_UNKNOWN) {
+                        left = true;
+                    } else {
                         int32_t dy, cy;
                         path_depth_count(a, y, r.w, dy, cy);
                         top1_merge(m, c, r.z, cy);
-                        const int32_t d = s + dy, len = d - skip_landmark_depth(d);
-                        int32_t anc = y;
-                        if (s < len) {
-                            // y lies in v's segment and shares its landmark: its record was written
-                            // before the summary (a sink child's is known: itself up to the sink)
-                            if (r.x < 0) {
-                                top2_add(seg, r.y);
-                                anc = -1;
-                            } else {
-                                acquire_rmax(&a.node[y]);
-                                const int4 sy = __ldcg(&a.skip[y]);
-                                skip_merge(seg, sy);
-                                anc = sy.x;
-                            }
-                        } else if (s > len) {   // the landmark lies before y: collect its segment again
-                            seg = Top2{q.y, 1, -1, 0};
-                            anc = q.x;
-                            for (int32_t i = 1; i < len; i++) {
-                                const int2 e = *reinterpret_cast<const int2 *>(&a.node[anc]);
-                                top2_add(seg, e.y);
-                                anc = e.x;
-                            }
-                        }
-                        publish_finite(a, v, d, m, c, anc, seg);
                         k = finite_key(m, c);
                         finite = true;
+                        const int32_t d = s + dy, len = d - skip_landmark_depth(d);
+                        a.st[v] = d;
+                        if (d >= kDeepPath) a.rdeep[v] = c;
+                        publish_summary(&a.node[v], m, path_word(d, c), d >= kDeepPath);
+                        // the segment from v to its landmark: by steps (the walk has just read
+                        // them) up to y, then y's record if the landmark lies beyond and the
+                        // record has arrived (its summary may have come first), else by steps
+                        Top2 seg = {q.y, 1, -1, 0};
+                        int32_t anc = q.x;
+                        for (int32_t i = 1; i < len; i++) {
+                            if (i == s) {
+                                const int4 sy = load_whole(&a.skip[y]);
+                                if (sy.x != SKIP_UNKNOWN && skip_epoch(sy.w) == epoch) {
+                                    skip_merge(seg, sy);
+                                    anc = sy.x;
+                                    break;
+                                }
+                            }
+                            const int2 e = *reinterpret_cast<const int2 *>(&a.node[anc]);
+                            top2_add(seg, e.y);
+                            anc = e.x;
+                        }
+                        store_whole(&a.skip[v], skip_pack(anc, seg, epoch));
                     }
                 }
             }
@@ -280,7 +283,7 @@ __device__ void settle_body(const EvalArgs &a, int32_t nl)
                         top2_add(seg, x.y);
                         anc = x.x;
                     }
-                    publish_finite(a, u, d, m, c, anc, seg);
+                    publish_finite(a, u, d, m, c, anc, seg, *a.epoch & kEpochMask);
                     k = finite_key(m, c);
                 } else {
                     const int4 f = __ldcg(&in[t]);
@@ -357,10 +360,13 @@ int device_sms()
     });
 }
 
-// enough blocks to fill the device a few times over
-unsigned capped_grid(int64_t items)
+// Many more blocks than are resident: walks differ in length, and short blocks
+// even that out (2^24 random game, ms per solve with 16, 64, 256 blocks per
+// SM: 36.6, 35.3, 35.2, long-path 25.1, 24.1, 23.1).  A gated launch whose
+// gate is closed pays for its blocks, 27 us at 256 per SM, so those keep to 64.
+unsigned walk_grid(const EvalArgs &a)
 {
-    const int64_t g = ceil_div(items, kBlock), cap = 16 * (int64_t)device_sms();
+    const int64_t g = ceil_div(a.n, kBlock), cap = (a.gate ? 64 : 256) * (int64_t)device_sms();
     return (unsigned)(g < 1 ? 1 : (g < cap ? g : cap));
 }
 
@@ -369,13 +375,13 @@ unsigned capped_grid(int64_t items)
 void launch_root_init(cudaStream_t s, const EvalArgs &a)
 {
     count_launch();
-    k_root_init<<<capped_grid(a.n), kBlock, 0, s>>>(a);
+    k_root_init<<<walk_grid(a), kBlock, 0, s>>>(a);
 }
 
 void launch_root_walk(cudaStream_t s, const EvalArgs &a)
 {
     count_launch();
-    k_root_walk<<<capped_grid(a.n), kWalkThreads, 0, s>>>(a);
+    k_root_walk<<<walk_grid(a), kWalkThreads, 0, s>>>(a);
 }
 
 int launch_root_settle(cudaStream_t s, const EvalArgs &a)

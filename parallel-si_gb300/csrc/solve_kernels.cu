@@ -68,28 +68,6 @@ constexpr int kMaxPasses = 64;
 constexpr int32_t kMaxLen = 1 << 24, kLen = (1 << 25) - 1;
 constexpr int32_t kNew = 1 << 30, kNewEven = 1 << 29;
 
-__device__ __forceinline__ int4 load_jump(const int4 *p)
-{
-    int4 r;
-    asm volatile("{\n\t.reg .b128 t;\n\t.reg .b64 lo, hi;\n\t"
-                 "ld.relaxed.gpu.global.b128 t, [%4];\n\t"
-                 "mov.b128 {lo, hi}, t;\n\t"
-                 "mov.b64 {%0, %1}, lo;\n\tmov.b64 {%2, %3}, hi;\n\t}"
-                 : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-                 : "l"(p)
-                 : "memory");
-    return r;
-}
-__device__ __forceinline__ void store_jump(int4 *p, const int4 r)
-{
-    asm volatile("{\n\t.reg .b128 t;\n\t.reg .b64 lo, hi;\n\t"
-                 "mov.b64 lo, {%1, %2};\n\tmov.b64 hi, {%3, %4};\n\t"
-                 "mov.b128 t, {lo, hi};\n\t"
-                 "st.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
-                 "r"(r.x), "r"(r.y), "r"(r.z), "r"(r.w)
-                 : "memory");
-}
-
 // One pass of v's record r; true when it is finished.
 __device__ __forceinline__ bool jump_pass(int4 *jump, int32_t n, int32_t v, int4 &r)
 {
@@ -98,10 +76,10 @@ __device__ __forceinline__ bool jump_pass(int4 *jump, int32_t n, int32_t v, int4
     for (int i = 1; i <= kJumps; i++) {
         bool cycle = (r.w & kLen) >= n;
         if (!cycle) {
-            const int4 q = load_jump(&jump[r.x]);
+            const int4 q = load_whole(&jump[r.x]);
             if (q.x <= kNegInf) {
                 r = make_int4(q.x, 0, 0, 0);
-                store_jump(&jump[v], r);
+                store_whole(&jump[v], r);
                 return true;
             }
             top1_merge(r.y, r.z, q.y, q.z);
@@ -117,7 +95,7 @@ __device__ __forceinline__ bool jump_pass(int4 *jump, int32_t n, int32_t v, int4
             const int32_t t0 = r.x;
             int32_t t = t0, len = 0, top = -1, code = 0;
             for (int j = 0; j < kJumps; j++) {
-                const int4 q = load_jump(&jump[t]);
+                const int4 q = load_whole(&jump[t]);
                 if (q.x <= kNegInf) {
                     code = q.x;
                     break;
@@ -132,15 +110,15 @@ __device__ __forceinline__ bool jump_pass(int4 *jump, int32_t n, int32_t v, int4
             }
             if (code) {
                 r = make_int4(code, 0, 0, 0);
-                store_jump(&jump[v], r);
+                store_whole(&jump[v], r);
                 return true;
             }
             r.w = kMaxLen | (r.w & ~kLen);   // a later pass goes on from the cycle
-            store_jump(&jump[v], r);
+            store_whole(&jump[v], r);
             return false;
         }
         if (r.x == kSink && (r.w & kNew)) r.w |= kNewEven;
-        store_jump(&jump[v], r);
+        store_whole(&jump[v], r);
         if (r.x == kSink) return true;
     }
     return false;
@@ -240,7 +218,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
     auto prepare = [&](int4 *j, int2 *p, const Own &o, int32_t code, bool fresh) {
         const int32_t t = (o.t >> 2) - 1;
         p[o.v] = make_int2(t, o.pri);
-        store_jump(&j[o.v], (o.t & kSolved) ? make_int4(code, 0, 0, 0) : make_int4(t, o.pri, 1, bits(o.t, fresh)));
+        store_whole(&j[o.v], (o.t & kSolved) ? make_int4(code, 0, 0, 0) : make_int4(t, o.pri, 1, bits(o.t, fresh)));
     };
     // The player's choice at a vertex (k_switch's rule): the successors in CSR
     // order, moving only on a strict improvement; that is the first best one,
@@ -329,7 +307,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
             for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
                 const Own o = get(w, i);
                 if (o.t & kSolved) continue;   // its record and key stay
-                int4 r = load_jump(&jump[o.v]);
+                int4 r = load_whole(&jump[o.v]);
                 if (!jump_pass(jump, n, o.v, r)) {
                     left = true;
                     continue;

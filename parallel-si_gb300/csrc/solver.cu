@@ -265,6 +265,7 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
     PSI_CUDA_TRY(cudaMallocHost((void **)&hw_, sizeof(Words)));
     PSI_CUDA_TRY(cudaMemsetAsync(dw_, 0, sizeof(Words), stream_));
     PSI_CUDA_TRY(cudaMemsetAsync(sync_, 0, sizeof(SolveSync), stream_));
+    PSI_CUDA_TRY(cudaMemsetAsync(skip_, 0, sizeof(int4) * (size_t)cap_n, stream_));   // of no evaluation (number 0)
     const GraphCtl fresh;
     // pageable source: staged before the call returns
     PSI_CUDA_TRY(cudaMemcpyAsync(ctl_, &fresh, sizeof fresh, cudaMemcpyHostToDevice, stream_));
@@ -488,6 +489,7 @@ PatchArgs Solver::patch_args()
     a.stats = dw_->patch;
     a.track = track();
     a.skip = skip_;
+    a.epoch = &sync_->epoch;
     return a;
 }
 
@@ -527,6 +529,7 @@ EvalArgs Solver::eval_args()
     a.node = node_;
     a.rdeep = rdeep_;
     a.skip = skip_;
+    a.epoch = &sync_->epoch;
     a.key = key_;
     a.ulist = ulist_;
     a.ucount = &dw_->ucount;
@@ -544,7 +547,8 @@ EvalArgs Solver::eval_args()
 // The full evaluation (root_kernels.cu), every kernel gated (ctl_->eval).
 int Solver::enqueue_full(bool timed)
 {
-    const EvalArgs a = eval_args();
+    EvalArgs a = eval_args();
+    if (!timed) a.gate = nullptr;   // in the graph's conditional node: it runs only when it has to
     if (timed) phase_begin(PH_BROADCAST);
     launch_root_init(stream_, a);
     launch_root_walk(stream_, a);
@@ -597,7 +601,7 @@ int Solver::mark_solved(int32_t player)
     return PSI_OK;   // ordered on the stream before the next call
 }
 
-int Solver::switch_strategy(int32_t player, int64_t *switched)
+int Solver::switch_strategy(int32_t player, int64_t *switched, bool count)
 {
     if (player != 0 && player != 1) return fail(PSI_ERR_INVALID, "player must be 0 or 1");
     if (!val_ready_) return fail(PSI_ERR_STATE, "switch_strategy before compute_valuation");
@@ -611,7 +615,7 @@ int Solver::switch_strategy(int32_t player, int64_t *switched)
     // jB_ is free until the next full evaluation: it holds the list of vertices to examine
     launch_switch(stream_, np, pl, player, off_, tgt_, strat_, st_, key_, node_, rdeep_, dw_->sw, game_of_, gcount_,
                   gmask_, &dw_->err, nullptr, need_, reinterpret_cast<int32_t *>(jB_), &dw_->cnt[2], changes(), tie_,
-                  watch_, skip_, switch_warp_, &dw_->claim, arena_ ? nullptr : owner_, n_);
+                  watch_, skip_, switch_warp_, &dw_->claim, arena_ ? nullptr : owner_, n_, count);
     phase_end(PH_SWITCH);
     rc = sync_and_check("switch_strategy");
     if (rc) return rc;
@@ -795,7 +799,7 @@ int Solver::solve(int32_t reset, int32_t *iters, int32_t *brs, int64_t max_evals
             rc = mark_solved(1);
             if (rc) return rc;
             int64_t sw = 0;
-            rc = switch_strategy(1, &sw);
+            rc = switch_strategy(1, &sw, false);
             if (rc) return rc;
             if (sw == 0) break;
             if (max_evals > 0 && br >= max_evals) {
@@ -809,7 +813,7 @@ int Solver::solve(int32_t reset, int32_t *iters, int32_t *brs, int64_t max_evals
         if (rc) return rc;
         it++;
         int64_t sw = 0;
-        rc = switch_strategy(0, &sw);
+        rc = switch_strategy(0, &sw, false);
         if (rc) return rc;
         if (sw == 0) break;
         if (max_evals > 0 && br >= max_evals) {
@@ -851,7 +855,7 @@ int Solver::solve_batch(int32_t *iters, int32_t *brs)
             rc = mark_solved(1);
             if (rc) return rc;
             int64_t sw = 0;
-            rc = switch_strategy(1, &sw);
+            rc = switch_strategy(1, &sw, false);
             if (rc) return rc;
             launch_batch_account(stream_, games_, 1, gstate_, gcount_);
             if (sw == 0) break;
@@ -860,7 +864,7 @@ int Solver::solve_batch(int32_t *iters, int32_t *brs)
         if (rc) return rc;
         launch_batch_account(stream_, games_, 2, gstate_, gcount_);
         int64_t sw = 0;
-        rc = switch_strategy(0, &sw);
+        rc = switch_strategy(0, &sw, false);
         if (rc) return rc;
         launch_batch_account(stream_, games_, 3, gstate_, gcount_);
         if (sw == 0) break;
@@ -1064,12 +1068,12 @@ int Solver::arena_step(bool reset, std::vector<int32_t> &done, std::vector<int32
     gmask_ = nullptr;                       // Odd's step: every resident game
     rc = mark_solved(1);
     int64_t sw = 0;
-    if (!rc) rc = switch_strategy(1, &sw);
+    if (!rc) rc = switch_strategy(1, &sw, false);
     gmask_ = mask;
     if (rc) return rc;
     launch_serve_account(stream_, games_, 1, gstate_, gcount_, gmask_);
     rc = mark_solved(0);                    // Even's step: games with gmask set
-    if (!rc) rc = switch_strategy(0, &sw);
+    if (!rc) rc = switch_strategy(0, &sw, false);
     if (rc) return rc;
     if (reset)
         launch_serve_reset_odd(stream_, np_ - np0_, plist_ + np0_, game_of_, gmask_, gcount_, off_, tgt_, strat_,

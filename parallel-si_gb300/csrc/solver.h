@@ -72,7 +72,9 @@ public:
     int compute_valuation();
     int compute_first_val() { return compute_valuation(); }
     int mark_solved(int32_t player);
-    int switch_strategy(int32_t player, int64_t *switched);
+    // count: *switched is the number of strict improvements; otherwise only
+    // whether it is zero matters (launch_switch's count_moves).
+    int switch_strategy(int32_t player, int64_t *switched, bool count = true);
     int get_winning(int32_t player, std::vector<int32_t> &out);
     // Device-side selection of the winning set, then a copy of its first k ids.
     int winning_ids(int32_t player, int64_t *count);
