@@ -157,6 +157,7 @@ struct SolveSync {
 };
 struct SolveArgs {
     int32_t n = 0, n_even = 0;    // plist: Even's n_even vertices, then Odd's
+    int64_t m = 0;
     const int8_t *owner = nullptr;
     const int32_t *pri = nullptr, *off = nullptr, *tgt = nullptr, *plist = nullptr;
     int32_t *strat = nullptr, *st = nullptr, *key = nullptr, *rdeep = nullptr;

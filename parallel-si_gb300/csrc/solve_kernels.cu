@@ -154,19 +154,21 @@ __device__ __forceinline__ int32_t bits(int32_t t, bool fresh)
 constexpr int kFirst = 5;       // successors kept per vertex
 constexpr int kWords = 5 + kFirst;
 constexpr int kMinThreads = 128;
-constexpr int32_t kOneBlock = 1024;   // games up to this size run in one block
+constexpr int kSmallBytes = 227 * 1024;   // all a block can have
+// Games below this size are solved there.  Solve in us, k_solve -> here: n = 100
+// 96 -> 62, 300 145 -> 91, 1,024 189 -> 152, 1,537 295 -> 263, 2,048 235 -> 241,
+// 4,000 308 -> 454 (one SM's issue slots).
+constexpr int32_t kSmall = 2000;
 constexpr int kMaxWaves = 32;   // vertices per thread (a bit mask)
 constexpr int kMaxCached = 5;   // vertices per thread kept (200 KB); further ones are read anew
 constexpr int kSharedBytes = 4 * kWords * kSolveThreads * kMaxCached;   // 200 KB
 
-// GRID: over the whole grid; otherwise one block with block barriers.
-template <bool GRID>
 __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
 {
     extern __shared__ int32_t own[];   // [wave][word][thread]
     const int32_t n = a.n;
-    const int32_t tid = GRID ? (int32_t)(blockIdx.x * blockDim.x + threadIdx.x) : (int32_t)threadIdx.x;
-    const int32_t nth = GRID ? (int32_t)(gridDim.x * blockDim.x) : (int32_t)blockDim.x;
+    const int32_t tid = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
+    const int32_t nth = (int32_t)(gridDim.x * blockDim.x);
     const int32_t budget = walk_budget(n, nth);
     // Barrier with two votes: whether any thread passed true.  Phase k uses the
     // words k % 3, which thread 0 clears in phase k - 1, when everyone has
@@ -184,8 +186,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
         }
         if (__syncthreads_or(mine) && threadIdx.x == 0) a.sync->vote[k] = 1;
         if (__syncthreads_or(mine2) && threadIdx.x == 0) a.sync->vote2[k] = 1;
-        if (GRID) cg::this_grid().sync();
-        else __syncthreads();
+        cg::this_grid().sync();
         err = __ldcg(&a.sync->errs[k]);
         voted = __ldcg(&a.sync->vote[k]) != 0;
         voted2 = __ldcg(&a.sync->vote2[k]) != 0;
@@ -438,6 +439,230 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
     }
 }
 
+// ---- the smallest games: one block, everything a phase reads in shared memory
+// (its latency is a tenth of L2's, a block barrier's a fortieth of a grid's).
+// Evaluations are plain pointer doubling between two buffers: in round r every
+// record is a window of 2^r vertices or finished, and once 2^r >= n what is
+// left is on or into a cycle that its target's window covers.  Vertices in id
+// order, v = thread, thread + threads, ...
+
+// low bits of the choice word: kSolved, kTouched, and the owner
+constexpr int32_t kOddBit = 4;
+
+struct SmallLayout {   // byte offsets in shared memory
+    int32_t jump[2], path, key, off, choice, tgt, total;
+};
+__host__ __device__ inline SmallLayout small_layout(int32_t n, int64_t m)
+{
+    SmallLayout l;
+    int32_t at = 0;
+    auto take = [&](int64_t bytes) {
+        const int32_t x = at;
+        at += (int32_t)((bytes + 15) & ~15ll);
+        return x;
+    };
+    l.jump[0] = take(16ll * n);
+    l.jump[1] = take(16ll * n);
+    l.path = take(8ll * n);
+    l.key = take(4ll * n);
+    l.off = take(4ll * (n + 1));
+    l.choice = take(4ll * n);
+    l.tgt = at;
+    l.total = at;
+    if (4 * m + at <= kSmallBytes) l.total = at + (int32_t)(4 * m);   // the successors too, if they fit
+    return l;
+}
+
+__global__ void __launch_bounds__(kSolveThreads, 1) k_solve_small(SolveArgs a)
+{
+    extern __shared__ __align__(16) unsigned char mem[];
+    const int32_t n = a.n, tid = threadIdx.x, nth = blockDim.x;
+    const SmallLayout l = small_layout(n, a.m);
+    int4 *jump[2] = {reinterpret_cast<int4 *>(mem + l.jump[0]), reinterpret_cast<int4 *>(mem + l.jump[1])};
+    int2 *path = reinterpret_cast<int2 *>(mem + l.path);
+    int32_t *key = reinterpret_cast<int32_t *>(mem + l.key), *off = reinterpret_cast<int32_t *>(mem + l.off);
+    int32_t *choice = reinterpret_cast<int32_t *>(mem + l.choice);
+    const bool held = l.total > l.tgt;
+    int32_t *held_tgt = reinterpret_cast<int32_t *>(mem + l.tgt);
+    const int32_t *tgt = held ? held_tgt : a.tgt;
+    int rounds = 0;
+    while ((1 << rounds) < n) rounds++;
+
+    for (int32_t v = tid; v <= n; v += nth) off[v] = a.off[v];
+    if (held)
+        for (int32_t e = tid; e < (int32_t)a.m; e += nth) held_tgt[e] = a.tgt[e];
+    for (int32_t v = tid; v < n; v += nth) {   // init_strat (cpu_parity.cpp:276-286)
+        const bool odd = a.owner[v] != 0;
+        const int32_t t = odd ? a.tgt[a.off[v]] : kSink;
+        choice[v] = (t + 1) * 8 + (odd ? kOddBit : 0) + kTouched;
+        path[v] = make_int2(t, a.pri[v]);
+    }
+    if (tid == 0) *a.ucount = 0;
+    bool all_new = true;   // every vertex counts as changed in the first evaluation
+    int32_t iters = 0, brs = 0, stop = GraphCtl::kRunning;
+    int4 *in = jump[0];
+    while (stop == GraphCtl::kRunning) {
+        // evaluation; bit w: the thread's vertex v = tid + w nth
+        in = jump[0];
+        int4 *out = jump[1];
+        uint32_t active = 0, fresh_done = 0;   // unfinished; finished in the last round (one buffer has it)
+        for (int32_t w = 0, v = tid; v < n; w++, v += nth) {
+            const int32_t c = choice[v], t = (c >> 3) - 1;
+            int2 p = path[v];
+            const bool fresh = all_new || p.x != t;
+            p.x = t;
+            path[v] = p;
+            const int32_t wd = 1 | (fresh ? kNew | kNewEven : 0) | ((c & kTouched) ? kNewEven : 0);
+            int4 x = make_int4(t, p.y, 1, wd);
+            if (c & kSolved) x = make_int4(key[v] == KEY_POS_INF ? kPosInf : kNegInf, 0, 0, 0);
+            else if (t == kSink) key[v] = finite_key(p.y, 1);
+            if (fresh) choice[v] = c | kTouched;
+            in[v] = x;
+            if (x.x >= 0) active |= 1u << w;
+            else out[v] = x;
+        }
+        all_new = false;
+        __syncthreads();
+        for (int r = 0;; r++) {
+            uint32_t done = 0;
+            for (uint32_t todo = active | fresh_done; todo; todo &= todo - 1) {
+                const int w = __ffs(todo) - 1;
+                const int32_t v = tid + w * nth;
+                int4 x = in[v];
+                if (active >> w & 1) {
+                    const int4 q = in[x.x];
+                    int32_t code = q.x <= kNegInf ? q.x : 0;
+                    if (q.x >= 0 && r == rounds) code = (q.y & 1) ? kNegInf : kPosInf;
+                    if (code) {
+                        x = make_int4(code, 0, 0, 0);
+                        key[v] = code == kPosInf ? KEY_POS_INF : KEY_NEG_INF;
+                    } else {
+                        top1_merge(x.y, x.z, q.y, q.z);
+                        x.z = min(x.z, kMaxLen);
+                        x.w = min((x.w & kLen) + (q.w & kLen), kMaxLen) | (x.w & kNewEven) | ((x.w | q.w) & kNew);
+                        x.x = q.x;
+                        if (x.x == kSink) {
+                            key[v] = finite_key(x.y, x.z);
+                            if (x.w & kNew) {
+                                x.w |= kNewEven;
+                                choice[v] |= kTouched;
+                            }
+                        }
+                    }
+                    if (x.x < 0) done |= 1u << w;
+                }
+                out[v] = x;
+            }
+            active &= ~done;
+            fresh_done = done;
+            int4 *t = in;
+            in = out;
+            out = t;
+            if (!__syncthreads_or(active != 0)) break;
+        }
+        brs++;
+        if (tid == 0 && a.inject_at > 0 && brs == a.inject_at) atomicOr(&a.sync->err, a.inject_bits);
+        // mark_solved and switch: Odd, and Even when Odd made no move
+        bool go;
+        int32_t player = 1;
+        for (;; player = 0) {
+            const int32_t code = player == 0 ? kPosInf : kNegInf, newbit = player == 0 ? kNewEven : kNew;
+            bool moved = false;
+            for (int32_t v = tid; v < n; v += nth) {
+                int32_t c = choice[v];
+                const int4 r = in[v];
+                if (r.x == code) c |= kSolved;
+                if (player == 0) c &= ~kTouched;
+                if (((c & kOddBit) != 0) == (player == 1)) {
+                    // the first best successor, the present one counting first (as k_solve)
+                    const int32_t e0 = off[v], e1 = off[v + 1], cur0 = (c >> 3) - 1;
+                    int32_t cur = cur0, kc = cur0 >= 0 ? key[cur0] : 0;
+                    bool tie = false;
+                    constexpr int kAt = 4;
+                    for (int32_t eb = e0; eb < e1; eb += kAt) {
+                        int32_t us[kAt], ks[kAt];
+#pragma unroll
+                        for (int j = 0; j < kAt; j++) us[j] = tgt[min(eb + j, e1 - 1)];   // (the last one again: no tie)
+#pragma unroll
+                        for (int j = 0; j < kAt; j++) ks[j] = key[us[j]];
+#pragma unroll
+                        for (int j = 0; j < kAt; j++) {
+                            if ((player == 0) ? ks[j] > kc : ks[j] < kc) {
+                                cur = us[j];
+                                kc = ks[j];
+                                tie = false;
+                            } else if (ks[j] == kc && us[j] != cur) {
+                                tie = true;
+                            }
+                        }
+                    }
+                    if (tie && !key_infinite(kc)) {
+                        const bool settled = cur == cur0 && !(c & kSolved) && !(r.w & newbit);
+                        int32_t loads = 0;
+                        bool after = cur == cur0;
+                        for (int32_t e = e0; e < e1; e++) {
+                            const int32_t u = tgt[e];
+                            if (!after) {
+                                after = u == cur;
+                                continue;
+                            }
+                            if (u == cur || key[u] != kc) continue;
+                            if (settled && cur == cur0 && !(in[u].w & newbit)) continue;
+                            const int x = compare_tied(in, path, nullptr, u, cur, loads, INT_MAX, &a.sync->err);
+                            if ((player == 0) ? x > 0 : x < 0) cur = u;
+                        }
+                    }
+                    if (cur != cur0) {
+                        moved = true;
+                        c = (cur + 1) * 8 + (c & 7);
+                    }
+                }
+                choice[v] = c;
+            }
+            go = __syncthreads_or(moved);
+            if (go || player == 0) break;
+        }
+        // the loop's control, as k_ctl_even (solver_graph.cu)
+        if (__syncthreads_or(tid == 0 && *(volatile uint32_t *)&a.sync->err != 0)) {
+            stop = GraphCtl::kDeviceError;
+        } else if (player == 0) {
+            iters++;
+            if (!go) stop = GraphCtl::kConverged;
+        }
+        if (stop == GraphCtl::kRunning && a.max_evals > 0 && brs >= a.max_evals) stop = GraphCtl::kEvalCap;
+        if (stop == GraphCtl::kRunning && brs >= a.guard) stop = GraphCtl::kRunaway;
+        if (stop == GraphCtl::kRunning && player == 0 && a.reset)   // cpu_parity.cpp:300-307
+            for (int32_t v = tid; v < n; v += nth) {
+                const int32_t c = choice[v];
+                if (c & kOddBit) choice[v] = (tgt[off[v]] + 1) * 8 + (c & 7);
+            }
+    }
+
+    for (int32_t v = tid; v < n; v += nth) {   // as k_solve leaves it
+        const int4 r = in[v];
+        const int2 q = path[v];
+        const int32_t c = choice[v];
+        const bool fin = r.x == kSink;
+        a.strat[v] = (c >> 3) - 1;
+        a.solved[v] = c & kSolved;
+        a.key[v] = key[v];
+        if (!fin && !(c & kSolved)) a.ulist[atomicAdd(a.ucount, 1)] = v;
+        a.st[v] = fin ? r.w & kLen : (r.x == kPosInf ? ST_POS_INF : ST_NEG_INF);
+        a.skip[v] = make_int4(SKIP_UNKNOWN, 0, 0, 0);
+        *reinterpret_cast<int4 *>(&a.node[v]) =
+            fin ? make_int4(q.x, q.y, r.y, path_word(r.w & kLen, r.z))
+                : make_int4(q.x, q.y, r.x == kPosInf ? RM_POS_INF : RM_NEG_INF, 0);
+    }
+    if (tid == 0) {
+        a.ctl->iters = iters;
+        a.ctl->brs = brs;
+        a.ctl->stop = stop;
+        a.ctl->mfrom[0] = a.ctl->mfrom[1] = 0;
+        *a.err = *(volatile uint32_t *)&a.sync->err;
+        a.sync->err = 0;
+    }
+}
+
 std::atomic<int> g_sms[kMaxCachedDevices];
 
 }  // namespace
@@ -457,23 +682,29 @@ int64_t solve_capacity() { return (int64_t)kMaxWaves * kSolveThreads * device_sm
 int launch_solve(cudaStream_t s, const SolveArgs &a)
 {
     const int sms = device_sms();
+    if (a.n < kSmall) {
+        const SmallLayout l = small_layout(a.n, a.m);
+        int threads = 64;
+        while (threads < a.n && threads < kSolveThreads) threads *= 2;
+        cudaError_t e = cudaFuncSetAttribute(k_solve_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallBytes);
+        if (e != cudaSuccess) return (int)e;
+        count_launch();
+        k_solve_small<<<1, threads, l.total, s>>>(a);
+        return (int)cudaGetLastError();
+    }
     // the vertices spread over all SMs, at least kMinThreads per block (n = 10^4:
-    // 0.63 ms per solve in ten blocks of 1,024, 0.53 ms in 79 of 128; one block
-    // up to kOneBlock vertices, where block barriers are worth more)
+    // 0.63 ms per solve in ten blocks of 1,024, 0.53 ms in 79 of 128)
     int threads = kSolveThreads;
     while (threads > kMinThreads && ceil_div(a.n, threads / 2) <= sms) threads /= 2;
     const int64_t need = ceil_div(a.n, threads);
-    const int grid = a.n <= kOneBlock ? 1 : (int)(need < sms ? need : sms);
-    if (grid == 1) threads = kSolveThreads;
+    const int grid = (int)(need < sms ? need : sms);
     const int64_t waves = ceil_div(a.n, (int64_t)grid * threads);
     const size_t smem = 4 * (size_t)kWords * threads * (size_t)(waves < kMaxCached ? waves : kMaxCached);
-    const void *kernel = grid == 1 ? (const void *)k_solve<false> : (const void *)k_solve<true>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBytes);
+    cudaError_t e = cudaFuncSetAttribute(k_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedBytes);
     if (e != cudaSuccess) return (int)e;
     void *args[] = {(void *)&a};
     count_launch();
-    if (grid == 1) return (int)cudaLaunchKernel(kernel, dim3(1), dim3(threads), args, smem, s);
-    return (int)cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(threads), args, smem, s);
+    return (int)cudaLaunchCooperativeKernel((const void *)k_solve, dim3(grid), dim3(threads), args, smem, s);
 }
 
 }  // namespace psi

@@ -276,6 +276,7 @@ int Solver::run_fused(bool reset, int64_t max_evals, GraphCtl *out)
     SolveArgs a;
     a.n = n_;
     a.n_even = np0_;
+    a.m = m_;
     a.owner = owner_;
     a.pri = pri_;
     a.off = off_;

@@ -1,6 +1,7 @@
 """psi_solve as one persistent kernel (solve_kernels.cu) at the sizes where
-its launch or its phases change: one block up to 1,024 vertices, blocks of 128
-threads and more above, two vertices per thread past 155,648 (152 SMs), more
+its launch or its phases change: one block with everything in shared memory
+below 2,000 vertices (its successors too, where they fit), blocks of 128 threads
+and more above, two vertices per thread past 155,648 (152 SMs), more
 than the five kept in shared memory past 778,240; jumps over deep chains and
 long cycles; and the state it leaves for the step-by-step calls."""
 import numpy as np
@@ -25,7 +26,7 @@ def _same(a, b):
         assert np.array_equal(x, y), f"output {k}: differ at {np.nonzero(x != y)[0][:10]}"
 
 
-GAMES = [("ring10", 10, 0)]
+GAMES = [("ring10", 10, 0), ("c4", 1999, 1), ("c4", 2000, 2), ("c3", 1999, 3)]
 GAMES += [("c4", n, n) for n in (20, 127, 128, 129, 1023, 1024, 1025, 2049, 19456, 19457)]
 GAMES += [("smallpri", n, n) for n in (64, 1024, 1025, 30000)]
 GAMES += [("c3", n, n) for n in (50, 1025, 20000)]
@@ -44,6 +45,25 @@ def test_solve_matches_the_oracle(fam, n, seed, reset):
         assert np.array_equal(s.get_strategy(), ref.get_strategy())
         assert np.array_equal(s.get_infinite(), ref.get_infinite())
         assert np.array_equal(s.get_winning(0), ref.get_winning(0))
+    s.close()
+    ref.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,deg", [(1, 0), (2, 1), (65, 64), (1500, 40), (1999, 45)])
+def test_small_games_of_any_degree(n, deg):
+    """Up to 1,999 vertices with few or many successors (past what shared
+    memory holds), self-loops and repeated successors among them."""
+    rng = np.random.default_rng(n)
+    size = rng.integers(1, deg + 2, n)
+    off = np.concatenate(([0], np.cumsum(size))).astype(np.int32)
+    g = psi.Game.from_csr(rng.integers(0, 2, n), rng.integers(0, 30, n), off, rng.integers(0, n, off[-1]))
+    ref = oracle.Sparse(*g.csr())
+    s = psi.GPUList(g)
+    for reset in (False, True):
+        assert s.solve(reset=reset) == ref.solve(reset=reset)
+        assert np.array_equal(s.get_strategy(), ref.get_strategy())
+        assert np.array_equal(s.get_infinite(), ref.get_infinite())
     s.close()
     ref.close()
 
