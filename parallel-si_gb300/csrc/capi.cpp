@@ -250,12 +250,8 @@ int psi_get_winning(psi_solver *s, int32_t player, int32_t *out, int64_t cap, in
     if (!s || !s->s) return psi::fail(PSI_ERR_INVALID, "null solver");
     PSI_GUARD_BEGIN
     int64_t total = 0;
-    int rc = s->s->winning_ids(player, &total);
+    int rc = s->s->get_winning(player, out, cap, &total);
     if (rc) return rc;
-    if (out && cap > 0) {
-        rc = s->s->copy_winning(out, total < cap ? total : cap);
-        if (rc) return rc;
-    }
     if (count) *count = total;
     return PSI_OK;
     PSI_GUARD_END
@@ -497,17 +493,9 @@ int psi_batch_get_winning(psi_batch *b, int32_t game, int32_t player, int32_t *o
     if (rc) return rc;
     if (player != 0 && player != 1) return psi::fail(PSI_ERR_INVALID, "player must be 0 or 1");
     PSI_GUARD_BEGIN
-    std::vector<int32_t> inf((size_t)n);
-    rc = b->s->get_infinite_range(v0, n, inf.data());
-    if (rc) return rc;
     int64_t k = 0;
-    for (int64_t i = 0; i < n; i++) {
-        bool w0 = inf[i] == 1;
-        if ((player == 0 && w0) || (player == 1 && !w0)) {
-            if (out && k < cap) out[k] = (int32_t)i;
-            k++;
-        }
-    }
+    rc = b->s->get_winning_range(v0, n, player, out, cap, &k);
+    if (rc) return rc;
     if (count) *count = k;
     return PSI_OK;
     PSI_GUARD_END

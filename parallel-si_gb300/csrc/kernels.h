@@ -114,8 +114,13 @@ void launch_narrow_owner(cudaStream_t s, int32_t n, const int32_t *in, int8_t *o
 // order); *n_even (device) = Even's count.  Returns a cudaError_t value.
 int partition_players(cudaStream_t s, int32_t n, const int8_t *owner, int32_t *plist, int32_t *n_even);
 // Winning set of `player` from the status words, in increasing vertex order
-// (out: up to n ids; *count on the device).  Returns a cudaError_t value.
-int select_winning(cudaStream_t s, int32_t n, int32_t player, const int32_t *st, int32_t *out, int32_t *count);
+// (out: up to n ids; *count on the device).  tmp: workspace of *bytes bytes;
+// nullptr: only *bytes is set.  Returns a cudaError_t value.
+int select_winning(cudaStream_t s, int32_t n, int32_t player, const int32_t *st, int32_t *out, int32_t *count,
+                   void *tmp, size_t *bytes);
+// The same for small games, in one block.
+constexpr int32_t kSelectSmall = 16384;
+void launch_select_small(cudaStream_t s, int32_t n, int32_t player, const int32_t *st, int32_t *out, int32_t *count);
 
 // ---- strategy set-up (gpu_parity.cu:38-56, cpu_parity.cpp:276-286, 300-307)
 void launch_init_strat(cudaStream_t s, int32_t n, const int8_t *owner, const int32_t *off,

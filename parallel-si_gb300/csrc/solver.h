@@ -75,15 +75,14 @@ public:
     // count: *switched is the number of strict improvements; otherwise only
     // whether it is zero matters (launch_switch's count_moves).
     int switch_strategy(int32_t player, int64_t *switched, bool count = true);
-    int get_winning(int32_t player, std::vector<int32_t> &out);
-    // Device-side selection of the winning set, then a copy of its first k ids.
-    int winning_ids(int32_t player, int64_t *count);
-    int copy_winning(int32_t *out, int64_t k);
+    // The winning set of `player`: at most cap ids to out, *count its size.
+    int get_winning(int32_t player, int32_t *out, int64_t cap, int64_t *count);
+    // The same of the vertices [v0, v0 + n) alone (a batch's game), as ids from v0 on.
+    int get_winning_range(int64_t v0, int64_t n, int32_t player, int32_t *out, int64_t cap, int64_t *count);
     int reset_opponent_strategy();
 
     int get_strategy(int32_t *out);
     int get_strategy_range(int64_t v0, int64_t count, int32_t *out);
-    int get_infinite_range(int64_t v0, int64_t count, int32_t *out);
     int set_strategy(const int32_t *in);
     int get_infinite(int32_t *out);
     int get_solved(int32_t *out);
@@ -163,6 +162,20 @@ private:
     ChangeList changes() const { return clist_ ? ChangeList{clist_, &ctl_->ccount, ccap_} : ChangeList(); }
     int build_graph(bool reset);
     int get_range(const int32_t *src, int64_t v0, int64_t count, int32_t *out);
+    // Device memory to the caller's, complete on return.  Small copies into
+    // pageable memory go through stage_: the driver's own path for them took
+    // 30 to 80 us, this one 12.
+    int copy_out(void *dst, const void *src, size_t bytes);
+    // Page-locked memory of at least `bytes` (at most kStageBytes): a part of
+    // hw_'s allocation up to small_stage_, else one of its own, made when first
+    // wanted.
+    int stage(size_t bytes, void **out);
+    int stage_in(const void *src, size_t bytes, const void **out);   // device memory there, complete on return
+    static constexpr size_t kStageBytes = 1 << 20;
+    size_t small_stage_ = 0;
+    void *stage_ = nullptr;
+    void *select_tmp_ = nullptr;       // workspace of the winning-set selection
+    size_t select_bytes_ = 0;
     int set_device();
 
     int device_ = 0;
@@ -235,7 +248,12 @@ private:
         int32_t cnt[3];             // list counters (EvalArgs, launch_switch)
         uint32_t claim;             // the switch kernel's work counter (launch_switch)
     };
-    Words *dw_ = nullptr, *hw_ = nullptr;
+    Words *dw_ = nullptr, *hw_ = nullptr;   // ctl_ follows dw_ on the device, hctl_ follows hw_
+    struct AllWords {
+        Words w;
+        GraphCtl ctl;
+    };
+    GraphCtl *hctl_ = nullptr;
     // graph-driven solve loop (solver_graph.cu)
     int run_graph(bool reset, int64_t max_evals, GraphCtl *out, int4 *gstate_out);
     int solve_batch_graph(std::vector<int4> &state);

@@ -228,13 +228,13 @@ int Solver::run_graph(bool reset, int64_t max_evals, GraphCtl *out, int4 *gstate
     init.inject_bits = inject_bits_;
     PSI_CUDA_TRY(cudaMemcpyAsync(ctl_, &init, sizeof init, cudaMemcpyHostToDevice, stream_));
     PSI_CUDA_TRY(cudaGraphLaunch(graph_exec_, stream_));
-    PSI_CUDA_TRY(cudaMemcpyAsync(out, ctl_, sizeof *out, cudaMemcpyDeviceToHost, stream_));
     if (gstate_out)
         PSI_CUDA_TRY(cudaMemcpyAsync(gstate_out, gstate_, sizeof(int4) * (size_t)games_, cudaMemcpyDeviceToHost,
                                      stream_));
     // the counts of the passes that ran are kept even when a pass failed
     rc = sync_and_check("solve (graph)");
     if (rc && rc != PSI_ERR_LIMIT) return rc;
+    *out = *hctl_;
     // every pass launches each kernel of the body once, those of the full
     // evaluation only when it is not a patch
     const long long patched = (long long)(hw_->patch[0] - patches_before);
@@ -305,9 +305,9 @@ int Solver::run_fused(bool reset, int64_t max_evals, GraphCtl *out)
     a.inject_bits = inject_bits_;
     int ce = launch_solve(stream_, a);
     if (ce) return fail(PSI_ERR_CUDA, std::string("solve kernel: ") + cudaGetErrorString((cudaError_t)ce));
-    PSI_CUDA_TRY(cudaMemcpyAsync(out, ctl_, sizeof *out, cudaMemcpyDeviceToHost, stream_));
     rc = sync_and_check("solve (kernel)");
     if (rc && rc != PSI_ERR_LIMIT) return rc;
+    *out = *hctl_;
     times_.evals += out->brs;
     times_.switches += out->brs + out->iters;
     strat_ready_ = true;
