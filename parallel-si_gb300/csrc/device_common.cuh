@@ -366,6 +366,79 @@ __device__ __forceinline__ void note_change(const ChangeList &c, int32_t v)
     if (p < c.cap) c.list[p] = v;
 }
 
+// Before an evaluation (one thread): decides between a patch and the full
+// evaluation (patch_kernels.cu) and resets what either starts from.
+__device__ __forceinline__ void patch_begin(const PatchArgs &a)
+{
+    EvalGates *g = a.g;
+    ++*a.epoch;
+    if (*a.quiet > 0) --*a.quiet;
+    const int32_t cc = g->ccount;
+    g->ccount = 0;   // the next switch steps list their changes afresh
+    g->csnap = cc;
+    g->acount = 0;
+    g->lcnt[0] = g->lcnt[1] = g->lcnt[2] = 0;
+    bool ok = g->try_patch && cc <= a.ccap && (int64_t)*a.ucount + a.acap <= a.ucap;
+    if (ok && g->skip > 0) {
+        g->skip--;
+        ok = false;
+    }
+    g->patch = ok ? 1 : 0;
+    g->eval = ok ? 0 : 1;
+    if (!ok) {
+        *a.ucount = 0;      // the full evaluation collects the unreached vertices afresh
+        g->mfrom[0] = g->mfrom[1] = 0;
+    }
+}
+
+// One event of a batch's per-game accounting (switch_kernels.cu says what
+// state and events are).
+__device__ __forceinline__ void batch_event(int32_t event, int4 &state, unsigned long long &gcount)
+{
+    int4 s = state;
+    if (event == 0) {
+        if (!s.w && !s.z) s.x++;
+    } else if (event == 1) {
+        if (!s.w && !s.z && gcount == 0) s.z = 1;
+        gcount = 0;
+    } else if (event == 2) {
+        if (!s.w) s.y++;
+    } else {
+        if (!s.w) {
+            if (gcount == 0) s.w = 1;
+            else s.z = 0;
+        }
+        gcount = 0;
+    }
+    state = s;
+}
+
+// mark_solved restricted to the last evaluation's unreached vertices: every
+// other non-solved vertex is finite.  Every thread of the grid calls it.
+// With game_of/gmask (served games), only vertices of games whose mask is set.
+__device__ __forceinline__ void mark_solved_pass(const MarkArgs &m)
+{
+    const int32_t nu = *m.ucount;
+    const int32_t i0 = m.from ? *m.from : 0;
+    const int32_t target = (m.player == 0) ? ST_POS_INF : ST_NEG_INF;
+    for (int64_t i = i0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nu; i += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t u = m.ulist[i];
+        if (m.gmask) {
+            const int32_t g = m.game_of[u];
+            if (g < 0 || !m.gmask[g]) continue;
+        }
+        if (m.st[u] == target) m.solved[u] = 1;
+    }
+    if (!m.from) return;
+    // the last block to finish (every block has read *from by then) moves
+    // the start past the entries scanned
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicInc(m.done, gridDim.x - 1) == gridDim.x - 1) *m.from = nu;
+    }
+}
+
 // Tour node ids (an Euler tour of the strategy forest, two nodes per vertex):
 // node 2v is v's "down" node (leaving v's subtree toward the sink), 2v+1 its
 // "up" node (entering it); 2n / 2n+1 are the sink's down / up nodes.  The list

@@ -484,42 +484,7 @@ __global__ void __launch_bounds__(kCycleBlock, kCycleMinBlocks) k_cycles(const i
     cycles_body<true>(nu, ulist, strat, pri, solved, st, key, ja, jb, la, lb, cnt, err, track);
 }
 
-// mark_solved restricted to the last evaluation's unreached vertices: every
-// other non-solved vertex is finite.
-// With game_of/gmask (served games), only vertices of games whose mask is set.
-__global__ void k_mark_solved(const int32_t *__restrict__ ucount, const int32_t *__restrict__ ulist,
-                              int32_t player, const int32_t *__restrict__ st, uint8_t *__restrict__ solved,
-                              const int32_t *__restrict__ game_of,
-                              const int32_t *__restrict__ gmask, const int32_t *__restrict__ gate,
-                              int32_t *__restrict__ from, uint32_t *__restrict__ done)
-{
-    if (gate && !*gate) return;
-    const int32_t nu = *ucount;
-    const int32_t i0 = from ? *from : 0;
-    const int32_t target = (player == 0) ? ST_POS_INF : ST_NEG_INF;
-    for (int32_t i = i0 + blockIdx.x * blockDim.x + threadIdx.x; i < nu; i += gridDim.x * blockDim.x) {
-        int32_t u = ulist[i];
-        if (gmask) {
-            int32_t g = game_of[u];
-            if (g < 0 || !gmask[g]) continue;
-        }
-        if (st[u] == target) solved[u] = 1;
-    }
-    if (!from) return;
-    // the last block to finish (every block has read *from by then) moves
-    // the start past the entries scanned
-    __shared__ bool last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        last = atomicAdd(done, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (last && threadIdx.x == 0) {
-        *from = nu;
-        *done = 0;
-    }
-}
+__global__ void k_mark_solved(MarkArgs m) { mark_solved_pass(m); }
 
 // Grid for the grid-stride kernels: enough blocks to fill the device a few
 // times over, not one block per 256 items (a kernel whose gate is closed then
@@ -644,13 +609,10 @@ int launch_cycles(cudaStream_t s, const int32_t *ucount, const int32_t *ulist, c
     return e == cudaSuccess ? 0 : (int)e;
 }
 
-void launch_mark_solved(cudaStream_t s, const int32_t *ucount, const int32_t *ulist, int32_t player,
-                        const int32_t *st, uint8_t *solved, const int32_t *game_of,
-                        const int32_t *gmask, const int32_t *gate, int32_t *from, uint32_t *done)
+void launch_mark_solved(cudaStream_t s, const MarkArgs &m)
 {
     count_launch();
-    k_mark_solved<<<608, kBlock, 0, s>>>(ucount, ulist, player, st, solved, game_of, gmask, gate, from,
-                                         done);
+    k_mark_solved<<<608, kBlock, 0, s>>>(m);
 }
 
 }  // namespace psi

@@ -19,7 +19,8 @@ struct GraphCtl;   // solver.h
 // successors' keys, except where equal keys tie at the best one, and such a
 // vertex keeps need = 1 (switch_kernels.cu).  need == nullptr: no tracking.
 // quiet (a device word, optional): while nonzero every need flag is already
-// set, and changed keys flag nothing (the first evaluation after a reset).
+// set, and changed keys flag nothing (the first evaluation after a reset sets
+// it to 2: launch_patch_begin counts it down).
 // tie (optional): vertices whose last switch examination rested on a walk
 // (equal keys at their best successor).  Such a vertex needs another look
 // when the exact value of a successor may have changed: after every full
@@ -220,18 +221,25 @@ int launch_cycles(cudaStream_t s, const int32_t *ucount, const int32_t *ulist, c
 // are scanned, and *from moves to the list's end: the entries before it were
 // scanned by this player's last mark_solved, and a vertex whose status has
 // changed since was appended again by a patch (EvalGates::mfrom).
-void launch_mark_solved(cudaStream_t s, const int32_t *ucount, const int32_t *ulist, int32_t player,
-                        const int32_t *st, uint8_t *solved, const int32_t *game_of = nullptr,
-                        const int32_t *gmask = nullptr, const int32_t *gate = nullptr,
-                        int32_t *from = nullptr, uint32_t *done = nullptr);
+struct MarkArgs {
+    const int32_t *ucount = nullptr, *ulist = nullptr;
+    int32_t player = 0;
+    const int32_t *st = nullptr;
+    uint8_t *solved = nullptr;
+    const int32_t *game_of = nullptr, *gmask = nullptr;
+    int32_t *from = nullptr;
+    uint32_t *done = nullptr;
+};
+void launch_mark_solved(cudaStream_t s, const MarkArgs &m);
 
 // ---- all-switches (gpu_parity.cu:191-317, cpu_parity.cpp:154-263)
 // Switches the np vertices listed in plist (all owned by `player`).
 // stats[0..3] += compared edges, walk loads, changed vertices, strict
 // improvements (those only with count_moves; otherwise one per changed vertex,
 // for fewer comparisons); with game_of (batches) also gcount[game] += them,
-// and with gmask only vertices of games whose mask is set switch.  With need
-// (and list: n entries, list_count: one counter) only the vertices of plist
+// and with gmask only vertices of games whose mask is set switch.  stats is
+// cleared first.  With need (and list: n entries, list_count: a counter that
+// is zero between calls, list_done: another) only the vertices of plist
 // whose need flag is set are examined (ChangeTrack); examined vertices get
 // need = 0, or 1 when a tie at their best successor leaves their choice to a
 // walk that a later evaluation may decide differently.  With changes.list,
@@ -239,7 +247,8 @@ void launch_mark_solved(cudaStream_t s, const int32_t *ucount, const int32_t *ul
 // word) and the need list, the thread kernel deals the list out to warps in
 // chunks through that counter instead of a fixed grid stride.  With owner
 // (and no gmask), the need list is collected from the n_all vertices' need
-// and owner bytes rather than through plist.
+// and owner bytes rather than through plist.  mark: a mark_solved done on the
+// way (the two touch different words).
 void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t player,
                    const int32_t *off, const int32_t *tgt, int32_t *strat, const int32_t *st,
                    const int32_t *key, const PathNode *node, const int32_t *rdeep,
@@ -249,12 +258,11 @@ void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t pla
                    int32_t *list_count = nullptr, ChangeList changes = ChangeList(), uint8_t *tie = nullptr,
                    uint8_t *watch = nullptr, const int4 *skip = nullptr, bool warp = false,
                    uint32_t *claim = nullptr, const int8_t *owner = nullptr, int32_t n_all = 0,
-                   bool count_moves = true);
+                   bool count_moves = true, uint32_t *list_done = nullptr, const MarkArgs *mark = nullptr);
 // ---- batches: per-game accounting of solve_si (state[g] = brs, iters,
 // odd_done, done; gcount[g] = strict improvements of the last switch step);
-// with gate, only when *gate is set
-void launch_batch_account(cudaStream_t s, int32_t games, int32_t event, int4 *state,
-                          unsigned long long *gcount, const int32_t *gate = nullptr);
+// the graph loop does the same in its control kernels
+void launch_batch_account(cudaStream_t s, int32_t games, int32_t event, int4 *state, unsigned long long *gcount);
 // ---- serving arena (serve_kernels.cu)
 // Places the games of one admission, uploaded as a packed union (game k owns
 // union vertices [ub[k], ub[k+1]); u_roff/u_rsrc: the union's reverse CSR), at
@@ -279,7 +287,7 @@ void launch_arena_clear(cudaStream_t s, int32_t vb, int32_t count, uint8_t *solv
 // Appends the vertices of `player` that belong to a game to plist (*count += k).
 void launch_build_plist(cudaStream_t s, int32_t n, int32_t player, const int8_t *owner, const int32_t *game_of,
                         int32_t *plist, int32_t *count);
-// Per-slot solve_si state machine: event 0 after an evaluation, 1 after
+// Per-slot solve_si state machine: event 1 after an evaluation and
 // switch(Odd), 2 after switch(Even) (see serve_kernels.cu).
 void launch_serve_account(cudaStream_t s, int32_t slots, int32_t event, int4 *state, unsigned long long *gcount,
                           int32_t *gmask);
@@ -319,11 +327,11 @@ struct PatchArgs {
     ChangeTrack track;
     int4 *skip = nullptr;       // landmark skips: a patched vertex's record becomes unknown
     uint32_t *epoch = nullptr;
+    int32_t *quiet = nullptr;
 };
-// Sets the gates the host decides before an evaluation (one thread).
-void launch_eval_gates(cudaStream_t s, EvalGates *g, int32_t try_patch);
 // One thread: decides between a patch and the full evaluation (gates).
-void launch_patch_begin(cudaStream_t s, const PatchArgs &a);
+// try_patch: whether the caller allows one; -1: as g->try_patch says.
+void launch_patch_begin(cudaStream_t s, const PatchArgs &a, int32_t try_patch);
 // Cooperative launches, gated on g->patch; return a cudaError_t value.
 int launch_patch_collect(cudaStream_t s, const PatchArgs &a);
 int launch_patch_values(cudaStream_t s, const PatchArgs &a);

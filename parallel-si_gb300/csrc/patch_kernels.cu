@@ -12,7 +12,7 @@
 // follow such a step: in Odd's best-response loop the number of changed
 // strategies falls by about an order of magnitude per step.
 //
-//  1. k_patch_begin (one thread) takes the changed vertices the switch steps
+//  1. patch_begin (one thread; a launch, or part of the graph loop's control) takes the changed vertices the switch steps
 //     listed since the last evaluation and opens either the patch's gate or
 //     the full evaluation's: a patch needs the list complete, the caller's
 //     permission (the list covers every change since the last
@@ -75,31 +75,10 @@ __device__ __forceinline__ int ceil_log2_i(int64_t x)
     return r;
 }
 
-__global__ void k_eval_gates(EvalGates *g, int32_t try_patch) { g->try_patch = try_patch; }
-
-__global__ void k_patch_begin(PatchArgs a)
+__global__ void k_patch_begin(PatchArgs a, int32_t try_patch)
 {
-    EvalGates *g = a.g;
-    ++*a.epoch;
-    const int32_t cc = g->ccount;
-    g->ccount = 0;   // the next switch steps list their changes afresh
-    g->csnap = cc;
-    g->acount = 0;
-    g->lcnt[0] = g->lcnt[1] = g->lcnt[2] = 0;
-    bool ok = g->try_patch && cc <= a.ccap && (int64_t)*a.ucount + a.acap <= a.ucap;
-    if (ok && g->skip > 0) {
-        g->skip--;
-        ok = false;
-    }
-    if (ok) {
-        g->eval = 0;
-        g->patch = 1;
-    } else {
-        g->eval = 1;
-        g->patch = 0;
-        *a.ucount = 0;      // the full evaluation collects the unreached vertices afresh
-        g->mfrom[0] = g->mfrom[1] = 0;
-    }
+    if (try_patch >= 0) a.g->try_patch = try_patch;
+    patch_begin(a);
 }
 
 // Warp-collective: the in-edges of the lanes' vertices x (valid ones, at
@@ -440,16 +419,10 @@ std::atomic<int> g_collect_blocks[kMaxCachedDevices], g_values_blocks[kMaxCached
 
 }  // namespace
 
-void launch_eval_gates(cudaStream_t s, EvalGates *g, int32_t try_patch)
+void launch_patch_begin(cudaStream_t s, const PatchArgs &a, int32_t try_patch)
 {
     count_launch();
-    k_eval_gates<<<1, 1, 0, s>>>(g, try_patch);
-}
-
-void launch_patch_begin(cudaStream_t s, const PatchArgs &a)
-{
-    count_launch();
-    k_patch_begin<<<1, 1, 0, s>>>(a);
+    k_patch_begin<<<1, 1, 0, s>>>(a, try_patch);
 }
 
 int launch_patch_collect(cudaStream_t s, const PatchArgs &a)

@@ -164,9 +164,10 @@ __global__ void k_build_plist(int32_t n, int32_t player, const int8_t *__restric
 // Per-slot solve_si state machine (main.cpp:20-55), one step of every
 // resident game per call sequence.  state[s] = (evaluations, iterations,
 // flags, 0) with flags bit 0 = resident, bit 1 = done.  A step is:
-//   evaluation                     -> event 0: evaluations++ (resident, not done)
-//   mark_solved(Odd), switch(Odd)  -> event 1: a game whose Odd made no strict
-//                                     improvement takes its Even step now: gmask[s] = 1
+//   evaluation, mark_solved(Odd), switch(Odd)
+//                                  -> event 1: evaluations++ (resident, not done); a game whose
+//                                     Odd made no strict improvement takes its Even step
+//                                     now: gmask[s] = 1
 //   mark_solved(Even), switch(Even) for games with gmask set
 //                                  -> event 2: iterations++; no Even improvement = done
 // which is exactly the solo sequence of each game (its switch(Odd) returning 0
@@ -178,9 +179,8 @@ __global__ void k_serve_account(int32_t slots, int32_t event, int4 *__restrict__
     if (s >= slots) return;
     int4 x = state[s];
     bool live = (x.z & 1) && !(x.z & 2);
-    if (event == 0) {
+    if (event == 1) {
         if (live) x.x++;
-    } else if (event == 1) {
         gmask[s] = (live && gcount[s] == 0) ? 1 : 0;
         gcount[s] = 0;
     } else {

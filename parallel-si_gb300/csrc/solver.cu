@@ -420,12 +420,12 @@ void Solver::reset_times()
 
 void Solver::reset_tracking()
 {
-    static const int32_t one = 1;
+    static const int32_t two = 2;   // patch_begin counts it down: nonzero in the next evaluation alone
     stale_ = false;
     cudaMemsetAsync(need_, 1, (size_t)n_, stream_);
     cudaMemsetAsync(tie_, 0, (size_t)n_, stream_);
     cudaMemsetAsync(watch_, 0, (size_t)n_, stream_);
-    cudaMemcpyAsync(&ctl_->quiet, &one, sizeof one, cudaMemcpyHostToDevice, stream_);
+    cudaMemcpyAsync(&ctl_->quiet, &two, sizeof two, cudaMemcpyHostToDevice, stream_);
 }
 
 // The same when a switch step may come before the next evaluation, which
@@ -493,25 +493,24 @@ PatchArgs Solver::patch_args()
     a.track = track();
     a.skip = skip_;
     a.epoch = &sync_->epoch;
+    a.quiet = &ctl_->quiet;
     return a;
 }
 
-int Solver::enqueue_eval(bool timed)
+int Solver::enqueue_eval(bool timed, int32_t try_patch)
 {
-    int rc = enqueue_patch(timed);
+    int rc = enqueue_patch(timed, try_patch);
     if (!rc) rc = enqueue_full(timed);
-    if (rc) return rc;
-    PSI_CUDA_TRY(cudaMemsetAsync(&ctl_->quiet, 0, sizeof(int32_t), stream_));
-    return PSI_OK;
+    return rc;
 }
 
 // 0. a patch, when the gates allow it and it succeeds; otherwise its
 //    kernels return at once and the full evaluation's gates are open
-int Solver::enqueue_patch(bool timed)
+int Solver::enqueue_patch(bool timed, int32_t try_patch)
 {
     if (timed) phase_begin(PH_PATCH);
     const PatchArgs pa = patch_args();
-    launch_patch_begin(stream_, pa);
+    if (timed) launch_patch_begin(stream_, pa, try_patch);   // (the graph loop's control has done so)
     if (incremental_ != PSI_INCR_OFF) {
         int pe = launch_patch_collect(stream_, pa);
         if (!pe) pe = launch_patch_values(stream_, pa);
@@ -571,10 +570,10 @@ int Solver::compute_valuation()
     refresh_tracking();
     // the last evaluation's state and the switch steps' change list since are
     // usable only if no strategy changed outside a switch step
-    launch_eval_gates(stream_, ctl_, (tracked_ && incremental_ != PSI_INCR_OFF) ? 1 : 0);
+    const int32_t try_patch = (tracked_ && incremental_ != PSI_INCR_OFF) ? 1 : 0;
     const unsigned long long patches_before = hw_->patch[0];
     phase_begin(PH_EVAL);
-    rc = enqueue_eval(true);
+    rc = enqueue_eval(true, try_patch);
     if (rc) return rc;
     phase_end(PH_EVAL);
     rc = sync_and_check("compute_valuation");
@@ -597,28 +596,45 @@ int Solver::mark_solved(int32_t player)
     if (!val_ready_) return fail(PSI_ERR_STATE, "mark_solved before compute_valuation");
     int rc = set_device();
     if (rc) return rc;
-    // a masked step (served games) scans the whole list
-    launch_mark_solved(stream_, &dw_->ucount, ulist_, player, st_, solved_, gmask_ ? game_of_ : nullptr,
-                       gmask_, nullptr, gmask_ ? nullptr : &ctl_->mfrom[player], &ctl_->mdone);
+    launch_mark_solved(stream_, mark_args(player));
     PSI_CUDA_TRY(cudaGetLastError());
     return PSI_OK;   // ordered on the stream before the next call
 }
 
-int Solver::switch_strategy(int32_t player, int64_t *switched, bool count)
+MarkArgs Solver::mark_args(int32_t player)
+{
+    MarkArgs m;
+    m.ucount = &dw_->ucount;
+    m.ulist = ulist_;
+    m.player = player;
+    m.st = st_;
+    m.solved = solved_;
+    if (gmask_) {   // a masked step (served games) scans the whole list
+        m.game_of = game_of_;
+        m.gmask = gmask_;
+    } else {
+        m.from = &ctl_->mfrom[player];
+        m.done = &ctl_->mdone;
+    }
+    return m;
+}
+
+int Solver::switch_strategy(int32_t player, int64_t *switched, bool count, bool mark)
 {
     if (player != 0 && player != 1) return fail(PSI_ERR_INVALID, "player must be 0 or 1");
     if (!val_ready_) return fail(PSI_ERR_STATE, "switch_strategy before compute_valuation");
     int rc = set_device();
     if (rc) return rc;
     refresh_tracking();
-    PSI_CUDA_TRY(cudaMemsetAsync(dw_->sw, 0, sizeof(dw_->sw), stream_));
+    const MarkArgs m = mark ? mark_args(player) : MarkArgs();
     phase_begin(PH_SWITCH);
     const int32_t np = (player == 0) ? np0_ : np_ - np0_;
     const int32_t *pl = plist_ + (player == 0 ? 0 : np0_);
     // jB_ is free until the next full evaluation: it holds the list of vertices to examine
     launch_switch(stream_, np, pl, player, off_, tgt_, strat_, st_, key_, node_, rdeep_, dw_->sw, game_of_, gcount_,
-                  gmask_, &dw_->err, nullptr, need_, reinterpret_cast<int32_t *>(jB_), &dw_->cnt[2], changes(), tie_,
-                  watch_, skip_, switch_warp_, &dw_->claim, arena_ ? nullptr : owner_, n_, count);
+                  gmask_, &dw_->err, nullptr, need_, reinterpret_cast<int32_t *>(jB_), &dw_->listcount, changes(), tie_,
+                  watch_, skip_, switch_warp_, &dw_->claim, arena_ ? nullptr : owner_, n_, count,
+                  &dw_->listdone, mark ? &m : nullptr);
     phase_end(PH_SWITCH);
     rc = sync_and_check("switch_strategy");
     if (rc) return rc;
@@ -856,10 +872,8 @@ int Solver::solve(int32_t reset, int32_t *iters, int32_t *brs, int64_t max_evals
             rc = first ? compute_first_val() : compute_valuation();
             if (rc) return rc;
             br++;
-            rc = mark_solved(1);
-            if (rc) return rc;
             int64_t sw = 0;
-            rc = switch_strategy(1, &sw, false);
+            rc = switch_strategy(1, &sw, false, true);
             if (rc) return rc;
             if (sw == 0) break;
             if (max_evals > 0 && br >= max_evals) {
@@ -869,11 +883,9 @@ int Solver::solve(int32_t reset, int32_t *iters, int32_t *brs, int64_t max_evals
             }
         }
         first = false;
-        rc = mark_solved(0);
-        if (rc) return rc;
         it++;
         int64_t sw = 0;
-        rc = switch_strategy(0, &sw, false);
+        rc = switch_strategy(0, &sw, false, true);
         if (rc) return rc;
         if (sw == 0) break;
         if (max_evals > 0 && br >= max_evals) {
@@ -912,19 +924,15 @@ int Solver::solve_batch(int32_t *iters, int32_t *brs)
             rc = compute_valuation();
             if (rc) return rc;
             launch_batch_account(stream_, games_, 0, gstate_, gcount_);
-            rc = mark_solved(1);
-            if (rc) return rc;
             int64_t sw = 0;
-            rc = switch_strategy(1, &sw, false);
+            rc = switch_strategy(1, &sw, false, true);
             if (rc) return rc;
             launch_batch_account(stream_, games_, 1, gstate_, gcount_);
             if (sw == 0) break;
         }
-        rc = mark_solved(0);
-        if (rc) return rc;
         launch_batch_account(stream_, games_, 2, gstate_, gcount_);
         int64_t sw = 0;
-        rc = switch_strategy(0, &sw, false);
+        rc = switch_strategy(0, &sw, false, true);
         if (rc) return rc;
         launch_batch_account(stream_, games_, 3, gstate_, gcount_);
         if (sw == 0) break;
@@ -1122,17 +1130,14 @@ int Solver::arena_step(bool reset, std::vector<int32_t> &done, std::vector<int32
     if (n_ == 0 || np_ == 0) return PSI_OK;
     int rc = compute_valuation();
     if (rc) return rc;
-    launch_serve_account(stream_, games_, 0, gstate_, gcount_, gmask_);
     int32_t *mask = gmask_;
     gmask_ = nullptr;                       // Odd's step: every resident game
-    rc = mark_solved(1);
     int64_t sw = 0;
-    if (!rc) rc = switch_strategy(1, &sw, false);
+    rc = switch_strategy(1, &sw, false, true);
     gmask_ = mask;
     if (rc) return rc;
     launch_serve_account(stream_, games_, 1, gstate_, gcount_, gmask_);
-    rc = mark_solved(0);                    // Even's step: games with gmask set
-    if (!rc) rc = switch_strategy(0, &sw, false);
+    rc = switch_strategy(0, &sw, false, true);   // Even's step: games with gmask set
     if (rc) return rc;
     if (reset)
         launch_serve_reset_odd(stream_, np_ - np0_, plist_ + np0_, game_of_, gmask_, gcount_, off_, tgt_, strat_,

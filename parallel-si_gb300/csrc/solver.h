@@ -74,7 +74,8 @@ public:
     int mark_solved(int32_t player);
     // count: *switched is the number of strict improvements; otherwise only
     // whether it is zero matters (launch_switch's count_moves).
-    int switch_strategy(int32_t player, int64_t *switched, bool count = true);
+    // mark: mark_solved(player) first.
+    int switch_strategy(int32_t player, int64_t *switched, bool count = true, bool mark = false);
     // The winning set of `player`: at most cap ids to out, *count its size.
     int get_winning(int32_t player, int32_t *out, int64_t cap, int64_t *count);
     // The same of the vertices [v0, v0 + n) alone (a batch's game), as ids from v0 on.
@@ -154,10 +155,11 @@ private:
     // One evaluation on the stream, no synchronisation: the patch kernels and
     // the full evaluation's, each set gated (which ones work is decided on
     // the device, k_patch_begin).
-    int enqueue_eval(bool timed);
-    int enqueue_patch(bool timed);
+    int enqueue_eval(bool timed, int32_t try_patch);
+    int enqueue_patch(bool timed, int32_t try_patch);
     int enqueue_full(bool timed);
     PatchArgs patch_args();
+    MarkArgs mark_args(int32_t player);
     EvalArgs eval_args();
     ChangeList changes() const { return clist_ ? ChangeList{clist_, &ctl_->ccount, ccap_} : ChangeList(); }
     int build_graph(bool reset);
@@ -245,7 +247,9 @@ private:
         int32_t ucount;             // vertices the sink did not reach
         int32_t selcount;           // size of a selected list (players, winning set)
         int32_t lcount;             // walks cut short in the last full evaluation
-        int32_t cnt[3];             // list counters (EvalArgs, launch_switch)
+        int32_t cnt[3];             // list counters (EvalArgs)
+        int32_t listcount;          // the switch steps' list (launch_switch): zero between steps
+        uint32_t listdone;
         uint32_t claim;             // the switch kernel's work counter (launch_switch)
     };
     Words *dw_ = nullptr, *hw_ = nullptr;   // ctl_ follows dw_ on the device, hctl_ follows hw_

@@ -10,6 +10,7 @@
 // when the loop is over, the node's condition.  A whole solve is one graph
 // launch and one synchronisation.  The kernels are the same as the host
 // loop's; gated ones return at once when their gate word is 0.
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -22,25 +23,44 @@ namespace psi {
 
 namespace {
 
-// after an evaluation: the next one may be a patch; one more evaluation
-__global__ void k_ctl_evaluated(GraphCtl *c, uint32_t *err)
+// A batch's per-game accounting in the control kernels (games == 0: none).
+struct Accounts {
+    int32_t games = 0;
+    int4 *state = nullptr;
+    unsigned long long *gcount = nullptr;
+};
+
+// After Odd's switch: one more evaluation; the next one may be a patch; Even
+// moves in this step iff Odd made no strict improvement.
+__global__ void k_ctl_odd(GraphCtl *c, const unsigned long long *sw, uint32_t *err, Accounts b)
 {
+    const int32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < b.games) {
+        batch_event(0, b.state[g], b.gcount[g]);
+        batch_event(1, b.state[g], b.gcount[g]);
+    }
+    if (g) return;
     c->try_patch = c->patch_on;
     c->reset = 0;
-    c->quiet = 0;
     c->brs++;
     if (c->inject_at > 0 && c->brs == c->inject_at) atomicOr(err, c->inject_bits);
+    c->even = (sw[3] == 0) ? 1 : 0;
 }
 
-// after Odd's switch: Even moves in this step iff Odd made no strict improvement
-__global__ void k_ctl_odd(GraphCtl *c, const unsigned long long *sw) { c->even = (sw[3] == 0) ? 1 : 0; }
-
-// after Even's (gated) switch: iteration count, termination, reset, caps.
-// A set bit of the device error word ends the loop after this pass: the
-// state it left may be inconsistent, and later passes must not build on it.
+// After Even's (gated) switch: iteration count, termination, reset, caps, and
+// where the loop goes on, the next evaluation's gates.  A set bit of the
+// device error word ends the loop after this pass: the state it left may be
+// inconsistent, and later passes must not build on it.
 __global__ void k_ctl_even(GraphCtl *c, const unsigned long long *sw, const uint32_t *err,
-                           cudaGraphConditionalHandle loop, int32_t reset_variant, int32_t guard)
+                           cudaGraphConditionalHandle loop, int32_t reset_variant, int32_t guard, Accounts b,
+                           PatchArgs next)
 {
+    const int32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g < b.games && c->even) {
+        batch_event(2, b.state[g], b.gcount[g]);
+        batch_event(3, b.state[g], b.gcount[g]);
+    }
+    if (g) return;
     if (*(volatile const uint32_t *)err) {
         c->stop = GraphCtl::kDeviceError;
         cudaGraphSetConditional(loop, 0);
@@ -65,7 +85,8 @@ __global__ void k_ctl_even(GraphCtl *c, const unsigned long long *sw, const uint
         c->stop = GraphCtl::kRunaway;
         go = false;
     }
-    if (!go) cudaGraphSetConditional(loop, 0);
+    if (go) patch_begin(next);
+    else cudaGraphSetConditional(loop, 0);
 }
 
 // A solve that needs more evaluations than this is treated as a runaway (the
@@ -108,8 +129,8 @@ int Solver::enqueue_step(cudaGraph_t body, cudaGraphConditionalHandle loop, bool
 
     // (A)
     PSI_CUDA_TRY(cudaStreamBeginCaptureToGraph(stream_, body, nullptr, nullptr, 0, mode));
-    launch_reset_odd(stream_, n_, owner_, off_, tgt_, strat_, &ctl_->reset, need_);
-    int rc = enqueue_patch(false);
+    if (reset) launch_reset_odd(stream_, n_, owner_, off_, tgt_, strat_, &ctl_->reset, need_);
+    int rc = enqueue_patch(false, 0);
     if (rc) return abort_capture(rc);
     count_launch();
     k_eval_cond<<<1, 1, 0, stream_>>>(ctl_, evalc);
@@ -137,41 +158,29 @@ int Solver::enqueue_step(cudaGraph_t body, cudaGraphConditionalHandle loop, bool
     if (rc) return abort_capture(rc);
     PSI_CUDA_TRY(cudaStreamEndCapture(stream_, &g));
 
-    // (C); a batch also advances every game's own solve_si counts
-    // (k_batch_account, at the points where the host loop calls it), and its
+    // (C); a batch also advances every game's own solve_si counts, and its
     // switch steps add each game's strict improvements to gcount_
     const bool batch = games_ > 0 && !arena_;
+    Accounts acc;
+    if (batch) acc = Accounts{games_, gstate_, gcount_};
+    const unsigned ctl_blocks = (unsigned)std::max<int64_t>(1, ceil_div(acc.games, kBlock));
     PSI_CUDA_TRY(cudaStreamBeginCaptureToGraph(stream_, body, &ifnode, nullptr, 1, mode));
-    count_launch();
-    k_ctl_evaluated<<<1, 1, 0, stream_>>>(ctl_, &dw_->err);
-    if (batch) launch_batch_account(stream_, games_, 0, gstate_, gcount_);
-    // Odd: mark_solved(1), switch(1)
-    launch_mark_solved(stream_, &dw_->ucount, ulist_, 1, st_, solved_, nullptr, nullptr, nullptr,
-                       &ctl_->mfrom[1], &ctl_->mdone);
-    e = cudaMemsetAsync(dw_->sw, 0, sizeof(dw_->sw), stream_);
-    if (e != cudaSuccess) return abort_capture(fail(PSI_ERR_CUDA, std::string("memset: ") + cudaGetErrorString(e)));
-    int32_t *todo = reinterpret_cast<int32_t *>(jB_);   // free until the next cycle pass
+    int32_t *todo = reinterpret_cast<int32_t *>(jB_);   // free until the next full evaluation
     unsigned long long *gc = batch ? gcount_ : nullptr;
-    launch_switch(stream_, np_ - np0_, plist_ + np0_, 1, off_, tgt_, strat_, st_, key_, node_, rdeep_, dw_->sw,
-                  batch ? game_of_ : nullptr, gc, nullptr, &dw_->err, nullptr, need_, todo, &dw_->cnt[2],
-                  changes(), tie_, watch_, skip_, switch_warp_, &dw_->claim, arena_ ? nullptr : owner_, n_,
-                  /*count_moves=*/false);
-    if (batch) launch_batch_account(stream_, games_, 1, gstate_, gcount_);
-    count_launch();
-    k_ctl_odd<<<1, 1, 0, stream_>>>(ctl_, dw_->sw);
-    // Even, when Odd made no strict improvement: mark_solved(0), switch(0)
-    launch_mark_solved(stream_, &dw_->ucount, ulist_, 0, st_, solved_, nullptr, nullptr, &ctl_->even,
-                       &ctl_->mfrom[0], &ctl_->mdone);
-    if (batch) launch_batch_account(stream_, games_, 2, gstate_, gcount_, &ctl_->even);
-    e = cudaMemsetAsync(dw_->sw, 0, sizeof(dw_->sw), stream_);
-    if (e != cudaSuccess) return abort_capture(fail(PSI_ERR_CUDA, std::string("memset: ") + cudaGetErrorString(e)));
-    launch_switch(stream_, np0_, plist_, 0, off_, tgt_, strat_, st_, key_, node_, rdeep_, dw_->sw,
-                  batch ? game_of_ : nullptr, gc, nullptr, &dw_->err, &ctl_->even, need_, todo,
-                  &dw_->cnt[2], changes(), tie_, watch_, skip_, switch_warp_, &dw_->claim,
-                  arena_ ? nullptr : owner_, n_, /*count_moves=*/false);
-    if (batch) launch_batch_account(stream_, games_, 3, gstate_, gcount_, &ctl_->even);
-    count_launch();
-    k_ctl_even<<<1, 1, 0, stream_>>>(ctl_, dw_->sw, &dw_->err, loop, reset ? 1 : 0, eval_guard(n_));
+    for (int32_t player = 1; player >= 0; player--) {   // Even's part when Odd made no strict improvement
+        const MarkArgs m = mark_args(player);
+        const int32_t np = player ? np_ - np0_ : np0_;
+        launch_switch(stream_, np, plist_ + (player ? np0_ : 0), player, off_, tgt_, strat_, st_, key_, node_, rdeep_,
+                      dw_->sw, batch ? game_of_ : nullptr, gc, nullptr, &dw_->err, player ? nullptr : &ctl_->even,
+                      need_, todo, &dw_->listcount, changes(), tie_, watch_, skip_, switch_warp_, &dw_->claim,
+                      arena_ ? nullptr : owner_, n_, /*count_moves=*/false, &dw_->listdone, &m);
+        count_launch();
+        if (player)
+            k_ctl_odd<<<ctl_blocks, kBlock, 0, stream_>>>(ctl_, dw_->sw, &dw_->err, acc);
+        else
+            k_ctl_even<<<ctl_blocks, kBlock, 0, stream_>>>(ctl_, dw_->sw, &dw_->err, loop, reset ? 1 : 0,
+                                                           eval_guard(n_), acc, patch_args());
+    }
     e = cudaGetLastError();
     if (e != cudaSuccess) return abort_capture(fail(PSI_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e)));
     PSI_CUDA_TRY(cudaStreamEndCapture(stream_, &g));
@@ -189,6 +198,18 @@ int Solver::build_graph(bool reset)
         graph_ = nullptr;
     }
     PSI_CUDA_TRY(cudaGraphCreate(&graph_, 0));
+    // the first evaluation's gates, then the loop
+    PSI_CUDA_TRY(cudaStreamBeginCaptureToGraph(stream_, graph_, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    launch_patch_begin(stream_, patch_args(), -1);
+    cudaStreamCaptureStatus status;
+    const cudaGraphNode_t *deps = nullptr;
+    size_t ndeps = 0;
+    cudaError_t ce = cudaStreamGetCaptureInfo(stream_, &status, nullptr, nullptr, &deps, nullptr, &ndeps);
+    std::vector<cudaGraphNode_t> first;
+    if (ce == cudaSuccess) first.assign(deps, deps + ndeps);
+    cudaGraph_t same = nullptr;
+    PSI_CUDA_TRY(cudaStreamEndCapture(stream_, &same));
+    PSI_CUDA_TRY(ce);
     cudaGraphConditionalHandle loop;
     PSI_CUDA_TRY(cudaGraphConditionalHandleCreate(&loop, graph_, 1, cudaGraphCondAssignDefault));
     cudaGraphNodeParams cp = {};
@@ -197,7 +218,7 @@ int Solver::build_graph(bool reset)
     cp.conditional.type = cudaGraphCondTypeWhile;
     cp.conditional.size = 1;
     cudaGraphNode_t node;
-    PSI_CUDA_TRY(cudaGraphAddNode(&node, graph_, nullptr, nullptr, 0, &cp));
+    PSI_CUDA_TRY(cudaGraphAddNode(&node, graph_, first.data(), nullptr, first.size(), &cp));
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     const long long before = launch_count();
     int rc = enqueue_step(body, loop, reset);
@@ -221,7 +242,7 @@ int Solver::run_graph(bool reset, int64_t max_evals, GraphCtl *out, int4 *gstate
         if (rc) return rc;
     }
     GraphCtl init;
-    init.quiet = 1;   // init_strat: every need flag is set
+    init.quiet = 2;   // init_strat: every need flag is set
     init.patch_on = incremental_ != PSI_INCR_OFF ? 1 : 0;
     init.max_evals = max_evals > 0 && max_evals < INT32_MAX ? (int32_t)max_evals : 0;
     init.inject_at = inject_at_;

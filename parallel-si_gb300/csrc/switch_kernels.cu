@@ -81,13 +81,34 @@ __device__ int compare_equal_keys(const PathNode *__restrict__ node, const int4 
 // blockDim apart, so every load is coalesced; plist + offset may not be
 // 16-byte aligned, so no vector loads): block_append_k per pass.
 constexpr int kNeedPer = 4;
+
+// What a step needs done before its switch kernel, in the launch that collects
+// its list: the work counter and the statistics cleared, and mark_solved
+// (launches of their own cost 2 us each and more where steps are small).
+__device__ __forceinline__ void need_prelude(uint32_t *claim, unsigned long long *stats, const MarkArgs &mark)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (claim) *claim = 0;
+        stats[0] = stats[1] = stats[2] = stats[3] = 0;
+    }
+    if (mark.ucount) mark_solved_pass(mark);
+}
+
+// The switch kernels' last block clears the list's counter for the next step:
+// every block calls it at its end, all its threads having read the counter.
+__device__ __forceinline__ void list_used(int32_t *count, uint32_t *done)
+{
+    if (!done) return;
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicInc(done, gridDim.x - 1) == gridDim.x - 1) *count = 0;
+}
 __global__ void k_need_list(int32_t np, const int32_t *__restrict__ plist, const uint8_t *__restrict__ need,
                             const int32_t *__restrict__ game_of, const int32_t *__restrict__ gmask,
                             const int32_t *__restrict__ gate, int32_t *__restrict__ list, int32_t *__restrict__ count,
-                            uint32_t *__restrict__ claim)
+                            uint32_t *__restrict__ claim, unsigned long long *__restrict__ stats, MarkArgs mark)
 {
     if (gate && !*gate) return;
-    if (claim && blockIdx.x == 0 && threadIdx.x == 0) *claim = 0;   // the switch kernel's work counter
+    need_prelude(claim, stats, mark);
     const int64_t pass = (int64_t)kNeedPer * blockDim.x;
     for (int64_t b0 = (int64_t)blockIdx.x * pass; b0 < np; b0 += (int64_t)gridDim.x * pass) {
         int32_t v[kNeedPer];
@@ -112,10 +133,11 @@ __global__ void k_need_list(int32_t np, const int32_t *__restrict__ plist, const
 constexpr int kVec = 16;
 __global__ void k_need_ids(int32_t n, int32_t player, const int8_t *__restrict__ owner,
                            const uint8_t *__restrict__ need, const int32_t *__restrict__ gate,
-                           int32_t *__restrict__ list, int32_t *__restrict__ count, uint32_t *__restrict__ claim)
+                           int32_t *__restrict__ list, int32_t *__restrict__ count, uint32_t *__restrict__ claim,
+                           unsigned long long *__restrict__ stats, MarkArgs mark)
 {
     if (gate && !*gate) return;
-    if (claim && blockIdx.x == 0 && threadIdx.x == 0) *claim = 0;   // the switch kernel's work counter
+    need_prelude(claim, stats, mark);
     const bool vec = aligned16(owner) && aligned16(need);
     const int64_t pass = (int64_t)kVec * blockDim.x;
     for (int64_t b0 = (int64_t)blockIdx.x * pass; b0 < n; b0 += (int64_t)gridDim.x * pass) {
@@ -163,7 +185,7 @@ __global__ void k_need_ids(int32_t n, int32_t player, const int8_t *__restrict__
 // registers instead of 64 measured 10.7, 10.9 and 11.0 ms.
 template <bool COUNT>
 __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__restrict__ plist,
-                                                   const int32_t *__restrict__ count, int32_t player,
+                                                   int32_t *__restrict__ count, int32_t player,
                                                    const int32_t *__restrict__ off, const int32_t *__restrict__ tgt,
                                                    int32_t *__restrict__ strat, const int32_t *__restrict__ st,
                                                    const int32_t *__restrict__ key,
@@ -177,13 +199,16 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
                                                    const int32_t *__restrict__ gate, uint8_t *__restrict__ need,
                                                    ChangeList changes, uint8_t *__restrict__ tie_out,
                                                    uint8_t *__restrict__ watch, const int4 *__restrict__ skip,
-                                                   uint32_t *__restrict__ claim)
+                                                   uint32_t *__restrict__ claim, uint32_t *__restrict__ list_done)
 {
     if (gate && !*gate) return;
-    if (count) np = *count;
+    if (count) np = *(volatile int32_t *)count;
     // a block past the list's end has nothing to count either (uniform per
     // block: the block reduction below is never left waiting)
-    if ((int64_t)blockIdx.x * blockDim.x >= np) return;
+    if ((int64_t)blockIdx.x * blockDim.x >= np) {
+        list_used(count, list_done);
+        return;
+    }
     // A bounded grid, so the work counters are reduced once per block (a few
     // thousand atomics per launch instead of a set per 256 vertices).  The
     // list is dealt out to warps in chunks of 32 entries: every warp takes
@@ -348,6 +373,7 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
         if (tot.z) atomicAdd(&stats[2], (unsigned long long)tot.z);
         if (tot.w) atomicAdd(&stats[3], (unsigned long long)tot.w);
     }
+    list_used(count, list_done);
 }
 
 // ---- warp-cooperative all-switches
@@ -373,7 +399,7 @@ struct ScoreArg {
 __device__ __forceinline__ ScoreArg first_max(ScoreArg a, ScoreArg b) { return (a.sc >= b.sc) ? a : b; }
 
 __global__ void __launch_bounds__(kBlock) k_switch_warp(int32_t np, const int32_t *__restrict__ plist,
-                                                        const int32_t *__restrict__ count, int32_t player,
+                                                        int32_t *__restrict__ count, int32_t player,
                                                         const int32_t *__restrict__ off,
                                                         const int32_t *__restrict__ tgt, int32_t *__restrict__ strat,
                                                         const int32_t *__restrict__ st,
@@ -387,12 +413,16 @@ __global__ void __launch_bounds__(kBlock) k_switch_warp(int32_t np, const int32_
                                                         uint32_t *__restrict__ err,
                                                         const int32_t *__restrict__ gate, uint8_t *__restrict__ need,
                                                         ChangeList changes, uint8_t *__restrict__ tie_out,
-                                                        uint8_t *__restrict__ watch, const int4 *__restrict__ skip)
+                                                        uint8_t *__restrict__ watch, const int4 *__restrict__ skip,
+                                                        uint32_t *__restrict__ list_done)
 {
     if (gate && !*gate) return;
-    if (count) np = *count;
+    if (count) np = *(volatile int32_t *)count;
     // a block past the list's end has nothing to count either (uniform per block)
-    if ((int64_t)blockIdx.x * blockDim.x >= np) return;
+    if ((int64_t)blockIdx.x * blockDim.x >= np) {
+        list_used(count, list_done);
+        return;
+    }
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -572,6 +602,7 @@ __global__ void __launch_bounds__(kBlock) k_switch_warp(int32_t np, const int32_
         if (tot.z) atomicAdd(&stats[2], (unsigned long long)tot.z);
         if (tot.w) atomicAdd(&stats[3], (unsigned long long)tot.w);
     }
+    list_used(count, list_done);
 }
 
 // Per-game accounting of the solve_si loop (main.cpp:20-55) run over a batch
@@ -588,27 +619,10 @@ __global__ void __launch_bounds__(kBlock) k_switch_warp(int32_t np, const int32_
 //   event 3: after switch(Even) -> a game whose Even made no improvement is done; the others
 //                                  re-enter their best-response loop
 __global__ void k_batch_account(int32_t games, int32_t event, int4 *__restrict__ state,
-                                unsigned long long *__restrict__ gcount, const int32_t *__restrict__ gate)
+                                unsigned long long *__restrict__ gcount)
 {
-    if (gate && !*gate) return;   // graph-driven loop: Even's events only when Even moves
     int32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= games) return;
-    int4 s = state[g];
-    if (event == 0) {
-        if (!s.w && !s.z) s.x++;
-    } else if (event == 1) {
-        if (!s.w && !s.z && gcount[g] == 0) s.z = 1;
-        gcount[g] = 0;
-    } else if (event == 2) {
-        if (!s.w) s.y++;
-    } else {
-        if (!s.w) {
-            if (gcount[g] == 0) s.w = 1;
-            else s.z = 0;
-        }
-        gcount[g] = 0;
-    }
-    state[g] = s;
+    if (g < games) batch_event(event, state[g], gcount[g]);
 }
 
 // Dense row of v: counts of the priorities on its strategy path (the reference
@@ -657,16 +671,20 @@ void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t pla
                    const int32_t *rdeep, unsigned long long *stats, const int32_t *game_of, unsigned long long *gcount,
                    const int32_t *gmask, uint32_t *err, const int32_t *gate, uint8_t *need,
                    int32_t *list, int32_t *list_count, ChangeList changes, uint8_t *tie, uint8_t *watch,
-                   const int4 *skip, bool warp, uint32_t *claim, const int8_t *owner, int32_t n_all, bool count_moves)
+                   const int4 *skip, bool warp, uint32_t *claim, const int8_t *owner, int32_t n_all, bool count_moves,
+                   uint32_t *list_done, const MarkArgs *mark)
 {
-    if (np <= 0) return;
+    const MarkArgs m = mark ? *mark : MarkArgs();
+    if (np <= 0) {
+        cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned long long), s);
+        if (mark) launch_mark_solved(s, m);
+        return;
+    }
     const int blocks = per_device(g_switch_blocks, switch_grid);   // one wave of resident blocks
     unsigned g = grid_for(np);
     g = g < (unsigned)blocks ? g : (unsigned)blocks;
-    const int32_t *items = plist, *count = nullptr;
-    if (need && list && list_count) {
-        // only the vertices whose need flag is set (ChangeTrack)
-        cudaMemsetAsync(list_count, 0, sizeof(int32_t), s);
+    // only the vertices whose need flag is set (ChangeTrack)
+    {
         count_launch();
         if (owner && !gmask) {
             // its own cap (four times the switch's one wave): the scan is one
@@ -674,32 +692,30 @@ void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t pla
             unsigned gn = grid_for(ceil_div(n_all, kVec));
             gn = gn < 4u * (unsigned)blocks ? gn : 4u * (unsigned)blocks;
             k_need_ids<<<gn, kBlock, 0, s>>>(n_all, player, owner, need, gate, list, list_count,
-                                             warp ? nullptr : claim);
+                                             warp ? nullptr : claim, stats, m);
         } else {
             unsigned gn = grid_for(ceil_div(np, kNeedPer));
             gn = gn < (unsigned)blocks ? gn : (unsigned)blocks;
             k_need_list<<<gn, kBlock, 0, s>>>(np, plist, need, game_of, gmask, gate, list, list_count,
-                                              warp ? nullptr : claim);
+                                              warp ? nullptr : claim, stats, m);
         }
-        items = list;
-        count = list_count;
     }
     count_launch();
     if (warp)
-        k_switch_warp<<<g, kBlock, 0, s>>>(np, items, count, player, off, tgt, strat, st, key, node, rdeep, stats,
-                                           game_of, gcount, gmask, err, gate, need, changes, tie, watch, skip);
+        k_switch_warp<<<g, kBlock, 0, s>>>(np, list, list_count, player, off, tgt, strat, st, key, node, rdeep, stats,
+                                           game_of, gcount, gmask, err, gate, need, changes, tie, watch, skip,
+                                           list_done);
     else
         (count_moves ? k_switch<true> : k_switch<false>)<<<g, kBlock, 0, s>>>(
-            np, items, count, player, off, tgt, strat, st, key, node, rdeep, stats, game_of, gcount, gmask, err, gate,
-            need, changes, tie, watch, skip, count ? claim : nullptr);
+            np, list, list_count, player, off, tgt, strat, st, key, node, rdeep, stats, game_of, gcount, gmask, err,
+            gate, need, changes, tie, watch, skip, claim, list_done);
 }
 
-void launch_batch_account(cudaStream_t s, int32_t games, int32_t event, int4 *state, unsigned long long *gcount,
-                          const int32_t *gate)
+void launch_batch_account(cudaStream_t s, int32_t games, int32_t event, int4 *state, unsigned long long *gcount)
 {
     if (games <= 0) return;
     count_launch();
-    k_batch_account<<<grid_for(games), kBlock, 0, s>>>(games, event, state, gcount, gate);
+    k_batch_account<<<grid_for(games), kBlock, 0, s>>>(games, event, state, gcount);
 }
 
 void launch_materialize(cudaStream_t s, int32_t v0, int32_t count, int32_t d, const int32_t *st,
