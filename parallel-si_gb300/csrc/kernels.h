@@ -145,6 +145,7 @@ struct EvalArgs {
     int32_t *la = nullptr, *lb = nullptr, *lcount = nullptr;   // walks cut short: two lists (n entries), a counter
     int4 *ja = nullptr, *jb = nullptr;             // their jump entries (n entries each)
     int32_t *cnt = nullptr;       // three counters
+    uint32_t *err = nullptr;
     ChangeTrack track;
     const int32_t *gate = nullptr;
 };
@@ -152,6 +153,11 @@ void launch_root_init(cudaStream_t s, const EvalArgs &a);
 void launch_root_walk(cudaStream_t s, const EvalArgs &a);
 // Cooperative launch; returns a cudaError_t value.
 int launch_root_settle(cudaStream_t s, const EvalArgs &a);
+
+// One full evaluation in one cooperative launch (solve_kernels.cu), with what
+// launch_patch_begin does before one; n < 2^20.  Returns a cudaError_t value.
+struct SolveSync;
+int launch_eval_jump(cudaStream_t s, const EvalArgs &a, SolveSync *sync, EvalGates *g, int32_t *quiet);
 
 // A whole solve_si of one game in one persistent launch (solve_kernels.cu).
 struct SolveSync {

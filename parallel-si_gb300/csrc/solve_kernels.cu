@@ -663,6 +663,95 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve_small(SolveArgs a)
     }
 }
 
+// ---- one full evaluation by the same jumps, for the step-by-step calls and the
+// served arena: init_records, jumps and results in one cooperative launch where
+// the walks (root_kernels.cu) take three and each walk its path's length (with
+// every vertex in flight at once no ancestor is finished yet).  It leaves what
+// they leave: status, path records, keys, landmark records, the unreached
+// list, need flags; and does what launch_patch_begin does before them.
+__global__ void __launch_bounds__(kSolveThreads, 1) k_eval_jump(EvalArgs a, SolveSync *sync, EvalGates *g,
+                                                                int32_t *quiet)
+{
+    const int32_t n = a.n, lane = threadIdx.x & 31;
+    const int32_t tid = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x), nth = (int32_t)(gridDim.x * blockDim.x);
+    uint32_t phase = sync->phase;
+    auto barrier = [&](bool mine) -> bool {   // with a vote, as k_solve's
+        const uint32_t k = phase % 3, k1 = (phase + 1) % 3;
+        phase++;
+        if (tid == 0) sync->vote[k1] = sync->vote2[k1] = 0;
+        if (__syncthreads_or(mine) && threadIdx.x == 0) sync->vote[k] = 1;
+        cg::this_grid().sync();
+        return __ldcg(&sync->vote[k]) != 0;
+    };
+    if (tid == 0) {
+        if (*quiet > 0) --*quiet;
+        g->ccount = g->csnap = 0;
+        g->patch = 0;
+        g->eval = 1;
+        g->mfrom[0] = g->mfrom[1] = 0;
+        *a.ucount = 0;
+    }
+    for (int32_t v = tid; v < n; v += nth) {
+        const int32_t t = a.strat[v], p = a.pri[v];
+        const bool solved = a.solved[v];
+        const int32_t st = solved ? a.st[v] : 0;
+        *reinterpret_cast<int4 *>(&a.node[v]) =
+            make_int4(solved ? -1 : t, p, !solved ? RM_UNKNOWN : (st == ST_POS_INF ? RM_POS_INF : RM_NEG_INF), 0);
+        store_whole(&a.ja[v], solved ? make_int4(st == ST_POS_INF ? kPosInf : kNegInf, 0, 0, 0) : make_int4(t, p, 1, 1));
+        if (a.track.tie && a.track.tie[v]) a.track.need[v] = 1;
+    }
+    bool more = true;
+    barrier(false);
+    for (int pass = 0; more; pass++) {
+        if (pass == kMaxPasses) {   // cannot happen: windows grow at least kJumps-fold per pass
+            if (tid == 0) atomicOr(a.err, DERR_WALK_CAP);
+            break;
+        }
+        bool left = false;
+        for (int32_t b = tid & ~31; b < n; b += nth) {   // whole warps: appends and flags are collective
+            const int32_t v = b + lane;
+            bool changed = false, infinite = false;
+            if (v < n && !a.solved[v]) {
+                int4 r = load_whole(&a.ja[v]);
+                // in later passes, what is finished has been dealt with
+                if (pass == 0 || r.x >= 0) {
+                    if (jump_pass(a.ja, n, v, r)) {
+                        const bool fin = r.x == kSink;
+                        const int32_t d = r.w & kLen;
+                        const int32_t k =
+                            fin ? finite_key(r.y, r.z) : (r.x == kPosInf ? KEY_POS_INF : KEY_NEG_INF);
+                        a.st[v] = fin ? d : (r.x == kPosInf ? ST_POS_INF : ST_NEG_INF);
+                        if (fin && d >= kDeepPath) a.rdeep[v] = r.z;
+                        *reinterpret_cast<int2 *>(&a.node[v].rmax) =
+                            fin ? make_int2(r.y, path_word(d, r.z))
+                                : make_int2(r.x == kPosInf ? RM_POS_INF : RM_NEG_INF, 0);
+                        if (fin) {
+                            Top2 seg = {-1, 0, -1, 0};
+                            int32_t anc = v;
+                            for (int32_t j = d - skip_landmark_depth(d); j > 0; j--) {
+                                const int2 q = *reinterpret_cast<const int2 *>(&a.node[anc]);
+                                top2_add(seg, q.y);
+                                anc = q.x;
+                            }
+                            a.skip[v] = skip_pack(anc, seg);
+                        }
+                        infinite = !fin;
+                        changed = a.key[v] != k;
+                        if (changed) a.key[v] = k;
+                    } else {
+                        left = true;
+                    }
+                }
+            }
+            const int32_t p = warp_reserve(infinite, a.ucount);
+            if (infinite) a.ulist[p] = v;
+            flag_in_neighbours(a.track, changed, v);
+        }
+        more = barrier(left);
+    }
+    if (tid == 0) sync->phase = phase;
+}
+
 std::atomic<int> g_sms[kMaxCachedDevices];
 
 }  // namespace
@@ -675,6 +764,18 @@ static int device_sms()
         cudaDeviceGetAttribute(&x, cudaDevAttrMultiProcessorCount, dev);
         return x > 0 ? x : 1;
     });
+}
+
+int launch_eval_jump(cudaStream_t s, const EvalArgs &a, SolveSync *sync, EvalGates *g, int32_t *quiet)
+{
+    const int sms = device_sms();
+    int threads = kSolveThreads;
+    while (threads > kMinThreads && ceil_div(a.n, threads / 2) <= sms) threads /= 2;
+    const int64_t need = ceil_div(a.n, threads);
+    const int grid = (int)(need < 1 ? 1 : (need < sms ? need : sms));
+    void *args[] = {(void *)&a, (void *)&sync, (void *)&g, (void *)&quiet};
+    count_launch();
+    return (int)cudaLaunchCooperativeKernel((const void *)k_eval_jump, dim3(grid), dim3(threads), args, 0, s);
 }
 
 int64_t solve_capacity() { return (int64_t)kMaxWaves * kSolveThreads * device_sms(); }

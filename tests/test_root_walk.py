@@ -1,5 +1,5 @@
-"""The full evaluation's walks (root_kernels.cu) at the sizes where they change
-path: walks that end just before, at and after the step cap of 128 (longer
+"""The full evaluation's walks (root_kernels.cu), and its jumps in one launch for
+games below 2^20 vertices (solve_kernels.cu), at the sizes where they change path: walks that end just before, at and after the step cap of 128 (longer
 ones go through pointer jumping, in one block up to 4,096 of them, over the
 grid above), cycles around the cap, paths longer than the 16-bit depth of a
 path record.  Checked against a plain restatement over the same strategy."""
@@ -67,16 +67,17 @@ def restated(strat, pri):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("mode", [0, 2])   # jumps in one launch (PSI_INCR_OFF); walks (PSI_INCR_ALWAYS, first evaluation)
 @pytest.mark.parametrize("chains,cycle", [
     ([1], 0), ([2, 3], 0), ([CAP - 2], 0), ([CAP - 1], 0), ([CAP], 0), ([CAP + 1, CAP + 2], 0), ([4 * CAP + 3] * 3, 0),
     ([4500, 4200, 70], 0), ([DEEP - 1, 40], 0), ([DEEP, 3], 0), ([DEEP + 1, 900], 0), ([70000], 0),
     ([1, 5], 1), ([40], 2), ([CAP], CAP - 1), ([CAP + 1], CAP), ([3], CAP + 1), ([60, 300], 1000), ([9], 5000),
     ([5000], 3), ([20000, 600], 4097),
 ])
-def test_walks_match_a_plain_restatement(chains, cycle):
+def test_walks_match_a_plain_restatement(chains, cycle, mode):
     g = paths_game(chains, len(chains) + cycle, cycle=cycle)
     _, pri, _, tgt = g.csr()
-    s = psi.GPUList(g, incremental=0)
+    s = psi.GPUList(g, incremental=mode)
     s.init_strat()
     s.compute_valuation()
     strat = tgt.copy()
