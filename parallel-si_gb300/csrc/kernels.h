@@ -177,7 +177,7 @@ struct SolveArgs {
     PathNode *node = nullptr;
     int4 *skip = nullptr;
     int4 *jump[2] = {nullptr, nullptr};       // n entries each
-    int2 *path[2] = {nullptr, nullptr};       // (strategy, priority), n entries each
+    int2 *path = nullptr;                     // (strategy, priority), n entries
     int32_t *ulist = nullptr, *ucount = nullptr;
     SolveSync *sync = nullptr;    // zero before the first solve
     GraphCtl *ctl = nullptr;      // receives iters, brs, stop

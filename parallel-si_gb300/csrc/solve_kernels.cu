@@ -26,7 +26,8 @@
 //  - Switch phase of one player.  mark_solved and the all-switches step touch
 //    different words, so they share a phase, and each vertex's thread also
 //    writes the next evaluation's initial records, into the other of two
-//    buffers (comparisons still read the current ones).
+//    buffers (comparisons still read the current ones).  The paths that
+//    comparisons walk change at the start of the jump phase.
 //  - Comparisons that walk far (equal summaries, paths that meet late) would
 //    hold up a whole phase, 30 to 500 us where the others take 5.  A vertex
 //    whose walks pass their budget of steps is left over; only if there are any, all
@@ -35,7 +36,7 @@
 //
 // A thread owns the same vertices in every phase (plist[tid], plist[tid +
 // threads], ...), so what a vertex's phases start from -- its id, CSR range,
-// priority, choice and first successors -- stays in shared memory, 40 bytes
+// choice and first successors -- stays in shared memory, 32 bytes
 // per vertex; the first dependent load of a phase is then a key or a record.
 //
 // Every vertex of the player is examined in every switch phase: with all keys
@@ -69,14 +70,15 @@ constexpr int32_t kMaxLen = 1 << 24, kLen = (1 << 25) - 1;
 constexpr int32_t kNew = 1 << 30, kNewEven = 1 << 29;
 
 // One pass of v's record r; true when it is finished.
-__device__ __forceinline__ bool jump_pass(int4 *jump, int32_t n, int32_t v, int4 &r)
+// q: its target's record, if it has one.
+__device__ __forceinline__ bool jump_pass(int4 *jump, int32_t n, int32_t v, int4 &r, int4 q)
 {
     if (r.x < 0) return true;
     int32_t mark = v;
     for (int i = 1; i <= kJumps; i++) {
         bool cycle = (r.w & kLen) >= n;
         if (!cycle) {
-            const int4 q = load_whole(&jump[r.x]);
+            if (i > 1) q = load_whole(&jump[r.x]);
             if (q.x <= kNegInf) {
                 r = make_int4(q.x, 0, 0, 0);
                 store_whole(&jump[v], r);
@@ -144,15 +146,20 @@ __device__ __forceinline__ int compare_tied(const int4 *jump, const int2 *path, 
 }
 
 constexpr int kSolveThreads = 1024;
-// low bits of a vertex's choice word: solved; its path touched since Even's
-// last examination
-constexpr int32_t kSolved = 1, kTouched = 2;
-__device__ __forceinline__ int32_t bits(int32_t t, bool fresh)
-{
-    return 1 | (fresh ? kNew | kNewEven : 0) | ((t & kTouched) ? kNewEven : 0);
-}
+// A vertex's choice word: (choice + 1) << kChoiceShift and bits.  Solved; its
+// path touched since Even's last examination, since the last evaluation; the
+// infinity its record ended in; its choice changed since the evaluation.  With
+// them a switch phase reads no record but those it compares: a phase is bound
+// by L2 sectors once a thread has several vertices (n = 7*10^5: own records,
+// paths and priorities were 0.3 of 0.85 million per 155,648 vertices; 62 -> 51
+// us per evaluation).
+constexpr int32_t kSolved = 1, kTouched = 2, kFresh = 4, kNeg = 8, kPos = 16, kChanged = 32;
+constexpr int kChoiceShift = 6;
+constexpr int32_t kChoiceBits = (1 << kChoiceShift) - 1;
+__device__ __forceinline__ int32_t chosen(int32_t t) { return (t >> kChoiceShift) - 1; }
 constexpr int kFirst = 5;       // successors kept per vertex
-constexpr int kWords = 5 + kFirst;
+constexpr int kWords = 3 + kFirst;
+constexpr int32_t kIdBits = 20, kManySuccessors = (1 << (32 - kIdBits)) - 1;
 constexpr int kMinThreads = 128;
 constexpr int kSmallBytes = 227 * 1024;   // all a block can have
 // Games below this size are solved there.  Solve in us, k_solve -> here: n = 100
@@ -160,8 +167,8 @@ constexpr int kSmallBytes = 227 * 1024;   // all a block can have
 // 4,000 308 -> 454 (one SM's issue slots).
 constexpr int32_t kSmall = 2000;
 constexpr int kMaxWaves = 32;   // vertices per thread (a bit mask)
-constexpr int kMaxCached = 5;   // vertices per thread kept (200 KB); further ones are read anew
-constexpr int kSharedBytes = 4 * kWords * kSolveThreads * kMaxCached;   // 200 KB
+constexpr int kMaxCached = 7;   // vertices per thread kept (224 KB); further ones are read anew
+constexpr int kSharedBytes = 4 * kWords * kSolveThreads * kMaxCached;   // 224 KB
 
 __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
 {
@@ -193,33 +200,38 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
     };
     // the thread's vertex in wave w (vertex i of plist): its words
     struct Own {
-        int32_t v, e0, deg, pri, t;   // t: (choice + 1) * 4 + kTouched + solved
+        int32_t v, e0, deg, t;   // t: choice word (kSolved ...)
     };
     auto word = [&](int32_t w, int k) -> int32_t & { return own[(w * kWords + k) * (int32_t)blockDim.x + threadIdx.x]; };
     auto get = [&](int32_t w, int32_t i) -> Own {
-        if (w < kMaxCached) return Own{word(w, 0), word(w, 1), word(w, 2), word(w, 3), word(w, 4)};
+        if (w < kMaxCached) {
+            const uint32_t x = (uint32_t)word(w, 0);
+            Own o{(int32_t)(x & ((1u << kIdBits) - 1)), word(w, 1), (int32_t)(x >> kIdBits), word(w, 2)};
+            if (o.deg == kManySuccessors) o.deg = a.off[o.v + 1] - o.e0;
+            return o;
+        }
         const int32_t v = a.plist[i], e0 = a.off[v];
-        return Own{v, e0, a.off[v + 1] - e0, a.pri[v], 4 * (a.strat[v] + 1) + a.solved[v]};
+        return Own{v, e0, a.off[v + 1] - e0, (a.strat[v] + 1) << kChoiceShift | a.solved[v]};
     };
     auto put = [&](int32_t w, int32_t v, int32_t t) {
         if (w < kMaxCached) {
-            word(w, 4) = t;
+            word(w, 2) = t;
         } else {
-            a.strat[v] = (t >> 2) - 1;
-            a.solved[v] = t & 3;   // (with kTouched until the end)
+            a.strat[v] = chosen(t);
+            a.solved[v] = (uint8_t)(t & kChoiceBits);   // (all the bits until the end)
         }
     };
     auto successor = [&](int32_t w, int32_t e0, int32_t j) -> int32_t {
-        return (w < kMaxCached && j < kFirst) ? word(w, 5 + j) : a.tgt[e0 + j];
+        return (w < kMaxCached && j < kFirst) ? word(w, 3 + j) : a.tgt[e0 + j];
     };
     // the records of the current evaluation, and those that switch phases prepare
     int4 *jump = a.jump[0], *jump_next = a.jump[1];
-    int2 *path = a.path[0], *path_next = a.path[1];
-    // fresh: the choice differs from the current evaluation's
-    auto prepare = [&](int4 *j, int2 *p, const Own &o, int32_t code, bool fresh) {
-        const int32_t t = (o.t >> 2) - 1;
-        p[o.v] = make_int2(t, o.pri);
-        store_whole(&j[o.v], (o.t & kSolved) ? make_int4(code, 0, 0, 0) : make_int4(t, o.pri, 1, bits(o.t, fresh)));
+    int2 *path = a.path;   // the current evaluation's (choice, priority)
+    auto prepare = [&](int4 *j, const Own &o) {
+        const bool fresh = o.t & kChanged;
+        const int32_t w = 1 | (fresh ? kNew : 0) | (fresh || (o.t & kTouched) ? kNewEven : 0);
+        store_whole(&j[o.v], (o.t & kSolved) ? make_int4((o.t & kPos) ? kPosInf : kNegInf, 0, 0, 0)
+                                             : make_int4(chosen(o.t), a.pri[o.v], 1, w));
     };
     // The player's choice at a vertex (k_switch's rule): the successors in CSR
     // order, moving only on a strict improvement; that is the first best one,
@@ -228,7 +240,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
     // was a best one at the last examination, so where it and the other path
     // are as they were then (newbit; solved vertices' records do not tell), it
     // stands.  False if the walks passed the budget.
-    auto choose = [&](int32_t w, const Own &o, int32_t player, const int4 *skip, int32_t budget, int32_t own_w,
+    auto choose = [&](int32_t w, const Own &o, int32_t player, const int4 *skip, int32_t budget,
                       int32_t &choice) -> bool {
         const int32_t cur0 = choice;
         int32_t cur = cur0, kc = (cur0 >= 0) ? a.key[cur0] : 0;
@@ -253,7 +265,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
         }
         if (tie && !key_infinite(kc)) {
             const int32_t newbit = player == 0 ? kNewEven : kNew;
-            const bool settled = cur == cur0 && !(o.t & kSolved) && !(own_w & newbit);
+            const bool settled = cur == cur0 && !(o.t & (kSolved | (player == 0 ? kTouched : kFresh)));
             int32_t loads = 0;
             bool after = cur == cur0;   // the candidates follow the first best one
             for (int32_t j = 0; j < o.deg; j++) {
@@ -280,18 +292,16 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
         o.v = a.plist[i];
         o.e0 = a.off[o.v];
         o.deg = a.off[o.v + 1] - o.e0;
-        o.pri = a.pri[o.v];
-        o.t = (i < a.n_even ? 0 : 4 * (a.tgt[o.e0] + 1)) | kTouched;
+        o.t = (i < a.n_even ? 0 : (a.tgt[o.e0] + 1) << kChoiceShift) | kTouched | kChanged;
         if (w < kMaxCached) {
-            word(w, 0) = o.v;
+            word(w, 0) = (int32_t)((uint32_t)o.v | (uint32_t)min(o.deg, kManySuccessors) << kIdBits);
             word(w, 1) = o.e0;
-            word(w, 2) = o.deg;
-            word(w, 3) = o.pri;
 #pragma unroll
-            for (int j = 0; j < kFirst; j++) word(w, 5 + j) = j < o.deg ? a.tgt[o.e0 + j] : 0;
+            for (int j = 0; j < kFirst; j++) word(w, 3 + j) = j < o.deg ? a.tgt[o.e0 + j] : 0;
         }
         put(w, o.v, o.t);
-        prepare(jump, path, o, 0, true);
+        path[o.v].y = a.pri[o.v];
+        prepare(jump, o);
     }
     barrier(false, false);
 
@@ -307,13 +317,26 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
             bool left = false;
             for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
                 const Own o = get(w, i);
-                if (o.t & kSolved) continue;   // its record and key stay
-                int4 r = load_whole(&jump[o.v]);
-                if (!jump_pass(jump, n, o.v, r)) {
-                    left = true;
+                int32_t t1 = o.t & ~kChanged;
+                if (pass == 0 && (o.t & kChanged)) path[o.v].x = chosen(o.t);   // (no phase that reads paths is on)
+                if (o.t & kSolved) {   // its record and key stay
+                    if (t1 != o.t) put(w, o.v, t1);
                     continue;
                 }
-                if (r.w & kNew) put(w, o.v, o.t | kTouched);
+                int4 r = load_whole(&jump[o.v]);
+                // in the first pass the target is the choice: its record arrives with the own one
+                const int32_t t = pass ? r.x : chosen(o.t);
+                int4 q = r;
+                if (t >= 0) q = load_whole(&jump[t]);
+                if (!jump_pass(jump, n, o.v, r, q)) {
+                    left = true;
+                    if (t1 != o.t) put(w, o.v, t1);
+                    continue;
+                }
+                t1 &= ~(kFresh | kNeg | kPos);
+                if (r.w & kNew) t1 |= kFresh | kTouched;
+                if (r.x != kSink) t1 |= r.x == kPosInf ? kPos : kNeg;
+                if (t1 != o.t) put(w, o.v, t1);
                 a.key[o.v] = r.x == kSink ? finite_key(r.y, r.z) : (r.x == kPosInf ? KEY_POS_INF : KEY_NEG_INF);
             }
             barrier(left, false);
@@ -324,31 +347,31 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
         int32_t player = 1;
         bool go;
         for (;; player = 0) {
-            const int32_t code = player == 0 ? kPosInf : kNegInf;
+            const int32_t code = player == 0 ? kPos : kNeg;
             uint32_t over = 0;   // the thread's vertices that are left over
             bool moved = false;
             for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
                 Own o = get(w, i);
-                const int4 r = jump[o.v];   // own record
                 const int32_t t0 = o.t;
-                bool fresh = false;
-                if (r.x == code) o.t |= kSolved;
-                if (player == 0) o.t &= ~kTouched;
+                if (o.t & code) o.t |= kSolved;
                 if ((i < a.n_even) == (player == 0)) {
-                    int32_t choice = (o.t >> 2) - 1;
-                    if (choose(w, o, player, nullptr, budget, r.w, choice)) o.t = 4 * (choice + 1) + (o.t & 3);
-                    else over |= 1u << w;
-                    fresh = (o.t >> 2) != (t0 >> 2);
-                    moved |= fresh;
+                    int32_t choice = chosen(o.t);
+                    if (!choose(w, o, player, nullptr, budget, choice)) {
+                        over |= 1u << w;
+                    } else if (choice != chosen(o.t)) {
+                        o.t = (choice + 1) << kChoiceShift | (o.t & kChoiceBits) | kChanged;
+                        moved = true;
+                    }
                 }
+                if (player == 0) o.t &= ~kTouched;   // (what changed now is new to the next examination)
                 if (o.t != t0) put(w, o.v, o.t);
-                prepare(jump_next, path_next, o, r.x, fresh);
+                prepare(jump_next, o);
             }
             barrier(moved, over != 0);
             go = voted;
             if (voted2) {
                 for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
-                    const int32_t v = w < kMaxCached ? word(w, 0) : a.plist[i];
+                    const int32_t v = get(w, i).v;
                     const int4 r = jump[v];
                     if (r.x != kSink) continue;
                     Top2 seg = {-1, 0, -1, 0};
@@ -366,14 +389,15 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
                 for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
                     if (!(over >> w & 1)) continue;
                     Own o = get(w, i);
-                    const int4 r = jump[o.v];
-                    int32_t choice = (o.t >> 2) - 1;
-                    choose(w, o, player, a.skip, INT_MAX, r.w, choice);
-                    if (choice != (o.t >> 2) - 1) {
+                    int32_t choice = chosen(o.t);
+                    if (player == 0) o.t |= kTouched;   // (cleared above; the examination is not over)
+                    choose(w, o, player, a.skip, INT_MAX, choice);
+                    if (player == 0) o.t &= ~kTouched;
+                    if (choice != chosen(o.t)) {
                         moved = true;
-                        o.t = 4 * (choice + 1) + (o.t & 3);
+                        o.t = (choice + 1) << kChoiceShift | (o.t & kChoiceBits) | kChanged;
                         put(w, o.v, o.t);
-                        prepare(jump_next, path_next, o, r.x, true);
+                        prepare(jump_next, o);
                     }
                 }
                 barrier(moved, false);
@@ -395,18 +419,18 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
             for (int32_t w = 0, i = tid; i < n; w++, i += nth) {
                 if (i < a.n_even) continue;
                 Own o = get(w, i);
-                o.t = 4 * (successor(w, o.e0, 0) + 1) + (o.t & 3);
-                put(w, o.v, o.t);
-                prepare(jump_next, path_next, o, jump_next[o.v].x, (o.t >> 2) - 1 != path[o.v].x);
+                const int32_t t = successor(w, o.e0, 0);
+                if (t != chosen(o.t)) {
+                    o.t = (t + 1) << kChoiceShift | (o.t & kChoiceBits) | kChanged;
+                    put(w, o.v, o.t);
+                    prepare(jump_next, o);
+                }
             }
             barrier(false, false);
         }
         int4 *j = jump;
         jump = jump_next;
         jump_next = j;
-        int2 *p = path;
-        path = path_next;
-        path_next = p;
     }
 
     // the last evaluation as a solver leaves it (device_common.cuh); the
@@ -417,7 +441,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
         const int4 r = jump[v];
         const int2 q = path[v];
         const bool fin = r.x == kSink;
-        if (w < kMaxCached) a.strat[v] = (o.t >> 2) - 1;
+        if (w < kMaxCached) a.strat[v] = chosen(o.t);
         a.solved[v] = o.t & kSolved;
         const int32_t d = r.w & kLen;
         if (!fin && !(o.t & kSolved)) a.ulist[atomicAdd(a.ucount, 1)] = v;   // (none once the loop has converged)
@@ -715,7 +739,9 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_eval_jump(EvalArgs a, Solv
                 int4 r = load_whole(&a.ja[v]);
                 // in later passes, what is finished has been dealt with
                 if (pass == 0 || r.x >= 0) {
-                    if (jump_pass(a.ja, n, v, r)) {
+                    int4 q = r;
+                    if (r.x >= 0) q = load_whole(&a.ja[r.x]);
+                    if (jump_pass(a.ja, n, v, r, q)) {
                         const bool fin = r.x == kSink;
                         const int32_t d = r.w & kLen;
                         const int32_t k =

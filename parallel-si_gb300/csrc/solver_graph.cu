@@ -312,8 +312,7 @@ int Solver::run_fused(bool reset, int64_t max_evals, GraphCtl *out)
     a.skip = skip_;
     a.jump[0] = jA_;
     a.jump[1] = jB_;
-    a.path[0] = paths_;
-    a.path[1] = paths_ + n_;
+    a.path = paths_;
     a.ulist = ulist_;
     a.ucount = &dw_->ucount;
     a.sync = sync_;
