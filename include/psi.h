@@ -101,7 +101,7 @@ typedef struct {
                                 strategy path passes through a changed one (the result is
                                 the same as a full evaluation's) */
     int32_t patch_limit;     /* PSI_INCR_AUTO: the most changed strategies after which a
-                                patch is tried (0, the default: max(1024, n/64)) */
+                                patch is tried (0, the default: max(1024, n/128)) */
     int32_t walk_block;      /* threads per block of the sublist walk: a multiple of 32 in
                                 [32, 1024] or 0 (the default); without effect, as sublist_len */
     int32_t switch_kernel;   /* PSI_SWITCH_*: how the all-switches step maps vertices to threads
@@ -116,9 +116,10 @@ typedef struct {
  * 3-4% faster on the 2^24 random game. */
 enum { PSI_SWITCH_THREAD = 0, PSI_SWITCH_WARP = 1 };
 
-/* incremental: PSI_INCR_AUTO (default) patches after steps that changed at
- * most patch_limit strategies, giving up for a full evaluation when more
- * than max(4096, n/8) vertices or 256 levels of descendants are affected;
+/* incremental: PSI_INCR_AUTO (default) patches, on games of 2^20 vertices or
+ * more and in batches, after steps that changed at most patch_limit
+ * strategies, giving up for a full evaluation when more than max(4096, n/16)
+ * vertices or n/20000 levels of descendants (32 to 256) are affected;
  * PSI_INCR_OFF evaluates in full every time; PSI_INCR_ALWAYS patches
  * whenever the previous evaluation's state allows it, without the size
  * limits (n extra entries of device memory per buffer; for tests). */
@@ -282,7 +283,7 @@ int psi_batch_get_winning(psi_batch *b, int32_t game, int32_t player, int32_t *o
  * count is 1 (psi_solve with base's graph setting), else all count games as
  * one batch (psi_batch_solve).  Coordinate descent from the defaults over
  * sublist_len {64,16,32,128,256}, walk_block {128,64,256,512} and
- * patch_limit max(1024, vertices/d) for d in {64,8,16,32,128,256} (skipped when
+ * patch_limit max(1024, vertices/d) for d in {128,8,16,32,64,256} (skipped when
  * base->incremental is PSI_INCR_OFF); each candidate is one untimed solve and
  * `repeats` timed ones scored by the least, and replaces the incumbent only
  * when at least 2% faster.  *out = *base with the three fields chosen.  The

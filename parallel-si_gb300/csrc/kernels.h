@@ -321,7 +321,12 @@ struct PatchArgs {
     int32_t *apos = nullptr;    // per vertex: its position in alist, -1 if none (n entries, -1 between patches)
     int4 *rel = nullptr;                 // per position of alist: seed, path summary to it (acap)
     int2 *arev = nullptr;                // per position of alist: the vertex's in-edge range (acap)
-    int4 *sja = nullptr, *sjb = nullptr; // pointer-jumping entries of the seeds (acap each)
+    int4 *sja = nullptr;                 // the seeds' jump records (acap)
+    int32_t *spill = nullptr, *spill2 = nullptr;   // positions still to be searched from (2 acap, acap)
+    int32_t *sizes = nullptr;            // per block (kPatchSizes)
+    SolveSync *sync = nullptr;
+    uint32_t *err = nullptr;
+    int32_t n = 0;
     int32_t acap = 0, ccap = 0, max_levels = 0;
     int64_t ucap = 0;           // capacity of ulist
     int32_t *st = nullptr;
@@ -338,9 +343,10 @@ struct PatchArgs {
 // One thread: decides between a patch and the full evaluation (gates).
 // try_patch: whether the caller allows one; -1: as g->try_patch says.
 void launch_patch_begin(cudaStream_t s, const PatchArgs &a, int32_t try_patch);
-// Cooperative launches, gated on g->patch; return a cudaError_t value.
-int launch_patch_collect(cudaStream_t s, const PatchArgs &a);
-int launch_patch_values(cudaStream_t s, const PatchArgs &a);
+// Cooperative launch, gated on g->patch; returns a cudaError_t value.  full: a
+// graph conditional it sets to whether the full evaluation is to run.
+constexpr int kPatchSizes = 1024;   // the most blocks
+int launch_patch(cudaStream_t s, const PatchArgs &a, const cudaGraphConditionalHandle *full = nullptr);
 
 }  // namespace psi
 

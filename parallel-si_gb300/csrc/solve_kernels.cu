@@ -49,6 +49,7 @@
 
 #include "compare.cuh"
 #include "device_common.cuh"
+#include "jump.cuh"
 #include "kernels.h"
 #include "solver.h"
 
@@ -57,74 +58,6 @@ namespace cg = cooperative_groups;
 namespace psi {
 
 namespace {
-
-// targets of finished records
-constexpr int32_t kSink = -1, kNegInf = -2, kPosInf = -3;
-// reads per vertex and pass
-constexpr int kJumps = 64;
-constexpr int kMaxPasses = 64;
-// a record's last word: the window's length (up to kMaxLen: n or more only say
-// "a cycle"; n < 2^20), whether a strategy in it has changed since the last
-// evaluation, and, once finished, since Even's last examination
-constexpr int32_t kMaxLen = 1 << 24, kLen = (1 << 25) - 1;
-constexpr int32_t kNew = 1 << 30, kNewEven = 1 << 29;
-
-// One pass of v's record r; true when it is finished.
-// q: its target's record, if it has one.
-__device__ __forceinline__ bool jump_pass(int4 *jump, int32_t n, int32_t v, int4 &r, int4 q)
-{
-    if (r.x < 0) return true;
-    int32_t mark = v;
-    for (int i = 1; i <= kJumps; i++) {
-        bool cycle = (r.w & kLen) >= n;
-        if (!cycle) {
-            if (i > 1) q = load_whole(&jump[r.x]);
-            if (q.x <= kNegInf) {
-                r = make_int4(q.x, 0, 0, 0);
-                store_whole(&jump[v], r);
-                return true;
-            }
-            top1_merge(r.y, r.z, q.y, q.z);
-            r.z = min(r.z, kMaxLen);
-            r.w = min((r.w & kLen) + (q.w & kLen), kMaxLen) | (r.w & kNewEven) | ((r.w | q.w) & kNew);
-            r.x = q.x;
-            cycle = r.x == mark;
-            if ((i & (i - 1)) == 0) mark = r.x;
-        }
-        if (cycle) {
-            // the target is on the cycle: the top priority of the windows from
-            // it, once around or n vertices
-            const int32_t t0 = r.x;
-            int32_t t = t0, len = 0, top = -1, code = 0;
-            for (int j = 0; j < kJumps; j++) {
-                const int4 q = load_whole(&jump[t]);
-                if (q.x <= kNegInf) {
-                    code = q.x;
-                    break;
-                }
-                top = max(top, q.y);
-                len = min(len + (q.w & kLen), kMaxLen);
-                t = q.x;
-                if (t == t0 || len >= n) {
-                    code = (top & 1) ? kNegInf : kPosInf;
-                    break;
-                }
-            }
-            if (code) {
-                r = make_int4(code, 0, 0, 0);
-                store_whole(&jump[v], r);
-                return true;
-            }
-            r.w = kMaxLen | (r.w & ~kLen);   // a later pass goes on from the cycle
-            store_whole(&jump[v], r);
-            return false;
-        }
-        if (r.x == kSink && (r.w & kNew)) r.w |= kNewEven;
-        store_whole(&jump[v], r);
-        if (r.x == kSink) return true;
-    }
-    return false;
-}
 
 // Steps of comparison walks per vertex before it is left over: a step is a
 // dependent read from L2, the second round costs the landmark records of all
@@ -328,7 +261,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
                 const int32_t t = pass ? r.x : chosen(o.t);
                 int4 q = r;
                 if (t >= 0) q = load_whole(&jump[t]);
-                if (!jump_pass(jump, n, o.v, r, q)) {
+                if (!jump_pass<true>(jump, n, o.v, r, q)) {
                     left = true;
                     if (t1 != o.t) put(w, o.v, t1);
                     continue;
@@ -741,7 +674,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_eval_jump(EvalArgs a, Solv
                 if (pass == 0 || r.x >= 0) {
                     int4 q = r;
                     if (r.x >= 0) q = load_whole(&a.ja[r.x]);
-                    if (jump_pass(a.ja, n, v, r, q)) {
+                    if (jump_pass<true>(a.ja, n, v, r, q)) {
                         const bool fin = r.x == kSink;
                         const int32_t d = r.w & kLen;
                         const int32_t k =

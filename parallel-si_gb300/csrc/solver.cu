@@ -192,15 +192,20 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
     if (rc) return rc;
     cap_n_ = cap_n;
     cap_m_ = cap_m;
-    // incremental evaluation: change-list capacity (larger lists mean a full
-    // evaluation), re-evaluated set capacity, level cap of its search
+    // Incremental evaluation: change-list capacity (larger lists mean a full
+    // evaluation), re-evaluated set capacity, level cap of its search.  A full
+    // evaluation takes about 50 us per 2^20 vertices, a patch 10 us and 1.5 us
+    // per level and block, more where levels are wide: n/128 changes, n/16
+    // vertices and n/20,000 levels.  Against n/64, n/8, 256, ms per solve: 2^20
+    // vertices 5.5 -> 4.9, 2*10^6 8.5 -> 7.8, 2^24 37.0 -> 35.1, long-path 2^23
+    // 17.8 -> 17.6, the 256-game batch 16.8 -> 17.2.
     if (incremental_ != PSI_INCR_OFF) {
         const bool always = incremental_ == PSI_INCR_ALWAYS;
-        const int64_t cc = always ? cap_n : patch_limit_ > 0 ? patch_limit_ : std::max<int64_t>(1024, cap_n >> 6);
-        const int64_t ac = always ? cap_n : std::max<int64_t>(4096, cap_n >> 3);
+        const int64_t cc = always ? cap_n : patch_limit_ > 0 ? patch_limit_ : std::max<int64_t>(1024, cap_n >> 7);
+        const int64_t ac = always ? cap_n : std::max<int64_t>(4096, cap_n >> 4);
         ccap_ = (int32_t)std::max<int64_t>(1, std::min(cc, cap_n));
         acap_ = (int32_t)std::max<int64_t>(1, std::min(ac, cap_n));
-        max_levels_ = always ? INT32_MAX : 256;
+        max_levels_ = always ? INT32_MAX : (int32_t)std::max<int64_t>(32, std::min<int64_t>(256, cap_n / 20000));
     }
     ucap_ = cap_n + acap_;
     PSI_CUDA_TRY(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
@@ -251,7 +256,7 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
             {(void **)&clist_, 4 * (size_t)ccap_},
             {(void **)&alist_, 4 * (size_t)acap_},
             {(void **)&apos_, 4 * (size_t)std::max<int64_t>(1, cap_n)},
-            {(void **)&pj_, (3 * sizeof(int4) + sizeof(int2)) * (size_t)acap_},
+            {(void **)&pj_, (3 * sizeof(int4) + sizeof(int2)) * (size_t)acap_ + 4 * (size_t)kPatchSizes},
         };
         for (const auto &a : patch) {
             cudaError_t e = device_alloc(a.ptr, a.bytes, stream_);
@@ -478,8 +483,15 @@ PatchArgs Solver::patch_args()
     a.apos = apos_;
     a.rel = pj_;
     a.sja = pj_ ? pj_ + acap_ : nullptr;
-    a.sjb = pj_ ? pj_ + 2 * (size_t)acap_ : nullptr;
-    a.arev = pj_ ? reinterpret_cast<int2 *>(pj_ + 3 * (size_t)acap_) : nullptr;
+    if (pj_) {
+        a.spill = reinterpret_cast<int32_t *>(pj_ + 2 * (size_t)acap_);
+        a.spill2 = a.spill + 2 * (size_t)acap_;
+        a.arev = reinterpret_cast<int2 *>(pj_ + 3 * (size_t)acap_);
+        a.sizes = reinterpret_cast<int32_t *>(a.arev + acap_);
+    }
+    a.sync = sync_;
+    a.err = &dw_->err;
+    a.n = n_;
     a.acap = acap_;
     a.ccap = ccap_;
     a.max_levels = max_levels_;
@@ -521,15 +533,14 @@ int Solver::enqueue_eval(bool timed, int32_t try_patch)
 
 // 0. a patch, when the gates allow it and it succeeds; otherwise its
 //    kernels return at once and the full evaluation's gates are open
-int Solver::enqueue_patch(bool timed, int32_t try_patch)
+int Solver::enqueue_patch(bool timed, int32_t try_patch, const cudaGraphConditionalHandle *full)
 {
     if (timed) phase_begin(PH_PATCH);
     const PatchArgs pa = patch_args();
     if (timed) launch_patch_begin(stream_, pa, try_patch);   // (the graph loop's control has done so)
     if (incremental_ != PSI_INCR_OFF) {
-        int pe = launch_patch_collect(stream_, pa);
-        if (!pe) pe = launch_patch_values(stream_, pa);
-        if (pe) return fail(PSI_ERR_CUDA, std::string("patch kernels: ") + cudaGetErrorString((cudaError_t)pe));
+        int pe = launch_patch(stream_, pa, full);
+        if (pe) return fail(PSI_ERR_CUDA, std::string("patch kernel: ") + cudaGetErrorString((cudaError_t)pe));
     }
     if (timed) phase_end(PH_PATCH);
     return PSI_OK;

@@ -156,7 +156,7 @@ private:
     // the full evaluation's, each set gated (which ones work is decided on
     // the device, k_patch_begin).
     int enqueue_eval(bool timed, int32_t try_patch);
-    int enqueue_patch(bool timed, int32_t try_patch);
+    int enqueue_patch(bool timed, int32_t try_patch, const cudaGraphConditionalHandle *full = nullptr);
     int enqueue_full(bool timed);
     PatchArgs patch_args();
     MarkArgs mark_args(int32_t player);

@@ -108,13 +108,12 @@ constexpr int32_t kFusedVertices = (1 << 20) - 1;
 
 }  // namespace
 
-// Opens the full evaluation's conditional node iff this evaluation is not a
-// patch (its gate word was set by k_patch_begin / k_patch_collect).
-__global__ void k_eval_cond(const GraphCtl *c, cudaGraphConditionalHandle h) { cudaGraphSetConditional(h, c->eval ? 1 : 0); }
+// Opens the full evaluation's conditional node where there are no patches
+// (launch_patch does it otherwise).
+__global__ void k_eval_cond(cudaGraphConditionalHandle h) { cudaGraphSetConditional(h, 1); }
 
 // One SI step captured into the loop body `body`, in three pieces: (A) Odd's
-// reset and the patch kernels, then a kernel that sets the condition of (B),
-// a conditional "if" node holding the full evaluation, so that a patched
+// reset and the patch kernel, which sets the condition of (B), a conditional "if" node holding the full evaluation, so that a patched
 // evaluation launches none of its kernels; (C) the rest of the step.
 int Solver::enqueue_step(cudaGraph_t body, cudaGraphConditionalHandle loop, bool reset)
 {
@@ -130,10 +129,12 @@ int Solver::enqueue_step(cudaGraph_t body, cudaGraphConditionalHandle loop, bool
     // (A)
     PSI_CUDA_TRY(cudaStreamBeginCaptureToGraph(stream_, body, nullptr, nullptr, 0, mode));
     if (reset) launch_reset_odd(stream_, n_, owner_, off_, tgt_, strat_, &ctl_->reset, need_);
-    int rc = enqueue_patch(false, 0);
+    int rc = enqueue_patch(false, 0, &evalc);
     if (rc) return abort_capture(rc);
-    count_launch();
-    k_eval_cond<<<1, 1, 0, stream_>>>(ctl_, evalc);
+    if (incremental_ == PSI_INCR_OFF) {
+        count_launch();
+        k_eval_cond<<<1, 1, 0, stream_>>>(evalc);
+    }
     cudaStreamCaptureStatus status;
     const cudaGraphNode_t *deps = nullptr;
     size_t ndeps = 0;
