@@ -116,3 +116,55 @@ def test_comparisons_on_deep_paths_match_the_oracle(length, incremental):
     lockstep(gpu, ref, rows=False, summary=True)
     gpu.close()
     ref.close()
+
+
+def comb_game(pairs, trunk, pad, seed):
+    """A trunk (a chain of Odd vertices to Even vertex 0) and pairs of equally
+    long chains that leave it at random vertices; an Odd vertex per pair chooses
+    between the two heads.  The trunk carries the top priorities, so the heads
+    tie and are told apart below the vertices where their chains meet the
+    trunk, hundreds of vertices apart.  Padded with Odd self-loops."""
+    rng = np.random.default_rng(seed)
+    succ, pri = [[0]], [2]
+    for i in range(trunk):
+        succ.append([len(succ) - 1 if i else 0])
+        pri.append(int(rng.integers(40, 64)))
+    for _ in range(pairs):
+        length, heads = int(rng.integers(1, 260)), []
+        at = int(rng.integers(trunk // 2, trunk)) + 1
+        for k in range(2):
+            prev = at if k == 0 or rng.random() < 0.5 else int(rng.integers(trunk // 2, trunk)) + 1
+            for _ in range(length):
+                succ.append([prev])
+                pri.append(int(rng.integers(0, 30)))
+                prev = len(succ) - 1
+            heads.append(prev)
+        if rng.random() < 0.3:      # the same private priorities: a tie to the end
+            n = len(succ)
+            pri[n - length:n] = pri[n - 2 * length:n - length]
+        succ.append(heads if rng.random() < 0.5 else heads[::-1])
+        pri.append(int(rng.integers(0, 30)))
+    size = np.array([len(x) for x in succ] + [1] * pad, np.int64)
+    n = len(size)
+    tgt = np.concatenate([np.array([u for x in succ for u in x]), np.arange(len(succ), n)]).astype(np.int32)
+    owner = np.ones(n, np.int32)
+    owner[0] = 0
+    pri = np.concatenate([pri, np.ones(pad)]).astype(np.int32)
+    return psi.Game.from_csr(owner, pri, np.concatenate(([0], np.cumsum(size))).astype(np.int32), tgt)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("trunk", [70, 700, 4000])
+@pytest.mark.parametrize("pad,incremental", [(0, 0), (0, 2), (1 << 20, 0), (1 << 20, 1)])
+def test_ties_far_from_where_the_paths_meet(trunk, pad, incremental):
+    """Small games compare on the jumps' records, larger ones along landmarks
+    (with patches, whose vertices have none, in between)."""
+    g = comb_game(400, trunk, pad, trunk + incremental)
+    gpu = psi.GPUList(g, incremental=incremental)
+    ref = oracle.Sparse(*g.csr())
+    lockstep(gpu, ref, rows=False, summary=True)
+    strat = ref.get_strategy()
+    gpu.solve()
+    assert np.array_equal(gpu.get_strategy(), strat)
+    gpu.close()
+    ref.close()
