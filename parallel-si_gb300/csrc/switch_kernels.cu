@@ -213,14 +213,23 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
     // thousand atomics per launch instead of a set per 256 vertices).  The
     // list is dealt out to warps in chunks of 32 entries: every warp takes
     // the chunk at its own index first, then -- with claim, a device word
-    // zeroed by k_need_list -- two chunks at a time from a counter, one atomic
-    // per claim, else the next chunk one grid's worth of warps further on.
-    // Claims keep a warp that meets a long comparison walk from holding up
-    // chunks that a fixed stride would have dealt to it as well (2^24 random
-    // game: 16.0 -> 14.8 ms of switch steps per solve); the first chunk at
-    // the warp's own index keeps short lists spread over the whole grid.  A
-    // thread's edge count is at most m (< 2^31).
-    constexpr int kClaimChunks = 2;
+    // zeroed by k_need_list -- from a counter, one atomic per claim, else the
+    // next chunk one grid's worth of warps further on.  Claims keep a warp
+    // that meets a long comparison walk from holding up chunks that a fixed
+    // stride would have dealt to it as well (2^24 random game: 16.0 -> 14.8 ms
+    // of switch steps per solve); the first chunk at the warp's own index
+    // keeps short lists spread over the whole grid.  All warps of the GPU
+    // claim from one address, so a claim takes half of what would be the
+    // warp's share of the rest, 2 to 16 chunks: large while there is much
+    // left, small at the end, where a walk would hold up the launch (2^24
+    // random games, ms per solve with 2, 4, 8, 16 chunks always: 12.6, 11.9,
+    // 11.5, 11.8 with few ties, 21.2, 20.7, 21.0, 22.5 with many, 2^22 vertices
+    // with 8 priorities 6.5, 6.8, 7.5, 9.2; so: 11.1, 19.8, 6.5).  The next
+    // entry's vertex, choice and edge range are read before the present one's
+    // successors and keys, which wait for theirs (11.1 -> 10.9, 8 priorities
+    // 6.5 -> 6.4, long-path 5.23 -> 5.10; its successors ahead as well: 11.3,
+    // 21.7, 6.9, for the registers).  A thread's edge count is at most m (< 2^31).
+    constexpr int kMinClaim = 2, kMaxClaim = 16;
     const int lane = threadIdx.x & 31;
     const int64_t nchunk = (np + 31) >> 5;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -228,15 +237,24 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
     int per = 1;
     int32_t t_edges = 0, t_loads = 0, t_changed = 0, t_moves = 0;
     while (base < nchunk) {
+        int32_t vn = -1, curn = 0, e0n = 0, e1n = 0;   // the next entry (-1: none)
+        auto ahead = [&](int k) {
+            const int64_t i = (base + k) * 32 + lane;
+            vn = (k < per && i < np) ? __ldcs(&plist[i]) : -1;   // one-use streams are evict-first: L2 keeps the keys
+            if (vn < 0) return;
+            curn = strat[vn];
+            e0n = __ldcs(&off[vn]);
+            e1n = __ldcs(&off[vn + 1]);
+        };
+        ahead(0);
         for (int k = 0; k < per; k++) {
-            const int64_t c = base + k;
-            const int64_t i = c * 32 + lane;
-            if (c >= nchunk || i >= np) continue;
-            const int32_t v = __ldcs(&plist[i]);   // one-use streams are evict-first: L2 keeps the keys
+            const int32_t v = vn;
+            int32_t cur = curn;
+            const int32_t e0 = e0n, e1 = e1n;
+            ahead(k + 1);
+            if (v < 0) continue;
             if (gmask && !gmask[game_of[v]]) continue;
-            int32_t cur = strat[v];
             int32_t kc = (cur >= 0) ? key[cur] : 0;
-            const int32_t e0 = __ldcs(&off[v]), e1 = __ldcs(&off[v + 1]);
             t_edges += e1 - e0;
             int32_t moves = 0;
             // best key over the start and all successors, and whether a second
@@ -353,10 +371,11 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
             }
         }
         if (claim) {
+            const int64_t share = (nchunk - base) / (2 * warps);
+            per = (int)(share < kMinClaim ? kMinClaim : (share < kMaxClaim ? share : kMaxClaim));
             uint32_t b = 0;
-            if (lane == 0) b = atomicAdd(claim, (uint32_t)kClaimChunks);
+            if (lane == 0) b = atomicAdd(claim, (uint32_t)per);
             base = warps + __shfl_sync(0xffffffffu, b, 0);
-            per = kClaimChunks;
         } else {
             base += warps;
         }

@@ -120,3 +120,20 @@ def test_steps_after_a_capped_solve(cap, reset):
         assert np.array_equal(a.get_solved(), b.get_solved())
     a.close()
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1 << 20, 933_888 + 300_001, 6_000_001])
+def test_claimed_switches_match_strided_ones(n):
+    """Odd owns seven of eight vertices, so the first switch lists just under and
+    over the entries (933,888 on 152 SMs) past which a warp claims more than
+    two chunks of the list, and past those where it claims sixteen; few
+    priorities, so that some walk.  The warp kernel deals by a fixed stride."""
+    rng = np.random.default_rng(n)
+    off = np.concatenate(([0], np.cumsum(rng.integers(1, 4, n)))).astype(np.int32)
+    g = psi.Game.from_csr((rng.integers(0, 8, n) > 0).astype(np.int32), rng.integers(0, 50, n).astype(np.int32), off,
+                          rng.integers(0, n, off[-1]).astype(np.int32))
+    a, b = psi.GPUList(g), psi.GPUList(g, switch_kernel=1)
+    _same(_solved(a), _solved(b))
+    a.close()
+    b.close()
