@@ -224,7 +224,10 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
     // left, small at the end, where a walk would hold up the launch (2^24
     // random games, ms per solve with 2, 4, 8, 16 chunks always: 12.6, 11.9,
     // 11.5, 11.8 with few ties, 21.2, 20.7, 21.0, 22.5 with many, 2^22 vertices
-    // with 8 priorities 6.5, 6.8, 7.5, 9.2; so: 11.1, 19.8, 6.5).  The next
+    // with 8 priorities 6.5, 6.8, 7.5, 9.2; so: 11.1, 19.8, 6.5).  In a batch
+    // chunks in a row belong to one game, whose walks may all be long: one at
+    // a time (256 games of 100 to 200,000 vertices, ms per solve: 17.3, with
+    // up to 16 18.1; 150 games up to 50,000: 4.43 and 4.59).  The next
     // entry's vertex, choice and edge range are read before the present one's
     // successors and keys, which wait for theirs (11.1 -> 10.9, 8 priorities
     // 6.5 -> 6.4, long-path 5.23 -> 5.10; its successors ahead as well: 11.3,
@@ -372,7 +375,7 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
         }
         if (claim) {
             const int64_t share = (nchunk - base) / (2 * warps);
-            per = (int)(share < kMinClaim ? kMinClaim : (share < kMaxClaim ? share : kMaxClaim));
+            per = game_of ? 1 : (int)(share < kMinClaim ? kMinClaim : (share < kMaxClaim ? share : kMaxClaim));
             uint32_t b = 0;
             if (lane == 0) b = atomicAdd(claim, (uint32_t)per);
             base = warps + __shfl_sync(0xffffffffu, b, 0);
