@@ -725,11 +725,28 @@ static int device_sms()
     });
 }
 
+// Threads per block that spread n vertices evenly over all SMs, at least
+// kMinThreads (n = 10^4: 0.63 ms per solve in ten blocks of 1,024, 0.53 ms in 79
+// of 128), and over as few vertices per thread as the SMs hold, evenly too: the
+// same for all threads, where blocks of 1,024 left SMs or most threads of the
+// last round idle (us per solve at 10^5, 1.8*10^5, 2^18, 3.5*10^5, 10^6 vertices:
+// 859, 1256, 1376, 1270, 4030 -> 801, 1123, 1307, 1228, 3990).  one_each: past so
+// many vertices per SM two per thread are better than one.  k_solve's are from
+// 600 (1.5*10^5: 1080 -> 1023; 10^5: 801 -> 771; 9*10^4 the same; three per thread
+// lose: 2^18 1307 -> 1500); a single evaluation's are not (15 to 20 calls at
+// 1.2*10^5: 2.58 -> 2.74 ms).
+constexpr int kOneEach = 600;
+static int spread_threads(int64_t n, int sms, int one_each)
+{
+    int64_t each = ceil_div(n, (int64_t)kSolveThreads * sms);
+    if (each == 1 && n > (int64_t)one_each * sms) each = 2;
+    const int64_t threads = 32 * ceil_div(ceil_div(n, sms * each), 32);
+    return (int)(threads > kMinThreads ? threads : kMinThreads);
+}
+
 int launch_eval_jump(cudaStream_t s, const EvalArgs &a, SolveSync *sync, EvalGates *g, int32_t *quiet)
 {
-    const int sms = device_sms();
-    int threads = kSolveThreads;
-    while (threads > kMinThreads && ceil_div(a.n, threads / 2) <= sms) threads /= 2;
+    const int sms = device_sms(), threads = spread_threads(a.n, sms, kSolveThreads);
     const int64_t need = ceil_div(a.n, threads);
     const int grid = (int)(need < 1 ? 1 : (need < sms ? need : sms));
     void *args[] = {(void *)&a, (void *)&sync, (void *)&g, (void *)&quiet};
@@ -752,10 +769,7 @@ int launch_solve(cudaStream_t s, const SolveArgs &a)
         k_solve_small<<<1, threads, l.total, s>>>(a);
         return (int)cudaGetLastError();
     }
-    // the vertices spread over all SMs, at least kMinThreads per block (n = 10^4:
-    // 0.63 ms per solve in ten blocks of 1,024, 0.53 ms in 79 of 128)
-    int threads = kSolveThreads;
-    while (threads > kMinThreads && ceil_div(a.n, threads / 2) <= sms) threads /= 2;
+    const int threads = spread_threads(a.n, sms, kOneEach);
     const int64_t need = ceil_div(a.n, threads);
     const int grid = (int)(need < sms ? need : sms);
     const int64_t waves = ceil_div(a.n, (int64_t)grid * threads);

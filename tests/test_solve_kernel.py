@@ -1,9 +1,9 @@
 """psi_solve as one persistent kernel (solve_kernels.cu) at the sizes where
 its launch or its phases change: one block with everything in shared memory
 below 2,000 vertices (its successors too, where they fit), blocks of 128 threads
-and more above, two vertices per thread past 155,648 (152 SMs), more
-than the five kept in shared memory past 778,240; jumps over deep chains and
-long cycles; and the state it leaves for the step-by-step calls."""
+and more above, two vertices per thread past 91,200 (152 SMs), three past
+311,296, up to seven; jumps over deep chains and long cycles; and the state it
+leaves for the step-by-step calls."""
 import numpy as np
 import pytest
 
@@ -69,7 +69,8 @@ def test_small_games_of_any_degree(n, deg):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n,pri", [(155648, 155648), (155649, 9), (778241, 778241), ((1 << 20) - 1, 1 << 20)])
+@pytest.mark.parametrize("n,pri", [(91200, 91200), (91201, 12), (155648, 155648), (155649, 9), (311296, 9),
+                                   (311297, 311297), (778241, 778241), ((1 << 20) - 1, 1 << 20)])
 def test_solve_matches_the_graph_loop(n, pri):
     """Against the same game through the graph (the warp-cooperative switch
     selects it), which other tests hold to the oracle at these sizes."""
