@@ -17,6 +17,26 @@ __device__ __forceinline__ int decide(int32_t p, int32_t ca, int32_t cb)
     return ca < cb ? 1 : -1;
 }
 
+// The next successor to compare exactly: ties holds which of the first 32
+// share the best key with the first best one; from the 32nd on all are asked
+// for (one that precedes the first best one has another key).  With it the
+// lanes of a warp come to their ties together, whatever their places in the
+// lists: in a loop over all successors each place was a turn of its own, in
+// which the lanes without a tie there waited for a walk (persistent solver,
+// 10^4, 10^5, 10^6 vertices and 2^18 with 8 priorities, us per solve: 281, 715,
+// 3837, 1928 -> 252, 670, 3648, 1600; graph, 2^24 with many ties, 2^22 with 8
+// priorities, ms: 43.4, 13.5 -> 40.2, 12.6).
+__device__ __forceinline__ int32_t next_tied(uint32_t &ties, int32_t &j)
+{
+    if (ties) {
+        j = __ffs(ties) - 1;
+        ties &= ties - 1;
+    } else if (j < 32) {
+        j = 32;
+    }
+    return j;
+}
+
 // Tier 3: walks to the lowest common ancestor of u and w (depths du, dw; w may
 // be the sink, -1 with depth 0).  Pass k finds the highest priority below the
 // last tie on each side's segment below the ancestor, and its count.  With
@@ -29,7 +49,10 @@ __device__ __forceinline__ int decide(int32_t p, int32_t ca, int32_t cb)
 // without branches on priorities: updating two diverged, about 0.12 us per
 // step on top of the loads, where a whole launch or phase waits for its
 // longest walk.  path: per vertex a record that begins with (parent,
-// priority).  Once loads passes budget: kUndecided.
+// priority).  Once loads passes budget: kUndecided.  Without SKIP a step is its
+// loads and little else, and they are issued before the checks (persistent
+// solver, sizes as above, against a test of skip at run time: 306, 770, 3993,
+// 2255 -> 281, 715, 3837, 1928).
 constexpr int kUndecided = 2;
 __device__ __forceinline__ void top_add(int32_t &m, int32_t &c, int32_t p, int32_t k, int32_t below)
 {
@@ -44,7 +67,7 @@ __device__ __forceinline__ bool top_jump(int32_t &m, int32_t &c, const int4 s, i
     top_add(m, c, first ? s.y : s.z, first ? skip_c1(s.w) : skip_c2(s.w), below);
     return true;
 }
-template <class Rec>
+template <bool SKIP, class Rec>
 static __device__ __noinline__ int lean_compare(const Rec *path, const int4 *skip, int32_t u, int32_t du, int32_t w,
                                                 int32_t dw, int32_t &loads, int32_t budget, uint32_t *err)
 {
@@ -61,13 +84,15 @@ static __device__ __noinline__ int lean_compare(const Rec *path, const int4 *ski
         }
         while (da > db) {
             if (a < 0 || ++loads > budget) break;
-            const int32_t l = skip_landmark_depth(da);
-            if (skip && l >= db) {
-                const int4 s = skip[a];
-                if (top_jump(ma, ca, s, below)) {
-                    a = s.x;
-                    da = l;
-                    continue;
+            if (SKIP) {
+                const int32_t l = skip_landmark_depth(da);
+                if (l >= db) {
+                    const int4 s = skip[a];
+                    if (top_jump(ma, ca, s, below)) {
+                        a = s.x;
+                        da = l;
+                        continue;
+                    }
                 }
             }
             const int2 q = *reinterpret_cast<const int2 *>(&path[a]);
@@ -75,9 +100,14 @@ static __device__ __noinline__ int lean_compare(const Rec *path, const int4 *ski
             a = q.x;
             da--;
         }
-        bool jumps = skip != nullptr;
+        bool jumps = SKIP;
         while (a != b) {
             if (a < 0 || b < 0) break;
+            int2 q, r;
+            if (!SKIP) {
+                q = *reinterpret_cast<const int2 *>(&path[a]);
+                r = *reinterpret_cast<const int2 *>(&path[b]);
+            }
             loads += 2;
             if (loads > budget) break;
             if (jumps) {
@@ -96,7 +126,10 @@ static __device__ __noinline__ int lean_compare(const Rec *path, const int4 *ski
                 // one landmark: the paths meet in this segment
                 jumps = s.x != t.x;
             }
-            const int2 q = *reinterpret_cast<const int2 *>(&path[a]), r = *reinterpret_cast<const int2 *>(&path[b]);
+            if (SKIP) {
+                q = *reinterpret_cast<const int2 *>(&path[a]);
+                r = *reinterpret_cast<const int2 *>(&path[b]);
+            }
             top_add(ma, ca, q.y, 1, below);
             top_add(mb, cb, r.y, 1, below);
             a = q.x;

@@ -75,7 +75,8 @@ __device__ __forceinline__ int compare_tied(const int4 *jump, const int2 *path, 
     const int4 rw = (w >= 0) ? jump[w] : make_int4(kSink, -1, 0, 0);   // w's length: 0
     if (ru.y != rw.y) return ru.y > rw.y ? decide(ru.y, ru.z, 0) : decide(rw.y, 0, rw.z);
     if (ru.z != rw.z) return decide(ru.y, ru.z, rw.z);
-    return lean_compare(path, skip, u, ru.w & kLen, w, rw.w & kLen, loads, budget, err);
+    return skip ? lean_compare<true>(path, skip, u, ru.w & kLen, w, rw.w & kLen, loads, budget, err)
+                : lean_compare<false>(path, skip, u, ru.w & kLen, w, rw.w & kLen, loads, budget, err);
 }
 
 constexpr int kSolveThreads = 1024;
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
         const int32_t cur0 = choice;
         int32_t cur = cur0, kc = (cur0 >= 0) ? a.key[cur0] : 0;
         bool tie = false;
+        uint32_t ties = 0;   // which of the first 32 successors share the best key with cur
         for (int32_t b = 0; b < o.deg; b += kFirst) {
             int32_t us[kFirst], ks[kFirst];
 #pragma unroll
@@ -191,8 +193,10 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
                     cur = us[j];
                     kc = ks[j];
                     tie = false;
+                    ties = 0;
                 } else if (ks[j] == kc && us[j] != cur) {
                     tie = true;
+                    if (b + j < 32) ties |= 1u << (b + j);
                 }
             }
         }
@@ -200,14 +204,10 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
             const int32_t newbit = player == 0 ? kNewEven : kNew;
             const bool settled = cur == cur0 && !(o.t & (kSolved | (player == 0 ? kTouched : kFresh)));
             int32_t loads = 0;
-            bool after = cur == cur0;   // the candidates follow the first best one
-            for (int32_t j = 0; j < o.deg; j++) {
+            for (int32_t j = 0;; j++) {
+                if (next_tied(ties, j) >= o.deg) break;
                 const int32_t u = successor(w, o.e0, j);
-                if (!after) {
-                    after = u == cur;
-                    continue;
-                }
-                if (u == cur || a.key[u] != kc) continue;
+                if (u == cur || (j >= 32 && a.key[u] != kc)) continue;
                 if (settled && cur == cur0 && !(jump[u].w & newbit)) continue;
                 const int c = compare_tied(jump, path, skip, u, cur, loads, budget, &a.sync->err);
                 if (c == kUndecided) return false;

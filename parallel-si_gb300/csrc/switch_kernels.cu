@@ -63,7 +63,7 @@ __device__ int compare_equal_keys(const PathNode *__restrict__ node, const int4 
     }
     if (ru.x != rw.x) return ru.x > rw.x ? decide(ru.x, cu, 0) : decide(rw.x, 0, cw);
     if (cu != cw) return decide(ru.x, cu, cw);
-    return lean_compare(node, skip, u, du, w, dw, loads, INT_MAX, err);
+    return lean_compare<true>(node, skip, u, du, w, dw, loads, INT_MAX, err);
 }
 
 // One thread per vertex of plist (all owned by `player`).  Per compared edge
@@ -264,6 +264,7 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
             // distinct vertex attains it (a tie)
             int32_t ext = kc, ext_v = cur;
             bool tie = false;
+            uint32_t ties = 0;   // which of the first 32 successors attain it, besides the first that does
             // Fast pass: successors in batches of kBatch -- all ids, then all
             // keys, before the comparisons (independent gathers in flight per
             // thread).  Equal keys of distinct finite vertices end it; the exact
@@ -288,8 +289,10 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
                         ext = ku;
                         ext_v = u;
                         tie = false;
+                        ties = 0;
                     } else if (ku == ext && u != ext_v) {
                         tie = true;
+                        if (!COUNT && eb - e0 + j < 32) ties |= 1u << (eb - e0 + j);
                     }
                     if (!COUNT) continue;
                     int c;
@@ -313,14 +316,10 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
                 // others that share it (none for an infinity)
                 cur = ext_v;
                 if (tie && !key_infinite(ext)) {
-                    bool after = cur == cur0;
-                    for (int32_t e = e0; e < e1; e++) {
-                        const int32_t u = tgt[e];
-                        if (!after) {
-                            after = u == cur;
-                            continue;
-                        }
-                        if (u == cur || key[u] != ext) continue;
+                    for (int32_t j = 0;; j++) {
+                        if (next_tied(ties, j) >= e1 - e0) break;
+                        const int32_t u = tgt[e0 + j];
+                        if (u == cur || (j >= 32 && key[u] != ext)) continue;
                         const int c = compare_equal_keys(node, skip, st, rdeep, u, cur, t_loads, err);
                         if ((player == 0) ? c > 0 : c < 0) cur = u;
                     }

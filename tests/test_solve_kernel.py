@@ -138,3 +138,27 @@ def test_claimed_switches_match_strided_ones(n):
     _same(_solved(a), _solved(b))
     a.close()
     b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [0, 2])   # the persistent solver; the graph (PSI_INCR_ALWAYS)
+@pytest.mark.parametrize("deg", [5, 31, 32, 33, 90])
+def test_ties_at_any_place_of_a_list(deg, mode):
+    """Ties among the first 32 successors are remembered, later ones asked for
+    again: lists of up to deg successors, repeated ones among them, with four
+    priorities, so that most best keys are shared."""
+    rng = np.random.default_rng(deg)
+    n = 2300
+    size = rng.integers(max(1, deg - 4), deg + 1, n)
+    off = np.concatenate(([0], np.cumsum(size))).astype(np.int32)
+    # successors near the end of the order make long common paths
+    tgt = np.minimum(n - 1, rng.integers(0, n, off[-1]) | rng.integers(0, n, off[-1])).astype(np.int32)
+    g = psi.Game.from_csr(rng.integers(0, 2, n), rng.integers(0, 4, n), off, tgt)
+    ref = oracle.Sparse(*g.csr())
+    s = psi.GPUList(g, incremental=mode)
+    for reset in (False, True):
+        assert s.solve(reset=reset) == ref.solve(reset=reset)
+        assert np.array_equal(s.get_strategy(), ref.get_strategy())
+        assert np.array_equal(s.get_infinite(), ref.get_infinite())
+    s.close()
+    ref.close()
