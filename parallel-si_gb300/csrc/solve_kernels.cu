@@ -61,11 +61,13 @@ namespace {
 
 // Steps of comparison walks per vertex before it is left over: a step is a
 // dependent read from L2, the second round costs the landmark records of all
-// vertices and two barriers.  Solve in us with 16, 64, 256 steps: 431, 382,
-// 323 (n = 10^4), 960, 940, 832 (10^5), 2782, 2537, 2640 (2^18 vertices, 8
-// priorities), but 5200, 5690, 6320 (10^6), where each thread has seven
-// vertices whose walks would add up.
-__device__ __forceinline__ int32_t walk_budget(int32_t n, int32_t threads) { return n <= 2 * threads ? 256 : 16; }
+// vertices and two barriers, and a warp's lanes walk together.  Solve in us
+// with 16, 64, 256, 1,024, 4,096 steps where a thread has more than two vertices:
+// 3640, 3622, 3448, 3248, 3250 (10^6), 6210, 5212, 5160, 5090, 4830 (9*10^5, 100
+// priorities), 3737, 3339, 2528, 2527, 2515 (10^6, long paths); with 256, 512, 1,024,
+// 4,096 where not: 669, 654, 653, 653 (10^5), 1600, 1542, 1433, 1424 (2^18, 8
+// priorities).  More is the same: few ties are that far apart.
+constexpr int32_t kWalkBudget = 4096;
 
 // Even's view of finite u against finite w (distinct, equal keys; -1: the sink).
 __device__ __forceinline__ int compare_tied(const int4 *jump, const int2 *path, const int4 *skip, int32_t u, int32_t w,
@@ -110,7 +112,6 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
     const int32_t n = a.n;
     const int32_t tid = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x);
     const int32_t nth = (int32_t)(gridDim.x * blockDim.x);
-    const int32_t budget = walk_budget(n, nth);
     // Barrier with two votes: whether any thread passed true.  Phase k uses the
     // words k % 3, which thread 0 clears in phase k - 1, when everyone has
     // read their last use (phase k - 3); the count goes on from solve to
@@ -289,7 +290,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
                 if (o.t & code) o.t |= kSolved;
                 if ((i < a.n_even) == (player == 0)) {
                     int32_t choice = chosen(o.t);
-                    if (!choose(w, o, player, nullptr, budget, choice)) {
+                    if (!choose(w, o, player, nullptr, kWalkBudget, choice)) {
                         over |= 1u << w;
                     } else if (choice != chosen(o.t)) {
                         o.t = (choice + 1) << kChoiceShift | (o.t & kChoiceBits) | kChanged;
