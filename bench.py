@@ -295,8 +295,9 @@ def phase_bytes(phase, n, m, nsub, counters, calls, n_even, n_odd, iters, brs):
         return 69 * n
     if phase == "walk":
         # records: strategy, priority, solved flag in, record out (25 B); walks: record and
-        # key in, status, summary, landmark record and key out (52 B)
-        return 77 * n
+        # key in, status, summary and key out (36 B; evaluations that write landmark
+        # records as well, 16 B, are not told apart)
+        return 61 * n
     if phase == "reduced":
         if nsub >= RULER_MIN:
             # ruling set: item entries in, (ruler, prefix) out and back in, the
@@ -1011,7 +1012,7 @@ def main():
     ap.add_argument("--no-tune", action="store_true",
                     help="skip the autotuner: sublist/walk/patch options from the flags")
     ap.add_argument("--patch-limit", type=int, default=0,
-                    help="psi_options.patch_limit (0: the library default, max(1024, n/64))")
+                    help="psi_options.patch_limit (0: the library default, max(1024, n/128))")
     ap.add_argument("--no-cpu", action="store_true", help="skip the CPU-baseline sample")
     ap.add_argument("--switch-kernel", choices=("thread", "warp"), default="thread",
                     help="psi_options.switch_kernel: thread-per-vertex (default) or warp-cooperative switch step")

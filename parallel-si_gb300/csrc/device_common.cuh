@@ -197,8 +197,8 @@ __device__ __forceinline__ void top2_add_n(Top2 &t, int32_t p, int32_t count)
 // segment from v up to the landmark, exclusive, one word: their counts, a
 // segment holds at most SKIP_K vertices, and the number of the evaluation that
 // wrote it).  Written by the walks of a full evaluation (root_kernels.cu) as
-// one 16-byte word; a patch marks its vertices' records unknown (the paths of
-// all other vertices are unchanged).  SKIP_K
+// one 16-byte word, where want_landmarks asks for them; a patch marks its
+// vertices' records unknown (the paths of all other vertices are unchanged).  SKIP_K
 // measured on GB300 (graph solve of the 2^24 random game, long-path 2^23):
 // 64: 63.8, 57.8 ms; 32: 62.8, 57.8; 16: 62.0, 57.0; 8: 61.6, 55.5; 4: 61.8,
 // 55.5 ms: shorter segments shorten the steps after the last jump more than
@@ -366,13 +366,30 @@ __device__ __forceinline__ void note_change(const ChangeList &c, int32_t v)
     if (p < c.cap) c.list[p] = v;
 }
 
+// Whether the coming full evaluation writes landmark records: a sixth to a
+// quarter of its time (2^24: 0.86 -> 0.64 ms), which pays where the comparisons
+// walk much (one switch step of 2^24 vertices with 5*10^7 jumps and steps 1.9
+// ms, without them over 5).  So it does when the last switch step took more
+// than n / 2 steps, or with records n / 8 jumps and steps, or a single vertex
+// had far to walk.  ms per solve, always -> so: 2^24 random games 32.9, 40.2,
+// 41.3, 37.5 -> 30.9, 38.8, 38.9, 35.7 (never: 31.5, 48.5, 38.7, 35.9), long-path
+// 2^23 17.6 -> 15.3, 256 games 16.9 -> 16.1; n and n / 8, n / 2 and n / 4, n / 8 and
+// n / 16 are within 2% of it.
+__device__ __forceinline__ bool want_landmarks(const EvalGates *g, const unsigned long long *sw, int32_t n)
+{
+    return g->lm_far || sw[1] > (unsigned long long)(g->lm_have ? n / 8 : n / 2);
+}
+
 // Before an evaluation (one thread): decides between a patch and the full
 // evaluation (patch_kernels.cu) and resets what either starts from.
 __device__ __forceinline__ void patch_begin(const PatchArgs &a)
 {
     EvalGates *g = a.g;
     ++*a.epoch;
-    if (*a.quiet > 0) --*a.quiet;
+    const bool fresh = *a.quiet > 0;   // after a reset: the statistics are of another solve
+    if (fresh) --*a.quiet;
+    g->lm_want = !fresh && want_landmarks(g, a.sw, a.n);
+    g->lm_far = 0;
     const int32_t cc = g->ccount;
     g->ccount = 0;   // the next switch steps list their changes afresh
     g->csnap = cc;

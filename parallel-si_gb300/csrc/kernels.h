@@ -51,6 +51,16 @@ struct EvalGates {
     int32_t skip = 0, backoff = 1;            // evaluations not to try a patch after a failed one
     int32_t mfrom[2] = {0, 0};   // per player: unreached-list index its next mark_solved scans from
     uint32_t mdone = 0;          // blocks of the running mark_solved that have finished
+    // landmark records (device_common.cuh): the next full evaluation is to write
+    // them, the last one has, a comparison since the last evaluation walked far
+    int32_t lm_want = 0, lm_have = 0, lm_far = 0;
+};
+
+// Landmark records as a switch step sees them.
+struct Landmarks {
+    const int4 *skip = nullptr;
+    const int32_t *have = nullptr;   // EvalGates::lm_have
+    int32_t *far = nullptr;          // EvalGates::lm_far
 };
 
 // A list of the vertices whose strategy a switch step changes (appended while
@@ -138,7 +148,9 @@ struct EvalArgs {
     int32_t *st = nullptr;        // status words (frozen where solved)
     PathNode *node = nullptr;
     int32_t *rdeep = nullptr;     // counts of paths too long for the record's word (n entries)
-    int4 *skip = nullptr;         // landmark skips (device_common.cuh)
+    int4 *skip = nullptr;         // landmark skips (device_common.cuh), written if g->lm_want
+    EvalGates *g = nullptr;
+    const unsigned long long *sw = nullptr;   // the last switch step's statistics (launch_switch)
     const uint32_t *epoch = nullptr;   // evaluation number (launch_patch_begin advances it)
     int32_t *key = nullptr;       // comparison keys
     int32_t *ulist = nullptr, *ucount = nullptr;   // the vertices the sink does not reach (*ucount 0 on entry)
@@ -262,7 +274,7 @@ void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t pla
                    unsigned long long *gcount, const int32_t *gmask, uint32_t *err,
                    const int32_t *gate = nullptr, uint8_t *need = nullptr, int32_t *list = nullptr,
                    int32_t *list_count = nullptr, ChangeList changes = ChangeList(), uint8_t *tie = nullptr,
-                   uint8_t *watch = nullptr, const int4 *skip = nullptr, bool warp = false,
+                   uint8_t *watch = nullptr, Landmarks marks = Landmarks(), bool warp = false,
                    uint32_t *claim = nullptr, const int8_t *owner = nullptr, int32_t n_all = 0,
                    bool count_moves = true, uint32_t *list_done = nullptr, const MarkArgs *mark = nullptr);
 // ---- batches: per-game accounting of solve_si (state[g] = brs, iters,
@@ -337,6 +349,7 @@ struct PatchArgs {
     unsigned long long *stats = nullptr;   // [0] += 1 per patch, [1] += vertices re-evaluated
     ChangeTrack track;
     int4 *skip = nullptr;       // landmark skips: a patched vertex's record becomes unknown
+    const unsigned long long *sw = nullptr;   // the last switch step's statistics
     uint32_t *epoch = nullptr;
     int32_t *quiet = nullptr;
 };

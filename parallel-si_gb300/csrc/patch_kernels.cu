@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(kPatchBlock, 1) k_patch(PatchArgs a, cudaGraph
             }
             // re-evaluated: a tied in-neighbour looks again even at an unchanged key
             mode = changed ? 2 : (watched ? 1 : 0);
-            if (a.skip) a.skip[v] = make_int4(SKIP_UNKNOWN, 0, 0, 0);   // its path changed: walks step here
+            if (a.g->lm_have) a.skip[v] = make_int4(SKIP_UNKNOWN, 0, 0, 0);   // its path changed: walks step here
             a.apos[v] = -1;
         }
         flag_in_neighbours(a.track, mode, v, &ev);

@@ -55,7 +55,10 @@ __device__ __forceinline__ int ceil_log2_dev(int64_t x)
 __global__ void k_root_init(EvalArgs a)
 {
     if (a.gate && !*a.gate) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *a.lcount = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *a.lcount = 0;
+        a.g->lm_have = a.g->lm_want;
+    }
     // the evaluation number wraps around: no record of the last round may look current
     const bool wrap = (*a.epoch & kEpochMask) == 0;
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < a.n; v += (int64_t)gridDim.x * blockDim.x) {
@@ -85,9 +88,9 @@ __device__ __forceinline__ void path_depth_count(const EvalArgs &a, int32_t y, i
 
 // Publishes a finite vertex: landmark record, status, summary.
 __device__ __forceinline__ void publish_finite(const EvalArgs &a, int32_t v, int32_t d, int32_t m, int32_t c,
-                                               int32_t anc, const Top2 &seg, uint32_t epoch)
+                                               int32_t anc, const Top2 &seg, uint32_t epoch, bool marks)
 {
-    store_whole(&a.skip[v], skip_pack(anc, seg, epoch));
+    if (marks) store_whole(&a.skip[v], skip_pack(anc, seg, epoch));
     a.st[v] = d;
     if (d >= kDeepPath) a.rdeep[v] = c;
     publish_summary(&a.node[v], m, path_word(d, c), d >= kDeepPath);
@@ -112,6 +115,7 @@ __global__ void __launch_bounds__(kWalkThreads, 8) k_root_walk(EvalArgs a)
     if (a.gate && !*a.gate) return;
     __shared__ int32_t ubuf[kWalkThreads / 32][kUnreachedBuf];
     const uint32_t epoch = *a.epoch & kEpochMask;
+    const bool marks = a.g->lm_want;
     const int lane = threadIdx.x & 31;
     int32_t *buf = ubuf[threadIdx.x >> 5];
     int nbuf = 0;   // uniform over the warp
@@ -135,7 +139,7 @@ __global__ void __launch_bounds__(kWalkThreads, 8) k_root_walk(EvalArgs a)
             if (q.z != RM_POS_INF && q.z != RM_NEG_INF) {   // not solved
                 if (q.x < 0) {   // a child of the sink, published by init: its skip and status are written here
                     a.st[v] = 1;
-                    a.skip[v] = skip_pack(-1, Top2{q.y, 1, -1, 0}, epoch);
+                    if (marks) a.skip[v] = skip_pack(-1, Top2{q.y, 1, -1, 0}, epoch);
                     k = finite_key(q.y, 1);
                     finite = true;
                 } else {
@@ -175,29 +179,32 @@ __global__ void __launch_bounds__(kWalkThreads, 8) k_root_walk(EvalArgs a)
                         top1_merge(m, c, r.z, cy);
                         k = finite_key(m, c);
                         finite = true;
-                        const int32_t d = s + dy, len = d - skip_landmark_depth(d);
+                        const int32_t d = s + dy;
                         a.st[v] = d;
                         if (d >= kDeepPath) a.rdeep[v] = c;
                         publish_summary(&a.node[v], m, path_word(d, c), d >= kDeepPath);
                         // the segment from v to its landmark: by steps (the walk has just read
                         // them) up to y, then y's record if the landmark lies beyond and the
                         // record has arrived (its summary may have come first), else by steps
-                        Top2 seg = {q.y, 1, -1, 0};
-                        int32_t anc = q.x;
-                        for (int32_t i = 1; i < len; i++) {
-                            if (i == s) {
-                                const int4 sy = load_whole(&a.skip[y]);
-                                if (sy.x != SKIP_UNKNOWN && skip_epoch(sy.w) == epoch) {
-                                    skip_merge(seg, sy);
-                                    anc = sy.x;
-                                    break;
+                        if (marks) {
+                            const int32_t len = d - skip_landmark_depth(d);
+                            Top2 seg = {q.y, 1, -1, 0};
+                            int32_t anc = q.x;
+                            for (int32_t i = 1; i < len; i++) {
+                                if (i == s) {
+                                    const int4 sy = load_whole(&a.skip[y]);
+                                    if (sy.x != SKIP_UNKNOWN && skip_epoch(sy.w) == epoch) {
+                                        skip_merge(seg, sy);
+                                        anc = sy.x;
+                                        break;
+                                    }
                                 }
+                                const int2 e = *reinterpret_cast<const int2 *>(&a.node[anc]);
+                                top2_add(seg, e.y);
+                                anc = e.x;
                             }
-                            const int2 e = *reinterpret_cast<const int2 *>(&a.node[anc]);
-                            top2_add(seg, e.y);
-                            anc = e.x;
+                            store_whole(&a.skip[v], skip_pack(anc, seg, epoch));
                         }
-                        store_whole(&a.skip[v], skip_pack(anc, seg, epoch));
                     }
                 }
             }
@@ -275,7 +282,9 @@ __device__ void settle_body(const EvalArgs &a, int32_t nl)
                     int32_t dt, ct, m = e.y, c = e.z;
                     path_depth_count(a, t, q.w, dt, ct);
                     top1_merge(m, c, q.z, ct);
-                    const int32_t d = (int32_t)((1u << r) + (uint32_t)dt), len = d - skip_landmark_depth(d);
+                    const bool marks = a.g->lm_want;
+                    const int32_t d = (int32_t)((1u << r) + (uint32_t)dt);
+                    const int32_t len = marks ? d - skip_landmark_depth(d) : 0;
                     Top2 seg = {-1, 0, -1, 0};
                     int32_t anc = u;
                     for (int32_t j = 0; j < len; j++) {
@@ -283,7 +292,7 @@ __device__ void settle_body(const EvalArgs &a, int32_t nl)
                         top2_add(seg, x.y);
                         anc = x.x;
                     }
-                    publish_finite(a, u, d, m, c, anc, seg, *a.epoch & kEpochMask);
+                    publish_finite(a, u, d, m, c, anc, seg, *a.epoch & kEpochMask, marks);
                     k = finite_key(m, c);
                 } else {
                     const int4 f = __ldcg(&in[t]);

@@ -381,7 +381,6 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
         if (!fin && !(o.t & kSolved)) a.ulist[atomicAdd(a.ucount, 1)] = v;   // (none once the loop has converged)
         a.st[v] = fin ? d : (r.x == kPosInf ? ST_POS_INF : ST_NEG_INF);
         if (fin && d >= kDeepPath) a.rdeep[v] = r.z;
-        a.skip[v] = make_int4(SKIP_UNKNOWN, 0, 0, 0);
         *reinterpret_cast<int4 *>(&a.node[v]) =
             fin ? make_int4(q.x, q.y, r.y, path_word(d, r.z))
                 : make_int4(q.x, q.y, r.x == kPosInf ? RM_POS_INF : RM_NEG_INF, 0);
@@ -391,6 +390,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
         a.ctl->brs = brs;
         a.ctl->stop = stop;
         a.ctl->mfrom[0] = a.ctl->mfrom[1] = 0;
+        a.ctl->lm_have = a.ctl->lm_far = 0;
         *a.err = *(volatile uint32_t *)&a.sync->err;
         a.sync->err = 0;
         a.sync->phase = phase;
@@ -606,7 +606,6 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve_small(SolveArgs a)
         a.key[v] = key[v];
         if (!fin && !(c & kSolved)) a.ulist[atomicAdd(a.ucount, 1)] = v;
         a.st[v] = fin ? r.w & kLen : (r.x == kPosInf ? ST_POS_INF : ST_NEG_INF);
-        a.skip[v] = make_int4(SKIP_UNKNOWN, 0, 0, 0);
         *reinterpret_cast<int4 *>(&a.node[v]) =
             fin ? make_int4(q.x, q.y, r.y, path_word(r.w & kLen, r.z))
                 : make_int4(q.x, q.y, r.x == kPosInf ? RM_POS_INF : RM_NEG_INF, 0);
@@ -616,6 +615,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve_small(SolveArgs a)
         a.ctl->brs = brs;
         a.ctl->stop = stop;
         a.ctl->mfrom[0] = a.ctl->mfrom[1] = 0;
+        a.ctl->lm_have = a.ctl->lm_far = 0;
         *a.err = *(volatile uint32_t *)&a.sync->err;
         a.sync->err = 0;
     }
@@ -642,7 +642,10 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_eval_jump(EvalArgs a, Solv
         return __ldcg(&sync->vote[k]) != 0;
     };
     if (tid == 0) {
-        if (*quiet > 0) --*quiet;
+        const bool fresh = *quiet > 0;
+        if (fresh) --*quiet;
+        g->lm_have = !fresh && want_landmarks(g, a.sw, n);
+        g->lm_far = 0;
         g->ccount = g->csnap = 0;
         g->patch = 0;
         g->eval = 1;
@@ -660,6 +663,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_eval_jump(EvalArgs a, Solv
     }
     bool more = true;
     barrier(false);
+    const bool marks = __ldcg(&g->lm_have) != 0;
     for (int pass = 0; more; pass++) {
         if (pass == kMaxPasses) {   // cannot happen: windows grow at least kJumps-fold per pass
             if (tid == 0) atomicOr(a.err, DERR_WALK_CAP);
@@ -685,7 +689,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_eval_jump(EvalArgs a, Solv
                         *reinterpret_cast<int2 *>(&a.node[v].rmax) =
                             fin ? make_int2(r.y, path_word(d, r.z))
                                 : make_int2(r.x == kPosInf ? RM_POS_INF : RM_NEG_INF, 0);
-                        if (fin) {
+                        if (fin && marks) {
                             Top2 seg = {-1, 0, -1, 0};
                             int32_t anc = v;
                             for (int32_t j = d - skip_landmark_depth(d); j > 0; j--) {

@@ -504,6 +504,7 @@ PatchArgs Solver::patch_args()
     a.stats = dw_->patch;
     a.track = track();
     a.skip = skip_;
+    a.sw = dw_->sw;
     a.epoch = &sync_->epoch;
     a.quiet = &ctl_->quiet;
     return a;
@@ -557,6 +558,8 @@ EvalArgs Solver::eval_args()
     a.node = node_;
     a.rdeep = rdeep_;
     a.skip = skip_;
+    a.g = ctl_;
+    a.sw = dw_->sw;
     a.epoch = &sync_->epoch;
     a.key = key_;
     a.ulist = ulist_;
@@ -660,7 +663,7 @@ int Solver::switch_strategy(int32_t player, int64_t *switched, bool count, bool 
     // jB_ is free until the next full evaluation: it holds the list of vertices to examine
     launch_switch(stream_, np, pl, player, off_, tgt_, strat_, st_, key_, node_, rdeep_, dw_->sw, game_of_, gcount_,
                   gmask_, &dw_->err, nullptr, need_, reinterpret_cast<int32_t *>(jB_), &dw_->listcount, changes(), tie_,
-                  watch_, skip_, switch_warp_, &dw_->claim, arena_ ? nullptr : owner_, n_, count,
+                  watch_, landmarks(), switch_warp_, &dw_->claim, arena_ ? nullptr : owner_, n_, count,
                   &dw_->listdone, mark ? &m : nullptr);
     phase_end(PH_SWITCH);
     rc = sync_and_check("switch_strategy");

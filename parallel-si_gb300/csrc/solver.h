@@ -158,6 +158,7 @@ private:
     int enqueue_eval(bool timed, int32_t try_patch);
     int enqueue_patch(bool timed, int32_t try_patch, const cudaGraphConditionalHandle *full = nullptr);
     int enqueue_full(bool timed);
+    Landmarks landmarks() const { return Landmarks{skip_, &ctl_->lm_have, &ctl_->lm_far}; }
     PatchArgs patch_args();
     MarkArgs mark_args(int32_t player);
     EvalArgs eval_args();

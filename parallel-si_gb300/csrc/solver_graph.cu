@@ -173,7 +173,7 @@ int Solver::enqueue_step(cudaGraph_t body, cudaGraphConditionalHandle loop, bool
         const int32_t np = player ? np_ - np0_ : np0_;
         launch_switch(stream_, np, plist_ + (player ? np0_ : 0), player, off_, tgt_, strat_, st_, key_, node_, rdeep_,
                       dw_->sw, batch ? game_of_ : nullptr, gc, nullptr, &dw_->err, player ? nullptr : &ctl_->even,
-                      need_, todo, &dw_->listcount, changes(), tie_, watch_, skip_, switch_warp_, &dw_->claim,
+                      need_, todo, &dw_->listcount, changes(), tie_, watch_, landmarks(), switch_warp_, &dw_->claim,
                       arena_ ? nullptr : owner_, n_, /*count_moves=*/false, &dw_->listdone, &m);
         count_launch();
         if (player)

@@ -42,10 +42,12 @@ inline unsigned grid_for(int64_t items, int block = kBlock)
     return (unsigned)(g < 1 ? 1 : g);
 }
 
+constexpr int32_t kFarWalk = 4096;   // steps after which landmarks are asked for (want_landmarks)
+
 // Even's view of finite u against finite w (u != w) when their keys are
 // equal: the exact summaries decide, else a walk to the lowest common
 // ancestor (w = -1 is the sink).
-__device__ int compare_equal_keys(const PathNode *__restrict__ node, const int4 *__restrict__ skip,
+__device__ int compare_equal_keys(const PathNode *__restrict__ node, const Landmarks &marks,
                                   const int32_t *__restrict__ st, const int32_t *__restrict__ rdeep, int32_t u, int32_t w, int32_t &loads,
                                   uint32_t *__restrict__ err)
 {
@@ -63,7 +65,11 @@ __device__ int compare_equal_keys(const PathNode *__restrict__ node, const int4 
     }
     if (ru.x != rw.x) return ru.x > rw.x ? decide(ru.x, cu, 0) : decide(rw.x, 0, cw);
     if (cu != cw) return decide(ru.x, cu, cw);
-    return lean_compare<true>(node, skip, u, du, w, dw, loads, INT_MAX, err);
+    const int32_t before = loads;
+    const int c = marks.skip ? lean_compare<true>(node, marks.skip, u, du, w, dw, loads, INT_MAX, err)
+                             : lean_compare<false>(node, nullptr, u, du, w, dw, loads, INT_MAX, err);
+    if (loads - before > kFarWalk) *marks.far = 1;
+    return c;
 }
 
 // One thread per vertex of plist (all owned by `player`).  Per compared edge
@@ -198,10 +204,11 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
                                                    uint32_t *__restrict__ err,
                                                    const int32_t *__restrict__ gate, uint8_t *__restrict__ need,
                                                    ChangeList changes, uint8_t *__restrict__ tie_out,
-                                                   uint8_t *__restrict__ watch, const int4 *__restrict__ skip,
+                                                   uint8_t *__restrict__ watch, Landmarks marks,
                                                    uint32_t *__restrict__ claim, uint32_t *__restrict__ list_done)
 {
     if (gate && !*gate) return;
+    if (!*marks.have) marks.skip = nullptr;
     if (count) np = *(volatile int32_t *)count;
     // a block past the list's end has nothing to count either (uniform per
     // block: the block reduction below is never left waiting)
@@ -320,7 +327,7 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
                         if (next_tied(ties, j) >= e1 - e0) break;
                         const int32_t u = tgt[e0 + j];
                         if (u == cur || (j >= 32 && key[u] != ext)) continue;
-                        const int c = compare_equal_keys(node, skip, st, rdeep, u, cur, t_loads, err);
+                        const int c = compare_equal_keys(node, marks, st, rdeep, u, cur, t_loads, err);
                         if ((player == 0) ? c > 0 : c < 0) cur = u;
                     }
                 }
@@ -344,7 +351,7 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
                     int c;
                     if (ku != kc) c = ku > kc ? 1 : -1;
                     else if (u == cur || key_infinite(ku)) c = 0;
-                    else c = compare_equal_keys(node, skip, st, rdeep, u, cur, t_loads, err);
+                    else c = compare_equal_keys(node, marks, st, rdeep, u, cur, t_loads, err);
                     if ((player == 0 && c > 0) || (player == 1 && c < 0)) {
                         cur = u;
                         kc = ku;
@@ -434,10 +441,11 @@ __global__ void __launch_bounds__(kBlock) k_switch_warp(int32_t np, const int32_
                                                         uint32_t *__restrict__ err,
                                                         const int32_t *__restrict__ gate, uint8_t *__restrict__ need,
                                                         ChangeList changes, uint8_t *__restrict__ tie_out,
-                                                        uint8_t *__restrict__ watch, const int4 *__restrict__ skip,
+                                                        uint8_t *__restrict__ watch, Landmarks marks,
                                                         uint32_t *__restrict__ list_done)
 {
     if (gate && !*gate) return;
+    if (!*marks.have) marks.skip = nullptr;
     if (count) np = *(volatile int32_t *)count;
     // a block past the list's end has nothing to count either (uniform per block)
     if ((int64_t)blockIdx.x * blockDim.x >= np) {
@@ -578,7 +586,7 @@ __global__ void __launch_bounds__(kBlock) k_switch_warp(int32_t np, const int32_
                 int cmp;
                 if (ku != kc) cmp = ku > kc ? 1 : -1;
                 else if (uu == cur || key_infinite(ku)) cmp = 0;
-                else cmp = compare_equal_keys(node, skip, st, rdeep, uu, cur, t_loads, err);
+                else cmp = compare_equal_keys(node, marks, st, rdeep, uu, cur, t_loads, err);
                 if ((player == 0 && cmp > 0) || (player == 1 && cmp < 0)) {
                     cur = uu;
                     kc = ku;
@@ -692,7 +700,7 @@ void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t pla
                    const int32_t *rdeep, unsigned long long *stats, const int32_t *game_of, unsigned long long *gcount,
                    const int32_t *gmask, uint32_t *err, const int32_t *gate, uint8_t *need,
                    int32_t *list, int32_t *list_count, ChangeList changes, uint8_t *tie, uint8_t *watch,
-                   const int4 *skip, bool warp, uint32_t *claim, const int8_t *owner, int32_t n_all, bool count_moves,
+                   Landmarks marks, bool warp, uint32_t *claim, const int8_t *owner, int32_t n_all, bool count_moves,
                    uint32_t *list_done, const MarkArgs *mark)
 {
     const MarkArgs m = mark ? *mark : MarkArgs();
@@ -724,12 +732,12 @@ void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t pla
     count_launch();
     if (warp)
         k_switch_warp<<<g, kBlock, 0, s>>>(np, list, list_count, player, off, tgt, strat, st, key, node, rdeep, stats,
-                                           game_of, gcount, gmask, err, gate, need, changes, tie, watch, skip,
+                                           game_of, gcount, gmask, err, gate, need, changes, tie, watch, marks,
                                            list_done);
     else
         (count_moves ? k_switch<true> : k_switch<false>)<<<g, kBlock, 0, s>>>(
             np, list, list_count, player, off, tgt, strat, st, key, node, rdeep, stats, game_of, gcount, gmask, err,
-            gate, need, changes, tie, watch, skip, claim, list_done);
+            gate, need, changes, tie, watch, marks, claim, list_done);
 }
 
 void launch_batch_account(cudaStream_t s, int32_t games, int32_t event, int4 *state, unsigned long long *gcount)

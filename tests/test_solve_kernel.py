@@ -162,3 +162,20 @@ def test_ties_at_any_place_of_a_list(deg, mode):
         assert np.array_equal(s.get_infinite(), ref.get_infinite())
     s.close()
     ref.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,pri", [(20000, 2), (100000, 6), (300000, 4), (300000, 60)])
+def test_landmarks_come_and_go(n, pri):
+    """The graph's evaluations write landmark records only after a switch step
+    that walked more than n / 2 steps (n / 8 with them) or far from one vertex:
+    games with few priorities cross both ways.  Against the persistent solver,
+    whose comparisons step; in full every time and with patches in between."""
+    g = psi.Game.random(n, 2, 5, pri, n + pri)
+    ref = psi.GPUList(g)
+    for kw in (dict(incremental=2), dict(incremental=0, switch_kernel=1), dict(incremental=2, graph=0)):
+        s = psi.GPUList(g, **kw)
+        for _ in range(2):
+            _same(_solved(s), _solved(ref))
+        s.close()
+    ref.close()
