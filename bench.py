@@ -11,9 +11,9 @@ stream).  e2e repeats the solve through the C ABI from page-locked host buffers
 (psi_host_alloc): upload of the game, the solve, and the read-back of the
 winning set and strategy are inside the timed region.  Prints one JSON line (rank 0).
 
-Before its warm-up the bench lets psi_autotune choose the sublist stride, the
-sublist walk's block size and the patch limit by timing trial solves of the
-same workload (--no-tune takes them from the flags); none of them changes a
+Before its warm-up the bench lets psi_autotune choose the patch limit (and the
+two options of the tour's list ranking, which change nothing any more) by timing
+trial solves of the same workload (--no-tune takes them from the flags); none of them changes a
 result.  After its timed regions it measures the random-access bound
 (psi_measure_random_access) at the size of the array the switch reads at
 random, and reports the kernel against it beside the
@@ -237,7 +237,7 @@ def random_accesses(phase, n, counters, n_even, n_odd, iters, brs):
     phase is a chase or a gather: the sublist walk reads one successor per
     tour node and writes one (sublist, prefix) entry per vertex; the switch
     gathers the key of every compared successor and of each vertex's current
-    choice, loads a parent per walk step, and sets two dirty flags per
+    choice, loads a parent per walk step, and writes two flags (need, tie) per
     changed vertex."""
     L = 2 * n + 2
     if phase == "sublist":
@@ -271,7 +271,7 @@ def phase_bytes(phase, n, m, nsub, counters, calls, n_even, n_odd, iters, brs):
         # per vertex of the player: plist, strategy, offsets, key of the current
         # choice (4 B each); per compared edge: target id and its key (8 B);
         # per walk step: parent and priority (8 B); per changed vertex: the
-        # strategy write and two dirty flags (6 B)
+        # strategy write and two flags (need, tie; 6 B)
         sw_calls = max(1, counters["switches"])
         player_vertices = brs * n_odd + iters * n_even
         total = (16 * player_vertices + 8 * counters["sw_edges"] + 8 * counters["sw_loads"]

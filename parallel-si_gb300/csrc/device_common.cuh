@@ -267,7 +267,7 @@ constexpr int kMaxBlockWarps = 32;
 // Block-aggregated append: every thread of the block calls it (no early
 // return before); one atomic on the shared counter per block instead of one
 // per warp, which serialises when most warps append (the sink's children,
-// the unreached vertices, the dirty parents).
+// the unreached vertices).
 __device__ __forceinline__ void block_append(bool flag, int32_t value, int32_t *__restrict__ list,
                                              int32_t *__restrict__ count)
 {

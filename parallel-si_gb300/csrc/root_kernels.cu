@@ -19,7 +19,8 @@
 //     meeting it again means one round of the cycle, whose top priority was
 //     collected since) -- the cycle parity of cpu_parity.cpp:35-52, 80-104.
 //     With threads in arbitrary order a walk is short: about two steps on
-//     random games, whose paths are 12 vertices long on average.
+//     random games, whose paths are 12 vertices long on average (ten for the
+//     longest of a warp's walks).  Landmark records only where wanted.
 //  3. k_root_settle: walks that did not end within kWalkCap steps (deep
 //     chains, long cycles, none on random games) are finished by pointer
 //     jumping over those vertices alone.
@@ -103,13 +104,16 @@ constexpr int kWalkThreads = 256;
 // atomic (one atomic per warp and pass on the list's counter would serialise)
 constexpr int kUnreachedBuf = 128;
 
-// Bound by the latency of dependent loads (2^22 random game: DRAM 25%, L2 32%,
-// issue slots 45% busy), so by how many walks are in flight: eight blocks per
-// SM at 32 registers; a summary is stored as soon as it is known and without a
+// Bound by dependent random reads (2^22 random game: DRAM 40%, L2 36%, issue
+// slots 60% busy; 2^24: 2.9 GB in 670 us, 4.1 TB/s), so eight blocks per SM at
+// 32 registers; a summary is stored as soon as it is known and without a
 // release (which waits for the thread's earlier stores: a third of the stalls),
-// the landmark record after it and tagged with the evaluation's number.  Walks
-// and init of a 2^24 solve 17.6 -> 14.1 ms (17 full evaluations), long-path
-// 11.0 -> 8.9 ms.
+// the landmark record, where wanted, after it and tagged with the evaluation's
+// number.  Walks and init of a 2^24 solve 17.6 -> 14.1 ms (17 full evaluations),
+// long-path 11.0 -> 8.9 ms, without landmark records 11.5 and 5.8.  Lanes that
+// take the next vertex as soon as their walk ends lose (solve 35.3 -> 35.6,
+// long-path 18.3 -> 20.5 ms): a walk's end is 60 instructions that then run at
+// almost every step.
 __global__ void __launch_bounds__(kWalkThreads, 8) k_root_walk(EvalArgs a)
 {
     if (a.gate && !*a.gate) return;

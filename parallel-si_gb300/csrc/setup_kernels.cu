@@ -1,6 +1,6 @@
 // setup_kernels.cu -- device set-up of a game and ordered selections: the
 // reverse CSR (distinct in-neighbours of every vertex, in increasing order)
-// that the tour build scans to link each parent's children without atomics,
+// that change tracking and patches follow from a changed vertex,
 // the owner narrowing and player lists built at upload, and the winning-set
 // selection read back at the end of a solve.
 #include <cub/block/block_reduce.cuh>

@@ -28,11 +28,10 @@
 //    writes the next evaluation's initial records, into the other of two
 //    buffers (comparisons still read the current ones).  The paths that
 //    comparisons walk change at the start of the jump phase.
-//  - Comparisons that walk far (equal summaries, paths that meet late) would
-//    hold up a whole phase, 30 to 500 us where the others take 5.  A vertex
-//    whose walks pass their budget of steps is left over; only if there are any, all
-//    threads write landmark records (device_common.cuh) and those vertices
-//    are done again with them.
+//  - Comparisons that walk far (equal summaries, paths that meet late) hold
+//    up a whole phase.  A vertex whose walks pass their budget of steps is left
+//    over; only if there are any, all threads write landmark records
+//    (device_common.cuh) and those vertices are done again with them.
 //
 // A thread owns the same vertices in every phase (plist[tid], plist[tid +
 // threads], ...), so what a vertex's phases start from -- its id, CSR range,

@@ -3,11 +3,11 @@
 // solves of that very workload on the device.
 //
 // None of the three knobs changes a result (every evaluation is exact, and a
-// patch gives the full evaluation's values), only the time: the stride trades
-// the walks' length against the size of the reduced list, the walk's block
-// size sets how its one-thread-per-sublist grid fills the SMs, and the patch
-// limit decides which switch steps are followed by a patch instead of a full
-// evaluation.  The reference fixes the stride at 64 (gpu_list_ranking.cu:19)
+// patch gives the full evaluation's values), only the time: the patch limit
+// decides which switch steps are followed by a patch instead of a full
+// evaluation.  The stride and the block size describe the list ranking of a
+// tour, which solvers no longer build; they are tried as before and change
+// nothing.  The reference fixes the stride at 64 (gpu_list_ranking.cu:19)
 // and has no incremental evaluation.
 //
 // Search: coordinate descent from the defaults, one knob at a time in the
