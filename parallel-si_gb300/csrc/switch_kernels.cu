@@ -187,8 +187,16 @@ __global__ void k_need_ids(int32_t n, int32_t player, const int8_t *__restrict__
 // the caller wants the number of strict improvements the scan makes, compares
 // equal keys on the way there too; otherwise a changed vertex counts as one.
 // With that and lean_compare for the walks, switch steps of the 2^24 random
-// game 12.0 -> 10.5 ms per solve (long-path 7.05 -> 6.85); 48, 40 or 32
-// registers instead of 64 measured 10.7, 10.9 and 11.0 ms.
+// game 12.0 -> 10.5 ms per solve (long-path 7.05 -> 6.85).  Blocks per SM: four
+// (64 registers) without COUNT, ms per solve against the five of 48 registers
+// and spills that the compiler chose: 2^24 30.8, 38.3, 38.6 -> 30.2, 37.5, 38.2,
+// long-path 2^23 14.7 -> 14.45; three (79 registers) with COUNT: 2^18 to 4*10^5
+// vertices step by step 2% faster than four.
+// COUNT's comparisons go from tie to tie too (a mask, as without): what the
+// scan's choice is at a tie follows from the places that set the best key
+// before it.  Step by step at 2*10^4, 5*10^4, 4*10^5 vertices and 5*10^4 with 8
+// priorities 2110, 2430, 5660, 4200 -> 1990, 2270, 5300, 3770 us against redoing
+// such a vertex successor by successor (kept past 32 successors).
 template <bool COUNT>
 __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__restrict__ plist,
                                                    int32_t *__restrict__ count, int32_t player,
@@ -271,17 +279,18 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
             // distinct vertex attains it (a tie)
             int32_t ext = kc, ext_v = cur;
             bool tie = false;
-            uint32_t ties = 0;   // which of the first 32 successors attain it, besides the first that does
-            // Fast pass: successors in batches of kBatch -- all ids, then all
+            // which of the first 32 successors attain it, besides the first that
+            // does; with COUNT, which attain the best key up to their place, and
+            // which set it
+            uint32_t ties = 0, sets = 0;
+            // Key pass: successors in batches of kBatch -- all ids, then all
             // keys, before the comparisons (independent gathers in flight per
-            // thread).  Equal keys of distinct finite vertices end it; the exact
-            // pass then redoes the vertex with summaries and walks.  Five
-            // per batch (one batch for out-degrees up to 5): switch steps
-            // 12.6 -> 12.1 ms per 2^24 solve against four; six the same as five.
+            // thread).  Five per batch (one batch for out-degrees up to 5): switch
+            // steps 12.6 -> 12.1 ms per 2^24 solve against four; six the same as five.
             constexpr int kBatch = 5;
             const int32_t cur0 = cur, kc0 = kc;
             bool exact = false;
-            for (int32_t eb = e0; eb < e1 && !exact; eb += kBatch) {
+            for (int32_t eb = e0; eb < e1; eb += kBatch) {
                 const int32_t cnt = min(kBatch, e1 - eb);
                 int32_t us[kBatch], ks[kBatch];
     #pragma unroll
@@ -291,37 +300,25 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
     #pragma unroll
                 for (int j = 0; j < kBatch; j++) {
                     if (j >= cnt) break;
-                    const int32_t u = us[j], ku = ks[j];
+                    const int32_t u = us[j], ku = ks[j], at = eb - e0 + j;
                     if ((player == 0) ? ku > ext : ku < ext) {
                         ext = ku;
                         ext_v = u;
                         tie = false;
-                        ties = 0;
+                        if (!COUNT) ties = 0;
+                        else if (at < 32) sets |= 1u << at;
+                        moves++;
                     } else if (ku == ext && u != ext_v) {
                         tie = true;
-                        if (!COUNT && eb - e0 + j < 32) ties |= 1u << (eb - e0 + j);
-                    }
-                    if (!COUNT) continue;
-                    int c;
-                    if (ku != kc) {
-                        c = ku > kc ? 1 : -1;
-                    } else if (u == cur || key_infinite(ku)) {
-                        c = 0;
-                    } else {
-                        exact = true;
-                        break;
-                    }
-                    if ((player == 0 && c > 0) || (player == 1 && c < 0)) {
-                        cur = u;
-                        kc = ku;
-                        moves++;
+                        if (at < 32) ties |= 1u << at;
+                        if (COUNT && !key_infinite(ku)) exact = true;
                     }
                 }
             }
+            // the first vertex at the best key, then exact comparisons with the
+            // others that share it (none for an infinity)
+            cur = ext_v;
             if (!COUNT) {
-                // the first vertex at the best key, then exact comparisons with the
-                // others that share it (none for an infinity)
-                cur = ext_v;
                 if (tie && !key_infinite(ext)) {
                     for (int32_t j = 0;; j++) {
                         if (next_tied(ties, j) >= e1 - e0) break;
@@ -332,22 +329,32 @@ __global__ void __launch_bounds__(kBlock) k_switch(int32_t np, const int32_t *__
                     }
                 }
                 moves = cur != cur0 ? 1 : 0;
+            } else if (exact && e1 - e0 <= 32) {
+                // the scan again, from tie to tie: each against the choice up to
+                // there, the last vertex that set the best key or one that won since
+                int32_t set = -1;
+                cur = cur0;
+                for (; ties; ties &= ties - 1) {
+                    const int32_t j = __ffs(ties) - 1, before = 31 - __clz(sets & ((1u << j) - 1));   // -1: none
+                    if (before != set) {
+                        set = before;
+                        cur = tgt[e0 + set];
+                    }
+                    const int32_t u = tgt[e0 + j];
+                    if (u == cur || key_infinite(key[u])) continue;
+                    const int c = compare_equal_keys(node, marks, st, rdeep, u, cur, t_loads, err);
+                    if ((player == 0) ? c > 0 : c < 0) {
+                        cur = u;
+                        moves++;
+                    }
+                }
+                if (31 - __clz(sets) != set) cur = ext_v;   // set after the last tie
             } else if (exact) {
                 cur = cur0;
                 kc = kc0;
                 moves = 0;
-                ext = kc0;
-                ext_v = cur0;
-                tie = false;
                 for (int32_t e = e0; e < e1; e++) {
                     const int32_t u = tgt[e], ku = key[u];
-                    if ((player == 0) ? ku > ext : ku < ext) {
-                        ext = ku;
-                        ext_v = u;
-                        tie = false;
-                    } else if (ku == ext && u != ext_v) {
-                        tie = true;
-                    }
                     int c;
                     if (ku != kc) c = ku > kc ? 1 : -1;
                     else if (u == cur || key_infinite(ku)) c = 0;
@@ -678,14 +685,15 @@ __global__ void k_materialize(int32_t v0, int32_t count, int32_t d, const int32_
     }
 }
 
-std::atomic<int> g_switch_blocks[kMaxCachedDevices];
+std::atomic<int> g_switch_blocks[2][kMaxCachedDevices];   // COUNT
 
+template <bool COUNT>
 int switch_grid()
 {
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_switch<true>, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_switch<COUNT>, kBlock, 0);
     // one wave of resident blocks: the chunk claims balance the work, and
     // fewer blocks reduce fewer counters (switch steps 13.2 -> 12.6 ms per
     // 2^24 solve against four waves)
@@ -709,7 +717,9 @@ void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t pla
         if (mark) launch_mark_solved(s, m);
         return;
     }
-    const int blocks = per_device(g_switch_blocks, switch_grid);   // one wave of resident blocks
+    // one wave of resident blocks
+    const int blocks = count_moves ? per_device(g_switch_blocks[1], switch_grid<true>)
+                                   : per_device(g_switch_blocks[0], switch_grid<false>);
     unsigned g = grid_for(np);
     g = g < (unsigned)blocks ? g : (unsigned)blocks;
     // only the vertices whose need flag is set (ChangeTrack)

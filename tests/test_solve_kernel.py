@@ -10,6 +10,7 @@ import pytest
 import oracle
 import psi
 from games import make
+from lockstep import lockstep
 from test_root_walk import paths_game
 
 PSI_ERR_LIMIT = 8
@@ -160,6 +161,7 @@ def test_ties_at_any_place_of_a_list(deg, mode):
         assert s.solve(reset=reset) == ref.solve(reset=reset)
         assert np.array_equal(s.get_strategy(), ref.get_strategy())
         assert np.array_equal(s.get_infinite(), ref.get_infinite())
+    lockstep(s, ref, rows=False)              # and the number of strict improvements of every step
     s.close()
     ref.close()
 
