@@ -612,7 +612,7 @@ int launch_cycles(cudaStream_t s, const int32_t *ucount, const int32_t *ulist, c
 void launch_mark_solved(cudaStream_t s, const MarkArgs &m)
 {
     count_launch();
-    k_mark_solved<<<608, kBlock, 0, s>>>(m);
+    k_mark_solved<<<kMarkBlocks, kBlock, 0, s>>>(m);
 }
 
 }  // namespace psi

@@ -248,6 +248,7 @@ struct MarkArgs {
     int32_t *from = nullptr;
     uint32_t *done = nullptr;
 };
+constexpr int kMarkBlocks = 608;   // blocks of a mark_solved that has a launch of its own
 void launch_mark_solved(cudaStream_t s, const MarkArgs &m);
 
 // ---- all-switches (gpu_parity.cu:191-317, cpu_parity.cpp:154-263)

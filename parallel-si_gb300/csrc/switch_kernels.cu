@@ -100,6 +100,15 @@ __device__ __forceinline__ void need_prelude(uint32_t *claim, unsigned long long
     if (mark.ucount) mark_solved_pass(mark);
 }
 
+// The same for a player without vertices, gated as its list would be: in the
+// solve graph Even's mark_solved waits for Odd's best response also where no
+// vertex is Even's.
+__global__ void k_need_none(const int32_t *__restrict__ gate, unsigned long long *__restrict__ stats, MarkArgs mark)
+{
+    if (gate && !*gate) return;
+    need_prelude(nullptr, stats, mark);
+}
+
 // The switch kernels' last block clears the list's counter for the next step:
 // every block calls it at its end, all its threads having read the counter.
 __device__ __forceinline__ void list_used(int32_t *count, uint32_t *done)
@@ -720,8 +729,8 @@ void launch_switch(cudaStream_t s, int32_t np, const int32_t *plist, int32_t pla
 {
     const MarkArgs m = mark ? *mark : MarkArgs();
     if (np <= 0) {
-        cudaMemsetAsync(stats, 0, 4 * sizeof(unsigned long long), s);
-        if (mark) launch_mark_solved(s, m);
+        count_launch();
+        k_need_none<<<mark ? kMarkBlocks : 1, kBlock, 0, s>>>(gate, stats, m);
         return;
     }
     // one wave of resident blocks

@@ -1,0 +1,95 @@
+"""The solve graph and the warp-cooperative switch on the edge games: single
+games below 2^20 vertices go to the persistent solver by default, so here they
+take the graph as a batch, with patches always, with the warp kernel, or padded
+to more than 2^20 vertices with Odd self-loops.  Each against the oracle, in
+counts, strategy and winning sets."""
+import numpy as np
+import pytest
+
+import oracle
+import psi
+from test_edge_cases import EDGE_GAMES
+
+
+def odd_leaves_even_loop():
+    """Odd's first choice leads to a loop Even wins, its other one to a loop
+    Odd wins: +inf until Odd's first switch, and no vertex is Even's."""
+    return psi.Game.from_csr([1, 1, 1], [0, 2, 1], [0, 2, 3, 4], [1, 2, 1, 2])
+
+
+def odd_leaves_even_loop_late(n=40):
+    """The same at the end of a chain: v0's better choice is a chain of Odd
+    vertices whose last one moves first."""
+    succ = [[1, 3], [1], [2]] + [[i + 1] for i in range(3, n - 1)] + [[1, 2]]
+    off = np.cumsum([0] + [len(x) for x in succ]).astype(np.int32)
+    pri = np.zeros(n, np.int32)
+    pri[[1, 2]] = 2, 1
+    return psi.Game.from_csr(np.ones(n, np.int32), pri, off, np.array([u for x in succ for u in x], np.int32))
+
+
+GAMES = {k: f for k, f in EDGE_GAMES.items() if k != "empty"}
+GAMES["odd_leaves_even_loop"] = odd_leaves_even_loop
+GAMES["odd_leaves_even_loop_late"] = odd_leaves_even_loop_late
+
+
+def padded(g, n):
+    """g and Odd self-loops of odd priority up to n vertices."""
+    owner, pri, off, tgt = g.csr()
+    k = n - g.n
+    return psi.Game.from_csr(np.concatenate([owner, np.ones(k, np.int32)]), np.concatenate([pri, np.ones(k, np.int32)]),
+                             np.concatenate([off, off[-1] + 1 + np.arange(k, dtype=np.int32)]),
+                             np.concatenate([tgt, g.n + np.arange(k, dtype=np.int32)]))
+
+
+def expected(g, reset=False):
+    ref = oracle.Sparse(*g.csr())
+    out = ref.solve(reset=reset), ref.get_strategy(), ref.get_winning(0), ref.get_winning(1)
+    ref.close()
+    return out
+
+
+def same(got, want):
+    assert got[0] == want[0]
+    for x, y in zip(got[1:], want[1:]):
+        assert np.array_equal(x, y)
+
+
+def solved(s, reset=False):
+    return s.solve(reset=reset), s.get_strategy(), s.get_winning(0), s.get_winning(1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw", [dict(incremental=2), dict(switch_kernel=1), dict(incremental=2, graph=0),
+                                dict(incremental=0, switch_kernel=1)])
+@pytest.mark.parametrize("name", sorted(GAMES))
+def test_graph_solves_match_the_oracle(name, kw):
+    g = GAMES[name]()
+    s = psi.GPUList(g, **kw)
+    for reset in (False, True):
+        same(solved(s, reset), expected(g, reset))
+    s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("names", [[k] for k in sorted(GAMES)] + [
+    ["all_odd", "odd_leaves_even_loop", "odd_self_loop_even"], ["all_even", "even_self_loop_odd"], sorted(GAMES)])
+@pytest.mark.parametrize("graph", [0, 1])
+def test_batches_match_the_oracle(names, graph):
+    games = [GAMES[k]() for k in names]
+    b = psi.Batch(games, graph=graph)
+    for _ in range(2):
+        iters, brs = b.solve()
+        for k, g in enumerate(games):
+            same(((iters[k], brs[k]), b.get_strategy(k), b.get_winning(k, 0), b.get_winning(k, 1)), expected(g))
+    b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["all_odd", "all_even", "odd_leaves_even_loop", "odd_leaves_even_loop_late", "two_cycle",
+                                  "cycle_forest", "odd_self_loop_even"])
+def test_large_games_match_the_oracle(name):
+    g = padded(GAMES[name](), (1 << 20) + 1)
+    s = psi.GPUList(g)
+    for reset in (False, True):
+        same(solved(s, reset), expected(g, reset))
+    s.close()
