@@ -51,6 +51,7 @@
 #include "jump.cuh"
 #include "kernels.h"
 #include "solver.h"
+#include "spread.h"
 
 namespace cg = cooperative_groups;
 
@@ -80,7 +81,6 @@ __device__ __forceinline__ int compare_tied(const int4 *jump, const int2 *path, 
                 : lean_compare<false>(path, skip, u, ru.w & kLen, w, rw.w & kLen, loads, budget, err);
 }
 
-constexpr int kSolveThreads = 1024;
 // A vertex's choice word: (choice + 1) << kChoiceShift and bits.  Solved; its
 // path touched since Even's last examination, since the last evaluation; the
 // infinity its record ended in; its choice changed since the evaluation.  With
@@ -95,7 +95,6 @@ __device__ __forceinline__ int32_t chosen(int32_t t) { return (t >> kChoiceShift
 constexpr int kFirst = 5;       // successors kept per vertex
 constexpr int kWords = 3 + kFirst;
 constexpr int32_t kIdBits = 20, kManySuccessors = (1 << (32 - kIdBits)) - 1;
-constexpr int kMinThreads = 128;
 constexpr int kSmallBytes = 227 * 1024;   // all a block can have
 // Games below this size are solved there.  Solve in us, k_solve -> here: n = 100
 // 96 -> 62, 300 145 -> 91, 1,024 189 -> 152, 1,537 295 -> 263, 2,048 235 -> 241,
@@ -727,25 +726,6 @@ static int device_sms()
         cudaDeviceGetAttribute(&x, cudaDevAttrMultiProcessorCount, dev);
         return x > 0 ? x : 1;
     });
-}
-
-// Threads per block that spread n vertices evenly over all SMs, at least
-// kMinThreads (n = 10^4: 0.63 ms per solve in ten blocks of 1,024, 0.53 ms in 79
-// of 128), and over as few vertices per thread as the SMs hold, evenly too: the
-// same for all threads, where blocks of 1,024 left SMs or most threads of the
-// last round idle (us per solve at 10^5, 1.8*10^5, 2^18, 3.5*10^5, 10^6 vertices:
-// 859, 1256, 1376, 1270, 4030 -> 801, 1123, 1307, 1228, 3990).  one_each: past so
-// many vertices per SM two per thread are better than one.  k_solve's are from
-// 600 (1.5*10^5: 1080 -> 1023; 10^5: 801 -> 771; 9*10^4 the same; three per thread
-// lose: 2^18 1307 -> 1500); a single evaluation's are not (15 to 20 calls at
-// 1.2*10^5: 2.58 -> 2.74 ms).
-constexpr int kOneEach = 600;
-static int spread_threads(int64_t n, int sms, int one_each)
-{
-    int64_t each = ceil_div(n, (int64_t)kSolveThreads * sms);
-    if (each == 1 && n > (int64_t)one_each * sms) each = 2;
-    const int64_t threads = 32 * ceil_div(ceil_div(n, sms * each), 32);
-    return (int)(threads > kMinThreads ? threads : kMinThreads);
 }
 
 int launch_eval_jump(cudaStream_t s, const EvalArgs &a, SolveSync *sync, EvalGates *g, int32_t *quiet)
