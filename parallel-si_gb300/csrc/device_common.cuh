@@ -366,6 +366,12 @@ __device__ __forceinline__ void note_change(const ChangeList &c, int32_t v)
     if (p < c.cap) c.list[p] = v;
 }
 
+// What a solver keeps of its count of grid barriers between launches
+// (SolveSync): phase k votes in word k % 3, so the remainder.  The count itself
+// would wrap around at 2^32, no multiple of 3, and two phases in a row, one of
+// which clears the other's votes, would share a word.
+__host__ __device__ __forceinline__ uint32_t kept_phase(uint32_t phase) { return phase % 3; }
+
 // Whether the coming full evaluation writes landmark records: a sixth to a
 // quarter of its time (2^24: 0.86 -> 0.64 ms), which pays where the comparisons
 // walk much (one switch step of 2^24 vertices with 5*10^7 jumps and steps 1.9

@@ -174,7 +174,7 @@ int launch_eval_jump(cudaStream_t s, const EvalArgs &a, SolveSync *sync, EvalGat
 // A whole solve_si of one game in one persistent launch (solve_kernels.cu).
 struct SolveSync {
     int32_t vote[3] = {0, 0, 0}, vote2[3] = {0, 0, 0};
-    uint32_t phase = 0;
+    uint32_t phase = 0;   // kept_phase
     uint32_t errs[3] = {0, 0, 0};
     uint32_t err = 0;
     uint32_t epoch = 0;   // evaluation number of the landmark records (EvalArgs)

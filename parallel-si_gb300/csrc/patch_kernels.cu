@@ -383,7 +383,7 @@ __global__ void __launch_bounds__(kPatchBlock, 1) k_patch(PatchArgs a, cudaGraph
             g->mfrom[0] = g->mfrom[1] = 0;
             g->skip = g->backoff;
             g->backoff = g->backoff < kBackoffMax ? 2 * g->backoff : kBackoffMax;
-            if (!solo) a.sync->phase = phase;
+            if (!solo) a.sync->phase = kept_phase(phase);
             if (in_graph) cudaGraphSetConditional(full, 1);
         }
         return;
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(kPatchBlock, 1) k_patch(PatchArgs a, cudaGraph
         g->nseeds = ns;
         a.stats[0] += 1;
         a.stats[1] += (unsigned long long)na;
-        if (!solo) a.sync->phase = phase;
+        if (!solo) a.sync->phase = kept_phase(phase);
         if (in_graph) cudaGraphSetConditional(full, 0);
     }
 }

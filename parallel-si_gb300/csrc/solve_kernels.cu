@@ -112,8 +112,8 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
     const int32_t nth = (int32_t)(gridDim.x * blockDim.x);
     // Barrier with two votes: whether any thread passed true.  Phase k uses the
     // words k % 3, which thread 0 clears in phase k - 1, when everyone has
-    // read their last use (phase k - 3); the count goes on from solve to
-    // solve.  err: the error bits thread 0 saw on its way into the barrier
+    // read their last use (phase k - 3); the count goes on from launch to
+    // launch (kept_phase).  err: the error bits thread 0 saw on its way into the barrier
     // (the same for all threads, as the loop's control has to be).
     uint32_t phase = a.sync->phase, err = 0;
     bool voted = false, voted2 = false;
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(SolveArgs a)
         a.ctl->lm_have = a.ctl->lm_far = 0;
         *a.err = *(volatile uint32_t *)&a.sync->err;
         a.sync->err = 0;
-        a.sync->phase = phase;
+        a.sync->phase = kept_phase(phase);
     }
 }
 
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_eval_jump(EvalArgs a, Solv
         }
         more = barrier(left);
     }
-    if (tid == 0) sync->phase = phase;
+    if (tid == 0) sync->phase = kept_phase(phase);
 }
 
 std::atomic<int> g_sms[kMaxCachedDevices];
