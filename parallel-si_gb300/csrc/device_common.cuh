@@ -381,14 +381,14 @@ __host__ __device__ __forceinline__ uint32_t kept_phase(uint32_t phase) { return
 // 41.3, 37.5 -> 30.9, 38.8, 38.9, 35.7 (never: 31.5, 48.5, 38.7, 35.9), long-path
 // 2^23 17.6 -> 15.3, 256 games 16.9 -> 16.1; n and n / 8, n / 2 and n / 4, n / 8 and
 // n / 16 are within 2% of it.
-__device__ __forceinline__ bool want_landmarks(const EvalGates *g, const unsigned long long *sw, int32_t n)
+__host__ __device__ __forceinline__ bool want_landmarks(const EvalGates *g, const unsigned long long *sw, int32_t n)
 {
     return g->lm_far || sw[1] > (unsigned long long)(g->lm_have ? n / 8 : n / 2);
 }
 
 // Before an evaluation (one thread): decides between a patch and the full
 // evaluation (patch_kernels.cu) and resets what either starts from.
-__device__ __forceinline__ void patch_begin(const PatchArgs &a)
+__host__ __device__ __forceinline__ void patch_begin(const PatchArgs &a)
 {
     EvalGates *g = a.g;
     ++*a.epoch;
@@ -402,6 +402,9 @@ __device__ __forceinline__ void patch_begin(const PatchArgs &a)
     g->acount = 0;
     g->lcnt[0] = g->lcnt[1] = g->lcnt[2] = 0;
     bool ok = g->try_patch && cc <= a.ccap && (int64_t)*a.ucount + a.acap <= a.ucap;
+    // the evaluation numbered 0 clears the landmark records of the last round
+    // (k_root_init), so it is a full one
+    if ((*a.epoch & kEpochMask) == 0) ok = false;
     if (ok && g->skip > 0) {
         g->skip--;
         ok = false;

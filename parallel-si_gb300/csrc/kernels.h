@@ -149,6 +149,7 @@ struct EvalArgs {
     PathNode *node = nullptr;
     int32_t *rdeep = nullptr;     // counts of paths too long for the record's word (n entries)
     int4 *skip = nullptr;         // landmark skips (device_common.cuh), written if g->lm_want
+    int64_t cap = 0;              // records there
     EvalGates *g = nullptr;
     const unsigned long long *sw = nullptr;   // the last switch step's statistics (launch_switch)
     const uint32_t *epoch = nullptr;   // evaluation number (launch_patch_begin advances it)

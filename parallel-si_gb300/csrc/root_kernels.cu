@@ -60,15 +60,17 @@ __global__ void k_root_init(EvalArgs a)
         *a.lcount = 0;
         a.g->lm_have = a.g->lm_want;
     }
-    // the evaluation number wraps around: no record of the last round may look current
-    const bool wrap = (*a.epoch & kEpochMask) == 0;
+    // the evaluation number wraps around: no record of the last round may look
+    // current, those past the arena's present extent among them
+    if ((*a.epoch & kEpochMask) == 0)
+        for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < a.cap; v += (int64_t)gridDim.x * blockDim.x)
+            a.skip[v] = make_int4(SKIP_UNKNOWN, 0, 0, 0);
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < a.n; v += (int64_t)gridDim.x * blockDim.x) {
         const int32_t t = a.strat[v], p = a.pri[v];
         int4 q = make_int4(t, p, RM_UNKNOWN, 0);
         if (a.solved[v]) q = make_int4(-1, p, a.st[v] == ST_POS_INF ? RM_POS_INF : RM_NEG_INF, 0);
         else if (t < 0) q = make_int4(-1, p, p, path_word(1, 1));
         *reinterpret_cast<int4 *>(&a.node[v]) = q;
-        if (wrap) a.skip[v] = make_int4(SKIP_UNKNOWN, 0, 0, 0);
         if (a.track.tie && a.track.tie[v]) a.track.need[v] = 1;
     }
 }

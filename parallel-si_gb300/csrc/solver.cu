@@ -558,6 +558,7 @@ EvalArgs Solver::eval_args()
     a.node = node_;
     a.rdeep = rdeep_;
     a.skip = skip_;
+    a.cap = cap_n_;
     a.g = ctl_;
     a.sw = dw_->sw;
     a.epoch = &sync_->epoch;

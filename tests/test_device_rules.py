@@ -22,3 +22,8 @@ def rules(tmp_path_factory):
 def test_barrier_words_past_four_billion_barriers(rules):
     r = rules("phases")
     assert r.returncode == 0, r.stdout
+
+
+def test_the_evaluation_numbered_zero_is_a_full_one(rules):
+    r = rules("numbers")
+    assert r.returncode == 0, r.stdout
