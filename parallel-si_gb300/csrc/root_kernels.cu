@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(kWalkThreads, 8) k_root_walk(EvalArgs a)
             if (q.z != RM_POS_INF && q.z != RM_NEG_INF) {   // not solved
                 if (q.x < 0) {   // a child of the sink, published by init: its skip and status are written here
                     a.st[v] = 1;
-                    if (marks) a.skip[v] = skip_pack(-1, Top2{q.y, 1, -1, 0}, epoch);
+                    if (marks) store_whole(&a.skip[v], skip_pack(-1, Top2{q.y, 1, -1, 0}, epoch));
                     k = finite_key(q.y, 1);
                     finite = true;
                 } else {

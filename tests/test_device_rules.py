@@ -1,6 +1,7 @@
 """Rules of the kernels that need no device, compiled for the host from
 csrc/device_common.cuh."""
 import os
+import re
 import shutil
 import subprocess
 
@@ -27,3 +28,11 @@ def test_barrier_words_past_four_billion_barriers(rules):
 def test_the_evaluation_numbered_zero_is_a_full_one(rules):
     r = rules("numbers")
     assert r.returncode == 0, r.stdout
+
+
+def test_walks_store_landmark_records_whole():
+    """Walks read each other's records in the launch that writes them."""
+    src = open(os.path.join(ROOT, "parallel-si_gb300", "csrc", "root_kernels.cu")).read()
+    walks = src[src.index("void publish_finite"):]
+    assert "load_whole(&a.skip[" in walks and walks.count("store_whole(&a.skip[") == 3
+    assert not re.search(r"a\.skip\[\w+\]\s*=[^=]", walks)
