@@ -254,10 +254,13 @@ private:
         uint32_t claim;             // the switch kernel's work counter (launch_switch)
     };
     Words *dw_ = nullptr, *hw_ = nullptr;   // ctl_ follows dw_ on the device, hctl_ follows hw_
-    struct AllWords {
+    // page-locked staging follows hw_'s (stage): aligned for what is read there
+    struct alignas(16) AllWords {
         Words w;
         GraphCtl ctl;
     };
+    static_assert(alignof(int4) <= alignof(AllWords) && sizeof(AllWords) % alignof(int4) == 0,
+                  "game states are read right behind the words");
     GraphCtl *hctl_ = nullptr;
     // graph-driven solve loop (solver_graph.cu)
     int run_graph(bool reset, int64_t max_evals, GraphCtl *out, int4 *gstate_out);
