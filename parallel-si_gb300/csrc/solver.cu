@@ -90,7 +90,7 @@ int Solver::create_arena(int64_t max_vertices, int64_t max_edges, int32_t slots,
     s->incremental_ = opt.incremental;
     s->patch_limit_ = opt.patch_limit;
     s->switch_warp_ = opt.switch_kernel == PSI_SWITCH_WARP;
-    rc = s->alloc_arrays(max_vertices, max_edges);
+    rc = s->alloc_arrays(max_vertices, max_edges, true);
     if (!rc) rc = s->init_arena(slots);
     if (rc) {
         delete s;
@@ -137,7 +137,7 @@ int Solver::create_union(const std::vector<const HostGame *> &gs, const psi_opti
     s->incremental_ = opt.incremental;
     s->patch_limit_ = opt.patch_limit;
     s->switch_warp_ = opt.switch_kernel == PSI_SWITCH_WARP;
-    rc = s->alloc_arrays(n, m);
+    rc = s->alloc_arrays(n, m, true);
     if (!rc) rc = s->upload_union(gs, table, base->back());
     if (rc) {
         delete s;
@@ -186,7 +186,7 @@ int Solver::upload_union(const std::vector<const HostGame *> &gs, const std::vec
 }
 
 // Device arrays for games of up to cap_n vertices and cap_m edges.
-int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
+int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m, bool many)
 {
     int rc = set_device();
     if (rc) return rc;
@@ -267,8 +267,10 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m)
         PSI_CUDA_TRY(cudaMemsetAsync(apos_, 0xff, 4 * (size_t)std::max<int64_t>(1, cap_n), stream_));   // -1: in no patch
     }
     ctl_ = &reinterpret_cast<AllWords *>(dw_)->ctl;
-    small_stage_ = 4 * (size_t)(std::min<int64_t>(cap_n, kSelectSmall) + 1);
-    PSI_CUDA_TRY(cudaMallocHost((void **)&hw_, sizeof(AllWords) + small_stage_));
+    // the small winning set; of a batch's or arena's games two words per vertex
+    stage_bytes_ = std::max(kStagedCopy, 4 * (size_t)(std::min<int64_t>(cap_n, kSelectSmall) + 1));
+    if (many) stage_bytes_ = std::max(stage_bytes_, std::min(kStageMost, 8 * (size_t)cap_n));
+    PSI_CUDA_TRY(cudaMallocHost((void **)&hw_, sizeof(AllWords) + stage_bytes_));
     hctl_ = &reinterpret_cast<AllWords *>(hw_)->ctl;
     PSI_CUDA_TRY(cudaMemsetAsync(dw_, 0, sizeof(Words), stream_));
     PSI_CUDA_TRY(cudaMemsetAsync(sync_, 0, sizeof(SolveSync), stream_));
@@ -339,7 +341,6 @@ Solver::~Solver()
     for (void *p : allocs_) cudaFreeAsync(p, stream_);   // back to the library's pool
     if (stream_) cudaStreamSynchronize(stream_);
     if (hw_) cudaFreeHost(hw_);
-    if (stage_) cudaFreeHost(stage_);
     for (auto &p : ph_) {
         if (p.a) cudaEventDestroy(p.a);
         if (p.b) cudaEventDestroy(p.b);
@@ -697,23 +698,10 @@ int Solver::get_depth(int32_t *out)
     return PSI_OK;
 }
 
-int Solver::stage(size_t bytes, void **out)
+int Solver::stage_in(const void *src, size_t bytes)
 {
-    *out = reinterpret_cast<AllWords *>(hw_) + 1;
-    if (bytes <= small_stage_) return PSI_OK;
-    if (!stage_) PSI_CUDA_TRY(cudaMallocHost(&stage_, kStageBytes));
-    *out = stage_;
-    return PSI_OK;
-}
-
-int Solver::stage_in(const void *src, size_t bytes, const void **out)
-{
-    void *p = nullptr;
-    int rc = stage(bytes, &p);
-    if (rc) return rc;
-    PSI_CUDA_TRY(cudaMemcpyAsync(p, src, bytes, cudaMemcpyDeviceToHost, stream_));
+    PSI_CUDA_TRY(cudaMemcpyAsync(stage(), src, bytes, cudaMemcpyDeviceToHost, stream_));
     PSI_CUDA_TRY(cudaStreamSynchronize(stream_));
-    *out = p;
     return PSI_OK;
 }
 
@@ -724,12 +712,11 @@ int Solver::copy_out(void *dst, const void *src, size_t bytes)
         return PSI_OK;
     }
     cudaPointerAttributes at = {};
-    const bool pageable = bytes <= kStageBytes && cudaPointerGetAttributes(&at, dst) == cudaSuccess &&
-                          at.type == cudaMemoryTypeUnregistered;
-    if (pageable) {
-        const void *p = nullptr;
-        int rc = stage_in(src, bytes, &p);
-        if (!rc) std::memcpy(dst, p, bytes);
+    const bool staged = bytes <= kStagedCopy && cudaPointerGetAttributes(&at, dst) == cudaSuccess &&
+                        at.type == cudaMemoryTypeUnregistered;
+    if (staged) {
+        int rc = stage_in(src, bytes);
+        if (!rc) std::memcpy(dst, stage(), bytes);
         return rc;
     }
     PSI_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream_));
@@ -746,10 +733,9 @@ int Solver::get_winning(int32_t player, int32_t *out, int64_t cap, int64_t *coun
     if (n_ <= kSelectSmall) {   // one block, size and ids in one copy
         launch_select_small(stream_, n_, player, st_, sel + 1, sel);
         PSI_CUDA_TRY(cudaGetLastError());
-        const void *p = nullptr;
-        rc = stage_in(sel, 4 * ((size_t)n_ + 1), &p);
+        rc = stage_in(sel, 4 * ((size_t)n_ + 1));
         if (rc) return rc;
-        const int32_t *h = static_cast<const int32_t *>(p);
+        const int32_t *h = static_cast<const int32_t *>(stage());
         *count = h[0];
         if (out && cap > 0) std::memcpy(out, h + 1, 4 * (size_t)std::min<int64_t>(cap, h[0]));
         return PSI_OK;
@@ -774,12 +760,8 @@ int Solver::get_winning_range(int64_t v0, int64_t n, int32_t player, int32_t *ou
     int rc = set_device();
     if (rc) return rc;
     // half of the staging memory for status words, half for the ids found in them
-    constexpr int64_t kPart = (int64_t)(kStageBytes / 8);
-    const int64_t part = std::min(n, kPart);
-    void *room = nullptr;
-    rc = stage(8 * (size_t)part, &room);
-    if (rc) return rc;
-    int32_t *st = static_cast<int32_t *>(room), *ids = st + part;
+    const int64_t part = std::min(n, (int64_t)(stage_bytes_ / 8));
+    int32_t *st = static_cast<int32_t *>(stage()), *ids = st + part;
     int64_t k = 0;
     for (int64_t at = 0; at < n; at += part) {
         const int64_t len = std::min(n - at, part);
@@ -1124,8 +1106,15 @@ int Solver::arena_export(int32_t vb, int32_t count, int32_t *strategy, int32_t *
     cudaError_t e = device_alloc((void **)&out, 8 * (size_t)count, stream_);
     if (e != cudaSuccess) return fail(PSI_ERR_NOMEM, "arena export buffer");
     launch_arena_export(stream_, vb, count, strat_, st_, out);
-    int rc = copy_out(strategy, out, 4 * (size_t)count);
-    if (!rc) rc = copy_out(infinite, out + count, 4 * (size_t)count);
+    // the caller's arrays are new memory: by way of the staging memory where they fit
+    auto get = [&](int32_t *dst, const int32_t *src) {
+        if (4 * (size_t)count > stage_bytes_) return copy_out(dst, src, 4 * (size_t)count);
+        int rc = stage_in(src, 4 * (size_t)count);
+        if (!rc) std::memcpy(dst, stage(), 4 * (size_t)count);
+        return rc;
+    };
+    int rc = get(strategy, out);
+    if (!rc) rc = get(infinite, out + count);
     cudaFreeAsync(out, stream_);
     return rc ? rc : sync_and_check("arena_export");
 }
@@ -1176,11 +1165,8 @@ int Solver::arena_step(bool reset, std::vector<int32_t> &done, std::vector<int32
     launch_serve_account(stream_, games_, 2, gstate_, gcount_, gmask_);
     std::vector<int4> big;
     int4 *st = nullptr;
-    if (sizeof(int4) * (size_t)games_ <= kStageBytes) {
-        void *room = nullptr;
-        rc = stage(sizeof(int4) * (size_t)games_, &room);
-        if (rc) return rc;
-        st = static_cast<int4 *>(room);
+    if (sizeof(int4) * (size_t)games_ <= stage_bytes_) {
+        st = static_cast<int4 *>(stage());
     } else {
         big.resize((size_t)games_);
         st = big.data();

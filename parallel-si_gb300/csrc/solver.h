@@ -144,7 +144,7 @@ public:
 
 private:
     Solver() = default;
-    int alloc_arrays(int64_t cap_n, int64_t cap_m);
+    int alloc_arrays(int64_t cap_n, int64_t cap_m, bool many = false);   // many: games in a batch or arena
     int upload_game(const CsrView &g, bool validate);
     int upload_union(const std::vector<const HostGame *> &gs, const std::vector<int32_t> &table, int64_t n);
     int finish_upload();
@@ -165,18 +165,19 @@ private:
     ChangeList changes() const { return clist_ ? ChangeList{clist_, &ctl_->ccount, ccap_} : ChangeList(); }
     int build_graph(bool reset);
     int get_range(const int32_t *src, int64_t v0, int64_t count, int32_t *out);
-    // Device memory to the caller's, complete on return.  Small copies into
-    // pageable memory go through stage_: the driver's own path for them took
-    // 30 to 80 us, this one 12.
+    // Device memory to the caller's, complete on return.  Into ordinary memory
+    // that the GPU has reached before, a copy straight into it takes 9 us up to
+    // 64 KB, 15 us for 1 MB; the first one into new memory 50 us and more.  By way
+    // of the staging memory 9 to 14 us up to 16 KB either way, but 13, 25, 73 us
+    // for 64 KB, 256 KB, 1 MB (new: 20, 40, 104; straight 50, 140, 195).  So up to
+    // kStagedCopy it goes there, where it costs nothing.
     int copy_out(void *dst, const void *src, size_t bytes);
-    // Page-locked memory of at least `bytes` (at most kStageBytes): a part of
-    // hw_'s allocation up to small_stage_, else one of its own, made when first
-    // wanted.
-    int stage(size_t bytes, void **out);
-    int stage_in(const void *src, size_t bytes, const void **out);   // device memory there, complete on return
-    static constexpr size_t kStageBytes = 1 << 20;
-    size_t small_stage_ = 0;
-    void *stage_ = nullptr;
+    // The staging memory, page-locked: a part of hw_'s allocation, sized for the
+    // solver's kind (alloc_arrays).  Allocating and freeing it apart took 190 us.
+    void *stage() const { return reinterpret_cast<AllWords *>(hw_) + 1; }
+    int stage_in(const void *src, size_t bytes);   // device memory there, complete on return
+    static constexpr size_t kStagedCopy = 16 << 10, kStageMost = 1 << 20;
+    size_t stage_bytes_ = 0;
     void *select_tmp_ = nullptr;       // workspace of the winning-set selection
     size_t select_bytes_ = 0;
     int set_device();
