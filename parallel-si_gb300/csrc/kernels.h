@@ -199,9 +199,9 @@ struct SolveArgs {
     int32_t inject_at = 0;
     uint32_t inject_bits = 0;
 };
-// The largest game it takes on the current device (over a million vertices
-// from 32 SMs on).
-int64_t solve_capacity();
+// Whether it takes a game of n vertices and m edges on the current device: any
+// up to six vertices per thread, further ones if they are sparse.
+bool solve_takes(int64_t n, int64_t m);
 // Returns a cudaError_t value.
 int launch_solve(cudaStream_t s, const SolveArgs &a);
 

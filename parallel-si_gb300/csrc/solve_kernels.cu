@@ -738,7 +738,22 @@ int launch_eval_jump(cudaStream_t s, const EvalArgs &a, SolveSync *sync, EvalGat
     return (int)cudaLaunchCooperativeKernel((const void *)k_eval_jump, dim3(grid), dim3(threads), args, 0, s);
 }
 
-int64_t solve_capacity() { return (int64_t)kMaxWaves * kSolveThreads * device_sms(); }
+// A switch phase reads every successor of the player's vertices, a thread its
+// own lists, so neighbouring reads of a list hit L1 only while the lists of a
+// block's 1,024 threads fit there.  With seven vertices per thread (933,889
+// vertices on 152 SMs) the kept words leave 32 KB of L1, and dense games lose to
+// the graph, whose steps examine what has changed: ms per solve here and there
+// at 10^6 vertices of mean degree 9, 12, 15, 24, 40, 100: 2.3, 2.3, 1.5, 2.1, 3.9,
+// 8.9 and 3.2, 2.6, 1.6, 1.7, 2.2, 4.7 (at 940,000, degrees 12 and 15: 2.0, 1.5 and
+// 1.9, 1.3; degree 200: 17 and 8.7).  With up to six it is the faster one: 930,000
+// vertices 1.7, 1.8, 0.8, 1.0, 1.6, 3.5 and 2.8, 3.4, 1.2, 1.5, 1.9, 3.5, 500,000 of
+// degree 300 8.8 and 18.5.
+constexpr int64_t kDenseDegree = 14;
+bool solve_takes(int64_t n, int64_t m)
+{
+    const int64_t round = (int64_t)kSolveThreads * device_sms();
+    return n <= kMaxWaves * round && (n <= (kMaxCached - 1) * round || m <= kDenseDegree * n);
+}
 
 int launch_solve(cudaStream_t s, const SolveArgs &a)
 {

@@ -288,7 +288,7 @@ int Solver::loop_ended(const GraphCtl &out)
 bool Solver::fused()
 {
     return games_ == 0 && n_ > 0 && n_ <= kFusedVertices && incremental_ != PSI_INCR_ALWAYS && !switch_warp_ &&
-           set_device() == PSI_OK && n_ <= solve_capacity();
+           set_device() == PSI_OK && solve_takes(n_, m_);
 }
 
 int Solver::run_fused(bool reset, int64_t max_evals, GraphCtl *out)

@@ -93,3 +93,21 @@ def test_large_games_match_the_oracle(name):
     for reset in (False, True):
         same(solved(s, reset), expected(g, reset))
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,deg,fused", [(1000003, 14, True), (1000003, 15, False), (900000, 15, True)])
+def test_dense_games_of_seven_vertices_per_thread_take_the_graph(n, deg, fused):
+    """Past 933,888 vertices (152 SMs) the persistent solver, one launch, has
+    games up to a mean degree of 14; the results are the same."""
+    g = psi.Game.random(n, deg, deg, n, deg)
+    s = psi.GPUList(g)
+    s.solve()                               # (the graph is built, which counts its launches)
+    before = psi.launch_count()
+    got = solved(s)
+    launches = psi.launch_count() - before  # of them three read the winning sets and initialise
+    assert (launches < 6) == fused, launches
+    w = psi.GPUList(g, switch_kernel=1)
+    same(got, solved(w))
+    w.close()
+    s.close()
