@@ -139,6 +139,16 @@ void launch_init_strat(cudaStream_t s, int32_t n, const int8_t *owner, const int
 void launch_reset_odd(cudaStream_t s, int32_t n, const int8_t *owner, const int32_t *off,
                       const int32_t *tgt, int32_t *strat, const int32_t *gate = nullptr, uint8_t *need = nullptr);
 
+// What the cooperative solver kernels share between blocks and keep between
+// launches; zero before the first.
+struct SolveSync {
+    int32_t vote[3] = {0, 0, 0}, vote2[3] = {0, 0, 0};
+    uint32_t phase = 0;   // kept_phase
+    uint32_t errs[3] = {0, 0, 0};
+    uint32_t err = 0;
+    uint32_t epoch = 0;   // evaluation number of the landmark records (EvalArgs)
+};
+
 // ---- evaluation (gpu_list_ranking.cu:52-277)
 // A full evaluation of the current strategy (root_kernels.cu).
 struct EvalArgs {
@@ -155,9 +165,9 @@ struct EvalArgs {
     const uint32_t *epoch = nullptr;   // evaluation number (launch_patch_begin advances it)
     int32_t *key = nullptr;       // comparison keys
     int32_t *ulist = nullptr, *ucount = nullptr;   // the vertices the sink does not reach (*ucount 0 on entry)
-    int32_t *la = nullptr, *lb = nullptr, *lcount = nullptr;   // walks cut short: two lists (n entries), a counter
-    int4 *ja = nullptr, *jb = nullptr;             // their jump entries (n entries each)
-    int32_t *cnt = nullptr;       // three counters
+    int32_t *la = nullptr, *lcount = nullptr;   // walks cut short: a list (n entries), its counter
+    int4 *ja = nullptr;           // jump records (n entries)
+    SolveSync *sync = nullptr;
     uint32_t *err = nullptr;
     ChangeTrack track;
     const int32_t *gate = nullptr;
@@ -169,17 +179,9 @@ int launch_root_settle(cudaStream_t s, const EvalArgs &a);
 
 // One full evaluation in one cooperative launch (solve_kernels.cu), with what
 // launch_patch_begin does before one; n < 2^20.  Returns a cudaError_t value.
-struct SolveSync;
-int launch_eval_jump(cudaStream_t s, const EvalArgs &a, SolveSync *sync, EvalGates *g, int32_t *quiet);
+int launch_eval_jump(cudaStream_t s, const EvalArgs &a, EvalGates *g, int32_t *quiet);
 
 // A whole solve_si of one game in one persistent launch (solve_kernels.cu).
-struct SolveSync {
-    int32_t vote[3] = {0, 0, 0}, vote2[3] = {0, 0, 0};
-    uint32_t phase = 0;   // kept_phase
-    uint32_t errs[3] = {0, 0, 0};
-    uint32_t err = 0;
-    uint32_t epoch = 0;   // evaluation number of the landmark records (EvalArgs)
-};
 struct SolveArgs {
     int32_t n = 0, n_even = 0;    // plist: Even's n_even vertices, then Odd's
     int64_t m = 0;
@@ -192,7 +194,7 @@ struct SolveArgs {
     int4 *jump[2] = {nullptr, nullptr};       // n entries each
     int2 *path = nullptr;                     // (strategy, priority), n entries
     int32_t *ulist = nullptr, *ucount = nullptr;
-    SolveSync *sync = nullptr;    // zero before the first solve
+    SolveSync *sync = nullptr;
     GraphCtl *ctl = nullptr;      // receives iters, brs, stop
     uint32_t *err = nullptr;
     int32_t reset = 0, max_evals = 0, guard = 0;

@@ -23,7 +23,7 @@
 //     longest of a warp's walks).  Landmark records only where wanted.
 //  3. k_root_settle: walks that did not end within kWalkCap steps (deep
 //     chains, long cycles, none on random games) are finished by pointer
-//     jumping over those vertices alone.
+//     jumping without barriers (jump.cuh) over those vertices alone.
 //
 // Against the tour upkeep, sublist walks, reduced-list ranking, depth
 // broadcast, summary walks and cycle rounds that this replaces, an evaluation
@@ -34,6 +34,7 @@
 #include <cooperative_groups.h>
 
 #include "device_common.cuh"
+#include "jump.cuh"
 #include "kernels.h"
 
 namespace cg = cooperative_groups;
@@ -41,13 +42,6 @@ namespace cg = cooperative_groups;
 namespace psi {
 
 namespace {
-
-__device__ __forceinline__ int ceil_log2_dev(int64_t x)
-{
-    int r = 0;
-    while (((int64_t)1 << r) < x) r++;
-    return r;
-}
 
 // Path records of a new evaluation: unknown, except the sink's children
 // (depth 1, their own priority) and the solved vertices (their frozen
@@ -89,22 +83,37 @@ __device__ __forceinline__ void path_depth_count(const EvalArgs &a, int32_t y, i
     }
 }
 
-// Publishes a finite vertex: landmark record, status, summary.
-__device__ __forceinline__ void publish_finite(const EvalArgs &a, int32_t v, int32_t d, int32_t m, int32_t c,
-                                               int32_t anc, const Top2 &seg, uint32_t epoch, bool marks)
-{
-    if (marks) store_whole(&a.skip[v], skip_pack(anc, seg, epoch));
-    a.st[v] = d;
-    if (d >= kDeepPath) a.rdeep[v] = c;
-    publish_summary(&a.node[v], m, path_word(d, c), d >= kDeepPath);
-}
-
 // A walk's step cap: longer walks are left to k_root_settle.
 constexpr int32_t kWalkCap = 128;
 constexpr int kWalkThreads = 256;
 // unreached vertices buffered per warp before they go to the list with one
 // atomic (one atomic per warp and pass on the list's counter would serialise)
 constexpr int kUnreachedBuf = 128;
+
+// A warp's buffer; its lanes call both together.
+struct Unreached {
+    int32_t *buf;
+    int held = 0;   // uniform over the warp
+    __device__ __forceinline__ void flush(const EvalArgs &a)
+    {
+        const int lane = threadIdx.x & 31;
+        int32_t base = 0;
+        if (lane == 0) base = atomicAdd(a.ucount, held);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int i = lane; i < held; i += 32) a.ulist[base + i] = buf[i];
+        __syncwarp();
+        held = 0;
+    }
+    __device__ __forceinline__ void add(const EvalArgs &a, bool infinite, int32_t v)
+    {
+        const unsigned m = __ballot_sync(0xffffffffu, infinite);
+        if (!m) return;
+        if (infinite) buf[held + __popc(m & ((1u << (threadIdx.x & 31)) - 1))] = v;
+        held += __popc(m);
+        __syncwarp();
+        if (held > kUnreachedBuf - 32) flush(a);
+    }
+};
 
 // Bound by dependent random reads (2^22 random game: DRAM 40%, L2 36%, issue
 // slots 60% busy; 2^24: 2.9 GB in 670 us, 4.1 TB/s), so eight blocks per SM at
@@ -123,16 +132,7 @@ __global__ void __launch_bounds__(kWalkThreads, 8) k_root_walk(EvalArgs a)
     const uint32_t epoch = *a.epoch & kEpochMask;
     const bool marks = a.g->lm_want;
     const int lane = threadIdx.x & 31;
-    int32_t *buf = ubuf[threadIdx.x >> 5];
-    int nbuf = 0;   // uniform over the warp
-    auto flush = [&] {
-        int32_t base = 0;
-        if (lane == 0) base = atomicAdd(a.ucount, nbuf);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        for (int i = lane; i < nbuf; i += 32) a.ulist[base + i] = buf[i];
-        __syncwarp();
-        nbuf = 0;
-    };
+    Unreached unreached{ubuf[threadIdx.x >> 5]};
     // every warp takes 32 consecutive vertices at a time
     for (int64_t b0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ll; b0 < a.n;
          b0 += (int64_t)gridDim.x * blockDim.x) {
@@ -218,149 +218,113 @@ __global__ void __launch_bounds__(kWalkThreads, 8) k_root_walk(EvalArgs a)
         const bool changed = (finite || infinite) && k != old;
         if (changed) a.key[v] = k;
         flag_in_neighbours(a.track, changed, v);
-        const unsigned um = __ballot_sync(0xffffffffu, infinite);
-        if (um) {
-            if (infinite) buf[nbuf + __popc(um & ((1u << lane) - 1))] = v;
-            nbuf += __popc(um);
-            __syncwarp();
-            if (nbuf > kUnreachedBuf - 32) flush();
-        }
+        unreached.add(a, infinite, v);
         const int32_t p = warp_reserve(left, a.lcount);
         if (left) a.la[p] = v;
     }
-    if (nbuf) flush();
+    if (unreached.held) unreached.flush(a);
 }
 
-// The vertices whose walk was cut short (list la, *lcount of them): pointer
-// jumping over them alone.  In round r an entry is (the vertex 2^r steps
-// ahead with kFlag possibly set, top priority of the 2^r vertices from u on,
-// its count, the largest id among the vertices that carry it).  A target that
-// is published settles u: a finite one with the window's summary merged, an
-// infinite one with its infinity.  Two windows back to back with the same top
-// (priority, id) vertex x mean that the walk meets x twice, so it is on x's
-// cycle from the target on, shorter than 2^(r+1): u is flagged, and in the
-// next round takes the parity of its target's window, which covers the
-// cycle.  After ceil(log2 |la|) + 1 rounds every window is longer than any
-// path through unpublished vertices: what is left is on a cycle.  A vertex
-// settled in an earlier round is published, so no round reads its entry again.
-constexpr int32_t kFlag = 1 << 30;   // vertex ids are below 2^30
-
-constexpr int kSmallSettle = 4096;   // up to this many: one block, no grid barrier
-
-template <bool GRID>
-__device__ void settle_body(const EvalArgs &a, int32_t nl)
-{
-    const int64_t tid = GRID ? (int64_t)blockIdx.x * blockDim.x + threadIdx.x : threadIdx.x;
-    const int64_t nth = GRID ? (int64_t)gridDim.x * blockDim.x : blockDim.x;
-    auto barrier = [] {
-        if (GRID) cg::this_grid().sync();
-        else __syncthreads();
-    };
-    for (int64_t i = tid; i < nl; i += nth) {
-        const int32_t u = a.la[i];
-        a.ja[u] = make_int4(a.node[u].parent, a.node[u].pri, 1, u);
-    }
-    if (tid == 0) a.cnt[0] = a.cnt[1] = a.cnt[2] = 0;
-    barrier();
-    const int32_t *act = a.la;
-    int32_t na = nl;
-    int4 *in = a.ja, *out = a.jb;
-    int32_t *next = a.lb, *spare = a.la;   // la is free after the first round
-    const int rounds = ceil_log2_dev(nl) + 2;
-    for (int r = 0; r < rounds && na > 0; r++) {
-        const bool last = r == rounds - 1;
-        int32_t *cnt = &a.cnt[r % 3];
-        if (tid == 0) a.cnt[(r + 1) % 3] = 0;    // next round's counter (last read two rounds ago)
-        for (int64_t b0 = tid - threadIdx.x; b0 < na; b0 += nth) {   // block-uniform passes
-            const int64_t i = b0 + threadIdx.x;
-            bool keep = false, changed = false, infinite = false;
-            int32_t u = -1;
-            if (i < na) {
-                u = act[i];
-                const int4 e = __ldcg(&in[u]);
-                const int32_t t = e.x & ~kFlag;
-                const int4 q = __ldcg(reinterpret_cast<const int4 *>(&a.node[t]));
-                int32_t code = 0, k = 0;
-                bool done = true;
-                if (q.z == RM_POS_INF || q.z == RM_NEG_INF) {
-                    code = q.z;
-                } else if (q.z != RM_UNKNOWN) {
-                    int32_t dt, ct, m = e.y, c = e.z;
-                    path_depth_count(a, t, q.w, dt, ct);
-                    top1_merge(m, c, q.z, ct);
-                    const bool marks = a.g->lm_want;
-                    const int32_t d = (int32_t)((1u << r) + (uint32_t)dt);
-                    const int32_t len = marks ? d - skip_landmark_depth(d) : 0;
-                    Top2 seg = {-1, 0, -1, 0};
-                    int32_t anc = u;
-                    for (int32_t j = 0; j < len; j++) {
-                        const int2 x = *reinterpret_cast<const int2 *>(&a.node[anc]);
-                        top2_add(seg, x.y);
-                        anc = x.x;
-                    }
-                    publish_finite(a, u, d, m, c, anc, seg, *a.epoch & kEpochMask, marks);
-                    k = finite_key(m, c);
-                } else {
-                    const int4 f = __ldcg(&in[t]);
-                    if ((e.x & kFlag) || last) {
-                        code = (f.y & 1) ? RM_NEG_INF : RM_POS_INF;
-                    } else {
-                        int4 o = make_int4(f.x & ~kFlag, e.y, e.z, e.w);
-                        if (f.y > e.y) {
-                            o.y = f.y;
-                            o.z = f.z;
-                            o.w = f.w;
-                        } else if (f.y == e.y) {
-                            o.z = (int32_t)((uint32_t)e.z + (uint32_t)f.z);   // may wrap on a cycle, where no count is used
-                            o.w = max(e.w, f.w);
-                            if (e.w == f.w) o.x |= kFlag;
-                        }
-                        out[u] = o;
-                        keep = true;
-                        done = false;
-                    }
-                }
-                if (code) {
-                    a.st[u] = (code == RM_POS_INF) ? ST_POS_INF : ST_NEG_INF;
-                    publish_summary(&a.node[u], code, 0);
-                    k = (code == RM_POS_INF) ? KEY_POS_INF : KEY_NEG_INF;
-                    infinite = true;
-                }
-                if (done && a.key[u] != k) {
-                    a.key[u] = k;
-                    changed = true;
-                }
-            }
-            flag_in_neighbours(a.track, changed, u);
-            block_append(infinite, u, a.ulist, a.ucount);
-            __syncthreads();
-            block_append(keep, u, next, cnt);
-            __syncthreads();
-        }
-        barrier();
-        na = *(volatile int32_t *)cnt;
-        act = next;
-        int32_t *l = next;
-        next = spare;
-        spare = l;
-        int4 *t = in;
-        in = out;
-        out = t;
-    }
-}
-
-// 1,024-thread blocks, one per SM: few blocks at each round's grid barrier.
-constexpr int kSettleThreads = 1024;
+// The vertices whose walk was cut short (list la, *lcount of them).  Their
+// successors are published, and give a finished record at once, or on the list
+// too, so from then on only the records (ja, 16 bytes) of vertices on the list
+// are read: one random read per jump and no rounds, where the pointer doubling
+// that this replaces read the target's path record as well, kept lists of
+// what was left and met at a barrier log2 n times.  One cycle of 4*10^6, 1.6*10^7
+// vertices (all of them left): 3.3 -> 0.55, 16.8 -> 3.0 ms.
+constexpr int kSettleThreads = 1024;   // one block per SM: few blocks at a pass's grid barrier
+constexpr int kSmallSettle = 4096;     // up to this many: one block, no grid barrier
 __global__ void __launch_bounds__(kSettleThreads, 1) k_root_settle(EvalArgs a)
 {
     if (a.gate && !*a.gate) return;   // every block returns: no grid barrier is left waiting
     const int32_t nl = *a.lcount;
-    if (nl == 0) return;
-    if (nl <= kSmallSettle) {
-        if (blockIdx.x == 0) settle_body<false>(a, nl);
-        return;
+    const bool one = nl <= kSmallSettle;
+    if (nl == 0 || (one && blockIdx.x)) return;
+    __shared__ int32_t ubuf[kSettleThreads / 32][kUnreachedBuf];
+    Unreached unreached{ubuf[threadIdx.x >> 5]};
+    const int64_t tid = (one ? 0 : (int64_t)blockIdx.x * kSettleThreads) + threadIdx.x;
+    const int64_t nth = one ? kSettleThreads : (int64_t)gridDim.x * kSettleThreads;
+    // barrier with a vote (k_solve's; one block: its own)
+    uint32_t phase = a.sync->phase;
+    auto barrier = [&](bool mine) -> bool {
+        if (one) return __syncthreads_or(mine);
+        const uint32_t k = phase % 3, k1 = (phase + 1) % 3;
+        phase++;
+        if (tid == 0) a.sync->vote[k1] = a.sync->vote2[k1] = 0;
+        if (__syncthreads_or(mine) && threadIdx.x == 0) a.sync->vote[k] = 1;
+        cg::this_grid().sync();
+        return __ldcg(&a.sync->vote[k]) != 0;
+    };
+    for (int64_t i = tid; i < nl; i += nth) {
+        const int32_t u = a.la[i];
+        const int2 p = *reinterpret_cast<const int2 *>(&a.node[u]);   // successor (not the sink), priority
+        const int4 q = *reinterpret_cast<const int4 *>(&a.node[p.x]);
+        int4 r = make_int4(p.x, p.y, 1, 1);
+        if (q.z == RM_POS_INF || q.z == RM_NEG_INF) {
+            r = make_int4(q.z == RM_POS_INF ? kPosInf : kNegInf, 0, 0, 0);
+        } else if (q.z != RM_UNKNOWN) {
+            int32_t d, c;
+            path_depth_count(a, p.x, q.w, d, c);
+            top1_merge(r.y, r.z, q.z, c);
+            r.x = kSink;
+            r.w += d;
+        }
+        store_whole(&a.ja[u], r);
     }
-    settle_body<true>(a, nl);
+    barrier(false);
+    const bool marks = a.g->lm_want;
+    const uint32_t epoch = *a.epoch & kEpochMask;
+    bool more = true;
+    for (int pass = 0; more; pass++) {
+        if (pass == kMaxPasses) {   // cannot happen: windows grow at least kJumps-fold per pass
+            if (tid == 0) atomicOr(a.err, DERR_WALK_CAP);
+            break;
+        }
+        bool left = false;
+        for (int64_t b = tid & ~31ll; b < nl; b += nth) {   // whole warps: flags and appends are collective
+            const int64_t i = b + (threadIdx.x & 31);
+            bool changed = false, infinite = false;
+            int32_t u = -1;
+            if (i < nl) {
+                u = a.la[i];
+                int4 r = load_whole(&a.ja[u]);
+                // in later passes, what is finished has been dealt with
+                if (pass == 0 || r.x >= 0) {
+                    int4 q = r;
+                    if (r.x >= 0) q = load_whole(&a.ja[r.x]);
+                    if (jump_pass<false>(a.ja, a.n, u, r, q)) {
+                        const bool fin = r.x == kSink;
+                        const int32_t d = r.w, code = r.x == kPosInf ? RM_POS_INF : RM_NEG_INF;
+                        const int32_t k = fin ? finite_key(r.y, r.z) : (r.x == kPosInf ? KEY_POS_INF : KEY_NEG_INF);
+                        a.st[u] = fin ? d : (r.x == kPosInf ? ST_POS_INF : ST_NEG_INF);
+                        if (fin && d >= kDeepPath) a.rdeep[u] = r.z;
+                        *reinterpret_cast<int2 *>(&a.node[u].rmax) =
+                            fin ? make_int2(r.y, path_word(d, r.z)) : make_int2(code, 0);
+                        if (fin && marks) {
+                            Top2 seg = {-1, 0, -1, 0};
+                            int32_t anc = u;
+                            for (int32_t j = d - skip_landmark_depth(d); j > 0; j--) {
+                                const int2 x = *reinterpret_cast<const int2 *>(&a.node[anc]);
+                                top2_add(seg, x.y);
+                                anc = x.x;
+                            }
+                            store_whole(&a.skip[u], skip_pack(anc, seg, epoch));
+                        }
+                        infinite = !fin;
+                        changed = a.key[u] != k;
+                        if (changed) a.key[u] = k;
+                    } else {
+                        left = true;
+                    }
+                }
+            }
+            flag_in_neighbours(a.track, changed, u);
+            unreached.add(a, infinite, u);
+        }
+        more = barrier(left);
+    }
+    if (unreached.held) unreached.flush(a);
+    if (tid == 0 && !one) a.sync->phase = kept_phase(phase);
 }
 
 std::atomic<int> g_sms[kMaxCachedDevices];

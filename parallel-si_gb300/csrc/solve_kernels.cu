@@ -625,11 +625,11 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve_small(SolveArgs a)
 // every vertex in flight at once no ancestor is finished yet).  It leaves what
 // they leave: status, path records, keys, landmark records, the unreached
 // list, need flags; and does what launch_patch_begin does before them.
-__global__ void __launch_bounds__(kSolveThreads, 1) k_eval_jump(EvalArgs a, SolveSync *sync, EvalGates *g,
-                                                                int32_t *quiet)
+__global__ void __launch_bounds__(kSolveThreads, 1) k_eval_jump(EvalArgs a, EvalGates *g, int32_t *quiet)
 {
     const int32_t n = a.n, lane = threadIdx.x & 31;
     const int32_t tid = (int32_t)(blockIdx.x * blockDim.x + threadIdx.x), nth = (int32_t)(gridDim.x * blockDim.x);
+    SolveSync *sync = a.sync;
     uint32_t phase = sync->phase;
     auto barrier = [&](bool mine) -> bool {   // with a vote, as k_solve's
         const uint32_t k = phase % 3, k1 = (phase + 1) % 3;
@@ -728,12 +728,12 @@ static int device_sms()
     });
 }
 
-int launch_eval_jump(cudaStream_t s, const EvalArgs &a, SolveSync *sync, EvalGates *g, int32_t *quiet)
+int launch_eval_jump(cudaStream_t s, const EvalArgs &a, EvalGates *g, int32_t *quiet)
 {
     const int sms = device_sms(), threads = spread_threads(a.n, sms, kSolveThreads);
     const int64_t need = ceil_div(a.n, threads);
     const int grid = (int)(need < 1 ? 1 : (need < sms ? need : sms));
-    void *args[] = {(void *)&a, (void *)&sync, (void *)&g, (void *)&quiet};
+    void *args[] = {(void *)&a, (void *)&g, (void *)&quiet};
     count_launch();
     return (int)cudaLaunchCooperativeKernel((const void *)k_eval_jump, dim3(grid), dim3(threads), args, 0, s);
 }

@@ -237,7 +237,7 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m, bool many)
         {(void **)&tie_, (size_t)cap_n},
         {(void **)&watch_, (size_t)cap_n},
         {(void **)&ulist_, 4 * (size_t)ucap_},
-        {(void **)&paths_, 2 * sizeof(int2) * (size_t)cap_n},
+        {(void **)&paths_, sizeof(int2) * (size_t)cap_n},
         {(void **)&jA_, sizeof(int4) * (size_t)cap_n},
         {(void **)&jB_, sizeof(int4) * (size_t)cap_n},
         {(void **)&dw_, sizeof(AllWords)},
@@ -523,7 +523,7 @@ int Solver::enqueue_eval(bool timed, int32_t try_patch)
 {
     if (n_ <= kJumpVertices && incremental_ != PSI_INCR_ALWAYS) {
         if (timed) phase_begin(PH_BROADCAST);
-        int ce = launch_eval_jump(stream_, eval_args(), sync_, ctl_, &ctl_->quiet);
+        int ce = launch_eval_jump(stream_, eval_args(), ctl_, &ctl_->quiet);
         if (ce) return fail(PSI_ERR_CUDA, std::string("evaluation kernel: ") + cudaGetErrorString((cudaError_t)ce));
         if (timed) phase_end(PH_BROADCAST);
         return PSI_OK;
@@ -567,11 +567,9 @@ EvalArgs Solver::eval_args()
     a.ulist = ulist_;
     a.ucount = &dw_->ucount;
     a.la = reinterpret_cast<int32_t *>(paths_);
-    a.lb = a.la + n_;
     a.lcount = &dw_->lcount;
     a.ja = jA_;
-    a.jb = jB_;
-    a.cnt = dw_->cnt;
+    a.sync = sync_;
     a.err = &dw_->err;
     a.track = track();
     a.gate = &ctl_->eval;

@@ -223,7 +223,7 @@ private:
     // evaluation scratch
     int32_t *ulist_ = nullptr;
     int32_t *rdeep_ = nullptr;   // counts of paths too long for the path record's word
-    int2 *paths_ = nullptr;      // 2n entries: path records (SolveArgs), or the lists of walks cut short (EvalArgs)
+    int2 *paths_ = nullptr;      // n entries: path records (SolveArgs), or the list of walks cut short (EvalArgs)
     uint8_t *need_ = nullptr;    // vertices their owner's next switch step must examine (ChangeTrack)
     uint8_t *tie_ = nullptr;     // vertices whose last examination rested on a walk (ChangeTrack)
     uint8_t *watch_ = nullptr;   // vertices such an examination rested on (ChangeTrack)
@@ -231,7 +231,7 @@ private:
     void refresh_tracking();     // after a fused solve: every vertex to be examined
     void reset_tracking();       // every vertex to be examined (need = 1, quiet until the next evaluation)
     int32_t *rev_off_ = nullptr, *rev_src_ = nullptr;   // distinct in-neighbours (static)
-    int4 *jA_ = nullptr, *jB_ = nullptr;   // jump entries of the walks cut short
+    int4 *jA_ = nullptr, *jB_ = nullptr;   // jump records; between evaluations jB_ holds the vertices to examine
     // incremental evaluation (patch_kernels.cu): the switch steps' change
     // list, the re-evaluated set and its positions, the jump entries
     int32_t incremental_ = 1;   // psi_options.incremental
@@ -249,7 +249,6 @@ private:
         int32_t ucount;             // vertices the sink did not reach
         int32_t selcount;           // size of a selected list (players, winning set)
         int32_t lcount;             // walks cut short in the last full evaluation
-        int32_t cnt[3];             // list counters (EvalArgs)
         int32_t listcount;          // the switch steps' list (launch_switch): zero between steps
         uint32_t listdone;
         uint32_t claim;             // the switch kernel's work counter (launch_switch)

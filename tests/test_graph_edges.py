@@ -9,6 +9,7 @@ import pytest
 import oracle
 import psi
 from test_edge_cases import EDGE_GAMES
+from test_root_walk import paths_game, restated
 
 
 def odd_leaves_even_loop():
@@ -110,4 +111,30 @@ def test_dense_games_of_seven_vertices_per_thread_take_the_graph(n, deg, fused):
     w = psi.GPUList(g, switch_kernel=1)
     same(got, solved(w))
     w.close()
+    s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("chains,cycle", [([3000, 1090], 0), ([3000, 1500], 0), ([200000, 150000, 60], 0),
+                                          ([5], 400000), ([170000, 100], 150000), ([40] * 9000, 7)])
+def test_walks_cut_short_in_numbers(chains, cycle):
+    """More of them than one block takes (4,096) and than the grid has threads
+    (155,648 on 152 SMs), in chains, on cycles and before them; in full twice,
+    the second time after a switch step."""
+    g = paths_game(chains, len(chains) + cycle, cycle=cycle)
+    _, pri, _, tgt = g.csr()
+    s = psi.GPUList(g, incremental=2)
+    s.init_strat()
+    strat = tgt.copy()
+    strat[0] = -1
+    depth, top, cnt, inf = restated(strat.tolist(), pri.tolist())
+    for again in range(2):
+        if again:
+            s.switch_strategy(1)
+            s.set_strategy(strat)             # not listed: the next evaluation is a full one
+        s.compute_valuation()
+        d, t, c = s.get_summary()
+        assert np.array_equal(s.get_infinite(), inf)
+        assert np.array_equal(d, depth) and np.array_equal(t, top) and np.array_equal(c, cnt)
+        assert s.unreached() == int((inf != 0).sum())
     s.close()
