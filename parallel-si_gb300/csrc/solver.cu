@@ -237,7 +237,7 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m, bool many)
         {(void **)&tie_, (size_t)cap_n},
         {(void **)&watch_, (size_t)cap_n},
         {(void **)&ulist_, 4 * (size_t)ucap_},
-        {(void **)&paths_, sizeof(int2) * (size_t)cap_n},
+        {(void **)&paths_, 2 * sizeof(int2) * (size_t)cap_n},
         {(void **)&jA_, sizeof(int4) * (size_t)cap_n},
         {(void **)&jB_, sizeof(int4) * (size_t)cap_n},
         {(void **)&dw_, sizeof(AllWords)},

@@ -223,7 +223,10 @@ private:
     // evaluation scratch
     int32_t *ulist_ = nullptr;
     int32_t *rdeep_ = nullptr;   // counts of paths too long for the path record's word
-    int2 *paths_ = nullptr;      // n entries: path records (SolveArgs), or the list of walks cut short (EvalArgs)
+    // n entries: path records (SolveArgs), or the list of walks cut short
+    // (EvalArgs).  Allocated at twice that, which places the arrays after it where
+    // they were: 8n bytes closer, solves took 5% less to 5% more, by the game.
+    int2 *paths_ = nullptr;
     uint8_t *need_ = nullptr;    // vertices their owner's next switch step must examine (ChangeTrack)
     uint8_t *tie_ = nullptr;     // vertices whose last examination rested on a walk (ChangeTrack)
     uint8_t *watch_ = nullptr;   // vertices such an examination rested on (ChangeTrack)
