@@ -83,8 +83,14 @@ __device__ __forceinline__ void path_depth_count(const EvalArgs &a, int32_t y, i
     }
 }
 
-// A walk's step cap: longer walks are left to k_root_settle.
-constexpr int32_t kWalkCap = 128;
+// A walk's step cap: longer walks are left to k_root_settle.  So are all of a
+// warp's if none of the 32 has ended after kWarpCap steps (the lanes that happen to
+// be together then: which walks are left changes no result).  In random games a
+// warp has walks that end; where the sink reaches few vertices, 128 steps each were
+// most of an evaluation: without, and with 8, 16, 32 steps, ms per solve of one
+// cycle of 1.6*10^7 27.5, 5.3, 6.8, 9.8, all Odd 11.1, 4.3, 5.4, 6.8; 2^24 random
+// 31.9, 31.8, 31.8, 31.9.  (As a second cap inside one loop: 2^24 random +1%.)
+constexpr int32_t kWalkCap = 128, kWarpCap = 8;
 constexpr int kWalkThreads = 256;
 // unreached vertices buffered per warp before they go to the list with one
 // atomic (one atomic per warp and pass on the list's counter would serialise)
@@ -152,14 +158,18 @@ __global__ void __launch_bounds__(kWalkThreads, 8) k_root_walk(EvalArgs a)
                     int32_t m = q.y, c = 1;
                     int32_t y = q.x, s = 1, mark = v;   // s vertices walked, y the next one; the marker
                     int4 r;
-                    while (true) {
-                        r = *reinterpret_cast<const int4 *>(&a.node[y]);
-                        if (r.z != RM_UNKNOWN || y == mark || s >= kWalkCap) break;
-                        if ((s & (s - 1)) == 0) mark = y;   // after 1, 2, 4, ... vertices the marker moves here
-                        top1_merge(m, c, r.y, 1);
-                        y = r.x;
-                        s++;
-                    }
+                    auto walk = [&](int32_t cap) {
+                        while (true) {
+                            r = *reinterpret_cast<const int4 *>(&a.node[y]);
+                            if (r.z != RM_UNKNOWN || y == mark || s >= cap) break;
+                            if ((s & (s - 1)) == 0) mark = y;   // after 1, 2, 4, ... vertices the marker moves here
+                            top1_merge(m, c, r.y, 1);
+                            y = r.x;
+                            s++;
+                        }
+                    };
+                    walk(kWarpCap);
+                    if (r.z == RM_UNKNOWN && y != mark && __activemask() != 0xffffffffu) walk(kWalkCap);
                     int32_t code = 0;                       // an infinity, where it is one
                     if (r.z == RM_POS_INF || r.z == RM_NEG_INF) {
                         code = r.z;
