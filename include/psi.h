@@ -119,7 +119,8 @@ enum { PSI_SWITCH_THREAD = 0, PSI_SWITCH_WARP = 1 };
 /* incremental: PSI_INCR_AUTO (default) patches, on games of 2^20 vertices or
  * more and in batches, after steps that changed at most patch_limit
  * strategies, giving up for a full evaluation when more than max(4096, n/16)
- * vertices or n/20000 levels of descendants (32 to 256) are affected;
+ * vertices (16,384 after at most 512 changed strategies) or n/20000 levels of
+ * descendants (32 to 256) are affected;
  * PSI_INCR_OFF evaluates in full every time; PSI_INCR_ALWAYS patches
  * whenever the previous evaluation's state allows it, without the size
  * limits (n extra entries of device memory per buffer; for tests). */

@@ -344,6 +344,7 @@ struct PatchArgs {
     uint32_t *err = nullptr;
     int32_t n = 0;
     int32_t acap = 0, ccap = 0, max_levels = 0;
+    int32_t solo_most = 0;      // vertices past which a patch in one block (few changes) gives up
     int64_t ucap = 0;           // capacity of ulist
     int32_t *st = nullptr;
     PathNode *node = nullptr;

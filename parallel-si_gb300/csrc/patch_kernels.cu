@@ -68,8 +68,6 @@ constexpr int32_t kBackoffMax = 64;
 // (16, 64, 512, 2,048: 9.42, 9.35, 9.26, 9.34 ms per solve of 2*10^6 vertices,
 // long-path 2^23 18.6, 18.4, 18.3, 18.6 ms)
 constexpr int32_t kSoloSeeds = 512;
-// and it gives up for the full evaluation past this many vertices of A
-constexpr int32_t kSoloMost = 16384;
 // levels between two meetings of the blocks (4, 8, 16, 32: 10.06, 9.35, 8.99,
 // 8.95 ms for 2*10^6 vertices, 39.1, 37.9, 37.4, 38.2 ms for 2^24)
 constexpr int32_t kEpochLevels = 16;
@@ -287,7 +285,7 @@ __global__ void __launch_bounds__(kPatchBlock, 1) k_patch(PatchArgs a, cudaGraph
             if (threadIdx.x == 0) {
                 if (sh.count[cur ^ 1] > kQueue) sh.count[cur ^ 1] = kQueue;
                 held += sh.count[cur ^ 1];
-                if (solo && held > kSoloMost) sh.bail = 1;
+                if (solo && held > a.solo_most) sh.bail = 1;
                 pending = sh.count[cur ^ 1] ? ns + atomicAdd(&g->lcnt[1], sh.count[cur ^ 1]) : 0;
             }
             placed = false;

@@ -185,6 +185,14 @@ int Solver::upload_union(const std::vector<const HostGame *> &gs, const std::vec
     return finish_upload();
 }
 
+// A patch after few changes runs in one block and, unless patches are always
+// wanted, gives up for the full evaluation past this many vertices, so that one
+// block's search stays well below a full evaluation.  No game of 12 measured
+// (random 1.2*10^6 to 2^24 vertices, few priorities, long paths) comes to it: the
+// same patches and times with 65,536 and without it; 4,096 costs one 2 of its 54
+// patches (2^24: 28.9 -> 29.9 ms).
+constexpr int32_t kSoloMost = 16384;
+
 // Device arrays for games of up to cap_n vertices and cap_m edges.
 int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m, bool many)
 {
@@ -206,6 +214,7 @@ int Solver::alloc_arrays(int64_t cap_n, int64_t cap_m, bool many)
         ccap_ = (int32_t)std::max<int64_t>(1, std::min(cc, cap_n));
         acap_ = (int32_t)std::max<int64_t>(1, std::min(ac, cap_n));
         max_levels_ = always ? INT32_MAX : (int32_t)std::max<int64_t>(32, std::min<int64_t>(256, cap_n / 20000));
+        solo_most_ = always ? INT32_MAX : kSoloMost;
     }
     ucap_ = cap_n + acap_;
     PSI_CUDA_TRY(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
@@ -496,6 +505,7 @@ PatchArgs Solver::patch_args()
     a.acap = acap_;
     a.ccap = ccap_;
     a.max_levels = max_levels_;
+    a.solo_most = solo_most_;
     a.ucap = ucap_;
     a.st = st_;
     a.node = node_;

@@ -242,7 +242,7 @@ private:
     bool switch_warp_ = false;          // psi_options.switch_kernel == PSI_SWITCH_WARP
     int32_t *clist_ = nullptr, *alist_ = nullptr, *apos_ = nullptr;
     int4 *pj_ = nullptr;
-    int32_t ccap_ = 0, acap_ = 0, max_levels_ = 0;
+    int32_t ccap_ = 0, acap_ = 0, max_levels_ = 0, solo_most_ = 0;
     int64_t ucap_ = 0;   // entries of ulist_
     // small device words + pinned host mirrors
     struct Words {
