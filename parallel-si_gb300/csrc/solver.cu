@@ -437,19 +437,20 @@ void Solver::reset_tracking()
 {
     static const int32_t two = 2;   // patch_begin counts it down: nonzero in the next evaluation alone
     stale_ = false;
+    fresh_ = true;
     cudaMemsetAsync(need_, 1, (size_t)n_, stream_);
     cudaMemsetAsync(tie_, 0, (size_t)n_, stream_);
     cudaMemsetAsync(watch_, 0, (size_t)n_, stream_);
     cudaMemcpyAsync(&ctl_->quiet, &two, sizeof two, cudaMemcpyHostToDevice, stream_);
 }
 
-// The same when a switch step may come before the next evaluation, which
-// then has to flag what it changes.
-void Solver::refresh_tracking()
+void Solver::refresh_tracking(bool switching)
 {
-    if (!stale_) return;
-    reset_tracking();
-    cudaMemsetAsync(&ctl_->quiet, 0, sizeof(int32_t), stream_);
+    if (stale_) reset_tracking();
+    // a switch step before the next evaluation takes flags away: the
+    // evaluation then has to flag what it changes
+    if (fresh_ && switching) cudaMemsetAsync(&ctl_->quiet, 0, sizeof(int32_t), stream_);
+    fresh_ = false;
 }
 
 int Solver::init_strat()
@@ -607,7 +608,7 @@ int Solver::compute_valuation()
     if (!strat_ready_) return fail(PSI_ERR_STATE, "compute_valuation before init_strat");
     int rc = set_device();
     if (rc) return rc;
-    refresh_tracking();
+    refresh_tracking(false);
     // the last evaluation's state and the switch steps' change list since are
     // usable only if no strategy changed outside a switch step
     const int32_t try_patch = (tracked_ && incremental_ != PSI_INCR_OFF) ? 1 : 0;
@@ -665,7 +666,7 @@ int Solver::switch_strategy(int32_t player, int64_t *switched, bool count, bool 
     if (!val_ready_) return fail(PSI_ERR_STATE, "switch_strategy before compute_valuation");
     int rc = set_device();
     if (rc) return rc;
-    refresh_tracking();
+    refresh_tracking(true);
     const MarkArgs m = mark ? mark_args(player) : MarkArgs();
     phase_begin(PH_SWITCH);
     const int32_t np = (player == 0) ? np0_ : np_ - np0_;

@@ -231,7 +231,8 @@ private:
     uint8_t *tie_ = nullptr;     // vertices whose last examination rested on a walk (ChangeTrack)
     uint8_t *watch_ = nullptr;   // vertices such an examination rested on (ChangeTrack)
     ChangeTrack track() const { return ChangeTrack{need_, rev_off_, rev_src_, &ctl_->quiet, tie_, watch_}; }
-    void refresh_tracking();     // after a fused solve: every vertex to be examined
+    // before an evaluation or (switching) a switch step
+    void refresh_tracking(bool switching);
     void reset_tracking();       // every vertex to be examined (need = 1, quiet until the next evaluation)
     int32_t *rev_off_ = nullptr, *rev_src_ = nullptr;   // distinct in-neighbours (static)
     int4 *jA_ = nullptr, *jB_ = nullptr;   // jump records; between evaluations jB_ holds the vertices to examine
@@ -274,6 +275,7 @@ private:
     static int loop_ended(const GraphCtl &out);
     SolveSync *sync_ = nullptr;
     bool stale_ = false;   // the tracking flags do not describe the state: reset before they are used
+    bool fresh_ = false;   // every vertex is to be examined, and nothing has been since they were reset
     bool use_graph_ = false, graph_reset_ = false;
     int32_t inject_at_ = 0;
     uint32_t inject_bits_ = 0;

@@ -244,6 +244,7 @@ int Solver::run_graph(bool reset, int64_t max_evals, GraphCtl *out, int4 *gstate
     }
     GraphCtl init;
     init.quiet = 2;   // init_strat: every need flag is set
+    fresh_ = false;
     init.patch_on = incremental_ != PSI_INCR_OFF ? 1 : 0;
     init.max_evals = max_evals > 0 && max_evals < INT32_MAX ? (int32_t)max_evals : 0;
     init.inject_at = inject_at_;
