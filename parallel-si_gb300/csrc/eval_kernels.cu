@@ -75,13 +75,12 @@ __global__ void k_reset_odd(int32_t n, const int8_t *__restrict__ owner, const i
 // list starts at sublist nsub-1.  A node's head index follows from its id,
 // and succ is never modified by the ranking (it persists between
 // evaluations).
-template <bool POW2>
+// The stride is a power of two.
 __device__ __forceinline__ int32_t head_index(int32_t x, int64_t L, int32_t nsub, int32_t stride)
 {
     if (x == L - 1) return nsub - 1;
-    int32_t j = POW2 ? (x >> (__ffs(stride) - 1)) : x / stride;
-    bool at = POW2 ? (x & (stride - 1)) == 0 : j * stride == x;
-    return (at && j < nsub - 1) ? j : -1;
+    const int32_t j = x >> (__ffs(stride) - 1);
+    return ((x & (stride - 1)) == 0 && j < nsub - 1) ? j : -1;
 }
 
 // One thread per sublist: walk from the head's successor up to and including
@@ -89,12 +88,10 @@ __device__ __forceinline__ int32_t head_index(int32_t x, int64_t L, int32_t nsub
 // -1 at its down node, 0 at the sink's nodes) and recording, at each up node,
 // the sublist and the inclusive local prefix.  red[j] = (next sublist or
 // TOUR_END, sublist total).
-template <bool POW2>
 __global__ void k_walk_sublists(int32_t nsub, int32_t n, int64_t L, int32_t stride,
                                 const int32_t *__restrict__ succ, int2 *__restrict__ vloc,
-                                int2 *__restrict__ red, uint32_t *__restrict__ err, const int32_t *__restrict__ gate)
+                                int2 *__restrict__ red, uint32_t *__restrict__ err)
 {
-    if (gate && !*gate) return;
     int32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= nsub) return;
     const int64_t h = (j == nsub - 1) ? L - 1 : (int64_t)j * stride;
@@ -111,7 +108,7 @@ __global__ void k_walk_sublists(int32_t nsub, int32_t n, int64_t L, int32_t stri
                 acc -= 1;
             }
         }
-        int32_t hx = head_index<POW2>(x, L, nsub, stride);
+        int32_t hx = head_index(x, L, nsub, stride);
         if (hx >= 0) {
             next = hx;
             break;
@@ -137,10 +134,8 @@ __global__ void k_walk_sublists(int32_t nsub, int32_t n, int64_t L, int32_t stri
 // 256)
 constexpr int kRankBlock = 1024;
 __global__ void __launch_bounds__(kRankBlock) k_rank_reduced(int32_t nsub, const int2 *__restrict__ red,
-                                                         int2 *__restrict__ a, int2 *__restrict__ b,
-                                                         const int32_t *__restrict__ gate)
+                                                         int2 *__restrict__ a, int2 *__restrict__ b)
 {
-    if (gate && !*gate) return;   // every block returns: no grid barrier is left waiting
     cg::grid_group g = cg::this_grid();
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t nth = (int64_t)gridDim.x * blockDim.x;
@@ -185,9 +180,8 @@ __device__ __forceinline__ int32_t ruler_index(int32_t j, int32_t nsub, int32_t 
 
 __global__ void __launch_bounds__(kRankBlock) k_rank_ruled(int32_t nsub, const int2 *__restrict__ red,
                                                        int2 *__restrict__ a, int2 *__restrict__ b,
-                                                       uint32_t *__restrict__ err, const int32_t *__restrict__ gate)
+                                                       uint32_t *__restrict__ err)
 {
-    if (gate && !*gate) return;   // every block returns: no grid barrier is left waiting
     cg::grid_group g = cg::this_grid();
     const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t nth = (int64_t)gridDim.x * blockDim.x;
@@ -274,9 +268,8 @@ __global__ void k_broadcast_depth(int32_t n, const int2 *__restrict__ vloc, cons
                                   const int32_t *__restrict__ strat, const int32_t *__restrict__ pri,
                                   const uint8_t *__restrict__ solved, int32_t *__restrict__ st,
                                   PathNode *__restrict__ node, int32_t *__restrict__ ulist,
-                                  int32_t *__restrict__ ucount, const int32_t *__restrict__ gate)
+                                  int32_t *__restrict__ ucount)
 {
-    if (gate && !*gate) return;
     const bool vec = aligned16(vloc) && aligned16(strat) && aligned16(pri) && aligned16(st) &&
                      ((uintptr_t)solved & 3) == 0;
     // grid-stride with block-uniform passes (block_append_k needs every thread)
@@ -363,9 +356,9 @@ constexpr int kSmallCycles = 4096;   // up to this many: one block, no grid barr
 template <bool GRID>
 __device__ void cycles_body(int32_t nu, const int32_t *__restrict__ ulist, const int32_t *__restrict__ strat,
                             const int32_t *__restrict__ pri, const uint8_t *__restrict__ solved,
-                            int32_t *__restrict__ st, int32_t *__restrict__ key, int4 *__restrict__ ja,
-                            int4 *__restrict__ jb, int32_t *__restrict__ la, int32_t *__restrict__ lb,
-                            int32_t *__restrict__ cnt, uint32_t *__restrict__ err, const ChangeTrack &track)
+                            int32_t *__restrict__ st, int4 *__restrict__ ja, int4 *__restrict__ jb,
+                            int32_t *__restrict__ la, int32_t *__restrict__ lb, int32_t *__restrict__ cnt,
+                            uint32_t *__restrict__ err)
 {
     const int64_t tid = GRID ? (int64_t)blockIdx.x * blockDim.x + threadIdx.x : threadIdx.x;
     const int64_t nth = GRID ? (int64_t)gridDim.x * blockDim.x : blockDim.x;
@@ -433,28 +426,14 @@ __device__ void cycles_body(int32_t nu, const int32_t *__restrict__ ulist, const
         in = out;
         out = t;
     }
-    // block-uniform iterations: flag_in_neighbours is warp-collective
-    for (int64_t b0 = tid - threadIdx.x; b0 < nu; b0 += nth) {
-        const int64_t i = b0 + threadIdx.x;
-        bool changed = false;
-        int32_t u = -1;
-        if (i < nu) {
-            u = ulist[i];
-            int32_t code = __ldcg(&in[u]).x;
-            if (code >= 0) {   // still walking after every round: its target is on the final cycle
-                const int4 e = __ldcg(&in[code]);
-                code = e.x < 0 ? e.x : cycle_code(e.y);
-            }
-            const int32_t su =
-                code <= kCycleOdd ? (code == kCycleEven ? ST_POS_INF : ST_NEG_INF) : st[-2 - code];
-            st[u] = su;
-            const int32_t k = (su == ST_POS_INF) ? KEY_POS_INF : KEY_NEG_INF;
-            if (key && key[u] != k) {
-                key[u] = k;
-                changed = true;
-            }
+    for (int64_t i = tid; i < nu; i += nth) {
+        const int32_t u = ulist[i];
+        int32_t code = __ldcg(&in[u]).x;
+        if (code >= 0) {   // still walking after every round: its target is on the final cycle
+            const int4 e = __ldcg(&in[code]);
+            code = e.x < 0 ? e.x : cycle_code(e.y);
         }
-        flag_in_neighbours(track, changed, u);
+        st[u] = code <= kCycleOdd ? (code == kCycleEven ? ST_POS_INF : ST_NEG_INF) : st[-2 - code];
     }
 }
 
@@ -468,20 +447,17 @@ __global__ void __launch_bounds__(kCycleBlock, kCycleMinBlocks) k_cycles(const i
                                                    const int32_t *__restrict__ strat,
                                                    const int32_t *__restrict__ pri,
                                                    const uint8_t *__restrict__ solved, int32_t *__restrict__ st,
-                                                   int32_t *__restrict__ key, int4 *__restrict__ ja,
-                                                   int4 *__restrict__ jb,
+                                                   int4 *__restrict__ ja, int4 *__restrict__ jb,
                                                    int32_t *__restrict__ la, int32_t *__restrict__ lb,
-                                                   int32_t *__restrict__ cnt, uint32_t *__restrict__ err,
-                                                   ChangeTrack track, const int32_t *__restrict__ gate)
+                                                   int32_t *__restrict__ cnt, uint32_t *__restrict__ err)
 {
-    if (gate && !*gate) return;   // every block returns: no grid barrier is left waiting
     int32_t nu = *ucount;
     if (nu == 0) return;
     if (nu <= kSmallCycles) {
-        if (blockIdx.x == 0) cycles_body<false>(nu, ulist, strat, pri, solved, st, key, ja, jb, la, lb, cnt, err, track);
+        if (blockIdx.x == 0) cycles_body<false>(nu, ulist, strat, pri, solved, st, ja, jb, la, lb, cnt, err);
         return;
     }
-    cycles_body<true>(nu, ulist, strat, pri, solved, st, key, ja, jb, la, lb, cnt, err, track);
+    cycles_body<true>(nu, ulist, strat, pri, solved, st, ja, jb, la, lb, cnt, err);
 }
 
 __global__ void k_mark_solved(MarkArgs m) { mark_solved_pass(m); }
@@ -545,27 +521,23 @@ void launch_reset_odd(cudaStream_t s, int32_t n, const int8_t *owner, const int3
 }
 
 void launch_walk_sublists(cudaStream_t s, int32_t nsub, int32_t n, int64_t L, int32_t stride, const int32_t *succ,
-                          int2 *vloc, int2 *red, uint32_t *err, const int32_t *gate, int block)
+                          int2 *vloc, int2 *red, uint32_t *err)
 {
     count_launch();
-    if ((stride & (stride - 1)) == 0)
-        k_walk_sublists<true><<<grid_for(nsub, block), block, 0, s>>>(nsub, n, L, stride, succ, vloc, red, err, gate);
-    else
-        k_walk_sublists<false><<<grid_for(nsub, block), block, 0, s>>>(nsub, n, L, stride, succ, vloc, red, err,
-                                                                      gate);
+    k_walk_sublists<<<grid_for(nsub, kWalkBlock), kWalkBlock, 0, s>>>(nsub, n, L, stride, succ, vloc, red, err);
 }
 
 int launch_rank_reduced(cudaStream_t s, int32_t nsub, const int2 *red, int2 *a, int2 *b, const int2 **fin,
-                        const int32_t *gate, uint32_t *err)
+                        uint32_t *err)
 {
-    if (err && nsub >= kRulerMin) {
+    if (nsub >= kRulerMin) {
         // the ruling set: the rulers' two jump buffers (2 nr entries) fit in b
         const int blocks =
             per_device(g_ruled_blocks, [] { return device_blocks((const void *)k_rank_ruled, kRankBlock); });
         int64_t need = ceil_div(nsub, kRankBlock);
         int grid = (int)(need < blocks ? need : blocks);
         *fin = a;
-        void *args[] = {(void *)&nsub, (void *)&red, (void *)&a, (void *)&b, (void *)&err, (void *)&gate};
+        void *args[] = {(void *)&nsub, (void *)&red, (void *)&a, (void *)&b, (void *)&err};
         count_launch();
         cudaError_t e =
             cudaLaunchCooperativeKernel((const void *)k_rank_ruled, dim3(grid), dim3(kRankBlock), args, 0, s);
@@ -579,7 +551,7 @@ int launch_rank_reduced(cudaStream_t s, int32_t nsub, const int2 *red, int2 *a, 
     while (((int64_t)1 << rounds) < nsub) rounds++;
     rounds += 1;
     *fin = (rounds % 2 == 1) ? a : b;
-    void *args[] = {(void *)&nsub, (void *)&red, (void *)&a, (void *)&b, (void *)&gate};
+    void *args[] = {(void *)&nsub, (void *)&red, (void *)&a, (void *)&b};
     count_launch();
     cudaError_t e =
         cudaLaunchCooperativeKernel((const void *)k_rank_reduced, dim3(grid), dim3(kRankBlock), args, 0, s);
@@ -588,22 +560,21 @@ int launch_rank_reduced(cudaStream_t s, int32_t nsub, const int2 *red, int2 *a, 
 
 void launch_broadcast_depth(cudaStream_t s, int32_t n, const int2 *vloc, const int2 *fin,
                             const int32_t *strat, const int32_t *pri, const uint8_t *solved,
-                            int32_t *st, PathNode *node, int32_t *ulist, int32_t *ucount, const int32_t *gate)
+                            int32_t *st, PathNode *node, int32_t *ulist, int32_t *ucount)
 {
     count_launch();
     k_broadcast_depth<<<capped_grid(ceil_div(n, kBcast)), kBlock, 0, s>>>(n, vloc, fin, strat, pri, solved, st, node,
-                                                                           ulist, ucount, gate);
+                                                                           ulist, ucount);
 }
 
 int launch_cycles(cudaStream_t s, const int32_t *ucount, const int32_t *ulist, const int32_t *strat,
-                  const int32_t *pri, const uint8_t *solved, int32_t *st, int32_t *key, int4 *ja, int4 *jb,
-                  int32_t *la, int32_t *lb, int32_t *cnt, uint32_t *err, ChangeTrack track, const int32_t *gate)
+                  const int32_t *pri, const uint8_t *solved, int32_t *st, int4 *ja, int4 *jb, int32_t *la, int32_t *lb,
+                  int32_t *cnt, uint32_t *err)
 {
     const int blocks =
         per_device(g_cycle_blocks, [] { return device_blocks((const void *)k_cycles, kCycleBlock); });
     void *args[] = {(void *)&ucount, (void *)&ulist, (void *)&strat, (void *)&pri, (void *)&solved,
-                    (void *)&st, (void *)&key, (void *)&ja, (void *)&jb, (void *)&la, (void *)&lb, (void *)&cnt,
-                    (void *)&err, (void *)&track, (void *)&gate};
+                    (void *)&st, (void *)&ja, (void *)&jb, (void *)&la, (void *)&lb, (void *)&cnt, (void *)&err};
     count_launch();
     cudaError_t e = cudaLaunchCooperativeKernel((const void *)k_cycles, dim3(blocks), dim3(kCycleBlock), args, 0, s);
     return e == cudaSuccess ? 0 : (int)e;

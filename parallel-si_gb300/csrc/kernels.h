@@ -46,7 +46,6 @@ struct EvalGates {
     int32_t ccount = 0;      // changed vertices the switch steps listed since the last evaluation
     int32_t csnap = 0;       // ccount as the current evaluation found it
     int32_t acount = 0;      // vertices the current patch re-evaluates
-    int32_t nseeds = 0;      // of them the changed ones (alist[0, nseeds))
     int32_t lcnt[3] = {0, 0, 0};              // per-level append counters of the patch's search
     int32_t skip = 0, backoff = 1;            // evaluations not to try a patch after a failed one
     int32_t mfrom[2] = {0, 0};   // per player: unreached-list index its next mark_solved scans from
@@ -209,33 +208,29 @@ int launch_solve(cudaStream_t s, const SolveArgs &a);
 
 // ---- list ranking of an Euler tour (gpu_list_ranking.cu:52-277), the
 // evaluation without allocation (noalloc.cu)
-// Sublist walks; heads are the nodes j*stride (j < nsub-1) and the list start.
-// One thread per sublist, `block` threads per block (a multiple of 32, <= 1024).
+// Sublist walks; heads are the nodes j*stride (j < nsub-1; stride: a power of
+// two) and the list start.  One thread per sublist.
 constexpr int kWalkBlock = 128;
 void launch_walk_sublists(cudaStream_t s, int32_t nsub, int32_t n, int64_t L, int32_t stride, const int32_t *succ,
-                          int2 *vloc, int2 *red, uint32_t *err, const int32_t *gate = nullptr,
-                          int block = kWalkBlock);
+                          int2 *vloc, int2 *red, uint32_t *err);
 // Ranks the reduced list red[0..nsub) (next, weight) in one cooperative
 // launch (a, b: nsub entries each): by Wyllie pointer jumping over all items,
-// or, with err and at least 4,096 items, through a ruling set (every 8th
-// item and the list start walk to the next ruler, Wyllie over the rulers;
-// err receives DERR_SUBLIST_CAP if a walk overruns).  *fin is set to the
-// buffer that will hold, per item, (TOUR_END if the list start reaches it,
-// else another value; inclusive suffix sum).  Returns a cudaError_t value.
+// or, from 4,096 items on, through a ruling set (every 8th item and the list
+// start walk to the next ruler, Wyllie over the rulers; err receives
+// DERR_SUBLIST_CAP if a walk overruns).  *fin is set to the buffer that will
+// hold, per item, (TOUR_END if the list start reaches it, else another value;
+// inclusive suffix sum).  Returns a cudaError_t value.
 int launch_rank_reduced(cudaStream_t s, int32_t nsub, const int2 *red, int2 *a, int2 *b, const int2 **fin,
-                        const int32_t *gate = nullptr, uint32_t *err = nullptr);
+                        uint32_t *err);
 void launch_broadcast_depth(cudaStream_t s, int32_t n, const int2 *vloc, const int2 *fin,
                             const int32_t *strat, const int32_t *pri, const uint8_t *solved,
-                            int32_t *st, PathNode *node, int32_t *ulist, int32_t *ucount,
-                            const int32_t *gate = nullptr);
-// Cycle parity of the *ucount vertices in ulist (cooperative launch), also
-// stored as their comparison keys when key != nullptr.  ja, jb: n entries;
-// la, lb: n entries (active lists); cnt: 3 counters.  Returns a cudaError_t
-// value.
+                            int32_t *st, PathNode *node, int32_t *ulist, int32_t *ucount);
+// Cycle parity of the *ucount vertices in ulist (cooperative launch).  ja, jb:
+// n entries; la, lb: n entries (active lists); cnt: 3 counters.  Returns a
+// cudaError_t value.
 int launch_cycles(cudaStream_t s, const int32_t *ucount, const int32_t *ulist, const int32_t *strat,
-                  const int32_t *pri, const uint8_t *solved, int32_t *st, int32_t *key, int4 *ja, int4 *jb,
-                  int32_t *la, int32_t *lb, int32_t *cnt, uint32_t *err, ChangeTrack track = ChangeTrack(),
-                  const int32_t *gate = nullptr);
+                  const int32_t *pri, const uint8_t *solved, int32_t *st, int4 *ja, int4 *jb, int32_t *la, int32_t *lb,
+                  int32_t *cnt, uint32_t *err);
 // mark_solved over the last evaluation's unreached vertices (cpu_parity.cpp:265-274);
 // with game_of/gmask only for games whose mask is set (nullptr: all).  With
 // from (a device word; done: a zeroed counter) only the entries from *from on

@@ -476,7 +476,6 @@ __global__ void __launch_bounds__(kPatchBlock, 1) k_patch(PatchArgs a, cudaGraph
     if (leader) {
         g->backoff = 1;
         g->acount = na;
-        g->nseeds = ns;
         a.stats[0] += 1;
         a.stats[1] += (unsigned long long)na;
         if (!solo) a.sync->phase = kept_phase(phase);
