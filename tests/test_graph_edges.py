@@ -138,3 +138,22 @@ def test_walks_cut_short_in_numbers(chains, cycle):
         assert np.array_equal(d, depth) and np.array_equal(t, top) and np.array_equal(c, cnt)
         assert s.unreached() == int((inf != 0).sum())
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2000, 9000, 100000])
+@pytest.mark.parametrize("kw", [dict(), dict(graph=0), dict(incremental=2)])
+def test_vertices_of_very_many_successors(n, kw):
+    """The persistent solver keeps a vertex's number of successors in 12 bits
+    and reads 4,095 and more anew: hubs about that size and far above it among
+    ordinary vertices, with ties at any place of their lists."""
+    rng = np.random.default_rng(n)
+    size = rng.integers(1, 5, n)
+    hubs = rng.choice(n, 12, replace=False)
+    size[hubs] = [4093, 4094, 4095, 4096, 4097, 8191, 5, 6, 31, 33, 30000, 12000]
+    off = np.concatenate(([0], np.cumsum(size))).astype(np.int32)
+    g = psi.Game.from_csr(rng.integers(0, 2, n), rng.integers(0, 40, n), off, rng.integers(0, n, off[-1]))
+    s = psi.GPUList(g, **kw)
+    for reset in (False, True):
+        same(solved(s, reset), expected(g, reset))
+    s.close()
