@@ -1,5 +1,5 @@
-// kernels.h -- host-side launchers of the sm_103a kernels (eval_kernels.cu,
-// switch_kernels.cu).  All launchers are asynchronous on the given stream.
+// kernels.h -- host-side launchers of the sm_103a kernels, and what host and
+// kernels share.  All launchers are asynchronous on the given stream.
 #ifndef PSI_KERNELS_H
 #define PSI_KERNELS_H
 
@@ -333,7 +333,7 @@ struct PatchArgs {
     int4 *rel = nullptr;                 // per position of alist: seed, path summary to it (acap)
     int2 *arev = nullptr;                // per position of alist: the vertex's in-edge range (acap)
     int4 *sja = nullptr;                 // the seeds' jump records (acap)
-    int32_t *spill = nullptr, *spill2 = nullptr;   // positions still to be searched from (2 acap, acap)
+    int32_t *spill = nullptr, *spill2 = nullptr;   // positions still to be searched from (2 acap each)
     int32_t *sizes = nullptr;            // per block (kPatchSizes)
     SolveSync *sync = nullptr;
     uint32_t *err = nullptr;

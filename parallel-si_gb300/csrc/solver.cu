@@ -525,9 +525,9 @@ PatchArgs Solver::patch_args()
 // Games up to this size are evaluated in full every time by one launch in the
 // host-driven calls: a patch takes three launches and a level of its search
 // longer than all the jumps.  Evaluation, mark_solved and switch step by step,
-// us per evaluation with patches and walks -> so: 136 -> 94 (n = 10^3), 141 ->
-// 99 (5*10^4), 159 -> 125 (4*10^5), 186 -> 166 (10^6); 24 served games 13.9 ->
-// 12.4 ms.
+// us per evaluation with patches and walks -> so: 118 -> 85 (n = 1,537), 117 -> 90
+// (10^4 and 10^5), 128 -> 100 (3*10^5), 153 -> 144 (10^6), 151 -> 140 (2^20 - 1); 24
+// served games 11.9 -> 11.4 ms.
 constexpr int32_t kJumpVertices = (1 << 20) - 1;
 
 int Solver::enqueue_eval(bool timed, int32_t try_patch)

@@ -99,11 +99,11 @@ inline int32_t eval_guard(int64_t n)
     return (int32_t)(g < (1 << 14) ? (1 << 14) : (g > (1 << 20) ? (1 << 20) : g));
 }
 
-// Games below 2^20 vertices are solved by one persistent kernel.  Solve and
-// read-back, graph -> kernel: n = 100 0.65 -> 0.17 ms, 10^4 1.41 -> 0.57 ms,
-// 10^5 (reset variant) 3.43 -> 1.18 ms, 10^6 9.0 -> 4.3 ms; at 2*10^6 both take
-// the same, and beyond, where full evaluations no longer run from L2, the
-// graph's patches win.
+// Games below 2^20 vertices are solved by one persistent kernel (dense ones of
+// that size by the graph, solve_takes).  Solve and read-back, graph -> kernel, us:
+// n = 100 274 -> 68, 1,537 1,131 -> 257, 10^4 924 -> 319, 10^5 (reset variant) 2,000
+// -> 697, 3*10^5 3,234 -> 1,245, 10^6 5,053 -> 3,745, 2^20 - 1 4,720 -> 3,385 (another
+// game 5,215 -> 4,205).  The kernel's 20-bit vertex ids end there, not its lead.
 constexpr int32_t kFusedVertices = (1 << 20) - 1;
 
 }  // namespace

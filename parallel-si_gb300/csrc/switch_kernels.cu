@@ -72,15 +72,6 @@ __device__ int compare_equal_keys(const PathNode *__restrict__ node, const Landm
     return c;
 }
 
-// One thread per vertex of plist (all owned by `player`).  Per compared edge
-// the common case is one 4-byte gather (the successor's comparison key) and
-// one integer comparison; equal keys of distinct finite vertices fall back to
-// the exact summaries and, rarely, a walk.  stats[0] += compared edges,
-// stats[1] += parent/priority loads of the walks, stats[2] += vertices whose
-// strategy changed, stats[3] += strict improvements.  For a batch of games
-// (game_of != nullptr) the strict improvements are also added to
-// gcount[game of the vertex]; with gmask only vertices of games whose mask is
-// set switch.
 // The vertices of plist whose need flag is set (and, with gmask, whose game
 // takes this step), appended to list with one atomic per block.  A block
 // pass covers kNeedPer * blockDim entries (each thread kNeedPer of them,
